@@ -371,6 +371,310 @@ __global__ void __launch_bounds__(kDdThreads) k_dedisperse(DedispArgs a)
     }
 }
 
+// ---------------------------------------------------------------------------
+// Shared partial sums.  The shifts of neighbouring DM trials differ by almost
+// the same amount in neighbouring channels: over S consecutive live channels
+// (a subband) the relative shifts D(d, c) - D(d, c0) of a block of up to 32 DM
+// trials take only a few distinct values (2 per pair of channels, 4 to 6 per
+// four at survey spacing).  So a CTA first forms, once per distinct vector
+// ("pattern") of relative shifts, the subband's own series
+//   Y[i] = sum over the S channels of x_c[t0 + smin + i + D(d,c) - D(d,c0)],
+// and each DM trial then adds one Y per subband instead of S channels.  The
+// sums are integers, so the result is the direct kernel's bit for bit.
+//
+// Layout.  A tile is 4Q outputs (2Q for 16-bit samples), Q = 256.  A staged
+// channel window is rearranged in shared memory into words
+// (x[i], x[i+Q], x[i+2Q], x[i+3Q]) ((x[i], x[i+Q]) for 16-bit samples), and a
+// pattern's Y is kept in the same arrangement: for 1..4-bit samples the same
+// words (the sum of four channels fits a byte), for 8-bit samples pairs of
+// words ((y[i], y[i+2Q]), (y[i+Q], y[i+3Q])) of 16-bit sums, for 16-bit
+// samples pairs (y[i], y[i+Q]) of 32-bit sums.  Every shift is then a whole
+// number of words, so no load needs a funnel shift and a warp's loads are
+// consecutive.
+//
+// Bound: the shared-memory port (71 % of its wavefronts; 46 % of them the
+// second level's, 2 bytes per output, subband and DM trial), then issue
+// (62 %).  Measured on B200 (us, the whole call, before and after): 256 DM
+// trials x 2^22 samples x 64 channels, 8 bits: 6311, 3227; 100 x 400,000 x
+// 1024, 4 bits: 3408, 1789.  Subbands of 8 channels have three times the
+// patterns; blocks of 64 DM trials leave half the warps.
+constexpr int kTrQ = 256;      // words of a row per (DM trial, YE or YO)
+constexpr int kTrWords = kTrQ / 32;
+// 16 warps of at most 64 registers, two CTAs to an SM (8 warps of 4 DM trials
+// each, the same work in half the warps, took 3407 us against 3162)
+constexpr int kTrThreads = 512;
+constexpr int kTrWarps = 16;
+constexpr int kTrMaxDms = 32;  // DM trials per CTA: at most 2 per warp
+// sample classes: 8-bit bytes (their sums need 16 bits at once), 1..4-bit
+// bytes (a subband's sum fits a byte), 16-bit samples (32-bit sums)
+enum { kTr8 = 0, kTrSmall = 1, kTr16 = 2 };
+constexpr int kTrS = 4;        // channels per subband
+constexpr int kTrRec = 8;      // ints of a pattern's record (32-byte aligned)
+inline int tr_tile(int el) { return el == 1 ? 4 * kTrQ : 2 * kTrQ; }
+
+struct TreeArgs {
+    const void* cm;
+    size_t pitch;
+    const int4* chan;  // [nblk * nlive] channel row, window start after t0 (samples),
+                       // first planar word in the stage, planar words / 4
+    int rawlen, pmax;  // words of the stage's windows, patterns of a stage at most
+    const int* dmrow;  // [ndm] output row of each DM trial in block order
+    const int* pstart; // [nblk * nq + 1] first pattern of (block, stage)
+    const int4* pat;   // [2 * patterns] planar word of each channel's source; first
+                       // group of 32 Y elements in the stage, groups
+    const int* gtot;   // [nblk * nq] groups of a stage
+    const int* yoff;   // [nblk * nq * (cc/S) * 16 DPW] Y element of a trial
+    int nlive, ndm, ndb, nblk, cc, nq, zero, zlen, plen, gmax;
+    float* out;
+    size_t out_pitch, nout;
+    float mid, scale;
+    int raw;
+    int p16;           // channels a 16-bit sum holds at the input's largest value
+    int p8s;           // subbands a byte holds (1..4-bit samples)
+};
+
+template <int MODE, int DPW, bool FLUSH>
+__global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
+{
+    constexpr int S = kTrS, W = kTrWords;
+    constexpr int kSlots = kTrWarps * DPW, kElem = MODE == kTr16 ? 2 : 1;
+    constexpr int kParts = MODE == kTr16 ? 2 : 4;      // outputs of one planar word
+    constexpr int kYWords = MODE == kTrSmall ? 1 : 2;  // words of one Y element
+    extern __shared__ __align__(16) uint32_t tsm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int blk = blockIdx.x % a.nblk;
+    const size_t t0 = (size_t)(blockIdx.x / a.nblk) * (kParts * kTrQ);
+    const int nsb = a.cc / S;       // subbands per stage
+    uint32_t* raw = tsm;            // the next stage's windows as they are in cm
+    uint32_t* pl = raw + a.rawlen;  // planar words of the stage's channels, zeros at a.zero
+    uint32_t* ysm = pl + a.plen;    // Y of the stage's patterns
+    int4* s_pat = reinterpret_cast<int4*>(ysm + a.gmax * 32 * kYWords);  // [2][pmax][2]
+    int* s_yoff = reinterpret_cast<int*>(s_pat + 4 * a.pmax);            // [2][nsb][kSlots]
+    // a window's words after its planar ones' first part; its place in raw
+    // follows from its place among the planar words
+    constexpr int kMore = MODE == kTr16 ? kTrQ / 2 : 3 * kTrQ / 4;
+    auto raw_at = [&](int c, const int4& ch) {
+        return raw + (MODE == kTr16 ? ch.z / 2 : ch.z / 4) + c * (kMore + 4);
+    };
+
+    // A stage's windows and tables, asynchronously.
+    auto load_stage = [&](int q) {
+        const int nch = min(a.cc, a.nlive - q * a.cc), bq = blk * a.nq + q;
+        for (int c = warp; c < nch; c += kTrWarps) {
+            const int4 ch = a.chan[(size_t)blk * a.nlive + q * a.cc + c];
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(
+                static_cast<const uint8_t*>(a.cm) + ((size_t)ch.x * a.pitch + t0 + ch.y) * kElem);
+            uint32_t* d = raw_at(c, ch);
+            const int n = (MODE == kTr16 ? 2 * ch.w : ch.w) + kMore;
+            for (int p = 4 * lane; p < n; p += 128) cp_async16(d + p, w + p);
+        }
+        const int p0 = a.pstart[bq], np = a.pstart[bq + 1] - p0;
+        int4* dp = s_pat + (q & 1) * 2 * a.pmax;
+        for (int k = threadIdx.x; k < 2 * np; k += kTrThreads) cp_async16(dp + k, a.pat + 2 * (size_t)p0 + k);
+        int* dy = s_yoff + (q & 1) * nsb * kSlots;
+        const int* sy = a.yoff + (size_t)bq * nsb * kSlots;
+        for (int k = threadIdx.x; k < nsb * (kSlots / 4); k += kTrThreads) cp_async16(dy + 4 * k, sy + 4 * k);
+        cp_async_commit();
+    };
+    // Windows -> planar words, four consecutive words per step.
+    auto to_planar = [&](int q) {
+        const int nch = min(a.cc, a.nlive - q * a.cc);
+        for (int c = warp; c < nch; c += kTrWarps) {
+            const int4 ch = a.chan[(size_t)blk * a.nlive + q * a.cc + c];
+            const uint32_t* w = raw_at(c, ch);
+            uint4* d = reinterpret_cast<uint4*>(pl + ch.z);
+            for (int p = lane; p < ch.w; p += 32) {
+                uint4 v;
+                if constexpr (MODE == kTr16) {
+                    const uint2 a0 = reinterpret_cast<const uint2*>(w)[p];
+                    const uint2 b0 = reinterpret_cast<const uint2*>(w)[p + kTrQ / 4];
+                    v.x = __byte_perm(a0.x, b0.x, 0x5410);
+                    v.y = __byte_perm(a0.x, b0.x, 0x7632);
+                    v.z = __byte_perm(a0.y, b0.y, 0x5410);
+                    v.w = __byte_perm(a0.y, b0.y, 0x7632);
+                } else {
+                    const uint32_t w0 = w[p], w1 = w[p + kTrQ / 4];
+                    const uint32_t w2 = w[p + kTrQ / 2], w3 = w[p + 3 * kTrQ / 4];
+                    const uint32_t l0 = __byte_perm(w0, w1, 0x5140), l1 = __byte_perm(w2, w3, 0x5140);
+                    const uint32_t h0 = __byte_perm(w0, w1, 0x7362), h1 = __byte_perm(w2, w3, 0x7362);
+                    v.x = __byte_perm(l0, l1, 0x5410);
+                    v.y = __byte_perm(l0, l1, 0x7632);
+                    v.z = __byte_perm(h0, h1, 0x5410);
+                    v.w = __byte_perm(h0, h1, 0x7632);
+                }
+                d[p] = v;
+            }
+        }
+    };
+
+    // packed 16-bit sums (32-bit for 16-bit samples): the pairs' first
+    // words, then their second words
+    uint32_t acc[DPW][2 * W];
+#pragma unroll
+    for (int j = 0; j < DPW; ++j)
+#pragma unroll
+        for (int k = 0; k < 2 * W; ++k) acc[j][k] = 0;
+    const int d0 = blk * a.ndb + warp;  // the warp's DM trials: d0, d0 + 16
+    const int dend = min(a.ndm, (blk + 1) * a.ndb);
+    bool flushed = false;
+    int since = 0;
+    // f(output of trial j after t0 + lane, sum) over the warp's outputs
+    auto each_of = [&](int j, auto in, auto f) {
+#pragma unroll
+        for (int k = 0; k < 2 * W; ++k) {
+            const int t = 32 * (k % W) + (k < W ? 0 : kTrQ);
+            if constexpr (MODE == kTr16) {
+                if (in(t)) f(t, acc[j][k]);
+            } else {
+                if (in(t)) f(t, acc[j][k] & 0xffffu);
+                if (in(t + 2 * kTrQ)) f(t + 2 * kTrQ, acc[j][k] >> 16);
+            }
+        }
+    };
+    auto each = [&](int j, auto f) {
+        if (t0 + kParts * kTrQ <= a.nout) {
+            each_of(j, [](int) { return true; }, f);
+        } else {
+            const int left = (int)(a.nout - t0) - lane;  // the last tile
+            each_of(j, [&](int t) { return t < left; }, f);
+        }
+    };
+
+    for (int k = threadIdx.x; k < a.zlen; k += kTrThreads) pl[a.zero + k] = 0;
+    load_stage(0);
+    cp_async_wait<0>();
+    __syncthreads();
+    to_planar(0);
+    for (int q = 0; q < a.nq; ++q) {
+        const int bq = blk * a.nq + q, nch = min(a.cc, a.nlive - q * a.cc);
+        const int np = a.pstart[bq + 1] - a.pstart[bq], ng = a.gtot[bq];
+        __syncthreads();
+        if (q + 1 < a.nq) load_stage(q + 1);
+        // the patterns' series: every warp takes an equal run of the stage's
+        // ng groups of 32 elements, starting inside pattern p
+        {
+            const int4* sp = s_pat + (q & 1) * 2 * a.pmax;
+            int g = ng * warp / kTrWarps;
+            const int gend = ng * (warp + 1) / kTrWarps;
+            int p = -1;
+            for (int b0 = 0; b0 < np; b0 += 32) {
+                const bool at = b0 + lane < np && sp[2 * (b0 + lane) + 1].x <= g;
+                p += __popc(__ballot_sync(0xffffffffu, at));
+            }
+            while (g < gend) {
+                const int4 src = sp[2 * p], rec = sp[2 * p + 1];
+                const int n = min(rec.x + rec.y, gend) - g, k = 32 * (g - rec.x) + lane;
+                const uint32_t* x0 = pl + src.x + k;
+                const uint32_t* x1 = pl + src.y + k;
+                const uint32_t* x2 = pl + src.z + k;
+                const uint32_t* x3 = pl + src.w + k;
+                uint32_t* y = ysm + (32 * g + lane) * kYWords;
+#pragma unroll 4
+                for (int m = 0; m < n; ++m) {
+                    const uint32_t v0 = x0[32 * m], v1 = x1[32 * m], v2 = x2[32 * m],
+                                   v3 = x3[32 * m];
+                    if constexpr (MODE == kTrSmall) {
+                        y[32 * m] = v0 + v1 + v2 + v3;
+                    } else if constexpr (MODE == kTr8) {
+                        // whole words summed modulo 2^32; the odd bytes' sums
+                        // taken out of that leave the even bytes' (both < 2^16)
+                        const uint32_t all = v0 + v1 + v2 + v3;
+                        const uint32_t o = __byte_perm(v0, 0, 0x4341) + __byte_perm(v1, 0, 0x4341) +
+                                           __byte_perm(v2, 0, 0x4341) + __byte_perm(v3, 0, 0x4341);
+                        reinterpret_cast<uint2*>(y)[32 * m] = make_uint2(all - o * 256u, o);
+                    } else {
+                        reinterpret_cast<uint2*>(y)[32 * m] =
+                            make_uint2((v0 & 0xffffu) + (v1 & 0xffffu) + (v2 & 0xffffu) + (v3 & 0xffffu),
+                                       (v0 >> 16) + (v1 >> 16) + (v2 >> 16) + (v3 >> 16));
+                    }
+                }
+                g += n;
+                ++p;
+            }
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        // the planar words are free: the next stage's go in beside the sums
+        if (q + 1 < a.nq) to_planar(q + 1);
+        if constexpr (FLUSH) {
+            // before a 16-bit sum can overflow: the sums so far go to the
+            // output rows as whole floats (exact: checked on the host)
+            if (since + nch > a.p16) {
+#pragma unroll
+                for (int j = 0; j < DPW; ++j) {
+                    if (d0 + j * kTrWarps < dend) {
+                        float* o = a.out + (size_t)a.dmrow[d0 + j * kTrWarps] * a.out_pitch + t0 + lane;
+                        each(j, [&](int t, uint32_t v) {
+                            o[t] = flushed ? o[t] + (float)v : (float)v;
+                        });
+                    }
+#pragma unroll
+                    for (int k = 0; k < 2 * W; ++k) acc[j][k] = 0;
+                }
+                flushed = true;
+                since = 0;
+            }
+            since += nch;
+        }
+        // one Y per subband and DM trial
+        const int nb = (nch + S - 1) / S;
+        const int* sy = s_yoff + (q & 1) * nsb * kSlots + warp;
+#pragma unroll
+        for (int j = 0; j < DPW; ++j) {
+            if (d0 + j * kTrWarps >= dend) continue;
+            if constexpr (MODE == kTrSmall) {
+                // bytes as they stand while they cannot overflow
+                for (int b0 = 0; b0 < nb; b0 += a.p8s) {
+                    uint32_t a8[W];
+#pragma unroll
+                    for (int k = 0; k < W; ++k) a8[k] = 0;
+                    const int b1 = min(nb, b0 + a.p8s);
+#pragma unroll 2
+                    for (int b = b0; b < b1; ++b) {
+                        const uint32_t* y = ysm + sy[b * kSlots + j * kTrWarps] + lane;
+#pragma unroll
+                        for (int k = 0; k < W; ++k) a8[k] += y[32 * k];
+                    }
+#pragma unroll
+                    for (int k = 0; k < W; ++k) {
+                        acc[j][k] += __byte_perm(a8[k], 0, 0x4240);
+                        acc[j][W + k] += __byte_perm(a8[k], 0, 0x4341);
+                    }
+                }
+            } else {
+#pragma unroll 2
+                for (int b = 0; b < nb; ++b) {
+                    const uint2* y = reinterpret_cast<const uint2*>(ysm) + sy[b * kSlots + j * kTrWarps] + lane;
+#pragma unroll
+                    for (int k = 0; k < W; ++k) {
+                        const uint2 v = y[32 * k];
+                        acc[j][k] += v.x;
+                        acc[j][W + k] += v.y;
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < DPW; ++j) {
+        if (d0 + j * kTrWarps >= dend) continue;
+        float* o = a.out + (size_t)a.dmrow[d0 + j * kTrWarps] * a.out_pitch + t0 + lane;
+        each(j, [&](int t, uint32_t v) {
+            if constexpr (FLUSH) {
+                if (flushed) v += (uint32_t)o[t];
+                o[t] = map_sum(v, a.mid, a.scale, a.raw);
+            } else if constexpr (MODE == kTr16) {
+                o[t] = map_sum(v, a.mid, a.scale, a.raw);
+            } else {
+                // a 16-bit whole number to float without the conversion unit
+                float f = __uint_as_float(0x4b000000u | v) - 8388608.0f;
+                if (!a.raw) f = __fadd_rn(__fmul_rn(__fsub_rn(f, a.mid), a.scale), 0.5f);
+                o[t] = f;
+            }
+        });
+    }
+}
+
 size_t round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }
 
 }  // namespace
@@ -386,10 +690,16 @@ struct psx_dedisp_plan {
     // derived tables for one sample width (elem bytes), rebuilt when dirty
     bool dirty = true;
     int elem = 0;
+    int kind = -1;          // sample class the tables were built for
     int nlive = 0, ndm_pad = 0, nblk = 0, group = 8, lwin = 0, cc = 0;
     size_t ngroups = 0, max_lo = 0;
     size_t scratch_limit = 4ull << 30;  // bytes of channel-major samples
     size_t flush_bytes = 0;             // shared 32-bit sums above 257 channels
+    // shared-partial-sum form (k_dedisperse_tree): 0 = the direct kernel,
+    // else S; DM trials in order of DM, ndb per block, dpw per warp
+    int tree = 0, dpw = 0, ndb = 0, nq = 0, zero = 0, zlen = 0, plen = 0, gmax = 0, pmax = 0, rawlen = 0,
+        tile = 0;
+    size_t tab_row = 0, tab_ps = 0, tab_gt = 0, tab_pat = 0, tab_yoff = 0;  // in h_tab
     std::vector<int> h_tab;
     int* d_tab = nullptr;
     size_t tab_cap = 0;
@@ -410,10 +720,13 @@ struct psx_dedisp_plan {
         return (size_t)std::floor((double)prod + 0.5);
     }
 
-    // Shift tables and the window shape for `el`-byte samples.
-    int build_tables(int el)
+    // Shift tables and the window shape for one class of samples.
+    int build_tables(int sample_kind)
     {
-        if (!dirty && el == elem) return PSX_OK;
+        if (!dirty && sample_kind == kind) return PSX_OK;
+        const int el = sample_kind == kTr16 ? 2 : 1;
+        kind = sample_kind;
+        dirty = true;
         if (dms.empty()) {
             set_error("psx_dedisp: no DM list set");
             return PSX_ERR_INVALID;
@@ -432,6 +745,13 @@ struct psx_dedisp_plan {
                 float p = dms[d] * delays[chans[i]];
                 shift[(size_t)d * nlive + i] = (int)std::nearbyint(p);
             }
+        tile = dd_tile(el);
+        if (nlive > 0 && build_tree(el, chans, shift)) {
+            elem = el;
+            dirty = true;  // tables must be uploaded
+            return PSX_OK;
+        }
+        tree = 0;
         // window shape for groups of G trials: lo = min shift aligned down,
         // lwin covers 512 outputs past the largest shift plus the read-ahead
         auto shape = [&](int G, std::vector<int>* lo_out, int* lwin_out, size_t* max_lo_out) {
@@ -498,8 +818,215 @@ struct psx_dedisp_plan {
         return PSX_OK;
     }
 
+    // Tables of the shared-partial-sum form, or false where the direct
+    // kernel is taken: the series do not fit shared memory, a sum could pass
+    // 2^24 where sums are kept as floats, or the patterns are so many (few
+    // or widely spaced DM trials) that it moves no fewer words through
+    // shared memory.  The words of a tile: S + 2 per pattern and word of its
+    // series, 2Q per DM trial and subband and 4 per planar word, against 2Q
+    // per DM trial and channel.  Measured on B200 (us, direct against this
+    // form, 64-128 channels x 500k samples, by that ratio, 8 / 2 / 16 bits):
+    // 0.50: 766/416, 661/351, 1496/829; 0.69: 146/120, 122/104, 260/192;
+    // 1.08: 145/157, 121/143, 261/263; 1.53: 155/208, 133/200, 321/357.
+    bool build_tree(int el, const std::vector<int>& chans, const std::vector<int>& shift)
+    {
+        constexpr int S = kTrS;
+        const int ndm = (int)dms.size();
+        if (el == 1 && (double)nlive * 255.0 >= 16777216.0) return false;
+        std::vector<int> order(ndm);
+        for (int d = 0; d < ndm; ++d) order[d] = d;
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return dms[x] < dms[y]; });
+        const int nb_ = (ndm + kTrMaxDms - 1) / kTrMaxDms;
+        const int per = (ndm + nb_ - 1) / nb_;       // DM trials per block, evenly
+        const int dw = (per + kTrWarps - 1) / kTrWarps, slots = kTrWarps * dw;
+        const int blocks = (ndm + per - 1) / per;
+        const int nsbt = (nlive + S - 1) / S, align = 16 / el;
+        struct Pat {
+            int first, lo, groups;  // a trial that has it, smallest reference shift, 32-word groups
+        };
+        // per (block, channel): window start, planar words / 4
+        std::vector<int> lo((size_t)blocks * nlive), quads((size_t)blocks * nlive);
+        std::vector<int> np((size_t)blocks * nsbt);
+        std::vector<Pat> pats;                       // in (block, subband) order
+        std::vector<uint8_t> which((size_t)ndm * nsbt);
+        int most = 0;
+        size_t mlo = 0, ngroups_ = 0, nquads = 0;
+        for (int g = 0; g < blocks; ++g) {
+            const int e0 = g * per, e1 = std::min(ndm, e0 + per);
+            int* l = &lo[(size_t)g * nlive];
+            std::vector<int> mx(shift.begin() + (size_t)order[e0] * nlive,
+                                shift.begin() + (size_t)(order[e0] + 1) * nlive);
+            std::copy(mx.begin(), mx.end(), l);
+            for (int e = e0 + 1; e < e1; ++e) {
+                const int* v = &shift[(size_t)order[e] * nlive];
+                for (int i = 0; i < nlive; ++i) {
+                    l[i] = std::min(l[i], v[i]);
+                    mx[i] = std::max(mx[i], v[i]);
+                }
+            }
+            for (int i = 0; i < nlive; ++i) {
+                l[i] = l[i] / align * align;
+                // a multiple of 16 planar words, so that the windows start 16-byte aligned
+                const int qd = (int)round_up((size_t)(kTrQ + mx[i] - l[i]), 16) / 4;
+                quads[(size_t)g * nlive + i] = qd;
+                most = std::max(most, qd);
+                nquads += qd;
+                mlo = std::max(mlo, (size_t)l[i]);
+            }
+            for (int b = 0; b < nsbt; ++b) {
+                const int c0 = b * S, nc = std::min(S, nlive - c0);
+                int first[kTrMaxDms], mn[kTrMaxDms], mxr[kTrMaxDms], n = 0, last = 0;
+                for (int e = e0; e < e1; ++e) {
+                    const int* v = &shift[(size_t)order[e] * nlive + c0];
+                    auto same = [&](int p) {
+                        const int* u = &shift[(size_t)order[first[p]] * nlive + c0];
+                        for (int c = 1; c < nc; ++c)
+                            if (v[c] - v[0] != u[c] - u[0]) return false;
+                        return true;
+                    };
+                    int p = last;
+                    if (n == 0 || !same(p))
+                        for (p = 0; p < n && !same(p);) ++p;
+                    if (p == n) {
+                        first[n] = e;
+                        mn[n] = mxr[n] = v[0];
+                        ++n;
+                    }
+                    mn[p] = std::min(mn[p], v[0]);
+                    mxr[p] = std::max(mxr[p], v[0]);
+                    which[(size_t)e * nsbt + b] = (uint8_t)p;
+                    last = p;
+                }
+                np[(size_t)g * nsbt + b] = n;
+                for (int p = 0; p < n; ++p) {
+                    const int gr = (kTrQ + mxr[p] - mn[p] + 31) / 32;
+                    pats.push_back({first[p], mn[p], gr});
+                    ngroups_ += gr;
+                }
+            }
+        }
+        const double q2 = 2.0 * kTrQ, cost_direct = (double)nlive * ndm * q2;
+        const double cost = (double)ngroups_ * 32 * (S + 2) + (double)nsbt * blocks * slots * q2 +
+                            16.0 * (double)nquads;
+        if (cost >= 0.9 * cost_direct) return false;
+        // channels per stage: the most that leave two CTAs on an SM
+        const int yw = kind == kTrSmall ? 1 : 2;
+        int c_ = 0, pm = 0, gm = 0, nm = 0;
+        const int more = el == 1 ? 3 * kTrQ / 4 : kTrQ / 2;
+        for (int c : {32, 16, 8, 4}) {
+            if (c > 4 && c / 2 >= nlive) continue;
+            pm = gm = nm = 0;
+            size_t at = 0;
+            for (int g = 0; g < blocks; ++g)
+                for (int b0 = 0; b0 < nsbt; b0 += c / S) {
+                    int gr = 0, pw = 0, n = 0;
+                    for (int b = b0; b < std::min(nsbt, b0 + c / S); ++b)
+                        for (int p = 0; p < np[(size_t)g * nsbt + b]; ++p, ++n) gr += pats[at++].groups;
+                    nm = std::max(nm, n);
+                    for (int i = b0 * S; i < std::min(nlive, b0 * S + c); ++i)
+                        pw += 4 * quads[(size_t)g * nlive + i];
+                    pm = std::max(pm, pw);
+                    gm = std::max(gm, gr);
+                }
+            // the last group of a pattern may read up to 31 words past a
+            // channel's: into the next one's, or the zeros
+            const size_t b = tree_bytes(raw_words(c, pm, more, el), pm + 4 * most + 32, gm, yw, nm,
+                                        c / S * slots);
+            if (b <= 112 * 1024 || (c == 4 && b <= 220 * 1024)) {
+                c_ = c;
+                break;
+            }
+        }
+        if (!c_) return false;
+        const int nq_ = (nlive + c_ - 1) / c_, sbs = c_ / S;
+        // tables: channel records, output rows, per stage the first pattern
+        // and the groups, pattern records, the trials' Y offsets
+        tab_row = 4 * (size_t)blocks * nlive;
+        tab_ps = tab_row + round_up((size_t)ndm, 4);
+        tab_gt = tab_ps + round_up((size_t)blocks * nq_ + 1, 4);
+        tab_pat = tab_gt + round_up((size_t)blocks * nq_, 4);
+        tab_yoff = tab_pat + pats.size() * kTrRec;
+        h_tab.assign(tab_yoff + (size_t)blocks * nq_ * sbs * slots, 0);
+        for (int g = 0; g < blocks; ++g)
+            for (int i = 0, at = 0; i < nlive; ++i) {
+                if (i % c_ == 0) at = 0;
+                int* ch = h_tab.data() + 4 * ((size_t)g * nlive + i);
+                ch[0] = chans[i];
+                ch[1] = lo[(size_t)g * nlive + i];
+                ch[2] = at;
+                ch[3] = quads[(size_t)g * nlive + i];
+                at += 4 * ch[3];
+            }
+        std::copy(order.begin(), order.end(), h_tab.begin() + tab_row);
+        int* ps = h_tab.data() + tab_ps;
+        int* gt = h_tab.data() + tab_gt;
+        int* yo = h_tab.data() + tab_yoff;
+        size_t at = 0;  // next pattern
+        for (int g = 0; g < blocks; ++g) {
+            const int e0 = g * per, e1 = std::min(ndm, e0 + per);
+            for (int b = 0; b < nsbt; ++b) {
+                const int q = b / sbs, c0 = b * S, n = np[(size_t)g * nsbt + b];
+                int& gr = gt[g * nq_ + q];
+                if (b % sbs == 0) {
+                    ps[g * nq_ + q] = (int)at;
+                    gr = 0;
+                }
+                int ybase[kTrMaxDms];
+                for (int p = 0; p < n; ++p) {
+                    const Pat& pt = pats[at + p];
+                    const int* u = &shift[(size_t)order[pt.first] * nlive];
+                    int* rec = h_tab.data() + tab_pat + (at + p) * kTrRec;
+                    for (int c = 0; c < S; ++c) {
+                        const int i = c0 + c;
+                        const int* ch = h_tab.data() + 4 * ((size_t)g * nlive + i);
+                        rec[c] = i < nlive ? ch[2] + pt.lo + (u[i] - u[c0]) - ch[1]
+                                           : pm;  // the zeros
+                    }
+                    rec[4] = gr;
+                    rec[5] = pt.groups;
+                    ybase[p] = 32 * gr - pt.lo;
+                    gr += pt.groups;
+                }
+                int* row = yo + (((size_t)g * nq_ + q) * sbs + b % sbs) * slots;
+                for (int e = e0; e < e1; ++e)
+                    row[e - e0] = ybase[which[(size_t)e * nsbt + b]] +
+                                  shift[(size_t)order[e] * nlive + c0];
+                at += n;
+            }
+        }
+        ps[blocks * nq_] = (int)at;
+        tree = S;
+        dpw = dw;
+        ndb = per;
+        nblk = blocks;
+        cc = c_;
+        nq = nq_;
+        zero = pm;
+        zlen = 4 * most + 32;
+        plen = zero + zlen;
+        gmax = gm;
+        pmax = nm;
+        rawlen = raw_words(c_, pm, more, el);
+        lwin = 4 * most + (el == 1 ? 3 : 1) * kTrQ;
+        max_lo = mlo;
+        tile = tr_tile(el);
+        return true;
+    }
+
+    // a stage's windows: the planar words' samples once, and per channel
+    // the parts after the first
+    static int raw_words(int c, int pm, int more, int el) { return pm / (el == 1 ? 4 : 2) + c * (more + 4); }
+
+    static size_t tree_bytes(int raw, int plen, int gmax, int yw, int pmax, int trials)
+    {
+        return 4ull * ((size_t)raw + plen + 32ull * gmax * yw + 2ull * pmax * kTrRec + 2ull * trials);
+    }
+
     size_t smem_bytes() const
     {
+        if (tree)
+            return tree_bytes(rawlen, plen, gmax, kind == kTrSmall ? 1 : 2, pmax,
+                              cc / kTrS * kTrWarps * dpw);
         return 2ull * cc * (kDdWarps / group) * lwin * elem + 2ull * kDdWarps * cc * sizeof(int) +
                flush_bytes;
     }
@@ -573,11 +1100,13 @@ int check_input(psx_dedisp_plan* p, size_t nsamps, int nbits, float* d_out, size
 // samples (a multiple of the CTA tile) so that cm, *pitch samples per
 // channel, stays within the plan's scratch limit; one gulp covers the
 // whole series when it fits.
-int prepare(psx_dedisp_plan* p, size_t nout, int el, cudaStream_t st, size_t* gulp,
+int prepare(psx_dedisp_plan* p, size_t nout, int nbits, cudaStream_t st, size_t* gulp,
             size_t* pitch)
 {
-    bool rebuilt = p->dirty || el != p->elem;
-    PSX_TRY(p->build_tables(el));
+    const int kind = nbits == 16 ? kTr16 : nbits <= 4 ? kTrSmall : kTr8;
+    const int el = nbits == 16 ? 2 : 1;
+    bool rebuilt = p->dirty || kind != p->kind;
+    PSX_TRY(p->build_tables(kind));
     if (rebuilt) {
         size_t bytes = p->h_tab.size() * sizeof(int);
         PSX_TRY(grow(reinterpret_cast<void**>(&p->d_tab), &p->tab_cap, std::max<size_t>(bytes, 4),
@@ -585,7 +1114,7 @@ int prepare(psx_dedisp_plan* p, size_t nout, int el, cudaStream_t st, size_t* gu
         PSX_CUDA(cudaMemcpyAsync(p->d_tab, p->h_tab.data(), bytes, cudaMemcpyHostToDevice, st));
         p->dirty = false;
     }
-    const size_t tile = dd_tile(el);
+    const size_t tile = (size_t)p->tile;
     const size_t md = p->max_delay();
     auto pitch_for = [&](size_t g) {
         size_t nt = (g + tile - 1) / tile;
@@ -632,9 +1161,72 @@ int unpack(int nbits, const uint8_t* rows, size_t nrows, size_t r0, size_t ncols
     }
 }
 
+template <int MODE, bool FLUSH>
+int launch_tree(const TreeArgs& a, int dpw, unsigned grid, size_t smem, cudaStream_t st)
+{
+    auto go = [&](auto kern) -> int {
+        PSX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+        kern<<<grid, kTrThreads, smem, st>>>(a);
+        return launch_status("k_dedisperse_tree");
+    };
+    return dpw == 1 ? go(k_dedisperse_tree<MODE, 1, FLUSH>) : go(k_dedisperse_tree<MODE, 2, FLUSH>);
+}
+
+// The shared-partial-sum form (p->tree).
+int dedisperse_tree(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, float* d_out,
+                    size_t out_pitch, int flags, cudaStream_t st)
+{
+    TreeArgs a;
+    a.cm = p->d_cm;
+    a.pitch = pitch;
+    a.chan = reinterpret_cast<const int4*>(p->d_tab);
+    a.dmrow = p->d_tab + p->tab_row;
+    a.pstart = p->d_tab + p->tab_ps;
+    a.pat = reinterpret_cast<const int4*>(p->d_tab + p->tab_pat);
+    a.gtot = p->d_tab + p->tab_gt;
+    a.yoff = p->d_tab + p->tab_yoff;
+    a.nlive = p->nlive;
+    a.ndm = (int)p->dms.size();
+    a.ndb = p->ndb;
+    a.nblk = p->nblk;
+    a.cc = p->cc;
+    a.nq = p->nq;
+    a.zero = p->zero;
+    a.zlen = p->zlen;
+    a.plen = p->plen;
+    a.gmax = p->gmax;
+    a.pmax = p->pmax;
+    a.rawlen = p->rawlen;
+    a.out = d_out;
+    a.out_pitch = out_pitch;
+    a.nout = nout;
+    const unsigned m = (1u << nbits) - 1u;
+    a.mid = (float)(0.5 * (double)p->nchans * (double)m);
+    a.scale = (float)(1.0 / ((double)m * std::sqrt((double)p->nchans)));
+    a.raw = (flags & PSX_DEDISP_RAW) ? 1 : 0;
+    a.p16 = (int)(65535u / m);
+    a.p8s = (int)(255u / m) / kTrS;
+    const size_t ntiles = (nout + p->tile - 1) / p->tile, nblocks = ntiles * (size_t)p->nblk;
+    if (nblocks > 0x7fffffffull) {
+        set_error("psx_dedisp: %zu blocks exceed one launch", nblocks);
+        return PSX_ERR_UNSUPPORTED;
+    }
+    const size_t smem = p->smem_bytes();
+    const unsigned grid = (unsigned)nblocks;
+    if (nbits == 16) return launch_tree<kTr16, false>(a, p->dpw, grid, smem, st);
+    const bool flush = p->nlive > a.p16;
+    if (nbits <= 4)
+        return flush ? launch_tree<kTrSmall, true>(a, p->dpw, grid, smem, st)
+                     : launch_tree<kTrSmall, false>(a, p->dpw, grid, smem, st);
+    return flush ? launch_tree<kTr8, true>(a, p->dpw, grid, smem, st)
+                 : launch_tree<kTr8, false>(a, p->dpw, grid, smem, st);
+}
+
 int dedisperse(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, float* d_out,
                size_t out_pitch, int flags, cudaStream_t st)
 {
+    if (p->tree) return dedisperse_tree(p, nbits, pitch, nout, d_out, out_pitch, flags, st);
     DedispArgs a;  // with every channel killed the sums are zero
     a.cm = p->d_cm;
     a.pitch = pitch;
@@ -818,8 +1410,7 @@ int psx_dedisp_execute(psx_dedisp_plan* p, size_t nsamps, const uint8_t* d_in, i
     PSX_TRY(check_input(p, nsamps, nbits, d_out, out_pitch, &nout));
     if (!d_in) return PSX_ERR_INVALID;
     cudaStream_t st = cs(stream);
-    const int el = nbits == 16 ? 2 : 1;
-    PSX_TRY(prepare(p, nout, el, st, &gulp, &pitch));
+    PSX_TRY(prepare(p, nout, nbits, st, &gulp, &pitch));
     const size_t row_bytes = p->nchans * (size_t)nbits / 8;
     const size_t md = p->max_delay();
     for (size_t g0 = 0; g0 < nout; g0 += gulp) {
@@ -838,8 +1429,7 @@ int psx_dedisp_execute_host(psx_dedisp_plan* p, size_t nsamps, const uint8_t* h_
     PSX_TRY(check_input(p, nsamps, nbits, d_out, out_pitch, &nout));
     if (!h_in) return PSX_ERR_INVALID;
     cudaStream_t st = cs(stream);
-    const int el = nbits == 16 ? 2 : 1;
-    PSX_TRY(prepare(p, nout, el, st, &gulp, &pitch));
+    PSX_TRY(prepare(p, nout, nbits, st, &gulp, &pitch));
     const size_t row_bytes = p->nchans * (size_t)nbits / 8;
     const size_t md = p->max_delay();
     // pieces of about 32 MB, a multiple of the unpack tile
