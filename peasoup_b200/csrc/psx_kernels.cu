@@ -253,18 +253,21 @@ static float stretch_step(size_t in_count, size_t out_count)
     return (float)(in_count - 1) / (float)(out_count - 1);
 }
 
-// Amplitudes of the complex spectrum X and their three median-of-5
-// levels in one pass: a CTA takes groups of 125 bins (5 * 25) at a time, so
+// The three median-of-5 levels of the amplitudes of a complex spectrum X
+// (AMP), or of the powers X as they are, in one pass: a CTA takes groups of 125 bins (5 * 25) at a time, so
 // every value of the 5-, 25- and 125-bin levels it writes is formed from
 // its own bins; the levels stop where the reference's floor(count / 5)
-// stops them.  The amplitudes themselves are never written.
+// stops them.  The amplitudes themselves are never written.  (One launch in
+// place of three for the powers: at 2^20 bins on B200 6.4 us of three
+// latency-bound kernels became 3.7.)
 constexpr int kScrGroups = 16;  // 125-bin groups per CTA step
 
-__global__ void __launch_bounds__(256) k_amp_scrunch3(const float* __restrict__ X, size_t nbins,
-                                                      float* __restrict__ m5, size_t n5,
-                                                      float* __restrict__ m25, size_t n25,
-                                                      float* __restrict__ m125, size_t n125,
-                                                      size_t x_stride = 0, size_t m_stride = 0)
+template <bool AMP>
+__global__ void __launch_bounds__(256) k_scrunch3(const float* __restrict__ X,
+                                                  float* __restrict__ m5, size_t n5,
+                                                  float* __restrict__ m25, size_t n25,
+                                                  float* __restrict__ m125, size_t n125,
+                                                  size_t x_stride = 0, size_t m_stride = 0)
 {
     // row blockIdx.y of a batch: its spectrum and its scratch (strides in floats)
     X += (size_t)blockIdx.y * x_stride;
@@ -280,12 +283,15 @@ __global__ void __launch_bounds__(256) k_amp_scrunch3(const float* __restrict__ 
             const size_t j = g0 * 25 + i;  // 5-level index
             float v = 0.f;
             if (j < n5) {
-                const float2* p = reinterpret_cast<const float2*>(X) + 5 * j;
                 float a[5];
 #pragma unroll
                 for (int t = 0; t < 5; ++t) {
-                    const float2 z = p[t];
-                    a[t] = amplitude(z.x, z.y);
+                    if constexpr (AMP) {
+                        const float2 z = reinterpret_cast<const float2*>(X)[5 * j + t];
+                        a[t] = amplitude(z.x, z.y);
+                    } else {
+                        a[t] = X[5 * j + t];
+                    }
                 }
                 v = med5(a[0], a[1], a[2], a[3], a[4]);
                 m5[j] = v;
@@ -359,7 +365,7 @@ int launch_running_median_spectrum(float* d_X, size_t nbins, double bin_width, f
     const size_t ngroups = (n5 + 24) / 25;
     const unsigned grid = (unsigned)std::min<size_t>((ngroups + kScrGroups - 1) / kScrGroups,
                                                      (size_t)sm_count() * 8);
-    k_amp_scrunch3<<<grid, 256, 0, s>>>(d_X, nbins, m5, n5, m25, n25, m125, n125);
+    k_scrunch3<true><<<grid, 256, 0, s>>>(d_X, m5, n5, m25, n25, m125, n125);
     PSX_TRY(launch_status("amplitude + scrunch kernel"));
     return median_apply(nbins, bin_width, b5, b25, nullptr, d_X, m5, m25, m125, s);
 }
@@ -376,29 +382,13 @@ int launch_running_median(const float* d_powers, size_t nbins, double bin_width,
     float* m5 = static_cast<float*>(d_scratch);
     float* m25 = m5 + up(nbins / 5 + 1);
     float* m125 = m25 + up(nbins / 25 + 1);
-    const size_t n5 = nbins / 5, n25 = nbins / 5 / 5, n125 = nbins / 5 / 5 / 5;
-    const unsigned T = 256;
-    k_scrunch5<<<grid_for(n5, T), T, 0, s>>>(d_powers, nbins, m5);
-    k_scrunch5<<<grid_for(n25, T), T, 0, s>>>(m5, n5, m25);
-    k_scrunch5<<<grid_for(n125, T), T, 0, s>>>(m25, n25, m125);
-    // reference dereddener.hpp:48-49: (int)(boundary / bin_width)
-    int pos5 = (int)((double)b5 / bin_width);
-    int pos25 = (int)((double)b25 / bin_width);
-    MedianLevels L;
-    L.m5 = m5;
-    L.m25 = m25;
-    L.m125 = m125;
-    L.n5 = (unsigned)n5;
-    L.n25 = (unsigned)n25;
-    L.n125 = (unsigned)n125;
-    L.step5 = stretch_step(n5, nbins);
-    L.step25 = stretch_step(n25, nbins);
-    L.step125 = stretch_step(n125, nbins);
-    L.pos5 = (unsigned)(pos5 < 0 ? 0 : (size_t)pos5 > nbins ? nbins : pos5);
-    L.pos25 = (unsigned)(pos25 < 0 ? 0 : (size_t)pos25 > nbins ? nbins : pos25);
-    if (L.pos25 < L.pos5) L.pos25 = L.pos5;
-    k_median_apply<<<grid_for(nbins, T), T, 0, s>>>(L, nbins, d_median, d_X);
-    return launch_status("running median kernels");
+    const size_t n5 = nbins / 5, n25 = n5 / 5, n125 = n25 / 5;
+    const size_t ngroups = (n5 + 24) / 25;
+    const unsigned grid = (unsigned)std::min<size_t>((ngroups + kScrGroups - 1) / kScrGroups,
+                                                     (size_t)sm_count() * 8);
+    k_scrunch3<false><<<grid, 256, 0, s>>>(d_powers, m5, n5, m25, n25, m125, n125);
+    PSX_TRY(launch_status("scrunch kernel"));
+    return median_apply(nbins, bin_width, b5, b25, d_median, d_X, m5, m25, m125, s);
 }
 
 // ------------------------------------------------------------------- zapping
@@ -780,8 +770,8 @@ int launch_running_median_spectrum_rows(float* d_X, size_t x_stride, int rows, s
     const size_t ngroups = (n5 + 24) / 25;
     const unsigned grid = (unsigned)std::min<size_t>((ngroups + kScrGroups - 1) / kScrGroups,
                                                      (size_t)sm_count() * 8);
-    k_amp_scrunch3<<<dim3(grid, rows), 256, 0, s>>>(d_X, nbins, m5, n5, m25, n25, m125, n125,
-                                                     x_stride, scratch_stride_floats);
+    k_scrunch3<true><<<dim3(grid, rows), 256, 0, s>>>(d_X, m5, n5, m25, n25, m125, n125, x_stride,
+                                                      scratch_stride_floats);
     PSX_TRY(launch_status("amplitude + scrunch kernel (rows)"));
     int pos5 = (int)((double)b5 / bin_width);
     int pos25 = (int)((double)b25 / bin_width);
@@ -843,7 +833,10 @@ int launch_stats(const float* d_x, bool interbinned, size_t first, size_t n, dou
 {
     const unsigned T = 256;
     const int nb = reduction_blocks();
-    if (interbinned)
+    if (!interbinned && (reinterpret_cast<uintptr_t>(d_x + first) & 15u) == 0)
+        k_partials_v4<<<nb, kVecThreads, 0, s>>>(d_x + first, n - first, d_partials, nullptr,
+                                                 nullptr);
+    else if (interbinned)
         k_sum_partials<InterbinSrc><<<nb, T, 0, s>>>(InterbinSrc{d_x}, first, n, d_partials);
     else
         k_sum_partials<PlainSrc><<<nb, T, 0, s>>>(PlainSrc{d_x}, first, n, d_partials);
@@ -852,11 +845,29 @@ int launch_stats(const float* d_x, bool interbinned, size_t first, size_t n, dou
 }
 
 // ------------------------------------------------------------- element-wise
-__global__ void k_normalise(float* __restrict__ x, float mean, float sigma, size_t n)
+// Four values per thread from one 128-bit load where x is 16-byte aligned
+// (VEC), the n % 4 last ones by block 0.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_normalise(float* __restrict__ x, float mean, float sigma,
+                                                   size_t n)
 {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        x[i] = normalise(x[i], mean, sigma);
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (VEC) {
+        float4* x4 = reinterpret_cast<float4*>(x);
+        for (size_t q = first; q < n / 4; q += stride) {
+            float4 v = x4[q];
+            v.x = normalise(v.x, mean, sigma);
+            v.y = normalise(v.y, mean, sigma);
+            v.z = normalise(v.z, mean, sigma);
+            v.w = normalise(v.w, mean, sigma);
+            x4[q] = v;
+        }
+        const size_t i = n / 4 * 4 + first;
+        if (blockIdx.x == 0 && i < n) x[i] = normalise(x[i], mean, sigma);
+    } else {
+        for (size_t i = first; i < n; i += stride) x[i] = normalise(x[i], mean, sigma);
+    }
 }
 
 __global__ void k_sub_scalar(float* __restrict__ x, size_t n, const float* __restrict__ v)
@@ -929,114 +940,166 @@ struct FoldPtrs {
     float* p[5];
 };
 
-// One thread per output bin, the running sum in the reference's order
-// (src/kernels.cu:41-96).
-__global__ void __launch_bounds__(256) k_harmonic_sum(const float* __restrict__ in,
-                                                      FoldPtrs out, unsigned n, int nharms)
+// Adds the fractions m/2^H (odd m, in the reference's order) of the bins
+// i + 32 k, k < K, to val: 32 m / 2^H is whole for H <= 5, so the K reads of
+// a fraction are one computed index and constant distances from it.
+template <int H, int K>
+__device__ __forceinline__ void add_fractions(const float* __restrict__ in, unsigned i, int take,
+                                              float (&val)[K])
 {
-    const unsigned stride = gridDim.x * blockDim.x;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        float val = in[i];
-        if (nharms > 0) {
-            val += in[frac_index<1>(i, 1)];
-            out.p[0][i] = val * rsqrt(2.0);
-        }
-        if (nharms > 1) {
-            val += in[frac_index<2>(i, 3)];
-            val += in[frac_index<2>(i, 1)];
-            out.p[1][i] = val * 0.5;
-        }
-        if (nharms > 2) {
 #pragma unroll
-            for (unsigned m = 1; m < 8; m += 2) val += in[frac_index<3>(i, m)];
-            out.p[2][i] = val * rsqrt(8.0);
-        }
-        if (nharms > 3) {
+    for (int r = 0; r < (1 << (H - 1)); ++r) {
+        const unsigned m = H == 2 ? (r == 0 ? 3u : 1u) : 2u * r + 1u;  // fold 2 adds 3/4 first
+        const float* p = in + frac_index<H>(i, m);
 #pragma unroll
-            for (unsigned m = 1; m < 16; m += 2) val += in[frac_index<4>(i, m)];
-            out.p[3][i] = val * 0.25;
-        }
-        if (nharms > 4) {
+        for (int k = 0; k < K; ++k)
+            if (k < take) val[k] += p[(size_t)k * (32u * m >> H)];
+    }
+}
+
+// The running sums in the reference's order (src/kernels.cu:41-96): a warp
+// takes 32 K consecutive bins, lane l the bins l + 32 k.  Bound by the loads'
+// L1 wavefronts (one or two per 32 reads); one bin per thread with every
+// index formed anew took 44 us at 2^21 bins and 5 folds on B200, this 19.
+constexpr int kHsBins = 4;
+
+template <int NH>
+__global__ void __launch_bounds__(256) k_harmonic_sum(const float* __restrict__ in, FoldPtrs out,
+                                                      unsigned n)
+{
+    constexpr int K = kHsBins;
+    const unsigned warps = gridDim.x * (blockDim.x / 32);
+    const unsigned nw = n / (32 * K) + (n % (32 * K) != 0);
+    for (unsigned w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; w < nw; w += warps) {
+        const unsigned i = w * (32 * K) + (threadIdx.x & 31);
+        // bins of this lane inside the spectrum
+        const int take = i >= n ? 0 : (int)min((unsigned)K, (n - 1 - i) / 32 + 1);
+        float val[K];
 #pragma unroll
-            for (unsigned m = 1; m < 32; m += 2) val += in[frac_index<5>(i, m)];
-            out.p[4][i] = val * rsqrt(32.0);
+        for (int k = 0; k < K; ++k) val[k] = k < take ? in[i + 32 * k] : 0.f;
+        auto put = [&](float* o, auto scale) {
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (k < take) o[i + 32 * k] = val[k] * scale;
+        };
+        add_fractions<1>(in, i, take, val);
+        put(out.p[0], rsqrt(2.0));
+        if constexpr (NH > 1) {
+            add_fractions<2>(in, i, take, val);
+            put(out.p[1], 0.5f);  // exact, as the double product is
+        }
+        if constexpr (NH > 2) {
+            add_fractions<3>(in, i, take, val);
+            put(out.p[2], rsqrt(8.0));
+        }
+        if constexpr (NH > 3) {
+            add_fractions<4>(in, i, take, val);
+            put(out.p[3], 0.25f);
+        }
+        if constexpr (NH > 4) {
+            add_fractions<5>(in, i, take, val);
+            put(out.p[4], rsqrt(32.0));
         }
     }
 }
 
 // ------------------------------------------------------------- compaction
 // Order-preserving stream compaction of (i, x[i]) with x[i] > thresh over
-// [start, n): per-tile counts, a single-block scan, then the scatter.
-constexpr int kCompactTile = 4096;
+// [start, n) in two kernels.  The bins are cut into one run per CTA (at most
+// kPeakRuns, a multiple of 256 bins each) and every run into one part per
+// warp.  The first kernel counts per part and per run; in the second a CTA
+// adds the counts of the runs before its own and its warps write their
+// parts.  Values above a threshold are rare, so most warps read their bins
+// once, in the first kernel.  (Counting per 4096 bins, a one-thread scan over
+// the tiles and a write that read every tile again took 7 + 10 + 9 us at 2^21
+// bins on B200, this 3.6 + 3.7.)
+constexpr int kPeakRuns = 1024;
+constexpr int kPeakWarps = 8;
+constexpr int kPeakInts = kPeakRuns * (1 + kPeakWarps) + 1;  // scratch: runs, parts, total
 
-__global__ void __launch_bounds__(256) k_compact_count(const float* __restrict__ x, int start,
-                                                       int n, float thresh, int* __restrict__ counts)
+__global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_count(const float* __restrict__ x,
+                                                                 int start, int n, int run,
+                                                                 float thresh,
+                                                                 int* __restrict__ counts)
 {
-    const int t0 = start + blockIdx.x * kCompactTile;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x / 32, part = run / kPeakWarps;
+    const long long a = start + (long long)blockIdx.x * run + (long long)warp * part;
+    const int len = (int)max(0LL, min((long long)part, (long long)n - a));
+    const float* p = x + a;
     int c = 0;
-    for (int i = t0 + threadIdx.x; i < n && i < t0 + kCompactTile; i += blockDim.x)
-        c += x[i] > thresh;
-    for (int o = 16; o; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    __shared__ int sh[8];
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x / 32] = c;
+#pragma unroll 8
+    for (int k = lane; k < len; k += 32) c += p[k] > thresh;
+    c = __reduce_add_sync(0xffffffffu, c);
+    __shared__ int sh[kPeakWarps];
+    if (lane == 0) {
+        sh[warp] = c;
+        counts[gridDim.x + blockIdx.x * kPeakWarps + warp] = c;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        int s = 0;
-        for (int w = 0; w < (int)(blockDim.x / 32); ++w) s += sh[w];
-        counts[blockIdx.x] = s;
+        int t = 0;
+        for (int w = 0; w < kPeakWarps; ++w) t += sh[w];
+        counts[blockIdx.x] = t;
     }
 }
 
-__global__ void k_compact_scan(int* __restrict__ counts, int ntiles, int* __restrict__ total)
+__global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_write(const float* __restrict__ x,
+                                                                 int start, int n, int run,
+                                                                 float thresh,
+                                                                 const int* __restrict__ counts,
+                                                                 int* __restrict__ total,
+                                                                 int* __restrict__ idx,
+                                                                 float* __restrict__ val, int cap)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int s = 0;
-    for (int i = 0; i < ntiles; ++i) {
-        const int c = counts[i];
-        counts[i] = s;
-        s += c;
-    }
-    *total = s;
-}
-
-__global__ void __launch_bounds__(256) k_compact_write(const float* __restrict__ x, int start,
-                                                       int n, float thresh,
-                                                       const int* __restrict__ offsets,
-                                                       int* __restrict__ idx, float* __restrict__ val,
-                                                       int cap)
-{
-    // one tile per block, processed in order by the block's warps in turn
-    const int t0 = start + blockIdx.x * kCompactTile;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x / 32, nw = blockDim.x / 32;
-    __shared__ int warp_base[8];
-    __shared__ int running;
-    if (threadIdx.x == 0) running = offsets[blockIdx.x];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x / 32, part = run / kPeakWarps;
+    const int own = counts[blockIdx.x];
+    const bool last = blockIdx.x == gridDim.x - 1;
+    if (own == 0 && !last) return;
+    __shared__ int sh[kPeakWarps];
+    int c = 0;  // hits of the runs before this one
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) c += counts[k];
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) sh[warp] = c;
     __syncthreads();
-    for (int c0 = t0; c0 < t0 + kCompactTile && c0 < n; c0 += (int)blockDim.x) {
-        const int i = c0 + threadIdx.x;
-        const bool hit = i < n && i < t0 + kCompactTile && x[i] > thresh;
+    int pos = 0;
+    for (int w = 0; w < kPeakWarps; ++w) pos += sh[w];
+    if (last && threadIdx.x == 0) *total = pos + own;
+    const int* parts = counts + gridDim.x + blockIdx.x * kPeakWarps;
+    for (int w = 0; w < warp; ++w) pos += parts[w];
+    int left = parts[warp];
+    const long long a = start + (long long)blockIdx.x * run + (long long)warp * part;
+    const int len = (int)max(0LL, min((long long)part, (long long)n - a));
+    for (int k = 0; k < len && left > 0; k += 32) {
+        const int i = k + lane;
+        const float v = i < len ? x[a + i] : 0.f;
+        const bool hit = i < len && v > thresh;
         const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) warp_base[warp] = __popc(m);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int s = running;
-            for (int w = 0; w < nw; ++w) {
-                const int c = warp_base[w];
-                warp_base[w] = s;
-                s += c;
-            }
-            running = s;
-        }
-        __syncthreads();
         if (hit) {
-            const int pos = warp_base[warp] + __popc(m & ((1u << lane) - 1));
-            if (pos < cap) {
-                idx[pos] = i;
-                val[pos] = x[i];
+            const int at = pos + __popc(m & ((1u << lane) - 1));
+            if (at < cap) {
+                idx[at] = (int)(a + i);
+                val[at] = v;
             }
         }
-        __syncthreads();
+        pos += __popc(m);
+        left -= __popc(m);
     }
+}
+
+// Both kernels over [start, n), n > start; `scratch` holds kPeakInts ints, its
+// last one the total.
+static int launch_peaks(const float* d_spec, int n, int start, float thresh, int* scratch,
+                        int* d_idx, float* d_val, int cap, cudaStream_t s)
+{
+    const long long bins = (long long)n - start;
+    // runs of at least 2048 bins, so that a short spectrum's few CTAs have work
+    long long run = (bins + kPeakRuns - 1) / kPeakRuns;
+    run = ((run < 2048 ? 2048 : run) + 255) / 256 * 256;
+    const unsigned g = (unsigned)((bins + run - 1) / run);
+    k_peaks_count<<<g, 32 * kPeakWarps, 0, s>>>(d_spec, start, n, (int)run, thresh, scratch);
+    k_peaks_write<<<g, 32 * kPeakWarps, 0, s>>>(d_spec, start, n, (int)run, thresh, scratch,
+                                                scratch + kPeakInts - 1, d_idx, d_val, cap);
+    return launch_status("compaction kernels");
 }
 
 }  // namespace psx
@@ -1267,7 +1330,10 @@ int psx_normalise(float* d_x, float mean, float sigma, size_t n, psx_stream_t st
         return PSX_ERR_INVALID;
     }
     if (n == 0) return PSX_OK;
-    k_normalise<<<grid_for(n, 256), 256, 0, cs(stream)>>>(d_x, mean, sigma, n);
+    if ((reinterpret_cast<uintptr_t>(d_x) & 15u) == 0)
+        k_normalise<true><<<grid_for((n + 3) / 4, 256), 256, 0, cs(stream)>>>(d_x, mean, sigma, n);
+    else
+        k_normalise<false><<<grid_for(n, 256), 256, 0, cs(stream)>>>(d_x, mean, sigma, n);
     return launch_status("normalise kernel");
 }
 
@@ -1281,15 +1347,34 @@ int psx_remove_baseline(float* d_x, size_t n, int* h_passes, psx_stream_t stream
     cudaStream_t s = cs(stream);
     const int nb = reduction_blocks();
     void* scratch = nullptr;
-    PSX_CUDA(cudaMallocAsync(&scratch, sizeof(double2) * nb + 2 * sizeof(double) + 16, s));
+    PSX_CUDA(cudaMallocAsync(&scratch, sizeof(double2) * 2 * nb + 2 * sizeof(double) + 64, s));
     double2* part = static_cast<double2*>(scratch);
-    double* sums = reinterpret_cast<double*>(part + nb);
+    double* sums = reinterpret_cast<double*>(part + 2 * nb);
     float* d_mean = reinterpret_cast<float*>(sums + 2);
+    unsigned* flags = reinterpret_cast<unsigned*>(d_mean + 2);  // as Slot::d_count of the search
     int rc = PSX_OK, count = 0;
     float mean = 0.f;
+    bool more = true;
     // reference src/kernels.cu:467-477: do { subtract mean } while
-    // (|mean| > 5e-7 n), leaving after the 102nd pass at most.
-    do {
+    // (|mean| > 5e-7 n), leaving after the 102nd pass at most.  A series
+    // rarely needs more than two passes: those run without the host (three
+    // kernels and one read-back, where a pass of its own takes four kernels
+    // and a read-back), the loop goes on from there.
+    if ((reinterpret_cast<uintptr_t>(d_x) & 15u) == 0) {
+        unsigned h[2] = {0, 0};
+        rc = launch_partials_v4(d_x, n, part, nullptr, flags + 4, s);
+        for (int pass = 0; pass < 2 && rc == PSX_OK; ++pass)
+            rc = launch_baseline_pass_v4(d_x, n, part + pass * nb, part + (1 - pass) * nb,
+                                         pass ? flags + 6 : flags + 4, flags + 6 + pass, flags + 5,
+                                         pass ? flags + 2 : nullptr, pass ? flags + 3 : nullptr, s);
+        if (rc == PSX_OK)
+            rc = cuda_status(cudaMemcpyAsync(h, flags + 2, sizeof h, cudaMemcpyDeviceToHost, s),
+                             "baseline copy");
+        if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "baseline");
+        more = h[0] != 0;
+        count = (int)h[1];
+    }
+    while (more && rc == PSX_OK) {
         rc = remove_baseline_pass(d_x, n, part, sums, d_mean, s);
         if (rc != PSX_OK) break;
         rc = cuda_status(cudaMemcpyAsync(&mean, d_mean, sizeof(float), cudaMemcpyDeviceToHost, s),
@@ -1297,7 +1382,8 @@ int psx_remove_baseline(float* d_x, size_t n, int* h_passes, psx_stream_t stream
         if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "baseline");
         if (rc != PSX_OK) break;
         if (count++ > 100) break;
-    } while (std::fabs(mean) > 5e-7 * (double)n);
+        more = std::fabs(mean) > 5e-7 * (double)n;
+    }
     cudaFreeAsync(scratch, s);
     if (h_passes) *h_passes = count;
     return rc;
@@ -1355,7 +1441,15 @@ int psx_harmonic_sum(const float* d_in, float* const* h_out_ptrs, size_t n, int 
         }
         o.p[h] = h_out_ptrs[h];
     }
-    k_harmonic_sum<<<grid_for(n, 256), 256, 0, cs(stream)>>>(d_in, o, (unsigned)n, nharms);
+    const unsigned g = grid_for((n + kHsBins - 1) / kHsBins, 256);
+    cudaStream_t s = cs(stream);
+    switch (nharms) {
+    case 1: k_harmonic_sum<1><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
+    case 2: k_harmonic_sum<2><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
+    case 3: k_harmonic_sum<3><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
+    case 4: k_harmonic_sum<4><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
+    default: k_harmonic_sum<5><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
+    }
     return launch_status("harmonic sum kernel");
 }
 
@@ -1371,16 +1465,12 @@ int psx_find_peaks(const float* d_spec, int n, int start, float thresh, int* d_i
     *h_count = 0;
     if (n <= start) return PSX_OK;
     cudaStream_t s = cs(stream);
-    const int ntiles = (n - start + kCompactTile - 1) / kCompactTile;
     int* scratch = nullptr;
-    PSX_CUDA(cudaMallocAsync((void**)&scratch, sizeof(int) * (ntiles + 1), s));
-    k_compact_count<<<ntiles, 256, 0, s>>>(d_spec, start, n, thresh, scratch);
-    k_compact_scan<<<1, 32, 0, s>>>(scratch, ntiles, scratch + ntiles);
-    k_compact_write<<<ntiles, 256, 0, s>>>(d_spec, start, n, thresh, scratch, d_idx, d_val, cap);
-    int rc = launch_status("compaction kernels");
+    PSX_CUDA(cudaMallocAsync((void**)&scratch, sizeof(int) * kPeakInts, s));
+    int rc = launch_peaks(d_spec, n, start, thresh, scratch, d_idx, d_val, cap, s);
     int total = 0;
     if (rc == PSX_OK)
-        rc = cuda_status(cudaMemcpyAsync(&total, scratch + ntiles, sizeof(int),
+        rc = cuda_status(cudaMemcpyAsync(&total, scratch + kPeakInts - 1, sizeof(int),
                                          cudaMemcpyDeviceToHost, s), "find_peaks copy");
     cudaFreeAsync(scratch, s);
     if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "find_peaks");
@@ -1396,8 +1486,8 @@ int psx_find_peaks(const float* d_spec, int n, int start, float thresh, int* d_i
 }  // extern "C"
 
 // ------------------------------------------------- peak finding, no allocation
-// psx_find_peaks_noalloc runs the three compaction kernels of psx_find_peaks
-// with their per-tile counts in a fixed device array instead of memory from
+// psx_find_peaks_noalloc runs the two compaction kernels of psx_find_peaks
+// with their counts in a fixed device array instead of memory from
 // cudaMallocAsync.  It serves callers that may not allocate device memory
 // while they search: hosts that have handed the whole of a GPU's memory to
 // their own pool or to another framework, hosts that forbid allocation
@@ -1406,18 +1496,19 @@ int psx_find_peaks(const float* d_spec, int n, int start, float thresh, int* d_i
 //
 // The array g_peak_tile_scratch is compiled into this library: every GPU
 // that loads the library holds its 256 KiB (+ 4 bytes) until the process
-// exits.  It has room for kNoAllocMaxTiles tile counts plus the total, so a
-// call may scan at most kNoAllocMaxTiles * kCompactTile = 2^28 bins
-// (n - start).  All calls on a device share the one array and it keeps the
-// last call's contents; nothing in it needs to start at zero, because
-// k_compact_count writes every tile count a call uses before k_compact_scan
-// reads it.  Calls whose GPU work overlaps (other streams, other host
+// exits.  A call may scan at most 2^28 bins (n - start), the documented limit
+// of the entry point (one count per 4096 bins would fill the array; the
+// kernels need kPeakInts ints of it).  All calls on a device share the one
+// array and it keeps the last call's contents; nothing in it needs to start
+// at zero, because k_peaks_count writes every count a call uses before
+// k_peaks_write reads it.  Calls whose GPU work overlaps (other streams, other host
 // threads) race on the array and give wrong results.
 namespace psx {
 namespace {
 
 constexpr int kNoAllocMaxTiles = 65536;
-constexpr long long kNoAllocMaxBins = (long long)kNoAllocMaxTiles * kCompactTile;
+constexpr long long kNoAllocMaxBins = (long long)kNoAllocMaxTiles * 4096;
+static_assert(kPeakInts <= kNoAllocMaxTiles + 1, "static scratch");
 constexpr int kNoAllocMaxDevices = 64;
 
 // Device-side storage.  In host code this name is only a handle for the
@@ -1478,14 +1569,10 @@ extern "C" int psx_find_peaks_noalloc(const float* d_spec, int n, int start, flo
     int rc = peak_scratch_address(&scratch);
     if (rc != PSX_OK) return rc;
     cudaStream_t s = cs(stream);
-    const int ntiles = (n - start + kCompactTile - 1) / kCompactTile;
-    k_compact_count<<<ntiles, 256, 0, s>>>(d_spec, start, n, thresh, scratch);
-    k_compact_scan<<<1, 32, 0, s>>>(scratch, ntiles, scratch + ntiles);
-    k_compact_write<<<ntiles, 256, 0, s>>>(d_spec, start, n, thresh, scratch, d_idx, d_val, cap);
-    rc = launch_status("compaction kernels");
+    rc = launch_peaks(d_spec, n, start, thresh, scratch, d_idx, d_val, cap, s);
     int total = 0;
     if (rc == PSX_OK)
-        rc = cuda_status(cudaMemcpyAsync(&total, scratch + ntiles, sizeof(int),
+        rc = cuda_status(cudaMemcpyAsync(&total, scratch + kPeakInts - 1, sizeof(int),
                                          cudaMemcpyDeviceToHost, s), "find_peaks_noalloc copy");
     if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "find_peaks_noalloc");
     if (rc != PSX_OK) return rc;
