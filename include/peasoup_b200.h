@@ -174,6 +174,12 @@ int psx_find_peaks(const float* d_spec, int n, int start, float thresh,
                    int* d_idx, float* d_val, int cap, int* h_count,
                    psx_stream_t stream);
 
+/* psx_find_peaks with the peaks returned in host arrays: the count and up to
+ * 1024 peaks come back in one copy.  PSX_ERR_OVERFLOW with the full count in
+ * *h_count (and nothing written) when cap is too small. */
+int psx_find_peaks_host(const float* d_spec, int n, int start, float thresh, int* h_idx,
+                        float* h_val, int cap, int* h_count, psx_stream_t stream);
+
 /* psx_find_peaks without any device allocation; no counterpart in the
    reference.  For callers that may not allocate GPU memory during a run
    (the device's memory is owned by their own pool or another framework,

@@ -16,6 +16,13 @@ int sm_count();
 void set_error(const char* fmt, ...);
 void clear_error();
 
+// Device scratch of one call, stream-ordered: allocated from a pool of the
+// library's own that keeps up to 64 MiB per device across synchronisations.
+// (The device's default pool gives everything back at each one, and the next
+// cudaMallocAsync then maps memory again: 0.25 ms on B200, more than the
+// kernels of most calls.)  Freed with cudaFreeAsync; any threads and streams.
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+
 inline cudaStream_t cs(psx_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Returns PSX_OK, or PSX_ERR_CUDA with the message recorded.

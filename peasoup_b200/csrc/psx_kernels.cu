@@ -4,6 +4,7 @@
 // Layout conventions: time series are float[N]; complex spectra are
 // interleaved float pairs (cufftComplex); all grids are grid-stride loops
 // sized to a multiple of the SM count (psx::grid_for).
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
@@ -34,6 +35,37 @@ void set_error(const char* fmt, ...)
 }
 
 void clear_error() { g_err.clear(); }
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s)
+{
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {nullptr};
+    static bool tried[64] = {false};
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!tried[dev]) {
+            tried[dev] = true;
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cuuint64_t keep = 64ull << 20;
+            if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess) {
+                pools[dev] = nullptr;
+            } else if (cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold,
+                                               &keep) != cudaSuccess) {
+                cudaMemPoolDestroy(pools[dev]);
+                pools[dev] = nullptr;
+            }
+        }
+        pool = pools[dev];
+    }
+    if (pool && cudaMallocFromPoolAsync(p, bytes, pool, s) == cudaSuccess) return cudaSuccess;
+    (void)cudaGetLastError();  // no pool (or one a device reset took): the default one
+    return cudaMallocAsync(p, bytes, s);
+}
 
 int sm_count()
 {
@@ -1156,7 +1188,7 @@ int psx_resampleII_batch(const float* d_in, float* d_out, size_t size, const flo
     std::vector<double> k(ntrials);
     for (int t = 0; t < ntrials; ++t) k[t] = accel_fact(h_accs[t], tsamp);
     double* d_k = nullptr;
-    PSX_CUDA(cudaMallocAsync((void**)&d_k, sizeof(double) * ntrials, cs(stream)));
+    PSX_CUDA(scratch_alloc((void**)&d_k, sizeof(double) * ntrials, cs(stream)));
     int rc = cuda_status(cudaMemcpyAsync(d_k, k.data(), sizeof(double) * ntrials,
                                          cudaMemcpyHostToDevice, cs(stream)),
                          "resampleII_batch copy");
@@ -1304,7 +1336,7 @@ int psx_stats(const float* d_x, size_t n, size_t first, float* h_mean, float* h_
     void* scratch = nullptr;
     const int nb = reduction_blocks();
     const size_t bytes = sizeof(double2) * nb + 2 * sizeof(double) + 8 * sizeof(float);
-    PSX_CUDA(cudaMallocAsync(&scratch, bytes, s));
+    PSX_CUDA(scratch_alloc(&scratch, bytes, s));
     double2* part = static_cast<double2*>(scratch);
     double* sums = reinterpret_cast<double*>(part + nb);
     float* stat = reinterpret_cast<float*>(sums + 2);
@@ -1347,7 +1379,7 @@ int psx_remove_baseline(float* d_x, size_t n, int* h_passes, psx_stream_t stream
     cudaStream_t s = cs(stream);
     const int nb = reduction_blocks();
     void* scratch = nullptr;
-    PSX_CUDA(cudaMallocAsync(&scratch, sizeof(double2) * 2 * nb + 2 * sizeof(double) + 64, s));
+    PSX_CUDA(scratch_alloc(&scratch, sizeof(double2) * 2 * nb + 2 * sizeof(double) + 64, s));
     double2* part = static_cast<double2*>(scratch);
     double* sums = reinterpret_cast<double*>(part + 2 * nb);
     float* d_mean = reinterpret_cast<float*>(sums + 2);
@@ -1466,7 +1498,7 @@ int psx_find_peaks(const float* d_spec, int n, int start, float thresh, int* d_i
     if (n <= start) return PSX_OK;
     cudaStream_t s = cs(stream);
     int* scratch = nullptr;
-    PSX_CUDA(cudaMallocAsync((void**)&scratch, sizeof(int) * kPeakInts, s));
+    PSX_CUDA(scratch_alloc((void**)&scratch, sizeof(int) * kPeakInts, s));
     int rc = launch_peaks(d_spec, n, start, thresh, scratch, d_idx, d_val, cap, s);
     int total = 0;
     if (rc == PSX_OK)
@@ -1481,6 +1513,57 @@ int psx_find_peaks(const float* d_spec, int n, int start, float thresh, int* d_i
         return PSX_ERR_OVERFLOW;
     }
     return PSX_OK;
+}
+
+int psx_find_peaks_host(const float* d_spec, int n, int start, float thresh, int* h_idx,
+                        float* h_val, int cap, int* h_count, psx_stream_t stream)
+{
+    clear_error();
+    if (!d_spec || !h_count || cap < 0 || (cap > 0 && (!h_idx || !h_val))) {
+        set_error("find_peaks_host: bad arguments");
+        return PSX_ERR_INVALID;
+    }
+    if (start < 0) start = 0;
+    *h_count = 0;
+    if (n <= start) return PSX_OK;
+    cudaStream_t s = cs(stream);
+    // the count and the first kFirst peaks come back in one copy
+    constexpr int kFirst = 1024;
+    int* scratch = nullptr;
+    PSX_CUDA(scratch_alloc((void**)&scratch, sizeof(int) * (kPeakInts + 2 * kFirst), s));
+    int* d_idx = scratch + kPeakInts;
+    float* d_val = reinterpret_cast<float*>(d_idx + kFirst);
+    int first[1 + 2 * kFirst];
+    int rc = launch_peaks(d_spec, n, start, thresh, scratch, d_idx, d_val, kFirst, s);
+    if (rc == PSX_OK)
+        rc = cuda_status(cudaMemcpyAsync(first, d_idx - 1, sizeof first, cudaMemcpyDeviceToHost, s),
+                         "find_peaks_host copy");
+    cudaFreeAsync(scratch, s);
+    if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "find_peaks_host");
+    if (rc != PSX_OK) return rc;
+    const int total = *h_count = first[0];
+    if (total > cap) {
+        set_error("find_peaks_host: %d values above threshold, buffer holds %d", total, cap);
+        return PSX_ERR_OVERFLOW;
+    }
+    if (total <= kFirst) {
+        if (total) std::memcpy(h_idx, first + 1, sizeof(int) * total);
+        if (total) std::memcpy(h_val, first + 1 + kFirst, sizeof(float) * total);
+        return PSX_OK;
+    }
+    PSX_CUDA(scratch_alloc((void**)&scratch, sizeof(int) * (kPeakInts + 2 * (size_t)total), s));
+    d_idx = scratch + kPeakInts;
+    d_val = reinterpret_cast<float*>(d_idx + total);
+    rc = launch_peaks(d_spec, n, start, thresh, scratch, d_idx, d_val, total, s);
+    if (rc == PSX_OK)
+        rc = cuda_status(cudaMemcpyAsync(h_idx, d_idx, sizeof(int) * total, cudaMemcpyDeviceToHost, s),
+                         "find_peaks_host copy");
+    if (rc == PSX_OK)
+        rc = cuda_status(cudaMemcpyAsync(h_val, d_val, sizeof(float) * total,
+                                         cudaMemcpyDeviceToHost, s), "find_peaks_host copy");
+    cudaFreeAsync(scratch, s);
+    if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "find_peaks_host");
+    return rc;
 }
 
 }  // extern "C"

@@ -2158,7 +2158,7 @@ int psx_harmonic_peaks(const float* d_spec, size_t pitch, size_t nbins, int rows
     cudaStream_t cs_ = cs(stream);
     PSX_TRY(configure_harm(nharms));
     unsigned* d_counter = nullptr;
-    PSX_CUDA(cudaMallocAsync((void**)&d_counter, sizeof(unsigned) * 2, cs_));
+    PSX_CUDA(scratch_alloc((void**)&d_counter, sizeof(unsigned) * 2, cs_));
     int rc = cuda_status(cudaMemsetAsync(d_counter, 0, sizeof(unsigned) * 2, cs_), "memset");
     if (rc == PSX_OK)
         rc = launch_harm(nharms, kHarmDefaultShape, d_spec, pitch, (unsigned)nbins, pk, 0, rows,

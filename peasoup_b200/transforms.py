@@ -19,7 +19,6 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import Candidate as _CandPOD
 from ._lib import PsxError, check, load
 
 __all__ = [
@@ -431,9 +430,12 @@ class PeakFinder:
         self.min_freq = float(min_freq)
         self.max_freq = float(max_freq)
         self.min_gap = int(min_gap)
-        self.cap = max(1024, int(size))
-        self.d_idx = torch.zeros(self.cap, dtype=torch.int32, device="cuda")
-        self.d_val = torch.zeros(self.cap, dtype=torch.float32, device="cuda")
+        self.cap = 4096  # grown on demand
+        self._alloc()
+
+    def _alloc(self) -> None:
+        self._idx, self._pidx = np.empty(self.cap, np.int32), np.empty(self.cap, np.int32)
+        self._val, self._pval = np.empty(self.cap, np.float32), np.empty(self.cap, np.float32)
 
     def find_candidates(self, spec, cands: SpectrumCandidates) -> None:
         if isinstance(spec, HarmonicSums):
@@ -447,36 +449,32 @@ class PeakFinder:
                                self.max_freq, C.byref(start), C.byref(end), C.byref(factor)),
               "peak_range")
         count = C.c_int()
-        rc = L.psx_find_peaks(_ptr(spec.data), end.value, start.value, self.threshold,
-                              _ptr(self.d_idx), _ptr(self.d_val), self.cap, C.byref(count),
-                              _stream())
-        if rc == _lib.PSX_ERR_OVERFLOW:
+        while True:
+            rc = L.psx_find_peaks_host(_ptr(spec.data), end.value, start.value, self.threshold,
+                                       self._idx.ctypes.data, self._val.ctypes.data, self.cap,
+                                       C.byref(count), _stream())
+            if rc != _lib.PSX_ERR_OVERFLOW:
+                break
             self.cap = int(count.value * 1.25) + 1024
-            self.d_idx = torch.zeros(self.cap, dtype=torch.int32, device="cuda")
-            self.d_val = torch.zeros(self.cap, dtype=torch.float32, device="cuda")
-            rc = L.psx_find_peaks(_ptr(spec.data), end.value, start.value, self.threshold,
-                                  _ptr(self.d_idx), _ptr(self.d_val), self.cap, C.byref(count),
-                                  _stream())
+            self._alloc()
         check(rc, "find_peaks")
         n = count.value
         if n == 0:
             return
-        idx = self.d_idx[:n].cpu().numpy()
-        val = self.d_val[:n].cpu().numpy()
-        pi = np.zeros(n, np.int32)
-        ps = np.zeros(n, np.float32)
-        npk = L.psx_identify_unique_peaks(idx.ctypes.data, val.ctypes.data, n, self.min_gap,
-                                          pi.ctypes.data, ps.ctypes.data)
-        freqs = (pi[:npk].astype(np.float32) * np.float32(factor.value)).astype(np.float32)
-        cands.append_peaks(ps[:npk].tolist(), freqs.tolist(), spec.get_nh())
+        npk = L.psx_identify_unique_peaks(self._idx.ctypes.data, self._val.ctypes.data, n,
+                                          self.min_gap, self._pidx.ctypes.data,
+                                          self._pval.ctypes.data)
+        freqs = (self._pidx[:npk].astype(np.float32) * np.float32(factor.value)).astype(np.float32)
+        cands.append_peaks(self._pval[:npk].tolist(), freqs.tolist(), spec.get_nh())
 
 
 # --------------------------------------------------------------- distillers
-def _to_pod(cands: Sequence[Candidate]):
-    arr = (_CandPOD * max(1, len(cands)))()
-    for i, c in enumerate(cands):
-        arr[i] = _CandPOD(*c.pod())
-    return arr
+_CAND_DTYPE = np.dtype([("dm", "<f4"), ("dm_idx", "<i4"), ("acc", "<f4"), ("nh", "<i4"),
+                        ("snr", "<f4"), ("freq", "<f4")])  # the layout of psx_candidate
+
+
+def _to_pod(cands: Sequence[Candidate]) -> np.ndarray:
+    return np.array([c.pod() for c in cands], dtype=_CAND_DTYPE)
 
 
 class _Distiller:
@@ -495,13 +493,13 @@ class _Distiller:
             return []
         arr = _to_pod(cands)
         na = np.zeros(n, np.int32)
-        keep = load().psx_distill(self.kind, arr, n, self.tol, self.max_harm, self.tobs,
-                                  int(self.keep_related), int(self.fractional), na.ctypes.data)
+        keep = load().psx_distill(self.kind, arr.ctypes.data, n, self.tol,
+                                  self.max_harm, self.tobs, int(self.keep_related),
+                                  int(self.fractional), na.ctypes.data)
         out = []
-        for i in range(keep):
-            a = arr[i]
-            c = Candidate(a.dm, a.dm_idx, a.acc, a.nh, a.snr, a.freq)
-            c.assoc = [Candidate()] * int(na[i])  # association count only
+        for a, k in zip(arr[:keep].tolist(), na[:keep].tolist()):
+            c = Candidate(*a)
+            c.assoc = [Candidate()] * k  # association count only
             out.append(c)
         return out
 

@@ -67,6 +67,12 @@ def test_find_peaks_runs_against_definition(psx, cuda, n, start, every):
         assert np.array_equal(idx.cpu().numpy()[:cap], want[:cap])
         assert np.array_equal(val.cpu().numpy()[:cap], x[want[:cap]])
         assert np.all(idx.cpu().numpy()[cap:] == -1)
+        hi, hv = np.full(len(want) + 1, -1, np.int32), np.zeros(len(want) + 1, np.float32)
+        rc = psx.psx_find_peaks_host(C.c_void_p(d.data_ptr()), n, start, 4.0, hi.ctypes.data,
+                                     hv.ctypes.data, cap, C.byref(cnt), None)
+        assert rc == (0 if cap == len(want) else 5) and cnt.value == len(want)
+        if rc == 0:
+            assert np.array_equal(hi[:-1], want) and np.array_equal(hv[:-1], x[want])
 
 
 @pytest.mark.parametrize("shift", [0, 1])
