@@ -127,6 +127,23 @@ __device__ __forceinline__ float stretch_at(const float* __restrict__ in,
     return lo + ((x - j > 1e-5f) ? (x - j) * (hi - lo) : 0.f);
 }
 
+// The three median levels, their stretch steps and the splice positions.
+struct MedianLevels {
+    const float* m5;
+    const float* m25;
+    const float* m125;
+    unsigned n5, n25, n125;
+    float step5, step25, step125;
+    unsigned pos5, pos25;
+};
+
+__device__ __forceinline__ float median_at(const MedianLevels& L, unsigned k)
+{
+    if (k < L.pos5) return stretch_at(L.m5, L.n5, k, L.step5);
+    if (k < L.pos25) return stretch_at(L.m25, L.n25, k, L.step25);
+    return stretch_at(L.m125, L.n125, k, L.step125);
+}
+
 // ---- harmonic sums (reference src/kernels.cu:34-100) ------------------
 // Index of fraction m/2^h of bin i: (int)(i*m/2^h + 0.5), exact in
 // integer arithmetic.

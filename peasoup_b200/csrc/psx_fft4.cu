@@ -35,8 +35,33 @@
 #include "psx_common.cuh"
 #include "psx_device.cuh"
 #include "psx_fft4.cuh"
+#include "psx_stages.cuh"
 
 namespace psx {
+
+// What a column pass reads and writes:
+//   kColGather   trials: the resample gather, forward twiddles, y
+//   kColDump     the gathered pairs z[e C + c] (the resampled series as it is
+//                read, interleaved) to y instead of transforming them (the
+//                debug tap)
+//   kColSeries   rows of series as they are (src), less up to three baseline
+//                means each, zero past ncopy; y as for trials
+//   kColInverse  the second pass of an inverse transform on conjugated data:
+//                y in place, the four-step twiddle W_M^(c k1) on the way in,
+//                the conjugate of the transform out (the real series)
+// kColSeries and kColInverse may write where they read: a CTA reads all its
+// columns before it writes them, and nobody else touches them.
+enum { kColGather = 0, kColDump = 1, kColSeries = 2, kColInverse = 3 };
+
+struct ColArgs {
+    const double* ktab;      // trials: resample factor of each
+    const unsigned* trow;    // trials of several series: trial -> row of x
+    size_t xpitch;           // rows of x are xpitch apart
+    SeriesRows src;          // kColSeries
+    size_t ncopy;
+    const float* means;      // kColSeries: 4 floats a row
+    unsigned offI;           // kColInverse: table of W_M^(J c q)
+};
 
 namespace {
 
@@ -173,18 +198,16 @@ __device__ __forceinline__ unsigned swz_a(unsigned e)
 
 // Column length R = 768 (stages of radix 16, 16, 3, for transform lengths
 // 3 * 2^k), 1024 (16, 16, 4), 2048 (16, 16, 8) or 4096 (16, 16, 16).
-// DUMP: write the gathered pairs z[e C + c] (the resampled series as it is
-// read, interleaved) to y instead of transforming them (the debug tap).
-template <int R, bool DUMP>
+template <int R, int KIND>
 __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THREADS)
-    k_fft4_cols(const float* __restrict__ x, unsigned long long n, const double* __restrict__ ktab,
-                const float2* __restrict__ tab, unsigned offA2, unsigned offA3, unsigned offQ,
-                unsigned offP, unsigned C, float2* __restrict__ y, size_t ypitch,
-                const unsigned* __restrict__ trow, size_t xpitch)
+    k_fft4_cols(const float* __restrict__ x, unsigned long long n, const float2* __restrict__ tab,
+                unsigned offA2, unsigned offA3, unsigned offQ, unsigned offP, unsigned C,
+                float2* y, size_t ypitch, const __grid_constant__ ColArgs a)
 {
     using S = ColShape<R>;
-    // trials of several series (trow: trial -> row of x, rows xpitch apart)
-    if (trow) x += (size_t)trow[blockIdx.y] * xpitch;
+    constexpr bool TRIAL = KIND == kColGather || KIND == kColDump;
+    if constexpr (TRIAL)
+        if (a.trow) x += (size_t)a.trow[blockIdx.y] * a.xpitch;
     static_assert(R == 768 || R == 1024 || R == 2048 || R == 4096, "column length");
     static_assert((S::THREADS == 512 || S::THREADS == 1024) && S::U * S::R3 <= 16,
                   "column shape");
@@ -192,12 +215,12 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
     extern __shared__ float2 sm_a[];
     const unsigned col = threadIdx.x % W, t = threadIdx.x / W;  // t in [0, TPC)
     const unsigned c = blockIdx.x * W + col;
-    const double k = ktab[blockIdx.y], size = (double)n;
+    const double k = TRIAL ? a.ktab[blockIdx.y] : 0.0, size = (double)n;
     // Table entries of the four-step twiddle (last step below), loaded first
     // so that their L2 latency passes under the three stages; for R = 4096
     // (one stage-3 butterfly per thread, fifteen entries W_M^(TPC c U q))
     // those are loaded where they are used instead.
-    constexpr bool EARLY = U > 1;
+    constexpr bool EARLY = U > 1 && KIND != kColInverse;
     const float2 wt = __ldg(tab + offQ + (size_t)t * C + c);
     float2 pu[U], pq[R3];
     if constexpr (EARLY) {
@@ -213,16 +236,54 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
     // stage 1 (radix 16, span 1): rows e = t + J q of column c, where
     // z[e C + c] = (x'[2m], x'[2m+1]); out[16 t + q]
     if (J == TPC || t < (unsigned)J) {  // every thread unless R = 768
-        const double i_first = 2.0 * ((double)t * (double)C + (double)c);
-        const double i_step = 2.0 * J * (double)C;
-        const unsigned n32 = (unsigned)n;
+        if constexpr (TRIAL) {
+            const double i_first = 2.0 * ((double)t * (double)C + (double)c);
+            const double i_step = 2.0 * J * (double)C;
+            const unsigned n32 = (unsigned)n;
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const double i0 = i_first + (double)q * i_step;  // exact: integers < 2^28
-            v[q].x = resampleII_read(x, i0, k, size, n32);
-            v[q].y = resampleII_read(x, i0 + 1.0, k, size, n32);
+            for (int q = 0; q < 16; ++q) {
+                const double i0 = i_first + (double)q * i_step;  // exact: integers < 2^28
+                v[q].x = resampleII_read(x, i0, k, size, n32);
+                v[q].y = resampleII_read(x, i0 + 1.0, k, size, n32);
+            }
+        } else if constexpr (KIND == kColSeries) {
+            const float* xr = a.src.p[blockIdx.y];
+            const float4 m = *reinterpret_cast<const float4*>(a.means + 4 * blockIdx.y);
+            auto less = [&](float f) { return ((f - m.x) - m.y) - m.z; };
+            const size_t s0 = 2 * ((size_t)t * C + c), step = 2 * (size_t)J * C;
+            const bool pairs = (reinterpret_cast<uintptr_t>(xr) & 7u) == 0;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const size_t i = s0 + q * step;
+                v[q] = make_float2(0.f, 0.f);
+                if (pairs && i + 1 < a.ncopy) {
+                    const float2 f = *reinterpret_cast<const float2*>(xr + i);
+                    v[q] = make_float2(less(f.x), less(f.y));
+                } else {
+                    if (i < a.ncopy) v[q].x = less(xr[i]);
+                    if (i + 1 < a.ncopy) v[q].y = less(xr[i + 1]);
+                }
+            }
+        } else {
+            const float2* yr = y + (size_t)blockIdx.y * ypitch;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = yr[(size_t)(t + J * q) * C + c];
+            // W_M^(c (t + J q)) = W_M^(c t) W_M^(J c (q mod 4)) W_M^(4 J c (q div 4))
+            const float2* ti = tab + a.offI + c;
+#pragma unroll
+            for (int l = 0; l < 4; ++l) {
+                const float2 w = l ? cmul(wt, __ldg(ti + l * (size_t)C)) : wt;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) v[4 * h + l] = cmul(v[4 * h + l], w);
+            }
+#pragma unroll
+            for (int h = 1; h < 4; ++h) {
+                const float2 w = __ldg(ti + 4 * h * (size_t)C);
+#pragma unroll
+                for (int l = 0; l < 4; ++l) v[4 * h + l] = cmul(v[4 * h + l], w);
+            }
         }
-        if constexpr (DUMP) {
+        if constexpr (KIND == kColDump) {
             float2* yo = y + (size_t)blockIdx.y * ypitch;
 #pragma unroll
             for (int q = 0; q < 16; ++q) yo[(size_t)(t + J * q) * C + c] = v[q];
@@ -232,7 +293,7 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
             for (int q = 0; q < 16; ++q) sm_a[swz_a<W>(16 * t + q) * W + col] = v[q];
         }
     }
-    if constexpr (DUMP) return;
+    if constexpr (KIND == kColDump) return;
     __syncthreads();
     // stage 2 (radix 16, span 16): in[t + J q] * W_256^((t mod 16) q),
     // out[(t / 16) 256 + t mod 16 + 16 q]
@@ -299,6 +360,15 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
     // W_M^(c t), W_M^(TPC c) and W_M^(TPC c U) instead of U R3 (R = 4096:
     // W_M^(c t) and the fifteen W_M^(TPC c q))
     float2* yo = y + (size_t)blockIdx.y * ypitch;
+    if constexpr (KIND == kColInverse) {
+#pragma unroll
+        for (int q = 0; q < R3; ++q)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                yo[(size_t)(t + TPC * (u + U * q)) * C + c] =
+                    make_float2(v[R3 * u + q].x, -v[R3 * u + q].y);
+        return;
+    }
 #pragma unroll
     for (int q = 0; q < R3; ++q) {
         const float2 wq =
@@ -371,8 +441,8 @@ __device__ __forceinline__ void row_stage(float2* s, unsigned t, const float2* _
 
 template <int LOGC>
 __global__ void __launch_bounds__(RowShape<LOGC>::THREADS, 1024 / RowShape<LOGC>::THREADS)
-    k_fft4_rows(const float2* __restrict__ y, size_t ypitch, float2* __restrict__ zt,
-                size_t zpitch, const float2* __restrict__ tw)
+    k_fft4_rows(const float2* y, size_t ypitch, float2* zt, size_t zpitch,
+                const float2* __restrict__ tw)  // zt may be y: a CTA reads its rows first
 {
     using S = RowShape<LOGC>;
     constexpr int C = S::C, T = S::T;
@@ -465,7 +535,8 @@ __device__ __forceinline__ void cp_async_wait()
 // block 0.  The split-step rotation (cos, sin)(pi j / M) is the product of
 // tabulated (cos, sin)(pi k1 / M) (k1 = -1 .. 1055, rv[k1 + 1]) and
 // (cos, sin)(pi k2 / C) (rk[k2]).
-template <unsigned R>
+// AMP: the amplitudes |X| instead (the running median's input).
+template <unsigned R, bool AMP>
 __global__ void __launch_bounds__(256, 8)  // 8 CTAs per SM: 32 registers
     k_unpack_form_norm_t(const float2* __restrict__ zt, size_t zpitch, unsigned C,
                          float* __restrict__ p, size_t ppitch,
@@ -474,7 +545,7 @@ __global__ void __launch_bounds__(256, 8)  // 8 CTAs per SM: 32 registers
 {
     __shared__ float2 lo_t[32][33], mi_t[32][33];
     // trials of several series: trial blockIdx.y's statistics at row trow[]
-    if (trow) stat += 8u * trow[blockIdx.y];
+    if (!AMP && trow) stat += 8u * trow[blockIdx.y];
     const unsigned M = R * C;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned gblocks = C / 64;
@@ -510,7 +581,8 @@ __global__ void __launch_bounds__(256, 8)  // 8 CTAs per SM: 32 registers
     __syncthreads();
     const int k1v = v0 + (int)lane;
     const float2 tv = __ldg(rv + (k1v + 1));
-    const float meanN = 2.0f * stat[3], stdN = 2.0f * stat[4];  // of 2X (exact)
+    // of 2X (exact)
+    const float meanN = AMP ? 0.f : 2.0f * stat[3], stdN = AMP ? 0.f : 2.0f * stat[4];
     const bool out = lane >= 1 && lane <= 30 && k1v < (int)R;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
@@ -519,6 +591,14 @@ __global__ void __launch_bounds__(256, 8)  // 8 CTAs per SM: 32 registers
         const float cs = tv.x * tk.x - tv.y * tk.y, sn = tv.y * tk.x + tv.x * tk.y;
         float2 lo, hi;
         unpack_one(lo_t[lane][cc], mi_t[lane][cc], cs, sn, lo, hi);
+        if constexpr (AMP) {
+            if (out) {
+                const unsigned j = (unsigned)k1v + R * k2;
+                o[j] = amplitude(0.5f * lo.x, 0.5f * lo.y);
+                o[M - j] = amplitude(0.5f * hi.x, 0.5f * hi.y);
+            }
+            continue;
+        }
         if (k1v < 0 && k2 == 0) lo = hi = make_float2(0.f, 0.f);
         const float plx = __shfl_up_sync(0xffffffffu, lo.x, 1);
         const float ply = __shfl_up_sync(0xffffffffu, lo.y, 1);
@@ -536,8 +616,163 @@ __global__ void __launch_bounds__(256, 8)  // 8 CTAs per SM: 32 registers
         const float2 r1 = __ldg(rv + 2);  // (cos, sin)(pi / M)
         float2 x0, x1, unused;
         unpack_one(zt_at<R>(z, C, jh), zt_at<R>(z, C, M - jh), 0.0f, 1.0f, x0, unused);
+        if constexpr (AMP) {
+            o[jh] = amplitude(0.5f * x0.x, 0.5f * x0.y);
+            return;
+        }
         unpack_one(zt_at<R>(z, C, jh - 1), zt_at<R>(z, C, M - jh + 1), r1.y, r1.x, x1, unused);
         o[jh] = normalise(interbin(x0.x, x0.y, x1.x, x1.y), meanN, stdN);
+    }
+}
+
+// ------------------------------------------------------- spectrum in place
+// Between the two transforms of the per-DM prologue, on the transposed
+// spectrum: from zt the real spectrum's bins X[j], X[M-j]; each divided by
+// the running median (bins 0..4 zeroed) and zapped (reference
+// src/kernels.cu's divide and zap kernels); the interbinned statistics of the result
+// (sums per CTA); and the input of the inverse transform,
+//   Z'[j] = (X[j] + conj X[M-j]) + i exp(i pi j / M) (X[j] - conj X[M-j]),
+// written conjugated at the transposed places of zo (the inverse runs the
+// forward passes on conjugated data).  Tiles as in k_unpack_form_norm_t:
+// lanes 1..30 own their bins, 0 and 31 bring the neighbours.  In place of
+// the interbin pass, the median pass, the zap and both of cuFFT's real-complex
+// steps: the spectrum is read and written once (five reads and three writes
+// before).  Bound by DRAM traffic and the divisions.
+struct MidArgs {
+    MedianLevels lev;        // of row 0; rows m_stride floats apart
+    size_t m_stride;
+    const unsigned* zap;     // bit per bin, or null
+    double2* parts;          // per row part_stride, one entry per CTA
+    size_t part_stride;
+};
+
+__device__ __forceinline__ float2 deredden(float2 x, unsigned j, const MidArgs& a)
+{
+    if (j < 5) {
+        x = make_float2(0.f, 0.f);
+    } else {
+        const cuComplex q = cuCdivf(make_cuComplex(x.x, x.y), make_cuComplex(median_at(a.lev, j), 0.f));
+        x = make_float2(q.x, q.y);
+    }
+    if (a.zap && (__ldg(a.zap + (j >> 5)) >> (j & 31) & 1u)) x = make_float2(1.f, 0.f);
+    return x;
+}
+
+template <unsigned R>
+__global__ void __launch_bounds__(256, 4)
+    k_deredden_t(const float2* __restrict__ zt, size_t zpitch, unsigned C, float2* __restrict__ zo,
+                 size_t opitch, const float2* __restrict__ rv, const float2* __restrict__ rk,
+                 MidArgs a)
+{
+    __shared__ float2 lo_t[32][33], mi_t[32][33];
+    __shared__ double2 sums[8];
+    a.lev.m5 += blockIdx.y * a.m_stride;
+    a.lev.m25 += blockIdx.y * a.m_stride;
+    a.lev.m125 += blockIdx.y * a.m_stride;
+    const unsigned M = R * C;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned gblocks = C / 64;
+    const unsigned wk = blockIdx.x / gblocks;
+    const unsigned k2a = (blockIdx.x % gblocks) * 32;
+    const int v0 = (int)(30 * wk) - 1;
+    const float2* z = zt + (size_t)blockIdx.y * zpitch;
+    float2* o = zo + (size_t)blockIdx.y * opitch;
+    if (v0 >= 1 && v0 + 31 < (int)R) {  // every row a real row: direct addresses
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const unsigned r = warp + 8 * e, v = (unsigned)v0 + r;
+            cp_async8(&lo_t[r][lane], z + (size_t)v * C + k2a + lane);
+            cp_async8(&mi_t[r][lane], z + (size_t)(R - v) * C + (C - 1 - k2a - lane));
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const unsigned r = warp + 8 * e;
+            const long long j = (long long)(v0 + (int)r) + (long long)R * (k2a + lane);
+            float2 p = make_float2(0.f, 0.f), q = p;  // X[-1] := 0
+            if (j >= 0) {
+                const unsigned jj = (unsigned)j;
+                p = zt_at<R>(z, C, jj);
+                q = zt_at<R>(z, C, jj ? M - jj : 0u);
+            }
+            lo_t[r][lane] = p;
+            mi_t[r][lane] = q;
+        }
+    }
+    __syncthreads();
+    const int k1v = v0 + (int)lane;
+    const float2 tv = __ldg(rv + (k1v + 1));
+    const bool out = lane >= 1 && lane <= 30 && k1v < (int)R;
+    double s = 0.0, s2 = 0.0;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const unsigned cc = 4 * warp + t, k2 = k2a + cc;
+        const float2 tk = __ldg(rk + k2);
+        const float cs = tv.x * tk.x - tv.y * tk.y, sn = tv.y * tk.x + tv.x * tk.y;
+        float2 lo, hi;
+        unpack_one(lo_t[lane][cc], mi_t[lane][cc], cs, sn, lo, hi);
+        if (k1v < 0 && k2 == 0) {
+            lo = hi = make_float2(0.f, 0.f);
+        } else {
+            const unsigned j = (unsigned)(k1v + (int)(R * k2));
+            lo = deredden(make_float2(0.5f * lo.x, 0.5f * lo.y), j, a);
+            hi = deredden(make_float2(0.5f * hi.x, 0.5f * hi.y), M - j, a);
+        }
+        const float plx = __shfl_up_sync(0xffffffffu, lo.x, 1);
+        const float ply = __shfl_up_sync(0xffffffffu, lo.y, 1);
+        const float nhx = __shfl_down_sync(0xffffffffu, hi.x, 1);
+        const float nhy = __shfl_down_sync(0xffffffffu, hi.y, 1);
+        if (out) {
+            const double p = interbin(lo.x, lo.y, plx, ply), q = interbin(hi.x, hi.y, nhx, nhy);
+            s += p + q;
+            s2 += p * p + q * q;
+        }
+        const float ax = lo.x + hi.x, ay = lo.y - hi.y;  // X[j] + conj X[M-j]
+        const float dx = lo.x - hi.x, dy = lo.y + hi.y;  // X[j] - conj X[M-j]
+        const float u = cs * dx - sn * dy, v = cs * dy + sn * dx;
+        lo_t[lane][cc] = make_float2(ax - v, -ay - u);
+        mi_t[lane][cc] = make_float2(ax + v, ay - u);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // bin M/2, its own mirror: Z' = 2 conj X
+        const unsigned jh = M / 2;
+        const float2 r1 = __ldg(rv + 2);  // (cos, sin)(pi / M)
+        float2 x0, x1, unused;
+        unpack_one(zt_at<R>(z, C, jh), zt_at<R>(z, C, M - jh), 0.0f, 1.0f, x0, unused);
+        unpack_one(zt_at<R>(z, C, jh - 1), zt_at<R>(z, C, M - jh + 1), r1.y, r1.x, x1, unused);
+        x0 = deredden(make_float2(0.5f * x0.x, 0.5f * x0.y), jh, a);
+        x1 = deredden(make_float2(0.5f * x1.x, 0.5f * x1.y), jh - 1, a);
+        const double p = interbin(x0.x, x0.y, x1.x, x1.y);
+        s += p;
+        s2 += p * p;
+        o[C / 2] = make_float2(2.0f * x0.x, 2.0f * x0.y);  // jh = R * (C / 2): row 0
+    }
+    for (int w = 16; w; w >>= 1) {
+        s += __shfl_down_sync(0xffffffffu, s, w);
+        s2 += __shfl_down_sync(0xffffffffu, s2, w);
+    }
+    if (lane == 0) sums[warp] = make_double2(s, s2);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double p = 0.0, q = 0.0;
+        for (int w = 0; w < 8; ++w) {
+            p += sums[w].x;
+            q += sums[w].y;
+        }
+        a.parts[blockIdx.y * a.part_stride + blockIdx.x] = make_double2(p, q);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const unsigned r = warp + 8 * e;
+        const int v = v0 + (int)r;
+        if (r < 1 || r > 30 || v >= (int)R) continue;  // (v >= 0 where r >= 1)
+        const unsigned k2 = k2a + lane;
+        o[(size_t)v * C + k2] = lo_t[r][lane];
+        if (v)
+            o[(size_t)(R - v) * C + (C - 1 - k2)] = mi_t[r][lane];
+        else if (k2)
+            o[C - k2] = mi_t[r][lane];
     }
 }
 
@@ -584,24 +819,35 @@ int configure_cols()
     // (the default shared/L1 split: measured on B200, forcing the largest
     // shared carve-out slowed the gather of pass 1 and the twiddle reads of
     // pass 2, both served from L1)
-    return cuda_status(cudaFuncSetAttribute(k_fft4_cols<R, false>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)S::SMEM),
-                       "fft4 column pass attribute");
+    auto one = [](auto kern) {
+        return cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)S::SMEM),
+                           "fft4 column pass attribute");
+    };
+    PSX_TRY(one(k_fft4_cols<R, kColGather>));
+    PSX_TRY(one(k_fft4_cols<R, kColSeries>));
+    return one(k_fft4_cols<R, kColInverse>);
 }
 
 }  // namespace
 
-template <int R, bool DUMP>
-void Fft4Plan::launch_cols(const Fft4Plan& f, const float* series, const double* ktab,
-                           int ntrials, float2* y, size_t ypitch, cudaStream_t s,
-                           const unsigned* trow, size_t xpitch)
+template <int KIND>
+int Fft4Plan::launch_cols(const float* x, int rows, float2* y, size_t ypitch, const ColArgs& a,
+                          cudaStream_t s) const
 {
-    using S = ColShape<R>;
-    dim3 ga(f.C / S::W, (unsigned)ntrials);
-    k_fft4_cols<R, DUMP><<<ga, S::THREADS, DUMP ? 0 : S::SMEM, s>>>(
-        series, (unsigned long long)f.n, ktab, f.d_tab, f.offA2, f.offA3, f.offQ, f.offP, f.C, y,
-        ypitch, trow, xpitch);
+    auto go = [&](auto kern, auto shape) {
+        using S = decltype(shape);
+        dim3 ga(C / S::W, (unsigned)rows);
+        kern<<<ga, S::THREADS, KIND == kColDump ? 0 : S::SMEM, s>>>(
+            x, (unsigned long long)n, d_tab, offA2, offA3, offQ, offP, C, y, ypitch, a);
+    };
+    switch (R) {
+    case 768: go(k_fft4_cols<768, KIND>, ColShape<768>{}); break;
+    case 1024: go(k_fft4_cols<1024, KIND>, ColShape<1024>{}); break;
+    case 2048: go(k_fft4_cols<2048, KIND>, ColShape<2048>{}); break;
+    default: go(k_fft4_cols<4096, KIND>, ColShape<4096>{}); break;
+    }
+    return launch_status("fft4 column pass");
 }
 
 bool Fft4Plan::supported(size_t n)
@@ -633,7 +879,8 @@ size_t Fft4Plan::table_floats2(size_t n)
     row_stages(lc, st);
     size_t rows = 0;
     for (auto& e : st) rows += (size_t)e.first * e.second;
-    return 256 + (size_t)(r / 256) * 256 + (size_t)cols_tpc(r) * c + 16 * (size_t)c +
+    return 256 + (size_t)(r / 256) * 256 + (size_t)cols_tpc(r) * c +
+           (cols_tpc(r) == r / 16 ? 16 : 32) * (size_t)c +
            (r + 33) + c / 2 + rows;
 }
 
@@ -678,6 +925,14 @@ int Fft4Plan::create(size_t n_)
     offP = (unsigned)h.size();  // [w * C + c] = W_M^(tpc c w), w < 16
     for (unsigned w = 0; w < 16; ++w)
         for (unsigned c = 0; c < Cn; ++c) h.push_back(W((unsigned long long)tpc * c * w, M));
+    // the same for W_M^(J c w), J = R / 16 (the inverse's input twiddle)
+    offI = offP;
+    if (tpc != Rn / 16) {
+        offI = (unsigned)h.size();
+        for (unsigned w = 0; w < 16; ++w)
+            for (unsigned c = 0; c < Cn; ++c)
+                h.push_back(W((unsigned long long)(Rn / 16) * c * w, M));
+    }
     // unpack rotations (cos, sin)(pi k1 / M), k1 = -1 .. R + 31, and (pi k2 / C)
     const double pi = two_pi / 2;
     offRv = (unsigned)h.size();
@@ -740,15 +995,35 @@ int Fft4Plan::exec_cols(const float* series, const double* ktab, int ntrials, fl
         set_error("fft4: bad arguments");
         return PSX_ERR_INVALID;
     }
-    const unsigned* tr = trow;
-    const size_t xp = xpitch;
-    switch (R) {
-    case 768: launch_cols<768, false>(*this, series, ktab, ntrials, y, ypitch, s, tr, xp); break;
-    case 1024: launch_cols<1024, false>(*this, series, ktab, ntrials, y, ypitch, s, tr, xp); break;
-    case 2048: launch_cols<2048, false>(*this, series, ktab, ntrials, y, ypitch, s, tr, xp); break;
-    default: launch_cols<4096, false>(*this, series, ktab, ntrials, y, ypitch, s, tr, xp); break;
+    ColArgs a{};
+    a.ktab = ktab;
+    a.trow = trow;
+    a.xpitch = xpitch;
+    return launch_cols<kColGather>(series, ntrials, y, ypitch, a, s);
+}
+
+int Fft4Plan::exec_series(const SeriesRows& src, int rows, size_t ncopy, const float* means,
+                          float2* y, size_t ypitch, float2* zt, size_t zpitch,
+                          cudaStream_t s) const
+{
+    if (!d_tab || !means || !y || rows <= 0 || rows > kSeriesRowsMax || ypitch < n / 2) {
+        set_error("fft4: bad arguments");
+        return PSX_ERR_INVALID;
     }
-    return launch_status("fft4 column pass");
+    ColArgs a{};
+    a.src = src;
+    a.ncopy = ncopy;
+    a.means = means;
+    PSX_TRY(launch_cols<kColSeries>(nullptr, rows, y, ypitch, a, s));
+    return exec_rows(y, ypitch, rows, zt, zpitch, s);
+}
+
+int Fft4Plan::exec_inverse(float2* z, size_t pitch, int rows, cudaStream_t s) const
+{
+    PSX_TRY(exec_rows(z, pitch, rows, z, pitch, s));
+    ColArgs a{};
+    a.offI = offI;
+    return launch_cols<kColInverse>(nullptr, rows, z, pitch, a, s);
 }
 
 int Fft4Plan::dump_gather(const float* series, const double* ktab, float* out,
@@ -758,14 +1033,9 @@ int Fft4Plan::dump_gather(const float* series, const double* ktab, float* out,
         set_error("fft4 dump: bad arguments");
         return PSX_ERR_INVALID;
     }
-    float2* o = reinterpret_cast<float2*>(out);
-    switch (R) {
-    case 768: launch_cols<768, true>(*this, series, ktab, 1, o, n / 2, s, nullptr, 0); break;
-    case 1024: launch_cols<1024, true>(*this, series, ktab, 1, o, n / 2, s, nullptr, 0); break;
-    case 2048: launch_cols<2048, true>(*this, series, ktab, 1, o, n / 2, s, nullptr, 0); break;
-    default: launch_cols<4096, true>(*this, series, ktab, 1, o, n / 2, s, nullptr, 0); break;
-    }
-    return launch_status("fft4 gather dump");
+    ColArgs a{};
+    a.ktab = ktab;
+    return launch_cols<kColDump>(series, 1, reinterpret_cast<float2*>(out), n / 2, a, s);
 }
 
 int Fft4Plan::exec_rows(const float2* y, size_t ypitch, int ntrials, float2* zt, size_t zpitch,
@@ -804,12 +1074,59 @@ int Fft4Plan::form(const float2* zt, size_t zpitch, int ntrials, float* p, size_
     const float2* rv = d_tab + offRv;
     const float2* rk = d_tab + offRk;
     switch (R) {
-    case 768: k_unpack_form_norm_t<768><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
-    case 1024: k_unpack_form_norm_t<1024><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
-    case 2048: k_unpack_form_norm_t<2048><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
-    default: k_unpack_form_norm_t<4096><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
+    case 768: k_unpack_form_norm_t<768, false><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
+    case 1024: k_unpack_form_norm_t<1024, false><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
+    case 2048: k_unpack_form_norm_t<2048, false><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
+    default: k_unpack_form_norm_t<4096, false><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
     }
     return launch_status("fft4 unpack kernel");
+}
+
+int Fft4Plan::amplitudes(const float2* zt, size_t zpitch, int rows, float* amp, size_t apitch,
+                         cudaStream_t s) const
+{
+    if (!d_tab || !zt || !amp || rows <= 0 || rows > 65535 || zpitch < n / 2 || apitch < n / 2 + 1) {
+        set_error("fft4 amplitudes: bad arguments");
+        return PSX_ERR_INVALID;
+    }
+    dim3 grid((R + 29) / 30 * (C / 64), (unsigned)rows);
+    const float2* rv = d_tab + offRv;
+    const float2* rk = d_tab + offRk;
+    switch (R) {
+    case 768: k_unpack_form_norm_t<768, true><<<grid, 256, 0, s>>>(zt, zpitch, C, amp, apitch, rv, rk, nullptr, nullptr); break;
+    case 1024: k_unpack_form_norm_t<1024, true><<<grid, 256, 0, s>>>(zt, zpitch, C, amp, apitch, rv, rk, nullptr, nullptr); break;
+    case 2048: k_unpack_form_norm_t<2048, true><<<grid, 256, 0, s>>>(zt, zpitch, C, amp, apitch, rv, rk, nullptr, nullptr); break;
+    default: k_unpack_form_norm_t<4096, true><<<grid, 256, 0, s>>>(zt, zpitch, C, amp, apitch, rv, rk, nullptr, nullptr); break;
+    }
+    return launch_status("fft4 amplitude kernel");
+}
+
+int Fft4Plan::deredden(const float2* zt, size_t zpitch, int rows, float2* zo, size_t opitch,
+                       const MedianLevels& lev, size_t m_stride, const unsigned* zap,
+                       double2* parts, size_t part_stride, cudaStream_t s) const
+{
+    if (!d_tab || !zt || !zo || zt == zo || rows <= 0 || rows > 65535 || zpitch < n / 2 ||
+        opitch < n / 2 || part_stride < stat_parts(n)) {
+        set_error("fft4 deredden: bad arguments");
+        return PSX_ERR_INVALID;
+    }
+    dim3 grid((R + 29) / 30 * (C / 64), (unsigned)rows);
+    const float2* rv = d_tab + offRv;
+    const float2* rk = d_tab + offRk;
+    const MidArgs a{lev, m_stride, zap, parts, part_stride};
+    switch (R) {
+    case 768: k_deredden_t<768><<<grid, 256, 0, s>>>(zt, zpitch, C, zo, opitch, rv, rk, a); break;
+    case 1024: k_deredden_t<1024><<<grid, 256, 0, s>>>(zt, zpitch, C, zo, opitch, rv, rk, a); break;
+    case 2048: k_deredden_t<2048><<<grid, 256, 0, s>>>(zt, zpitch, C, zo, opitch, rv, rk, a); break;
+    default: k_deredden_t<4096><<<grid, 256, 0, s>>>(zt, zpitch, C, zo, opitch, rv, rk, a); break;
+    }
+    return launch_status("fft4 deredden kernel");
+}
+
+size_t Fft4Plan::stat_parts(size_t n)
+{
+    const unsigned r = rows_for(n);
+    return (size_t)((r + 29) / 30) * (n / 2 / r / 64);
 }
 
 }  // namespace psx

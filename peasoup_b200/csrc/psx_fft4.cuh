@@ -7,9 +7,12 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>
+#include "psx_device.cuh"
+#include "psx_stages.cuh"
 
 namespace psx {
 
+struct ColArgs;
 
 struct Fft4Plan {
     size_t n = 0;      // real samples N
@@ -19,7 +22,7 @@ struct Fft4Plan {
     int logc = 0;
     float2* d_tab = nullptr;  // twiddle tables (offsets below, in float2)
     size_t tab_len = 0;
-    unsigned offA2 = 0, offA3 = 0, offQ = 0, offP = 0, offB = 0, offRv = 0, offRk = 0;
+    unsigned offA2 = 0, offA3 = 0, offQ = 0, offP = 0, offI = 0, offB = 0, offRv = 0, offRk = 0;
 
     // N = 2^19 .. 2^27 (R = 1024, 2048, 4096) or 3 * 2^17 .. 3 * 2^23
     // (R = 768), i.e. C = 2^8 .. 2^14.
@@ -58,11 +61,30 @@ struct Fft4Plan {
     int form(const float2* zt, size_t zpitch, int ntrials, float* p, size_t ppitch,
              const float* stat, cudaStream_t s, const unsigned* trow = nullptr) const;
 
+    // The per-DM prologue's transforms, on `rows` series at once.
+    // Forward: series src.p[r] less its baseline means (means[4 r + 0..2],
+    // subtracted in turn), zero from ncopy on, left transposed in zt as exec
+    // leaves it; y may be where the series are.
+    int exec_series(const SeriesRows& src, int rows, size_t ncopy, const float* means, float2* y,
+                    size_t ypitch, float2* zt, size_t zpitch, cudaStream_t s) const;
+    // |X| of bins 0..M of each row.
+    int amplitudes(const float2* zt, size_t zpitch, int rows, float* amp, size_t apitch,
+                   cudaStream_t s) const;
+    // zt's spectrum divided by the running median, zapped, and its
+    // interbinned statistics' partial sums (stat_parts(n) of them a row);
+    // zo receives the inverse's input.
+    int deredden(const float2* zt, size_t zpitch, int rows, float2* zo, size_t opitch,
+                 const MedianLevels& lev, size_t m_stride, const unsigned* zap, double2* parts,
+                 size_t part_stride, cudaStream_t s) const;
+    static size_t stat_parts(size_t n);
+    // The real series (unnormalised, as a C2R transform leaves it) from
+    // deredden's output, in place.
+    int exec_inverse(float2* z, size_t pitch, int rows, cudaStream_t s) const;
+
 private:
-    template <int R, bool DUMP>
-    static void launch_cols(const Fft4Plan& f, const float* series, const double* ktab,
-                            int ntrials, float2* y, size_t ypitch, cudaStream_t s,
-                            const unsigned* trow, size_t xpitch);
+    template <int KIND>
+    int launch_cols(const float* x, int rows, float2* y, size_t ypitch, const ColArgs& a,
+                    cudaStream_t s) const;
 };
 
 }  // namespace psx

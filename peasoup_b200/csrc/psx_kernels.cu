@@ -5,6 +5,7 @@
 // interleaved float pairs (cufftComplex); all grids are grid-stride loops
 // sized to a multiple of the SM count (psx::grid_for).
 #include <cuda.h>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
@@ -207,25 +208,8 @@ __global__ void __launch_bounds__(256) k_scrunch5(const float* __restrict__ in, 
     }
 }
 
-// Stretch of the three median levels, spliced at pos5/pos25; with X given
-// the spectrum is divided by the median in place (bins 0..4 zeroed),
+// The median spliced from its three levels (median_at); with X given the spectrum is divided by the median in place (bins 0..4 zeroed),
 // otherwise the median itself is written.
-struct MedianLevels {
-    const float* m5;
-    const float* m25;
-    const float* m125;
-    unsigned n5, n25, n125;
-    float step5, step25, step125;
-    unsigned pos5, pos25;
-};
-
-__device__ __forceinline__ float median_at(const MedianLevels& L, unsigned k)
-{
-    if (k < L.pos5) return stretch_at(L.m5, L.n5, k, L.step5);
-    if (k < L.pos25) return stretch_at(L.m25, L.n25, k, L.step25);
-    return stretch_at(L.m125, L.n125, k, L.step125);
-}
-
 __global__ void __launch_bounds__(256) k_median_apply(MedianLevels L, size_t nbins,
                                                       float* __restrict__ median_out,
                                                       float* __restrict__ X, size_t x_stride = 0,
@@ -283,6 +267,27 @@ static float stretch_step(size_t in_count, size_t out_count)
 {
     // reference src/kernels.cu:1016: float(in_count-1)/(out_count-1)
     return (float)(in_count - 1) / (float)(out_count - 1);
+}
+
+MedianLevels median_levels(size_t nbins, double bin_width, float b5, float b25, float* scratch)
+{
+    auto up = [](size_t v) { return (v + 63) / 64 * 64; };
+    // reference dereddener.hpp:48-49: (int)(boundary / bin_width)
+    const int pos5 = (int)((double)b5 / bin_width), pos25 = (int)((double)b25 / bin_width);
+    MedianLevels L;
+    L.m5 = scratch;
+    L.m25 = scratch + up(nbins / 5 + 1);
+    L.m125 = L.m25 + up(nbins / 25 + 1);
+    L.n5 = (unsigned)(nbins / 5);
+    L.n25 = L.n5 / 5;
+    L.n125 = L.n25 / 5;
+    L.step5 = stretch_step(L.n5, nbins);
+    L.step25 = stretch_step(L.n25, nbins);
+    L.step125 = stretch_step(L.n125, nbins);
+    L.pos5 = (unsigned)(pos5 < 0 ? 0 : (size_t)pos5 > nbins ? nbins : pos5);
+    L.pos25 = (unsigned)(pos25 < 0 ? 0 : (size_t)pos25 > nbins ? nbins : pos25);
+    if (L.pos25 < L.pos5) L.pos25 = L.pos5;
+    return L;
 }
 
 // The three median-of-5 levels of the amplitudes of a complex spectrum X
@@ -358,24 +363,9 @@ namespace {
 // The stretch, splice and division of launch_running_median once the three
 // levels are in the scratch.
 int median_apply(size_t nbins, double bin_width, float b5, float b25, float* d_median, float* d_X,
-                 float* m5, float* m25, float* m125, cudaStream_t s)
+                 float* m5, cudaStream_t s)
 {
-    const size_t n5 = nbins / 5, n25 = nbins / 5 / 5, n125 = nbins / 5 / 5 / 5;
-    int pos5 = (int)((double)b5 / bin_width);
-    int pos25 = (int)((double)b25 / bin_width);
-    MedianLevels L;
-    L.m5 = m5;
-    L.m25 = m25;
-    L.m125 = m125;
-    L.n5 = (unsigned)n5;
-    L.n25 = (unsigned)n25;
-    L.n125 = (unsigned)n125;
-    L.step5 = stretch_step(n5, nbins);
-    L.step25 = stretch_step(n25, nbins);
-    L.step125 = stretch_step(n125, nbins);
-    L.pos5 = (unsigned)(pos5 < 0 ? 0 : (size_t)pos5 > nbins ? nbins : pos5);
-    L.pos25 = (unsigned)(pos25 < 0 ? 0 : (size_t)pos25 > nbins ? nbins : pos25);
-    if (L.pos25 < L.pos5) L.pos25 = L.pos5;
+    const MedianLevels L = median_levels(nbins, bin_width, b5, b25, m5);
     k_median_apply<<<grid_for(nbins, 256), 256, 0, s>>>(L, nbins, d_median, d_X);
     return launch_status("median apply kernel");
 }
@@ -399,7 +389,7 @@ int launch_running_median_spectrum(float* d_X, size_t nbins, double bin_width, f
                                                      (size_t)sm_count() * 8);
     k_scrunch3<true><<<grid, 256, 0, s>>>(d_X, m5, n5, m25, n25, m125, n125);
     PSX_TRY(launch_status("amplitude + scrunch kernel"));
-    return median_apply(nbins, bin_width, b5, b25, nullptr, d_X, m5, m25, m125, s);
+    return median_apply(nbins, bin_width, b5, b25, nullptr, d_X, m5, s);
 }
 
 int launch_running_median(const float* d_powers, size_t nbins, double bin_width, float b5,
@@ -420,10 +410,22 @@ int launch_running_median(const float* d_powers, size_t nbins, double bin_width,
                                                      (size_t)sm_count() * 8);
     k_scrunch3<false><<<grid, 256, 0, s>>>(d_powers, m5, n5, m25, n25, m125, n125);
     PSX_TRY(launch_status("scrunch kernel"));
-    return median_apply(nbins, bin_width, b5, b25, d_median, d_X, m5, m25, m125, s);
+    return median_apply(nbins, bin_width, b5, b25, d_median, d_X, m5, s);
 }
 
 // ------------------------------------------------------------------- zapping
+// Bins [low, high) of a birdie (reference src/kernels.cu, zap kernel).
+__device__ __forceinline__ bool zap_range(float freq, float width, float bin_width, unsigned nbins,
+                                          int& low_bin, int& high_bin)
+{
+    low_bin = __float2int_rd((freq - width) / bin_width);
+    high_bin = __float2int_ru((freq + width) / bin_width);
+    if (low_bin < 0) low_bin = 0;
+    if (low_bin >= (int)nbins) return false;
+    if (high_bin >= (int)nbins) high_bin = (int)nbins - 1;
+    return true;
+}
+
 // One warp per birdie; lanes stride the birdie's bin range.
 __global__ void k_zap(float* __restrict__ X, const float* __restrict__ freqs,
                       const float* __restrict__ widths, float bin_width, unsigned nbirdies,
@@ -433,13 +435,8 @@ __global__ void k_zap(float* __restrict__ X, const float* __restrict__ freqs,
     const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const unsigned lane = threadIdx.x & 31;
     if (warp >= nbirdies) return;
-    const float freq = freqs[warp];
-    const float width = widths[warp];
-    int low_bin = __float2int_rd((freq - width) / bin_width);
-    int high_bin = __float2int_ru((freq + width) / bin_width);
-    if (low_bin < 0) low_bin = 0;
-    if (low_bin >= (int)nbins) return;
-    if (high_bin >= (int)nbins) high_bin = (int)nbins - 1;
+    int low_bin, high_bin;
+    if (!zap_range(freqs[warp], widths[warp], bin_width, nbins, low_bin, high_bin)) return;
     float2* c = reinterpret_cast<float2*>(X);
     for (int k = low_bin + (int)lane; k < high_bin; k += 32) c[k] = make_float2(1.0f, 0.0f);
 }
@@ -494,11 +491,25 @@ __global__ void __launch_bounds__(256) k_sum_partials(Src src, size_t first, siz
     }
 }
 
+// The reference's float statistics {mean, rms, std, mean*scale, std*scale} of
+// `count` values with sums a and (of squares) b, computed exactly as its host
+// code does (stats.hpp:20-31 and src/kernels.cu:443,458), without contraction.
+__device__ __forceinline__ void write_stats(double a, double b, double count,
+                                            float* __restrict__ stat, float scale)
+{
+    const float cnt = (float)count;
+    const float mean = __fdiv_rn((float)a, cnt);
+    const float rms = sqrtf(__fdiv_rn((float)b, cnt));
+    const float sd = sqrtf(__fsub_rn(__fmul_rn(rms, rms), __fmul_rn(mean, mean)));
+    stat[0] = mean;
+    stat[1] = rms;
+    stat[2] = sd;
+    stat[3] = __fmul_rn(mean, scale);
+    stat[4] = __fmul_rn(sd, scale);
+}
+
 // Adds `nparts` partials (one warp, fixed order); writes the totals to sums[0..1]
-// and, when stat != nullptr, the reference's float statistics
-// {mean, rms, std, mean*scale, std*scale} computed exactly as its host
-// code does (stats.hpp:20-31 and src/kernels.cu:443,458), without
-// contraction.
+// and, when stat != nullptr, the statistics of write_stats.
 __global__ void k_finish_stats(const double2* __restrict__ partials, int nparts, double count,
                                double* __restrict__ sums, float* __restrict__ stat, float scale,
                                size_t part_stride = 0, size_t sums_stride = 0,
@@ -514,17 +525,7 @@ __global__ void k_finish_stats(const double2* __restrict__ partials, int nparts,
     if (threadIdx.x != 0) return;
     sums[0] = a;
     sums[1] = b;
-    if (stat) {
-        const float cnt = (float)count;
-        const float mean = __fdiv_rn((float)a, cnt);
-        const float rms = sqrtf(__fdiv_rn((float)b, cnt));
-        const float sd = sqrtf(__fsub_rn(__fmul_rn(rms, rms), __fmul_rn(mean, mean)));
-        stat[0] = mean;
-        stat[1] = rms;
-        stat[2] = sd;
-        stat[3] = __fmul_rn(mean, scale);
-        stat[4] = __fmul_rn(sd, scale);
-    }
+    if (stat) write_stats(a, b, count, stat, scale);
 }
 
 struct PlainSrc {
@@ -732,6 +733,235 @@ __global__ void __launch_bounds__(kVecThreads) k_interbin_partials_v4(const floa
 
 int reduction_blocks() { return sm_count() * 2; }
 
+// Sum of (x - m0) - m1 over [0, n) by the CTAs of a row, with 128-bit loads
+// where x is 16-byte aligned (x - 0 is x).
+__device__ __forceinline__ double sum_less(const float* __restrict__ x, size_t n, float m0, float m1)
+{
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    size_t done = 0;
+    double s = 0.0;
+    auto less = [&](float v) { return (double)((v - m0) - m1); };
+    if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+        done = n / 4 * 4;
+        const float4* x4 = reinterpret_cast<const float4*>(x);
+#pragma unroll 8
+        for (size_t q = first; q < n / 4; q += stride) {
+            const float4 v = x4[q];
+            s += (less(v.x) + less(v.y)) + (less(v.z) + less(v.w));
+        }
+    }
+#pragma unroll 4
+    for (size_t i = done + first; i < n; i += stride) s += less(x[i]);
+    return s;
+}
+
+// The device-side baseline loop (reference src/kernels.cu:463-479) without
+// writing the series: every pass finds the float mean that the reference
+// would subtract next, from the sums of the series less the means found so
+// far (the subtraction itself, in the same order and so with the same
+// roundings, is done by the transform's loads).  Pass 0 (FIRST) sums the
+// series; pass p forms mean p - 1 from the previous pass's partials and,
+// while |mean| > 5e-7 n, sums again.  Row blockIdx.y of a batch; `cnt` as
+// Slot::d_count (16 words a row: [2] still active after the last pass, [3]
+// passes, [6 + p] pass p's flag), `means` 4 floats a row.
+template <bool FIRST>
+__global__ void __launch_bounds__(kVecThreads) k_baseline_means(
+    SeriesRows rows, size_t n, double2* __restrict__ parts, size_t part_stride, int nparts,
+    unsigned* __restrict__ cnt, float* __restrict__ means, int pass, int last)
+{
+    const float* x = rows.p[blockIdx.y];
+    unsigned* c = cnt + 16 * blockIdx.y;
+    float* m = means + 4 * blockIdx.y;
+    double2* out = parts + (size_t)blockIdx.y * part_stride + (pass & 1) * nparts;
+    double s = 0.0;
+    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
+    if constexpr (FIRST) {
+        if (one) {
+            c[6] = 1u;
+            for (int k = 0; k < 4; ++k) m[k] = 0.f;
+        }
+        s = sum_less(x, n, 0.f, 0.f);
+    } else {
+        // (mean p - 1 is read by nobody else in this pass: every CTA forms it)
+        const bool active = c[6 + pass - 1] != 0u;
+        if (!active) {
+            if (one) {
+                c[6 + pass] = 0u;
+                if (last) c[2] = 0u;
+            }
+            return;
+        }
+        __shared__ float s_mean;
+        if (threadIdx.x < 32) {
+            double a, b;
+            warp_sum_partials(parts + (size_t)blockIdx.y * part_stride + ((pass - 1) & 1) * nparts,
+                              nparts, a, b);
+            if (threadIdx.x == 0) s_mean = __fdiv_rn((float)a, (float)(double)n);
+        }
+        __syncthreads();
+        const float mean = s_mean;
+        const bool more = fabsf(mean) > 5e-7 * (double)n;
+        if (one) {
+            m[pass - 1] = mean;
+            c[6 + pass] = more ? 1u : 0u;
+            c[3] = (unsigned)pass;
+            if (last) c[2] = more ? 1u : 0u;
+        }
+        if (!more || last) return;
+        s = pass > 1 ? sum_less(x, n, m[0], mean) : sum_less(x, n, mean, 0.f);
+    }
+    block_partials<kVecThreads>(s, 0.0, out);
+}
+static_assert(kBaselineMeans == 3, "the third mean needs no sum after it");
+
+// The same loop for short series in one launch: a cluster of kMeanCtas CTAs
+// per row sums, exchanges its partial sums through distributed shared memory
+// and goes round again while the mean is above the threshold.  Eight SMs read
+// a row slower than the whole device, so it is taken up to 2^20 samples and,
+// where the rows of a group read side by side, 2^21.  A call of 1, 3, 12 and
+// 48 DM trials with two passes each on B200 (us, four launches against one):
+// 2^19: 172/161, 339/303, 516/383, 1220/750; 2^20: 171/169, 360/332, 622/512,
+// 1818/1359; 2^21: 179/189, 399/427, 895/812, 2839/2513.
+constexpr int kMeanCtas = 8;
+constexpr int kMeanThreads = 1024;
+constexpr size_t kMeanMaxSamples = (size_t)1 << 20;  // twice that from 4 rows on
+
+__global__ void __launch_bounds__(kMeanThreads) k_baseline_means_cluster(
+    SeriesRows rows, size_t n, unsigned* __restrict__ cnt, float* __restrict__ means)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const float* x = rows.p[blockIdx.y];
+    __shared__ double warp_sum[kMeanThreads / 32];
+    __shared__ double part[kBaselineMeans];  // this CTA's sum of each pass
+    float m[kBaselineMeans] = {0.f, 0.f, 0.f};
+    int pass = 0;
+    bool more = true;
+#pragma unroll
+    for (int p = 0; p < kBaselineMeans; ++p) {
+        if (!more) break;  // the same in every thread of the cluster
+        double s = sum_less(x, n, m[0], m[1]);
+        for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x / 32] = s;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            double t = warp_sum[threadIdx.x];
+            for (int o = 16; o; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+            if (threadIdx.x == 0) part[p] = t;
+        }
+        cl.sync();
+        double total = 0.0;
+        for (int c = 0; c < kMeanCtas; ++c) total += *cl.map_shared_rank(&part[p], c);
+        m[p] = __fdiv_rn((float)total, (float)(double)n);
+        more = fabsf(m[p]) > 5e-7 * (double)n;
+        pass = p + 1;
+    }
+    if (cl.block_rank() == 0 && threadIdx.x == 0) {
+        unsigned* c = cnt + 16 * blockIdx.y;
+        c[2] = more ? 1u : 0u;
+        c[3] = (unsigned)pass;
+        for (int k = 0; k < kBaselineMeans; ++k) means[4 * blockIdx.y + k] = m[k];
+    }
+    cl.sync();  // no CTA leaves while another reads its partial sums
+}
+
+int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* d_parts,
+                          size_t part_stride, unsigned* d_cnt, float* d_means, cudaStream_t s)
+{
+    if (n <= kMeanMaxSamples * (nrows >= 4 ? 2 : 1)) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kMeanCtas, nrows);
+        cfg.blockDim = dim3(kMeanThreads);
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim = {kMeanCtas, 1, 1};
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cuda_status(cudaLaunchKernelEx(&cfg, k_baseline_means_cluster, rows, n, d_cnt,
+                                              d_means),
+                           "baseline mean kernel");
+    }
+    const int nb = reduction_blocks();
+    const dim3 grid(nb, nrows);
+    k_baseline_means<true><<<grid, kVecThreads, 0, s>>>(rows, n, d_parts, part_stride, nb, d_cnt,
+                                                        d_means, 0, 0);
+    for (int pass = 1; pass <= kBaselineMeans; ++pass)
+        k_baseline_means<false><<<grid, kVecThreads, 0, s>>>(rows, n, d_parts, part_stride, nb,
+                                                             d_cnt, d_means, pass,
+                                                             pass == kBaselineMeans);
+    return launch_status("baseline mean kernels");
+}
+
+// Median levels of `rows` amplitude spectra (strides in floats).
+int launch_scrunch_rows(const float* d_amp, size_t stride, int rows, size_t nbins, float* d_scratch,
+                        size_t scratch_stride, cudaStream_t s)
+{
+    auto up = [](size_t v) { return (v + 63) / 64 * 64; };
+    float* m25 = d_scratch + up(nbins / 5 + 1);
+    float* m125 = m25 + up(nbins / 25 + 1);
+    const size_t n5 = nbins / 5, n25 = n5 / 5, n125 = n25 / 5, ngroups = (n5 + 24) / 25;
+    const unsigned grid = (unsigned)std::min<size_t>((ngroups + kScrGroups - 1) / kScrGroups,
+                                                     (size_t)sm_count() * 8);
+    k_scrunch3<false><<<dim3(grid, rows), 256, 0, s>>>(d_amp, d_scratch, n5, m25, n25, m125, n125,
+                                                       stride, scratch_stride);
+    return launch_status("scrunch kernel (rows)");
+}
+
+// k_finish_stats for many partials: 32 warps, each a fixed run of them.
+__global__ void __launch_bounds__(1024) k_finish_stats_wide(const double2* __restrict__ partials,
+                                                            int nparts, double count,
+                                                            float* __restrict__ stat, float scale,
+                                                            size_t part_stride, size_t stat_stride)
+{
+    partials += (size_t)blockIdx.y * part_stride;
+    stat += (size_t)blockIdx.y * stat_stride;
+    __shared__ double2 sh[32];
+    const int w = threadIdx.x / 32, per = (nparts + 31) / 32;
+    const int p0 = min(nparts, w * per), np = min(nparts, p0 + per) - p0;
+    double a, b;
+    warp_sum_partials(partials + p0, np, a, b);
+    if ((threadIdx.x & 31) == 0) sh[w] = make_double2(a, b);
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    warp_sum_partials(sh, 32, a, b);
+    if (threadIdx.x == 0) write_stats(a, b, count, stat, scale);
+}
+
+int launch_finish_stats_rows(const double2* d_partials, int nparts, size_t part_stride, int rows,
+                             size_t count, float* d_stat, size_t stat_stride, float scale,
+                             cudaStream_t s)
+{
+    k_finish_stats_wide<<<dim3(1, rows), 1024, 0, s>>>(d_partials, nparts, (double)count, d_stat,
+                                                       scale, part_stride, stat_stride);
+    return launch_status("statistics kernel (rows)");
+}
+
+// Bits of the bins that k_zap sets (the same ranges), for kernels that zap
+// as they go.
+__global__ void k_zap_mask(unsigned* __restrict__ mask, const float* __restrict__ freqs,
+                           const float* __restrict__ widths, float bin_width, unsigned nbirdies,
+                           unsigned nbins)
+{
+    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    if (warp >= nbirdies) return;
+    int lo, hi;
+    if (!zap_range(freqs[warp], widths[warp], bin_width, nbins, lo, hi)) return;
+    for (int k = lo + (int)(threadIdx.x & 31); k < hi; k += 32)
+        atomicOr(mask + (k >> 5), 1u << (k & 31));
+}
+
+int launch_zap_mask(unsigned* d_mask, const float* d_freqs, const float* d_widths, float bin_width,
+                    size_t nbirdies, size_t nbins, cudaStream_t s)
+{
+    PSX_CUDA(cudaMemsetAsync(d_mask, 0, (nbins + 31) / 32 * sizeof(unsigned), s));
+    if (nbirdies == 0) return PSX_OK;
+    k_zap_mask<<<(unsigned)((nbirdies * 32 + 255) / 256), 256, 0, s>>>(
+        d_mask, d_freqs, d_widths, bin_width, (unsigned)nbirdies, (unsigned)nbins);
+    return launch_status("zap mask kernel");
+}
+
 int launch_partials_v4(const float* d_x, size_t n, double2* d_partials, float* d_copy,
                        unsigned* d_state, cudaStream_t s)
 {
@@ -805,21 +1035,7 @@ int launch_running_median_spectrum_rows(float* d_X, size_t x_stride, int rows, s
     k_scrunch3<true><<<dim3(grid, rows), 256, 0, s>>>(d_X, m5, n5, m25, n25, m125, n125, x_stride,
                                                       scratch_stride_floats);
     PSX_TRY(launch_status("amplitude + scrunch kernel (rows)"));
-    int pos5 = (int)((double)b5 / bin_width);
-    int pos25 = (int)((double)b25 / bin_width);
-    MedianLevels L;
-    L.m5 = m5;
-    L.m25 = m25;
-    L.m125 = m125;
-    L.n5 = (unsigned)n5;
-    L.n25 = (unsigned)n25;
-    L.n125 = (unsigned)n125;
-    L.step5 = stretch_step(n5, nbins);
-    L.step25 = stretch_step(n25, nbins);
-    L.step125 = stretch_step(n125, nbins);
-    L.pos5 = (unsigned)(pos5 < 0 ? 0 : (size_t)pos5 > nbins ? nbins : pos5);
-    L.pos25 = (unsigned)(pos25 < 0 ? 0 : (size_t)pos25 > nbins ? nbins : pos25);
-    if (L.pos25 < L.pos5) L.pos25 = L.pos5;
+    const MedianLevels L = median_levels(nbins, bin_width, b5, b25, m5);
     k_median_apply<<<dim3(grid_for(nbins, 256), rows), 256, 0, s>>>(
         L, nbins, nullptr, d_X, x_stride, scratch_stride_floats);
     return launch_status("median apply kernel (rows)");

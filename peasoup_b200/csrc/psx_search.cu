@@ -44,6 +44,10 @@
 #include "psx_host.h"
 #include "psx_stages.cuh"
 
+extern "C" {
+static int effective_form(const psx_search_config* c);
+}
+
 namespace psx {
 
 // Host threads that cluster and distil one DM's records trial by trial.
@@ -382,28 +386,36 @@ static int launch_harm(int F, int shape, const float* p, size_t ppitch, unsigned
 }
 
 constexpr int kDeviceBaselinePasses = 4;
+// launches of prologue_own: baseline means, two forward passes, amplitudes,
+// medians, dereddening, statistics, two inverse passes
+constexpr int kOwnPrologueLaunches = 1 + kBaselineMeans + 8;
 
 // Grouped prologue: DM trials per group by default, the largest transform
 // it applies to by default, and the most acceleration trials per DM trial
-// (averaged over a call) for which the default groups.  Measured on B200
-// with 1-3 trials per DM trial: 4 rows take the per-DM cost from 89 to
-// 55 us at 2^19 points and from 93 to 65 us at 2^20 (8 and 16 rows a
-// little less), 150 to 141 us at 2^22, nothing at 2^23, where the
-// prologue's launches are long enough to fill the device on their own.
-// With many trials per DM trial the trials outweigh the prologue and the
-// two slots' overlap already hides it.
+// (averaged over a call) for which the default groups.  With many trials per
+// DM trial the trials outweigh the prologue and the two slots' overlap
+// already hides it; at 2^23 points the prologue's launches fill the device
+// on their own.
 constexpr int kGroupRowsDefault = 4;
-constexpr int kGroupRowsMax = 16;
+constexpr int kGroupRowsMax = kSeriesRowsMax;
 constexpr size_t kGroupMaxPoints = (size_t)1 << 22;
 constexpr double kGroupMaxTrials = 32.0;
 
 // Rows of the group sets an instance of this configuration may use (0: it
-// never groups).
+// never groups).  By default as many as make a launch of the own-transform
+// prologue fill the device: us per call of 48 DM trials with one trial each
+// on B200, in groups of 4, 8 and 16: 1162, 830, 789 at 2^19 points; 1526,
+// 1364, 1285 at 2^20 (with five trials each 2882, 2650, 2709); 2638, 2400,
+// 2325 at 2^21; 4957, 4804, 4748 at 2^22, where 4 rows already take 800 MB.
+// cuFFT's batched plans transform every row of a set, used or not: 4.
 static int group_rows_for(const psx_search_config* c)
 {
     if (c->mode != PSX_MODE_BATCHED || c->group_dms == 1) return 0;
     if (c->group_dms >= 2) return c->group_dms;
-    return c->fft_size <= kGroupMaxPoints ? kGroupRowsDefault : 0;
+    if (c->fft_size > kGroupMaxPoints) return 0;
+    if (effective_form(c) != 3) return kGroupRowsDefault;
+    return c->fft_size <= ((size_t)1 << 19) ? 16 : c->fft_size <= ((size_t)1 << 21) ? 8
+                                                                                  : kGroupRowsDefault;
 }
 
 // Tensor maps of a spectrum buffer of `rows` rows of `pitch` floats for
@@ -500,7 +512,7 @@ struct Slot {
     double* d_sums = nullptr;
     float* d_stat = nullptr;  // interbin statistics: [3] mean*N, [4] std*N
     float* d_mean = nullptr;
-    FftPlan* r2c = nullptr;   // batch-1 plans of the prologue
+    FftPlan* r2c = nullptr;   // batch-1 plans of the prologue (cuFFT forms)
     FftPlan* c2r = nullptr;
     cudaStream_t pst = nullptr;
     cudaEvent_t ready = nullptr;  // prologue complete (on pst)
@@ -530,12 +542,12 @@ struct GroupSet {
     float* tim = nullptr;     // G x N dereddened series
     float* Xp = nullptr;      // G x 2 Bp prologue spectra
     float* med = nullptr;     // G x med_floats median scratch
-    double2* part = nullptr;  // G x 2 nb partial sums
+    double2* part = nullptr;  // G x part_len partial sums
     double* sums = nullptr;   // G x 2
     float* stat = nullptr;    // G x 8
-    unsigned* count = nullptr;  // G x 16 counters and flags
-    float* mean = nullptr;    // G x 2
-    FftPlan r2c, c2r;         // batch-G plans over the rows
+    unsigned* count = nullptr;  // G x 16 counters and flags, then d_cnt's 4 words
+    float* mean = nullptr;    // G x 4
+    FftPlan r2c, c2r;         // batch-G plans over the rows (cuFFT forms)
     // Trial schedule spanning the chunk's DM trials (two-pass transform):
     // the trials of all its DM trials in one list (DM trial i's at
     // [off[i], off[i+1])), each with its factor and its series row, and one
@@ -543,9 +555,9 @@ struct GroupSet {
     int4* d_rec = nullptr;
     int4* h_rec = nullptr;
     size_t rec_cap = 0;
-    unsigned* d_cnt = nullptr;  // [0] hits, [1] staging error
-    unsigned* h_cnt = nullptr;  // d_cnt's two words, then the rows' 16 counters each
-    double* d_ktab = nullptr;
+    unsigned* d_cnt = nullptr;  // [0] hits, [1] staging error (after the rows' counters)
+    unsigned* h_cnt = nullptr;  // the rows' 16 counters each, then d_cnt's words
+    double* d_ktab = nullptr;   // tab_cap factors, then tab_cap series rows (one copy)
     double* h_ktab = nullptr;
     unsigned* d_trow = nullptr;
     unsigned* h_trow = nullptr;
@@ -609,7 +621,9 @@ struct psx_search {
     Slot slot[2];
     // grouped prologue (0 = off): two sets of kGroupRows slots, used in turn
     int group_rows = 0;
-    size_t med_floats = 0;
+    size_t med_floats = 0;             // floats of one DM trial's median scratch
+    size_t part_len = 0;               // partial sums of one DM trial (double2)
+    unsigned* d_zap = nullptr;         // own-transform prologue: bit per zapped bin
     GroupSet gset[2];
     FftPlan r2c1;                      // plain-mode trials and the debug tap
     Fft4Plan f4;                       // the hand-written transform (fft_form 3)
@@ -666,11 +680,12 @@ struct psx_search {
             m.clear();
         }
         r2c1.destroy();
-        void* dev[] = {d_trl[0], d_Xl[0], d_pl[0], d_trl[1], d_Xl[1], d_pl[1], d_bf, d_bw};
+        void* dev[] = {d_trl[0], d_Xl[0], d_pl[0], d_trl[1], d_Xl[1], d_pl[1], d_bf, d_bw, d_zap};
         for (void* q : dev)
             if (q) cudaFree(q);
         for (int l = 0; l < 2; ++l) d_trl[l] = d_Xl[l] = d_pl[l] = nullptr;
         d_tr = d_X = d_p = d_bf = d_bw = nullptr;
+        d_zap = nullptr;
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         ev_fork = ev_join = nullptr;
@@ -722,7 +737,14 @@ struct psx_search {
     int grow_ktab(Slot& s, size_t need);
     int ensure_events(Slot& s, int groups);
     int prologue(Slot& s);
+    bool readable(const Slot& s) const;
+    int make_zap_mask();
+    int host_baseline_loop(Slot& s, size_t ncopy, cudaStream_t ps);
+    int prologue_own(float* tim, float* Xp, void* med, double2* part, float* stat,
+                     unsigned* count, float* mean, const SeriesRows& src, size_t ncopy, int rows,
+                     bool host_baseline, cudaStream_t ps);
     int prologue_group(GroupSet& g, int count, cudaStream_t ps);
+    int prologue_done(GroupSet& g, int count, int launches, int ffts, cudaStream_t ps);
     int prep(Slot& s, const float* series, size_t nsamps, bool on_device, float dm, int dm_idx);
     int enqueue_trials(Slot& s);
     int alloc_groups();
@@ -824,7 +846,7 @@ int psx_search::grow_records(Slot& s, size_t need)
     PSX_CUDA(cudaMalloc(&s.d_rec, sizeof(int4) * cap));
     PSX_CUDA(cudaMallocHost(&s.h_rec, sizeof(int4) * cap));
     s.rec_cap = cap;
-    drop_graphs();  // captured schedules hold the old buffer
+    if (!s.grouped) drop_graphs();  // captured schedules hold the old buffer
     return PSX_OK;
 }
 
@@ -856,14 +878,80 @@ int psx_search::ensure_events(Slot& s, int groups)
     return PSX_OK;
 }
 
+// The baseline loop with the host in it (rare), on the series in s.d_tim.
+int psx_search::host_baseline_loop(Slot& s, size_t ncopy, cudaStream_t ps)
+{
+    int count = 0;
+    do {
+        PSX_TRY(remove_baseline_pass(s.d_tim, ncopy, s.d_part, s.d_sums, s.d_mean, ps));
+        s.launches += 4;
+        PSX_CUDA(cudaMemcpyAsync(h_mean, s.d_mean, sizeof(float), cudaMemcpyDeviceToHost, ps));
+        PSX_CUDA(cudaStreamSynchronize(ps));
+        if (count++ > 100) break;
+    } while (std::fabs(*h_mean) > 5e-7 * (double)ncopy);
+    return PSX_OK;
+}
+
 // src/pipeline_multi.cu:170-238 for one series, on the slot's own stream.
 // It starts once the caller's work queued before this call (call_start)
 // and the slot's previous DM (whose trials read s.d_tim) are done, and
 // records s.ready; the trials wait for s.ready on the compute stream.  So
 // the prologue of DM d+1 runs alongside the trials of DM d.
+// Whether the kernels can read the job's series where it lies: this
+// device's own memory, whole floats.  Anything else is copied first.
+bool psx_search::readable(const Slot& s) const
+{
+    if (!s.on_device || (reinterpret_cast<uintptr_t>(s.series) & 3u)) return false;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, s.series) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == device;
+}
+
+int psx_search::make_zap_mask()
+{
+    if (!d_zap || bf.empty()) return PSX_OK;
+    PSX_CUDA(cudaStreamSynchronize(nullptr));  // the birdie list's copies
+    return launch_zap_mask(d_zap, d_bf, d_bw, bin_width_f, bf.size(), B, st);
+}
+
+// src/pipeline_multi.cu:170-238 on the library's own transform, for `rows`
+// series at once (row strides N floats, Bp complex, med_floats, part_len, 8,
+// 16 and 4 elements): the means of the baseline loop, then the two forward
+// passes (their loads subtract the means and pad), amplitudes, median
+// levels, one kernel from spectrum to dereddened spectrum with its
+// statistics, and the two inverse passes.  `tim` holds in turn the forward
+// intermediate, the amplitudes, the inverse's input and the series; src may
+// lie there.  Twelve launches and about 13 N floats of traffic per DM trial,
+// where cuFFT's transforms with the passes between them took 22 launches and
+// 22 N (103 us per DM trial at 2^22 points on B200, now 61).
+int psx_search::prologue_own(float* tim, float* Xp, void* med, double2* part, float* stat,
+                             unsigned* count, float* mean, const SeriesRows& src, size_t ncopy,
+                             int rows, bool host_baseline, cudaStream_t ps)
+{
+    float2* z = reinterpret_cast<float2*>(Xp);
+    float2* t2 = reinterpret_cast<float2*>(tim);
+    float* m = static_cast<float*>(med);
+    if (host_baseline)
+        PSX_CUDA(cudaMemsetAsync(mean, 0, sizeof(float) * 4 * (size_t)rows, ps));
+    else
+        PSX_TRY(launch_baseline_means(src, rows, ncopy, part, part_len, count, mean, ps));
+    PSX_TRY(f4.exec_series(src, rows, ncopy, mean, t2, N / 2, z, Bp, ps));
+    PSX_TRY(f4.amplitudes(z, Bp, rows, tim, N, ps));
+    PSX_TRY(launch_scrunch_rows(tim, N, rows, B, m, med_floats, ps));
+    PSX_TRY(f4.deredden(z, Bp, rows, t2, N / 2,
+                        median_levels(B, bin_width, cfg.boundary_5_freq, cfg.boundary_25_freq, m),
+                        med_floats, bf.empty() ? nullptr : d_zap, part, part_len, ps));
+    PSX_TRY(launch_finish_stats_rows(part, (int)Fft4Plan::stat_parts(N), part_len, rows, B, stat, 8,
+                                     (float)N, ps));
+    return f4.exec_inverse(t2, N / 2, rows, ps);
+}
+
 int psx_search::prologue(Slot& s)
 {
-    if (!s.r2c) {  // a grouped slot run on its own (a retry): batch-1 plans on first need
+    if (!s.r2c && !use_f4) {  // a grouped slot run on its own (a retry): batch-1 plans on first need
         s.r2c = new (std::nothrow) FftPlan;
         s.c2r = new (std::nothrow) FftPlan;
         if (!s.r2c || !s.c2r) return PSX_ERR_ALLOC;
@@ -875,6 +963,23 @@ int psx_search::prologue(Slot& s)
     PSX_CUDA(cudaStreamWaitEvent(ps, s.done, 0));
     if (s.profiled) PSX_CUDA(cudaEventRecord(s.ev[0], ps));
     const size_t ncopy = std::min(s.nsamps, N);
+    if (use_f4) {
+        SeriesRows src{};
+        src.p[0] = s.series;
+        if (s.host_baseline || !readable(s)) {
+            PSX_CUDA(cudaMemcpyAsync(s.d_tim, s.series, sizeof(float) * ncopy,
+                                     s.on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                                     ps));
+            src.p[0] = s.d_tim;
+        }
+        if (s.host_baseline) PSX_TRY(host_baseline_loop(s, ncopy, ps));
+        PSX_TRY(prologue_own(s.d_tim, s.d_Xp, s.d_med, s.d_part, s.d_stat, s.d_count, s.d_mean,
+                             src, ncopy, 1, s.host_baseline, ps));
+        s.launches += s.host_baseline ? 8 : kOwnPrologueLaunches;
+        if (s.profiled) PSX_CUDA(cudaEventRecord(s.ev[1], ps));
+        PSX_CUDA(cudaEventRecord(s.ready, ps));
+        return PSX_OK;
+    }
     // a device series 16-byte aligned is copied by the first baseline pass
     const bool fused_copy =
         s.on_device && !s.host_baseline && (reinterpret_cast<uintptr_t>(s.series) & 15u) == 0;
@@ -905,16 +1010,7 @@ int psx_search::prologue(Slot& s)
             ++s.launches;
         }
     } else {
-        int count = 0;
-        float mean = 0.f;
-        do {
-            PSX_TRY(remove_baseline_pass(s.d_tim, ncopy, s.d_part, s.d_sums, s.d_mean, ps));
-            s.launches += 4;
-            PSX_CUDA(cudaMemcpyAsync(h_mean, s.d_mean, sizeof(float), cudaMemcpyDeviceToHost, ps));
-            PSX_CUDA(cudaStreamSynchronize(ps));
-            mean = *h_mean;
-            if (count++ > 100) break;
-        } while (std::fabs(mean) > 5e-7 * (double)ncopy);
+        PSX_TRY(host_baseline_loop(s, ncopy, ps));
     }
     // zero padding (pipeline_multi.cu:179-187)
     if (ncopy < N) {
@@ -964,17 +1060,15 @@ int psx_search::grow_span_tables(GroupSet& g, size_t need)
     if (need <= g.tab_cap) return PSX_OK;
     const size_t cap = round_up(need + need / 4, 256);
     PSX_CUDA(cudaStreamSynchronize(st));
-    for (void* q : {(void*)g.d_ktab, (void*)g.d_trow})
-        if (q) cudaFree(q);
-    for (void* q : {(void*)g.h_ktab, (void*)g.h_trow})
-        if (q) cudaFreeHost(q);
+    if (g.d_ktab) cudaFree(g.d_ktab);
+    if (g.h_ktab) cudaFreeHost(g.h_ktab);
     g.d_ktab = g.h_ktab = nullptr;
     g.d_trow = g.h_trow = nullptr;
     g.tab_cap = 0;
-    PSX_CUDA(cudaMalloc((void**)&g.d_ktab, sizeof(double) * cap));
-    PSX_CUDA(cudaMalloc((void**)&g.d_trow, sizeof(unsigned) * cap));
-    PSX_CUDA(cudaMallocHost(&g.h_ktab, sizeof(double) * cap));
-    PSX_CUDA(cudaMallocHost(&g.h_trow, sizeof(unsigned) * cap));
+    PSX_CUDA(cudaMalloc((void**)&g.d_ktab, (sizeof(double) + sizeof(unsigned)) * cap));
+    PSX_CUDA(cudaMallocHost(&g.h_ktab, (sizeof(double) + sizeof(unsigned)) * cap));
+    g.d_trow = reinterpret_cast<unsigned*>(g.d_ktab + cap);
+    g.h_trow = reinterpret_cast<unsigned*>(g.h_ktab + cap);
     g.tab_cap = cap;
     return PSX_OK;
 }
@@ -988,15 +1082,10 @@ int psx_search::grow_span_tables(GroupSet& g, size_t need)
 int psx_search::trials_span(GroupSet& g, int cnt)
 {
     const int T = g.off[cnt];
-    for (int i = 0; i < cnt; ++i) {
-        Slot& sl = g.slots[i];
-        PSX_CUDA(cudaStreamWaitEvent(st, sl.ready, 0));
-        // each slot keeps its own factors too (the debug tap reads them)
-        PSX_CUDA(cudaMemcpyAsync(sl.d_ktab, sl.h_ktab, sizeof(double) * sl.accs.size(),
-                                 cudaMemcpyHostToDevice, st));
-    }
-    PSX_CUDA(cudaMemcpyAsync(g.d_ktab, g.h_ktab, sizeof(double) * T, cudaMemcpyHostToDevice, st));
-    PSX_CUDA(cudaMemcpyAsync(g.d_trow, g.h_trow, sizeof(unsigned) * T, cudaMemcpyHostToDevice, st));
+    for (int i = 0; i < cnt; ++i) PSX_CUDA(cudaStreamWaitEvent(st, g.slots[i].ready, 0));
+    // factors and series rows in one copy
+    PSX_CUDA(cudaMemcpyAsync(g.d_ktab, g.h_ktab, sizeof(double) * g.tab_cap + sizeof(unsigned) * T,
+                             cudaMemcpyHostToDevice, st));
     PSX_CUDA(cudaMemsetAsync(g.d_cnt, 0, sizeof(unsigned) * 2, st));
     const bool span = pk.hi > pk.lo;
     float* tr = d_trl[0];
@@ -1030,9 +1119,8 @@ int psx_search::trials_span(GroupSet& g, int cnt)
         t0 += b;
         ++g.groups;
     }
-    // the hit counter, and every row's prologue counters (baseline flags)
-    PSX_CUDA(cudaMemcpyAsync(g.h_cnt, g.d_cnt, sizeof(unsigned) * 2, cudaMemcpyDeviceToHost, st));
-    PSX_CUDA(cudaMemcpyAsync(g.h_cnt + 2, g.count, sizeof(unsigned) * 16 * (size_t)cnt,
+    // every row's prologue counters (baseline flags) and the hit counter
+    PSX_CUDA(cudaMemcpyAsync(g.h_cnt, g.count, sizeof(unsigned) * (16 * g.slots.size() + 2),
                              cudaMemcpyDeviceToHost, st));
     PSX_CUDA(cudaEventRecord(g.done, st));
     for (int i = 0; i < cnt; ++i) PSX_CUDA(cudaEventRecord(g.slots[i].done, st));
@@ -1046,23 +1134,24 @@ int psx_search::trials_span(GroupSet& g, int cnt)
 // through the per-DM path with the host loop.
 int psx_search::finish_span(GroupSet& g, int cnt, std::vector<DmRecords>& jobs)
 {
+    const unsigned* hits = g.h_cnt + 16 * g.slots.size();  // [0] hits, [1] staging error
     for (int attempt = 0;; ++attempt) {
         const auto t_wait = std::chrono::steady_clock::now();
         PSX_CUDA(cudaEventSynchronize(g.done));
         prof.host_wait_ms += ms_since(t_wait);
-        if (g.h_cnt[1] != 0) {
-            set_error("search: harmonic-sum staging did not complete (status 0x%x)", g.h_cnt[1]);
+        if (hits[1] != 0) {
+            set_error("search: harmonic-sum staging did not complete (status 0x%x)", hits[1]);
             return PSX_ERR_CUDA;
         }
-        if (g.h_cnt[0] <= g.rec_cap) break;
+        if (hits[0] <= g.rec_cap) break;
         if (attempt == 2) {
             set_error("search: could not complete DM trials %d..", g.slots[0].dm_idx);
             return PSX_ERR_OVERFLOW;
         }
-        PSX_TRY(grow_span_records(g, g.h_cnt[0]));
+        PSX_TRY(grow_span_records(g, hits[0]));
         PSX_TRY(trials_span(g, cnt));
     }
-    const size_t nrec = g.h_cnt[0];
+    const size_t nrec = hits[0];
     if (nrec) {
         PSX_CUDA(cudaStreamWaitEvent(cst, g.done, 0));
         PSX_CUDA(cudaMemcpyAsync(g.h_rec, g.d_rec, sizeof(int4) * nrec, cudaMemcpyDeviceToHost,
@@ -1091,7 +1180,7 @@ int psx_search::finish_span(GroupSet& g, int cnt, std::vector<DmRecords>& jobs)
     info.fft_launches += g.slots[0].ffts;
     info.above_threshold += (long long)nrec;
     for (int i = 0; i < cnt; ++i) {
-        const unsigned* c = g.h_cnt + 2 + 16 * (size_t)i;
+        const unsigned* c = g.h_cnt + 16 * (size_t)i;
         Slot& sl = g.slots[i];
         info.baseline_passes = (int)c[3];
         if (c[2] != 0) {  // rare: the baseline loop needs the host
@@ -1124,25 +1213,24 @@ int psx_search::alloc_groups_sets()
 {
     const int G = group_rows_for(&cfg);
     if (G < 2) return PSX_OK;
-    const size_t nb = (size_t)reduction_blocks();
-    med_floats = median_scratch_bytes(B) / sizeof(float);
     for (GroupSet& g : gset) {
         PSX_CUDA(cudaMalloc((void**)&g.tim, sizeof(float) * N * G));
         PSX_CUDA(cudaMalloc((void**)&g.Xp, sizeof(float) * 2 * Bp * G));
         PSX_CUDA(cudaMalloc((void**)&g.med, sizeof(float) * med_floats * G));
-        PSX_CUDA(cudaMalloc((void**)&g.part, sizeof(double2) * 2 * nb * G));
+        PSX_CUDA(cudaMalloc((void**)&g.part, sizeof(double2) * part_len * G));
         PSX_CUDA(cudaMalloc((void**)&g.sums, sizeof(double) * 2 * G));
         PSX_CUDA(cudaMalloc((void**)&g.stat, sizeof(float) * 8 * G));
-        PSX_CUDA(cudaMalloc((void**)&g.count, sizeof(unsigned) * 16 * G));
-        PSX_CUDA(cudaMalloc((void**)&g.mean, sizeof(float) * 2 * G));
+        PSX_CUDA(cudaMalloc((void**)&g.count, sizeof(unsigned) * (16 * G + 4)));
+        PSX_CUDA(cudaMalloc((void**)&g.mean, sizeof(float) * 4 * G));
         // rows past a call's last DM trial are transformed too (the plans
         // hold G rows): they start as zeros, never as uninitialised memory
         PSX_CUDA(cudaMemsetAsync(g.tim, 0, sizeof(float) * N * G, st));
         PSX_CUDA(cudaMemsetAsync(g.Xp, 0, sizeof(float) * 2 * Bp * G, st));
-        PSX_TRY(g.r2c.create(N, G, PSX_FFT_R2C, N, Bp));
-        PSX_TRY(g.c2r.create(N, G, PSX_FFT_C2R, Bp, N));
-        if (use_f4) {  // the spanning trial schedule's counters and event
-            PSX_CUDA(cudaMalloc((void**)&g.d_cnt, sizeof(unsigned) * 4));
+        if (!use_f4) {
+            PSX_TRY(g.r2c.create(N, G, PSX_FFT_R2C, N, Bp));
+            PSX_TRY(g.c2r.create(N, G, PSX_FFT_C2R, Bp, N));
+        } else {  // the spanning trial schedule's counters and event
+            g.d_cnt = g.count + 16 * G;
             PSX_CUDA(cudaMallocHost(&g.h_cnt, sizeof(unsigned) * (2 + 16 * (size_t)G)));
             PSX_CUDA(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming));
             PSX_TRY(grow_span_records(g, (size_t)1 << 20));
@@ -1155,16 +1243,18 @@ int psx_search::alloc_groups_sets()
             sl.d_tim = g.tim + (size_t)i * N;
             sl.d_Xp = g.Xp + (size_t)i * 2 * Bp;
             sl.d_med = g.med + (size_t)i * med_floats;
-            sl.d_part = g.part + (size_t)i * 2 * nb;
+            sl.d_part = g.part + (size_t)i * part_len;
             sl.d_sums = g.sums + 2 * i;
             sl.d_stat = g.stat + 8 * i;
             sl.d_count = g.count + 16 * i;
-            sl.d_mean = g.mean + 2 * i;
+            sl.d_mean = g.mean + 4 * i;
             PSX_CUDA(cudaMallocHost(&sl.h_count, sizeof(unsigned) * 4));
             PSX_CUDA(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
             PSX_CUDA(cudaEventCreateWithFlags(&sl.copied, cudaEventDisableTiming));
             PSX_CUDA(cudaEventCreateWithFlags(&sl.ready, cudaEventDisableTiming));
-            PSX_TRY(grow_records(sl, (size_t)1 << 18));
+            // with one list of trials per group a slot's own records are for a
+            // DM trial run again alone: made on first need
+            if (!use_f4) PSX_TRY(grow_records(sl, (size_t)1 << 18));
             PSX_TRY(grow_ktab(sl, 64));
         }
     }
@@ -1190,13 +1280,14 @@ void psx_search::free_groups()
             delete s.c2r;
         }
         g.slots.clear();
-        for (void* q : {(void*)g.d_rec, (void*)g.d_cnt, (void*)g.d_ktab, (void*)g.d_trow})
+        for (void* q : {(void*)g.d_rec, (void*)g.d_ktab})
             if (q) cudaFree(q);
-        for (void* q : {(void*)g.h_rec, (void*)g.h_cnt, (void*)g.h_ktab, (void*)g.h_trow})
+        for (void* q : {(void*)g.h_rec, (void*)g.h_cnt, (void*)g.h_ktab})
             if (q) cudaFreeHost(q);
         if (g.done) cudaEventDestroy(g.done);
         g.d_rec = g.h_rec = nullptr;
-        g.d_cnt = g.h_cnt = g.d_trow = g.h_trow = nullptr;
+        g.d_cnt = g.h_cnt = nullptr;
+        g.d_trow = g.h_trow = nullptr;
         g.d_ktab = g.h_ktab = nullptr;
         g.rec_cap = g.tab_cap = 0;
         g.done = nullptr;
@@ -1214,20 +1305,23 @@ void psx_search::free_groups()
 
 // Rows per grouped prologue for a call over these DM trials (0: one
 // prologue per DM trial).  A call groups when it has more DM trials than a
-// group holds; by default also only when its DM trials average at most
-// kGroupMaxTrials acceleration trials.
+// group holds (by default, than kGroupRowsDefault); by default also only when
+// its DM trials average at most kGroupMaxTrials acceleration trials, and in
+// at least three groups where it can, so that one group's prologue runs
+// beside another's trials.
 int psx_search::group_rows_for_call(const float* dms, int ndm) const
 {
     const int G = group_rows_for(&cfg);
-    if (G < 2 || ndm <= G) return 0;
-    if (cfg.group_dms >= 2) return G;
+    if (cfg.group_dms >= 2) return ndm > G ? G : 0;
+    if (G < 2 || ndm <= kGroupRowsDefault) return 0;
     const psx_search_config& c = cfg;
     double total = 0.0;
     for (int d = 0; d < ndm; ++d)
         total += (double)accel_list(c.acc_lo, c.acc_hi, c.acc_tol, c.acc_pulse_width, N, c.tsamp,
                                     c.cfreq_hz, c.ch_bw_hz, dms[d], c.cdm)
                      .size();
-    return total <= kGroupMaxTrials * ndm ? G : 0;
+    if (total > kGroupMaxTrials * ndm) return 0;
+    return std::min(G, std::max(kGroupRowsDefault, (ndm + 2) / 3));
 }
 
 // The prologues of the first `count` slots of a group set as one batch:
@@ -1243,6 +1337,22 @@ int psx_search::prologue_group(GroupSet& g, int count, cudaStream_t ps)
     Slot& s0 = g.slots[0];
     if (s0.profiled) PSX_CUDA(cudaEventRecord(s0.ev[0], ps));
     const size_t ncopy = std::min(s0.nsamps, N);  // one length for every series of a call
+    if (use_f4) {
+        SeriesRows src{};
+        for (int i = 0; i < count; ++i) {
+            Slot& sl = g.slots[i];
+            sl.pst = ps;
+            src.p[i] = sl.series;
+            if (readable(sl)) continue;
+            PSX_CUDA(cudaMemcpyAsync(sl.d_tim, sl.series, sizeof(float) * ncopy,
+                                     sl.on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                                     ps));
+            src.p[i] = sl.d_tim;
+        }
+        PSX_TRY(prologue_own(g.tim, g.Xp, g.med, g.part, g.stat, g.count, g.mean, src, ncopy, count,
+                             false, ps));
+        return prologue_done(g, count, kOwnPrologueLaunches, 0, ps);
+    }
     for (int i = 0; i < count; ++i) {
         Slot& sl = g.slots[i];
         sl.pst = ps;
@@ -1252,7 +1362,7 @@ int psx_search::prologue_group(GroupSet& g, int count, cudaStream_t ps)
     }
     // baseline removal (timeseries.hpp:282-287, src/kernels.cu:463-479):
     // the device loop of prologue(), row by row
-    const size_t nb = (size_t)reduction_blocks(), pst_ = 2 * nb;
+    const size_t nb = (size_t)reduction_blocks(), pst_ = part_len;
     unsigned* c = g.count;
     PSX_TRY(launch_partials_rows(g.tim, ncopy, N, count, g.part, pst_, c + 4, 16, ps));
     for (int pass = 0; pass < kDeviceBaselinePasses; ++pass) {
@@ -1276,12 +1386,16 @@ int psx_search::prologue_group(GroupSet& g, int count, cudaStream_t ps)
     PSX_TRY(launch_interbin_stats_rows(g.Xp, 2 * Bp, count, B, g.part, pst_, g.sums, 2, g.stat, 8,
                                        (float)N, ps));
     PSX_TRY(g.c2r.exec(g.Xp, g.tim, ps));
-    const int launches = 5 + (ncopy < N ? 1 : 0) + 2 + (bf.empty() ? 0 : 1) + 2;
+    return prologue_done(g, count, 5 + (ncopy < N ? 1 : 0) + 2 + (bf.empty() ? 0 : 1) + 2, 2, ps);
+}
+
+int psx_search::prologue_done(GroupSet& g, int count, int launches, int ffts, cudaStream_t ps)
+{
     for (int i = 0; i < count; ++i) {
         Slot& sl = g.slots[i];
         // the batch's launches and transforms are counted once, on row 0
         sl.launches += i == 0 ? launches : 0;
-        sl.ffts += i == 0 ? 2 : 0;
+        sl.ffts += i == 0 ? ffts : 0;
         // profiling: the batch's span is row 0's prologue, the other rows
         // get an empty one
         if (sl.profiled) {
@@ -1521,6 +1635,7 @@ int psx_search::prep(Slot& s, const float* series, size_t nsamps, bool on_device
 int psx_search::enqueue_trials(Slot& s)
 {
     const int nacc = (int)s.accs.size();
+    if (!s.rec_cap) PSX_TRY(grow_records(s, (size_t)1 << 18));
     PSX_CUDA(cudaStreamWaitEvent(st, s.ready, 0));
     PSX_CUDA(cudaMemcpyAsync(s.d_ktab, s.h_ktab, sizeof(double) * nacc, cudaMemcpyHostToDevice, st));
     PSX_TRY(run_trials(s, nacc));
@@ -1857,8 +1972,6 @@ static int check_config(const psx_search_config* c)
     return PSX_OK;
 }
 
-static int effective_form(const psx_search_config* c);
-
 // Trials per launch group: the configured count (or the default), rounded
 // down to a power of two where cuFFT plans carry the trials (they exist for
 // powers of two only); the two-pass transform takes any count.
@@ -1890,6 +2003,14 @@ static int effective_lanes(const psx_search_config* c)
     return c->lanes ? c->lanes : 1;
 }
 
+// Partial sums of one DM trial: the two halves of the baseline passes, or the
+// own-transform prologue's statistics, one per CTA.
+static size_t part_len_for(const psx_search_config* c)
+{
+    const size_t base = 2 * (size_t)reduction_blocks();
+    return effective_form(c) == 3 ? std::max(base, Fft4Plan::stat_parts(c->fft_size)) : base;
+}
+
 size_t psx_search_footprint(const psx_search_config* c)
 {
     if (check_config(c) != PSX_OK) return 0;
@@ -1904,11 +2025,12 @@ size_t psx_search_footprint(const psx_search_config* c)
     bytes += L * sizeof(float) * Bp * b;              // normalised spectra, per lane
     bytes += 2 * sizeof(int4) * ((size_t)1 << 20);    // two initial record slots
     // cuFFT work areas: about one transform's worth per batched plan size and
-    // lane (none with the two-pass transform, which has twiddle tables
-    // instead), plus the batch-1 plans of the two slots' prologues and the
-    // plain path
-    if (effective_form(c) == 3)
-        bytes += sizeof(float) * 2 * Bp * 6 + sizeof(float2) * Fft4Plan::table_floats2(N);
+    // lane, plus the batch-1 plans of the two slots' prologues and the plain
+    // path (the two-pass transform has twiddle tables instead)
+    const bool own = effective_form(c) == 3;
+    bytes += 2 * sizeof(double2) * part_len_for(c);   // partial sums, per slot
+    if (own)
+        bytes += sizeof(float2) * Fft4Plan::table_floats2(N) + B / 8 + 4;  // and the zap mask
     else
         bytes += sizeof(float) * 2 * Bp * (2 * b * L + 6);
     // two group sets of G rows (made with the instance): series,
@@ -1918,9 +2040,10 @@ size_t psx_search_footprint(const psx_search_config* c)
     if (G >= 2)
         bytes += 2 * G *
                      (sizeof(float) * (N + 2 * Bp) + median_scratch_bytes(B) +
-                      sizeof(int4) * ((size_t)1 << 18) + 2 * sizeof(float) * 2 * Bp) +
+                      sizeof(int4) * ((size_t)1 << 18) + sizeof(double2) * part_len_for(c) +
+                      2 * sizeof(float) * 2 * Bp) +
                  // the spanning schedule's first record buffer per set
-                 (effective_form(c) == 3 ? 2 * sizeof(int4) * ((size_t)1 << 20) : 0);
+                 (own ? 2 * sizeof(int4) * ((size_t)1 << 20) : 0);
     return bytes;
 }
 
@@ -2014,7 +2137,8 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
         return fail(rc);
     const size_t N = s->N, Bp = s->Bp;
     const size_t b = (size_t)s->batch;
-    const int nb = reduction_blocks();
+    s->med_floats = median_scratch_bytes(s->B) / sizeof(float);
+    s->part_len = part_len_for(cfg);
 #define ALLOC(ptr, bytes)                                                        \
     if ((rc = cuda_status(cudaMalloc((void**)&(ptr), (bytes)), "cudaMalloc")) != \
         PSX_OK)                                                                  \
@@ -2037,11 +2161,12 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
         ALLOC(sl.d_tim, sizeof(float) * N);
         ALLOC(sl.d_Xp, sizeof(float) * 2 * Bp);
         ALLOC(sl.d_med, median_scratch_bytes(s->B));
-        ALLOC(sl.d_part, sizeof(double2) * 2 * nb);  // two halves: baseline passes alternate
+        ALLOC(sl.d_part, sizeof(double2) * s->part_len);  // two halves: baseline passes alternate
         ALLOC(sl.d_sums, sizeof(double) * 2);
         ALLOC(sl.d_stat, sizeof(float) * 8);
-        ALLOC(sl.d_mean, sizeof(float) * 2);
+        ALLOC(sl.d_mean, sizeof(float) * 4);
     }
+    if (s->use_f4) ALLOC(s->d_zap, sizeof(unsigned) * ((s->B + 31) / 32));
     if (!s->bf.empty()) {
         ALLOC(s->d_bf, sizeof(float) * s->bf.size());
         ALLOC(s->d_bw, sizeof(float) * s->bw.size());
@@ -2059,11 +2184,13 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
         if ((rc = cuda_status(cudaStreamCreateWithFlags(&sl.pst, cudaStreamNonBlocking),
                               "cudaStreamCreate")) != PSX_OK)
             return fail(rc);
-        sl.r2c = new (std::nothrow) FftPlan;
-        sl.c2r = new (std::nothrow) FftPlan;
-        if (!sl.r2c || !sl.c2r) return fail(PSX_ERR_ALLOC);
-        if ((rc = sl.r2c->create(N, 1, PSX_FFT_R2C, 0, 0)) != PSX_OK) return fail(rc);
-        if ((rc = sl.c2r->create(N, 1, PSX_FFT_C2R, 0, 0)) != PSX_OK) return fail(rc);
+        if (!s->use_f4) {
+            sl.r2c = new (std::nothrow) FftPlan;
+            sl.c2r = new (std::nothrow) FftPlan;
+            if (!sl.r2c || !sl.c2r) return fail(PSX_ERR_ALLOC);
+            if ((rc = sl.r2c->create(N, 1, PSX_FFT_R2C, 0, 0)) != PSX_OK) return fail(rc);
+            if ((rc = sl.c2r->create(N, 1, PSX_FFT_C2R, 0, 0)) != PSX_OK) return fail(rc);
+        }
         if ((rc = s->grow_records(sl, (size_t)1 << 20)) != PSX_OK) return fail(rc);
         if ((rc = s->grow_ktab(sl, 1024)) != PSX_OK) return fail(rc);
     }
@@ -2089,7 +2216,8 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
     }
     if (cudaEventCreateWithFlags(&s->call_start, cudaEventDisableTiming) != cudaSuccess)
         return fail(PSX_ERR_CUDA);
-    if ((rc = s->r2c1.create(N, 1, PSX_FFT_R2C, 0, 0)) != PSX_OK) return fail(rc);
+    if (!s->use_f4 && (rc = s->r2c1.create(N, 1, PSX_FFT_R2C, 0, 0)) != PSX_OK) return fail(rc);
+    if ((rc = s->make_zap_mask()) != PSX_OK) return fail(rc);
     if (s->fft4()) {
         if ((rc = s->f4.create(N)) != PSX_OK) return fail(rc);
     } else if (s->batched()) {
@@ -2225,6 +2353,8 @@ int psx_search_retarget(psx_search* s, const psx_search_config* cfg)
         PSX_CUDA(cudaMemcpy(s->d_bw, s->bw.data(), sizeof(float) * s->bw.size(),
                             cudaMemcpyHostToDevice));
     }
+    PSX_TRY(s->make_zap_mask());
+    PSX_CUDA(cudaStreamSynchronize(s->st));  // the prologues run on streams of their own
     // captured schedules hold the old search ranges by value
     s->drop_graphs();
     return PSX_OK;
@@ -2471,6 +2601,9 @@ int psx_search_debug_tap(psx_search* s, int trial, float* h_tim_dered, float* h_
             set_error("debug_tap: trial %d out of range", trial);
             return PSX_ERR_INVALID;
         }
+        if (sl.grouped)  // its trials ran from the group's list of factors
+            PSX_CUDA(cudaMemcpyAsync(sl.d_ktab, sl.h_ktab, sizeof(double) * accs.size(),
+                                     cudaMemcpyHostToDevice, s->st));
         if (s->fft4())  // what the trials' own pass 1 gathers
             PSX_TRY(s->f4.dump_gather(sl.d_tim, sl.d_ktab + trial, s->d_tr, s->st));
         else

@@ -6,6 +6,30 @@
 
 namespace psx {
 
+// Rows of a batch that lie where their callers have them.
+constexpr int kSeriesRowsMax = 16;
+struct SeriesRows {
+    const float* p[kSeriesRowsMax];
+};
+struct MedianLevels;
+
+// The grouped (and per-DM) prologue on the library's own transform: the means
+// the baseline loop subtracts (at most kBaselineMeans), the median levels of
+// amplitude rows, the statistics of many partials and the mask of the zapped
+// bins.
+constexpr int kBaselineMeans = 3;
+int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* d_parts,
+                          size_t part_stride, unsigned* d_cnt, float* d_means, cudaStream_t s);
+int launch_scrunch_rows(const float* d_amp, size_t stride, int rows, size_t nbins, float* d_scratch,
+                        size_t scratch_stride, cudaStream_t s);
+int launch_finish_stats_rows(const double2* d_partials, int nparts, size_t part_stride, int rows,
+                             size_t count, float* d_stat, size_t stat_stride, float scale,
+                             cudaStream_t s);
+int launch_zap_mask(unsigned* d_mask, const float* d_freqs, const float* d_widths, float bin_width,
+                    size_t nbirdies, size_t nbins, cudaStream_t s);
+// Levels in `scratch` (median_scratch_bytes) with the splice positions.
+MedianLevels median_levels(size_t nbins, double bin_width, float b5, float b25, float* scratch);
+
 double accel_fact(float acc, float tsamp);
 
 // ntrials outputs; trial t uses d_ktab[t] (or k when d_ktab is null) and is

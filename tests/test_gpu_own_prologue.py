@@ -1,0 +1,101 @@
+"""The per-DM prologue on the library's own transform (batched mode, fft_form
+3) against the same instance on cuFFT's (fft_form 1): the dereddened series
+and the statistics, over lengths with every column shape, padded and odd
+series, unaligned and host input, birdies at both ends of the spectrum, means
+that take several baseline passes and more than the device makes.
+
+Tolerance: single-precision transforms of either library are within about
+1e-6 of the result's RMS of the exact ones (forward and back), so the two
+agree within 1e-5 of it; mean and deviation, sums over all bins, within 1e-5
+relative."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _series(n, seed, mean):
+    rng = np.random.default_rng(seed)
+    t = np.arange(n)
+    x = rng.standard_normal(n) + mean + 0.3 * np.sin(t * 0.02) + 2.0 * np.sin(t * 2e-5)
+    return x.astype(np.float32)
+
+
+def _tap(n, series, form, **kw):
+    from peasoup_b200 import search, synth
+    s = search.AccelSearch(search.SearchParams(
+        fft_size=n, tsamp=64e-6, cfreq_hz=synth.CFREQ_HZ, ch_bw_hz=synth.CH_BW_HZ, acc_lo=0.0,
+        acc_hi=0.0, nharmonics=2, min_snr=8.0, batch=2, fft_form=form, **kw))
+    s.search(series)
+    info = s.info()
+    assert info["fft_form"] == form
+    tim, _, _, norm = s.debug_tap(0)
+    s.close()
+    return tim, norm, info
+
+
+# length, samples, mean, birdie edges (Hz; the last above Nyquist)
+BIRDIES = np.array([0.0, 0.05, 60.0, 7812.4, 9000.0], np.float32)
+CASES = [(1 << 19, 1 << 19, 0.0), (1 << 19, 400_001, 100.0), (3 << 17, 3 << 17, 50.0),
+         (3 << 18, (3 << 18) - 1, 1e4), (1 << 21, 2_000_003, 128.0), (1 << 20, (1 << 20) + 77, 5.0),
+         (1 << 26, (1 << 26) - 3, 3.0)]
+
+
+@pytest.mark.parametrize("n,nsamps,mean", CASES)
+def test_matches_cufft_prologue(cuda, n, nsamps, mean):
+    torch = cuda
+    x = _series(nsamps, n % 1009 + nsamps % 7, mean)
+    kw = dict(birdie_freqs=BIRDIES, birdie_widths=np.full(len(BIRDIES), 0.3, np.float32))
+    tim, norm, info = _tap(n, x, 3, **kw)
+    want, wnorm, winfo = _tap(n, x, 1, **kw)
+    assert info["baseline_passes"] == winfo["baseline_passes"]
+    assert np.max(np.abs(tim - want)) <= 1e-5 * np.sqrt(np.mean(want.astype(np.float64) ** 2))
+    assert np.all(np.abs(norm - wnorm) <= 1e-5 * np.abs(wnorm))
+    if n > 1 << 22:
+        return
+    # device series, aligned and one float past it: the same bits
+    buf = torch.zeros(nsamps + 1, device="cuda")
+    for shift in (0, 1):
+        d = buf[shift:shift + nsamps]
+        d.copy_(torch.from_numpy(x))
+        got, gnorm, _ = _tap(n, d, 3, **kw)
+        assert np.array_equal(got, tim) and np.array_equal(gnorm, norm)
+
+
+def test_more_baseline_passes_than_the_device_makes(cuda):
+    """A mean of 1e12 leaves residual means far above the threshold after
+    each float subtraction: the host's loop takes over."""
+    n = 1 << 19
+    x = (_series(n, 3, 0.0) * 1e9 + np.float32(1e12)).astype(np.float32)
+    tim, norm, info = _tap(n, x, 3)
+    want, wnorm, winfo = _tap(n, x, 1)
+    assert np.max(np.abs(tim - want)) <= 1e-5 * np.sqrt(np.mean(want.astype(np.float64) ** 2))
+    assert np.all(np.abs(norm - wnorm) <= 1e-5 * np.abs(wnorm))
+
+
+def test_retarget_replaces_the_birdies(cuda):
+    """A retargeted instance zaps the new list, or none."""
+    import ctypes as C
+    from peasoup_b200 import search, synth
+    from peasoup_b200._lib import check, load
+    n = 1 << 19
+    x = _series(n, 9, 10.0)
+    base = dict(fft_size=n, tsamp=64e-6, cfreq_hz=synth.CFREQ_HZ, ch_bw_hz=synth.CH_BW_HZ,
+                nharmonics=2, min_snr=8.0, batch=2)
+    lists = [np.zeros(0, np.float32), np.array([50.0, 160.0], np.float32),
+             np.array([700.0], np.float32), np.zeros(0, np.float32)]
+    s = search.AccelSearch(search.SearchParams(**base))
+    for f in lists:
+        p = search.SearchParams(birdie_freqs=f, birdie_widths=np.full(len(f), 2.0, np.float32),
+                                **base)
+        cfg, keep = p.to_c()
+        check(load().psx_search_retarget(s._handle, C.byref(cfg)), "retarget")
+        s.search(x)
+        got = s.debug_tap(0)
+        fresh = search.AccelSearch(p)
+        fresh.search(x)
+        want = fresh.debug_tap(0)
+        fresh.close()
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[3], want[3])
+        del keep
+    s.close()
