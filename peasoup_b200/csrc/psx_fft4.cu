@@ -651,8 +651,12 @@ __device__ __forceinline__ float2 deredden(float2 x, unsigned j, const MidArgs& 
     if (j < 5) {
         x = make_float2(0.f, 0.f);
     } else {
-        const cuComplex q = cuCdivf(make_cuComplex(x.x, x.y), make_cuComplex(median_at(a.lev, j), 0.f));
-        x = make_float2(q.x, q.y);
+        // X / m as X (1 / m): one division per bin where the reference's
+        // complex division makes two; a median without a finite reciprocal
+        // (0, infinite, subnormal) gives NaN, as it does there
+        const float m = median_at(a.lev, j), r = 1.0f / m, t = m * r;
+        const float w = t > 0.5f && t < 2.0f ? r : __int_as_float(0x7fffffff);
+        x = make_float2(x.x * w, x.y * w);
     }
     if (a.zap && (__ldg(a.zap + (j >> 5)) >> (j & 31) & 1u)) x = make_float2(1.f, 0.f);
     return x;

@@ -311,25 +311,45 @@ __global__ void __launch_bounds__(256) k_scrunch3(const float* __restrict__ X,
     m5 += (size_t)blockIdx.y * m_stride;
     m25 += (size_t)blockIdx.y * m_stride;
     m125 += (size_t)blockIdx.y * m_stride;
+    constexpr int kStep = kScrGroups * 125;  // bins of a CTA step, a multiple of 4
+    __shared__ __align__(16) float buf[kStep];
     __shared__ float s5[kScrGroups * 25];
     __shared__ float s25[kScrGroups * 5];
+    const bool vec = (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
     const size_t ngroups = (n5 + 24) / 25;  // groups holding any 5-level value
     for (size_t g0 = (size_t)blockIdx.x * kScrGroups; g0 < ngroups;
          g0 += (size_t)gridDim.x * kScrGroups) {
+        // the step's bins through shared memory (reading five neighbours per
+        // thread straight from X touches every line five times)
+        const size_t e0 = g0 * 125;
+        const int cnt = (int)min((size_t)kStep, 5 * n5 - e0);
+        int done = 0;
+        if (vec) {
+            if constexpr (AMP) {
+                done = cnt & ~1;
+                const float4* x4 = reinterpret_cast<const float4*>(X + 2 * e0);
+#pragma unroll 4
+                for (int i = threadIdx.x; i < cnt / 2; i += blockDim.x) {
+                    const float4 z = x4[i];
+                    reinterpret_cast<float2*>(buf)[i] =
+                        make_float2(amplitude(z.x, z.y), amplitude(z.z, z.w));
+                }
+            } else {
+                done = cnt & ~3;
+                const float4* x4 = reinterpret_cast<const float4*>(X + e0);
+#pragma unroll 2
+                for (int i = threadIdx.x; i < cnt / 4; i += blockDim.x)
+                    reinterpret_cast<float4*>(buf)[i] = x4[i];
+            }
+        }
+        for (int i = done + threadIdx.x; i < cnt; i += blockDim.x)
+            buf[i] = AMP ? amplitude(X[2 * (e0 + i)], X[2 * (e0 + i) + 1]) : X[e0 + i];
+        __syncthreads();
         for (int i = threadIdx.x; i < kScrGroups * 25; i += blockDim.x) {
             const size_t j = g0 * 25 + i;  // 5-level index
             float v = 0.f;
             if (j < n5) {
-                float a[5];
-#pragma unroll
-                for (int t = 0; t < 5; ++t) {
-                    if constexpr (AMP) {
-                        const float2 z = reinterpret_cast<const float2*>(X)[5 * j + t];
-                        a[t] = amplitude(z.x, z.y);
-                    } else {
-                        a[t] = X[5 * j + t];
-                    }
-                }
+                const float* a = buf + 5 * i;
                 v = med5(a[0], a[1], a[2], a[3], a[4]);
                 m5[j] = v;
             }
@@ -815,17 +835,19 @@ __global__ void __launch_bounds__(kVecThreads) k_baseline_means(
 }
 static_assert(kBaselineMeans == 3, "the third mean needs no sum after it");
 
-// The same loop for short series in one launch: a cluster of kMeanCtas CTAs
-// per row sums, exchanges its partial sums through distributed shared memory
-// and goes round again while the mean is above the threshold.  Eight SMs read
-// a row slower than the whole device, so it is taken up to 2^20 samples and,
-// where the rows of a group read side by side, 2^21.  A call of 1, 3, 12 and
-// 48 DM trials with two passes each on B200 (us, four launches against one):
-// 2^19: 172/161, 339/303, 516/383, 1220/750; 2^20: 171/169, 360/332, 622/512,
-// 1818/1359; 2^21: 179/189, 399/427, 895/812, 2839/2513.
-constexpr int kMeanCtas = 8;
+// The same loop in one launch: a cluster of CTAs per row sums, exchanges its
+// partial sums through distributed shared memory and goes round again while
+// the mean is above the threshold.  Clusters of 16 (8 for more than 8 rows,
+// where 16 would take two waves); a few SMs read a long row slower than the
+// whole device, so fewer than 4 rows take it up to 2^21 samples, 4 and more
+// up to 2^23.  A call of 1, 12 and 48 DM trials on B200 (us; four launches,
+// one with clusters of 8, of 16): 2^19: 171/162/164, 513/397/379,
+// 1225/744/793; 2^20: 173/170/164, 614/508/494, 1797/1370/1346; 2^21:
+// 178/187/176, 887/808/777, 2828/2497/2416; 2^22: 231/300/258,
+// 1428/1435/1356, 5093/5001/4872.
 constexpr int kMeanThreads = 1024;
-constexpr size_t kMeanMaxSamples = (size_t)1 << 20;  // twice that from 4 rows on
+inline unsigned mean_ctas(int rows) { return rows > 8 ? 8u : 16u; }
+inline size_t mean_max_samples(int rows) { return (size_t)1 << (rows < 4 ? 21 : 23); }
 
 __global__ void __launch_bounds__(kMeanThreads) k_baseline_means_cluster(
     SeriesRows rows, size_t n, unsigned* __restrict__ cnt, float* __restrict__ means)
@@ -852,7 +874,7 @@ __global__ void __launch_bounds__(kMeanThreads) k_baseline_means_cluster(
         }
         cl.sync();
         double total = 0.0;
-        for (int c = 0; c < kMeanCtas; ++c) total += *cl.map_shared_rank(&part[p], c);
+        for (unsigned c = 0; c < cl.num_blocks(); ++c) total += *cl.map_shared_rank(&part[p], c);
         m[p] = __fdiv_rn((float)total, (float)(double)n);
         more = fabsf(m[p]) > 5e-7 * (double)n;
         pass = p + 1;
@@ -866,22 +888,47 @@ __global__ void __launch_bounds__(kMeanThreads) k_baseline_means_cluster(
     cl.sync();  // no CTA leaves while another reads its partial sums
 }
 
+// Whether this device runs such clusters (asked once per device and size:
+// 16 is above the portable 8).
+static bool mean_clusters_fit(const cudaLaunchConfig_t* cfg, unsigned ctas)
+{
+    static std::mutex mu;
+    static int table[64][2] = {};  // 1 yes, 2 no
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    std::lock_guard<std::mutex> lock(mu);
+    int& known = table[dev][ctas > 8];
+    if (!known) {
+        int n = 0;
+        const bool ok = cudaFuncSetAttribute(k_baseline_means_cluster,
+                                             cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                             1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, k_baseline_means_cluster, cfg) ==
+                            cudaSuccess && n > 0;
+        (void)cudaGetLastError();
+        known = ok ? 1 : 2;
+    }
+    return known == 1;
+}
+
 int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* d_parts,
                           size_t part_stride, unsigned* d_cnt, float* d_means, cudaStream_t s)
 {
-    if (n <= kMeanMaxSamples * (nrows >= 4 ? 2 : 1)) {
+    if (n <= mean_max_samples(nrows)) {
+        const unsigned ctas = mean_ctas(nrows);
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kMeanCtas, nrows);
+        cfg.gridDim = dim3(ctas, nrows);
         cfg.blockDim = dim3(kMeanThreads);
         cfg.stream = s;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim = {kMeanCtas, 1, 1};
+        at[0].val.clusterDim = {ctas, 1, 1};
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        return cuda_status(cudaLaunchKernelEx(&cfg, k_baseline_means_cluster, rows, n, d_cnt,
-                                              d_means),
-                           "baseline mean kernel");
+        if (mean_clusters_fit(&cfg, ctas))
+            return cuda_status(cudaLaunchKernelEx(&cfg, k_baseline_means_cluster, rows, n, d_cnt,
+                                                  d_means),
+                               "baseline mean kernel");
     }
     const int nb = reduction_blocks();
     const dim3 grid(nb, nrows);
