@@ -43,80 +43,105 @@ constexpr int kDdTile8 = 1024; // output samples per CTA, 1..8-bit samples
 constexpr int kDdTile16 = 512; // output samples per CTA, 16-bit samples
 inline int dd_tile(int elem) { return elem == 1 ? kDdTile8 : kDdTile16; }
 constexpr int kUpRows = 64;    // unpack tile: samples
-constexpr int kUpChans = 64;   // unpack tile: channels
 constexpr float kDmConst = 4.15e3f;
 
 template <int NBITS> struct Sample { using T = uint8_t; };
 template <> struct Sample<16> { using T = uint16_t; };
 
-// Channel c of a SIGPROC row: below 8 bits the first channel sits in the
-// least significant bits of its byte; 16-bit samples are little-endian.
-template <int NBITS>
-__device__ __forceinline__ unsigned sigproc_value(const uint8_t* row, int c)
-{
-    if constexpr (NBITS == 8) {
-        return row[c];
-    } else if constexpr (NBITS == 16) {
-        return (unsigned)row[2 * c] | ((unsigned)row[2 * c + 1] << 8);
-    } else {
-        unsigned bit = (unsigned)c * NBITS;
-        return (row[bit >> 3] >> (bit & 7)) & ((1u << NBITS) - 1u);
-    }
-}
-
+// A SIGPROC row: below 8 bits the first channel sits in the least significant
+// bits of its byte; 16-bit samples are little-endian.
+//
 // Rows [r0, r0 + nrows) of the packed input (rows[0] is row r0) become
 // columns of cm; columns [r0 + nrows, r0 + ncols) are zeroed.  One CTA per
-// 64 samples x 64 channels, transposed through shared memory; every store
-// is 16 bytes.  r0 and ncols' rounding to 64 stay inside the pitch.
+// 64 samples x the channels of 64 bytes of a row (64 channels at 16 bits);
+// every store is 16 bytes.  r0 and ncols' rounding to 64 stay inside the
+// pitch.
+//
+// A thread takes one 32-bit word of four consecutive rows, splits it into
+// bytes of one channel class each (1, 2 or 4 bits: shift and mask) and turns
+// 4 channels x 4 samples around with eight byte permutes, so the tile is
+// written a word (four samples of a channel) at a time.  The words of a
+// channel are XOR-ed by the row word's index, so that neither side's accesses
+// meet in a bank more than twice.  Where rows do not start on 4-byte
+// boundaries (vec 0) the words are put together from bytes.  (Writing the
+// tile a byte at a time, 64 samples x 64 channels, took 146 us for 2^22
+// samples x 64 channels of 8 bits on B200 and 234 for 400,000 x 1024 of 4
+// bits; this takes 121 and 136, 4.5 TB/s.)
+template <int NBITS>
+struct UnpackTile {
+    static constexpr int kElem = NBITS == 16 ? 2 : 1;
+    static constexpr int kWords = NBITS == 16 ? 32 : 16;         // of a row's segment
+    static constexpr int kPer = 32 / NBITS;                      // channels of a word
+    static constexpr int kChans = kWords * kPer;
+    static constexpr int kChanWords = kUpRows * kElem / 4;       // of a channel's samples
+};
+
 template <int NBITS>
 __global__ void __launch_bounds__(256) k_unpack_chanmajor(
     const uint8_t* __restrict__ rows, size_t row_bytes, size_t nrows, size_t r0, size_t ncols,
     int nchans, typename Sample<NBITS>::T* __restrict__ cm, size_t pitch, int vec)
 {
-    using T = typename Sample<NBITS>::T;
-    constexpr int kPad = 16 / (int)sizeof(T) / 4;  // row stride 68 B (u8) or 132 B (u16)
-    constexpr int kStride = kUpRows + kPad;
-    __shared__ __align__(16) T tile[kUpChans * kStride];
+    using U = UnpackTile<NBITS>;
+    __shared__ __align__(16) uint32_t tile[U::kChans * U::kChanWords];
     const size_t col0 = (size_t)blockIdx.x * kUpRows;
-    const int c0 = blockIdx.y * kUpChans;
-    if (vec) {
-        // 32-bit loads: a row's 64 channels are 2*NBITS words (rows 4-byte aligned)
-        constexpr int kWords = 2 * NBITS;
-        constexpr int kPerWord = 32 / NBITS;
-        const size_t seg = (size_t)c0 * NBITS / 8;
-        for (int i = threadIdx.x; i < kUpRows * kWords; i += blockDim.x) {
-            int r = i / kWords, q = i % kWords;
-            size_t rr = col0 + r;
-            size_t byte = seg + 4 * (size_t)q;
-            uint32_t w = 0;
-            if (rr < nrows && byte < row_bytes)
-                w = *reinterpret_cast<const uint32_t*>(rows + rr * row_bytes + byte);
+    const int c0 = blockIdx.y * U::kChans;
+    const size_t seg = (size_t)c0 * NBITS / 8;  // first byte of the CTA's part of a row
+    constexpr int kRows = NBITS == 16 ? 2 : 4;  // rows of a thread's step: one word of samples
+    const int words = (int)min((size_t)U::kWords, (row_bytes - seg + 3) / 4);
+    for (int i = threadIdx.x; i < (kUpRows / kRows) * words; i += blockDim.x) {
+        const int q = i % words, g = i / words;  // row word, group of rows
+        const size_t byte = seg + 4 * (size_t)q;
+        uint32_t w[kRows];
 #pragma unroll
-            for (int k = 0; k < kPerWord; ++k) {
-                unsigned v;
-                if constexpr (NBITS == 16) v = (w >> (16 * k)) & 0xffffu;
-                else v = (w >> (k * NBITS)) & ((1u << NBITS) - 1u);
-                tile[(q * kPerWord + k) * kStride + r] = (T)v;
+        for (int r = 0; r < kRows; ++r) {
+            const size_t rr = col0 + kRows * g + r;
+            w[r] = 0;
+            if (rr < nrows && byte < row_bytes) {
+                const uint8_t* p = rows + rr * row_bytes + byte;
+                if (vec) {
+                    w[r] = *reinterpret_cast<const uint32_t*>(p);
+                } else {
+                    for (int k = 0; k < 4; ++k)
+                        if (byte + k < row_bytes) w[r] |= (uint32_t)p[k] << (8 * k);
+                }
             }
         }
-    } else {
-        for (int i = threadIdx.x; i < kUpRows * kUpChans; i += blockDim.x) {
-            int r = i / kUpChans, c = i % kUpChans;
-            size_t rr = col0 + r;
-            unsigned v = 0;
-            if (rr < nrows && c0 + c < nchans) v = sigproc_value<NBITS>(rows + rr * row_bytes, c0 + c);
-            tile[c * kStride + r] = (T)v;
+        uint32_t* t = tile + (q * U::kPer) * U::kChanWords;
+        const int at = g ^ (q & (U::kChanWords - 1));
+        if constexpr (NBITS == 16) {
+            t[at] = __byte_perm(w[0], w[1], 0x5410);
+            t[U::kChanWords + at] = __byte_perm(w[0], w[1], 0x7632);
+        } else {
+            // class k: channels k, k + kPer/4, ... of the word, one per byte
+            constexpr int kClasses = U::kPer / 4;
+            constexpr uint32_t kMask = 0x01010101u * ((1u << NBITS) - 1u);
+#pragma unroll
+            for (int k = 0; k < kClasses; ++k) {
+                uint32_t b[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) b[r] = NBITS == 8 ? w[r] : (w[r] >> (NBITS * k)) & kMask;
+                const uint32_t l0 = __byte_perm(b[0], b[1], 0x5140), l1 = __byte_perm(b[2], b[3], 0x5140);
+                const uint32_t h0 = __byte_perm(b[0], b[1], 0x7362), h1 = __byte_perm(b[2], b[3], 0x7362);
+                // byte j of a word holds its channel j * kClasses + k
+                t[(0 * kClasses + k) * U::kChanWords + at] = __byte_perm(l0, l1, 0x5410);
+                t[(1 * kClasses + k) * U::kChanWords + at] = __byte_perm(l0, l1, 0x7632);
+                t[(2 * kClasses + k) * U::kChanWords + at] = __byte_perm(h0, h1, 0x5410);
+                t[(3 * kClasses + k) * U::kChanWords + at] = __byte_perm(h0, h1, 0x7632);
+            }
         }
     }
     __syncthreads();
-    constexpr int kVec = 16 / (int)sizeof(T);           // samples per 16-byte store
-    constexpr int kPer = kUpRows / kVec;                // stores per channel
-    for (int i = threadIdx.x; i < kUpChans * kPer; i += blockDim.x) {
-        int c = i / kPer, q = i % kPer;
-        if (c0 + c >= nchans || col0 + (size_t)q * kVec >= ncols) continue;
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(tile + c * kStride + q * kVec);
-        uint4 w = make_uint4(src[0], src[1], src[2], src[3]);
-        *reinterpret_cast<uint4*>(cm + (size_t)(c0 + c) * pitch + r0 + col0 + (size_t)q * kVec) = w;
+    constexpr int kPer16 = U::kChanWords / 4;  // 16-byte stores per channel
+    constexpr int kVec = 16 / U::kElem;        // samples of one
+    const int chans = min(U::kChans, nchans - c0);
+    for (int i = threadIdx.x; i < chans * kPer16; i += blockDim.x) {
+        const int c = i / kPer16, v = i % kPer16, x = (c / U::kPer) & (U::kChanWords - 1);
+        if (col0 + (size_t)v * kVec >= ncols) continue;
+        // words 4 v + 0..3 lie at (4 v + j) ^ x: one 16-byte group, its words XOR-ed
+        uint4 w = *reinterpret_cast<const uint4*>(tile + c * U::kChanWords + ((4 * v) ^ (x & ~3)));
+        if (x & 1) w = make_uint4(w.y, w.x, w.w, w.z);
+        if (x & 2) w = make_uint4(w.z, w.w, w.x, w.y);
+        *reinterpret_cast<uint4*>(cm + (size_t)(c0 + c) * pitch + r0 + col0 + (size_t)v * kVec) = w;
     }
 }
 
@@ -1139,7 +1164,7 @@ int launch_unpack(const uint8_t* rows, size_t nrows, size_t r0, size_t ncols, ps
     using T = typename Sample<NBITS>::T;
     size_t row_bytes = p->nchans * NBITS / 8;
     dim3 grid((unsigned)((ncols + kUpRows - 1) / kUpRows),
-              (unsigned)((p->nchans + kUpChans - 1) / kUpChans));
+              (unsigned)((p->nchans + UnpackTile<NBITS>::kChans - 1) / UnpackTile<NBITS>::kChans));
     // word loads when every row starts 4-byte aligned; channels past the
     // last whole word of a row then read as zero and are never stored
     const int vec = (row_bytes % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 3) == 0) ? 1 : 0;

@@ -158,6 +158,30 @@ def test_shared_partial_sums_equal_oracle(psx, cuda, oracle, nchans, nbits, ndm,
         psx.psx_dedisp_destroy(h)
 
 
+# The transposition of rows into channels: rows that are not whole words
+# (every load from bytes), fewer channels than a CTA's segment holds and a few
+# more than one, sample counts around the 64-row tile
+@pytest.mark.parametrize("nchans,nbits", [(8, 1), (520, 1), (4, 2), (260, 2), (6, 4), (130, 4),
+                                          (1, 8), (3, 8), (65, 8), (1, 16), (65, 16), (66, 16)])
+@pytest.mark.parametrize("extra", [1, 63, 65])
+def test_unpack_edges_equal_oracle(psx, cuda, oracle, nchans, nbits, extra):
+    torch = cuda
+    tsamp, fch1, foff = 64e-6, 1500.0, -100.0 / nchans
+    h = _plan(psx, nchans, tsamp, fch1, foff)
+    try:
+        dms = np.array([0.0, 7.5], np.float32)
+        assert psx.psx_dedisp_set_dm_list(h, dms.ctypes.data, dms.size) == 0
+        delays = oracle.delay_table(nchans, tsamp, fch1, foff)
+        ns = oracle.max_delay(delays, dms) + extra
+        v = np.random.default_rng(nchans).integers(0, 1 << nbits, (ns, nchans), dtype=np.uint32)
+        rows = sigproc.pack_samples(v, nbits)
+        want = oracle.dedisperse(rows, nbits, nchans, delays, dms, raw=True)
+        for host in (False, True):
+            assert np.array_equal(_run(psx, torch, h, rows, nbits, 2, extra, True, host=host), want)
+    finally:
+        psx.psx_dedisp_destroy(h)
+
+
 def test_dedisperser_class_on_a_file(psx, cuda, oracle, tmp_path):
     from peasoup_b200.dedisperse import Dedisperser
     spec = synth.FilterbankSpec(nsamps=20000, tsamp=64e-6, nbits=4, dm=50.0,
