@@ -425,8 +425,9 @@ typedef struct {
                                   3 = the library's own two-pass transform of
                                   the interleaved pairs with the resample
                                   gather in its first pass, then the unpack
-                                  kernel (fft_size 2^19 .. 2^25 or
-                                  3 * 2^17 .. 3 * 2^23) */
+                                  kernel, also for the per-DM prologue
+                                  (fft_size 2^19 .. 2^27 or 3 * 2^17 ..
+                                  3 * 2^23; by default 2^17 and 2^18 too) */
     int group_dms;             /* batched: DM trials of a psx_search_block
                                   call whose per-DM prologues (baseline
                                   removal through the inverse transform) run

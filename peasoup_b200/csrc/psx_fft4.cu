@@ -178,7 +178,7 @@ template <int R>
 struct ColShape {
     static constexpr int W = R >= 2048 ? 4 : 8;
     static constexpr int J = R / 16;
-    static constexpr int TPC = J < 64 ? 64 : J;
+    static constexpr int TPC = R == 256 ? 16 : J < 64 ? 64 : J;
     static constexpr int R3 = R / 256;
     static constexpr int U = 256 / TPC;
     static constexpr int THREADS = W * TPC;
@@ -196,7 +196,8 @@ __device__ __forceinline__ unsigned swz_a(unsigned e)
     return e ^ ((e >> 4) & (16u / W - 1u));
 }
 
-// Column length R = 768 (stages of radix 16, 16, 3, for transform lengths
+// Column length R = 256 (stages of radix 16, 16; transforms of 2^17 and 2^18
+// points), 768 (stages of radix 16, 16, 3, for transform lengths
 // 3 * 2^k), 1024 (16, 16, 4), 2048 (16, 16, 8) or 4096 (16, 16, 16).
 template <int R, int KIND>
 __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THREADS)
@@ -208,8 +209,9 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
     constexpr bool TRIAL = KIND == kColGather || KIND == kColDump;
     if constexpr (TRIAL)
         if (a.trow) x += (size_t)a.trow[blockIdx.y] * a.xpitch;
-    static_assert(R == 768 || R == 1024 || R == 2048 || R == 4096, "column length");
-    static_assert((S::THREADS == 512 || S::THREADS == 1024) && S::U * S::R3 <= 16,
+    static_assert(R == 256 || R == 768 || R == 1024 || R == 2048 || R == 4096, "column length");
+    static_assert((S::THREADS == 128 || S::THREADS == 512 || S::THREADS == 1024) &&
+                      S::U * S::R3 <= 16,
                   "column shape");
     constexpr int W = S::W, J = S::J, TPC = S::TPC, R3 = S::R3, U = S::U;
     extern __shared__ float2 sm_a[];
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
     // so that their L2 latency passes under the three stages; for R = 4096
     // (one stage-3 butterfly per thread, fifteen entries W_M^(TPC c U q))
     // those are loaded where they are used instead.
-    constexpr bool EARLY = U > 1 && KIND != kColInverse;
+    constexpr bool EARLY = U > 1 && R3 > 1 && KIND != kColInverse;
     const float2 wt = __ldg(tab + offQ + (size_t)t * C + c);
     float2 pu[U], pq[R3];
     if constexpr (EARLY) {
@@ -315,10 +317,38 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
             v[q] = cmul(v[q], !qh ? lo[ql] : !ql ? hi[qh] : cmul(lo[ql], hi[qh]));
         }
         dft<16>(v);
-        const unsigned base2 = (t >> 4) * 256 + (t & 15);
+        if constexpr (R3 > 1) {
+            const unsigned base2 = (t >> 4) * 256 + (t & 15);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) sm_a[swz_a<W>(base2 + 16 * q) * W + col] = v[q];
+            for (int q = 0; q < 16; ++q) sm_a[swz_a<W>(base2 + 16 * q) * W + col] = v[q];
+        }
     }
+    float2* yo = y + (size_t)blockIdx.y * ypitch;
+    if constexpr (R3 == 1) {
+        // R = 256: v[q] is row k1 = t + 16 q already; four-step twiddle
+        // W_M^(c t) P^q, P = W_M^(16 c), as the products of P^(q mod 4) and
+        // P^(4 (q div 4)) in turn
+        if constexpr (KIND != kColInverse) {
+            const float2* tp = tab + offP + c;
+#pragma unroll
+            for (int l = 0; l < 4; ++l) {
+                const float2 w = l ? cmul(wt, __ldg(tp + l * (size_t)C)) : wt;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) v[4 * h + l] = cmul(v[4 * h + l], w);
+            }
+#pragma unroll
+            for (int h = 1; h < 4; ++h) {
+                const float2 w = __ldg(tp + 4 * h * (size_t)C);
+#pragma unroll
+                for (int l = 0; l < 4; ++l) v[4 * h + l] = cmul(v[4 * h + l], w);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+            yo[(size_t)(t + 16 * q) * C + c] =
+                KIND == kColInverse ? make_float2(v[q].x, -v[q].y) : v[q];
+        return;
+    } else {
     __syncthreads();
     // stage 3 (radix R3, span 256): butterflies j = t + TPC u, in[j + 256 q]
     // * W_R^(j q), out[j + 256 q] = row k1 = t + TPC (u + U q)
@@ -359,7 +389,6 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
     // W_M^(c t) * W_M^(TPC c U q) * W_M^(TPC c u), from the entries of
     // W_M^(c t), W_M^(TPC c) and W_M^(TPC c U) instead of U R3 (R = 4096:
     // W_M^(c t) and the fifteen W_M^(TPC c q))
-    float2* yo = y + (size_t)blockIdx.y * ypitch;
     if constexpr (KIND == kColInverse) {
 #pragma unroll
         for (int q = 0; q < R3; ++q)
@@ -367,18 +396,19 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
             for (int u = 0; u < U; ++u)
                 yo[(size_t)(t + TPC * (u + U * q)) * C + c] =
                     make_float2(v[R3 * u + q].x, -v[R3 * u + q].y);
-        return;
-    }
+    } else {
 #pragma unroll
-    for (int q = 0; q < R3; ++q) {
-        const float2 wq =
-            q ? cmul(wt, EARLY ? pq[q] : __ldg(tab + offP + (size_t)(U * q) * C + c)) : wt;
+        for (int q = 0; q < R3; ++q) {
+            const float2 wq =
+                q ? cmul(wt, EARLY ? pq[q] : __ldg(tab + offP + (size_t)(U * q) * C + c)) : wt;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const unsigned w = u + U * q;
-            const float2 tw = u ? cmul(wq, pu[u]) : wq;
-            yo[(size_t)(t + TPC * w) * C + c] = cmul(v[R3 * u + q], tw);
+            for (int u = 0; u < U; ++u) {
+                const unsigned w = u + U * q;
+                const float2 tw = u ? cmul(wq, pu[u]) : wq;
+                yo[(size_t)(t + TPC * w) * C + c] = cmul(v[R3 * u + q], tw);
+            }
         }
+    }
     }
 }
 
@@ -846,6 +876,7 @@ int Fft4Plan::launch_cols(const float* x, int rows, float2* y, size_t ypitch, co
             x, (unsigned long long)n, d_tab, offA2, offA3, offQ, offP, C, y, ypitch, a);
     };
     switch (R) {
+    case 256: go(k_fft4_cols<256, KIND>, ColShape<256>{}); break;
     case 768: go(k_fft4_cols<768, KIND>, ColShape<768>{}); break;
     case 1024: go(k_fft4_cols<1024, KIND>, ColShape<1024>{}); break;
     case 2048: go(k_fft4_cols<2048, KIND>, ColShape<2048>{}); break;
@@ -857,22 +888,24 @@ int Fft4Plan::launch_cols(const float* x, int rows, float2* y, size_t ypitch, co
 bool Fft4Plan::supported(size_t n)
 {
     auto pow2 = [](size_t v) { return v && (v & (v - 1)) == 0; };
-    if (pow2(n)) return n >= (size_t(1) << 19) && n <= (size_t(1) << 27);
+    if (pow2(n)) return n >= (size_t(1) << 17) && n <= (size_t(1) << 27);
     return n % 3 == 0 && pow2(n / 3) && n / 3 >= (size_t(1) << 17) && n / 3 <= (size_t(1) << 23);
 }
 
-// Rows of the four-step split: 768 for 3 * 2^k, else 1024 up to M = 2^24
+// Rows of the four-step split: 256 up to N = 2^18 (a row of pass 2 is at
+// least 256 points), 768 for 3 * 2^k, else 1024 up to M = 2^24
 // (N = 2^25), 2048 at M = 2^25 and 4096 at M = 2^26, so that the row length
 // C = M / R never exceeds 2^14 (one CTA's shared memory).
 unsigned Fft4Plan::rows_for(size_t n)
 {
     const size_t m = n / 2;
     if (n % 3 == 0) return 768u;
+    if (n < (size_t(1) << 19)) return 256u;
     return m <= (size_t(1) << 24) ? 1024u : m == (size_t(1) << 25) ? 2048u : 4096u;
 }
 
 // Threads per column of pass 1 (the range of t in the four-step twiddle).
-static unsigned cols_tpc(unsigned r) { return r / 16 < 64 ? 64u : r / 16; }
+static unsigned cols_tpc(unsigned r) { return r == 256 ? 16u : r / 16 < 64 ? 64u : r / 16; }
 
 size_t Fft4Plan::table_floats2(size_t n)
 {
@@ -900,7 +933,7 @@ int Fft4Plan::create(size_t n_)
 {
     destroy();
     if (!supported(n_)) {
-        set_error("fft4: unsupported length %zu (2^19 .. 2^27 or 3 * 2^17 .. 3 * 2^23)", n_);
+        set_error("fft4: unsupported length %zu (2^17 .. 2^27 or 3 * 2^17 .. 3 * 2^23)", n_);
         return PSX_ERR_INVALID;
     }
     const unsigned long long M = n_ / 2;
@@ -963,6 +996,7 @@ int Fft4Plan::create(size_t n_)
     R = Rn;
     logc = lc;
     switch (R) {
+    case 256: PSX_TRY(configure_cols<256>()); break;
     case 768: PSX_TRY(configure_cols<768>()); break;
     case 1024: PSX_TRY(configure_cols<1024>()); break;
     case 2048: PSX_TRY(configure_cols<2048>()); break;
@@ -1078,6 +1112,7 @@ int Fft4Plan::form(const float2* zt, size_t zpitch, int ntrials, float* p, size_
     const float2* rv = d_tab + offRv;
     const float2* rk = d_tab + offRk;
     switch (R) {
+    case 256: k_unpack_form_norm_t<256, false><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
     case 768: k_unpack_form_norm_t<768, false><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
     case 1024: k_unpack_form_norm_t<1024, false><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
     case 2048: k_unpack_form_norm_t<2048, false><<<grid, 256, 0, s>>>(zt, zpitch, C, p, ppitch, rv, rk, stat, trow); break;
@@ -1097,6 +1132,7 @@ int Fft4Plan::amplitudes(const float2* zt, size_t zpitch, int rows, float* amp, 
     const float2* rv = d_tab + offRv;
     const float2* rk = d_tab + offRk;
     switch (R) {
+    case 256: k_unpack_form_norm_t<256, true><<<grid, 256, 0, s>>>(zt, zpitch, C, amp, apitch, rv, rk, nullptr, nullptr); break;
     case 768: k_unpack_form_norm_t<768, true><<<grid, 256, 0, s>>>(zt, zpitch, C, amp, apitch, rv, rk, nullptr, nullptr); break;
     case 1024: k_unpack_form_norm_t<1024, true><<<grid, 256, 0, s>>>(zt, zpitch, C, amp, apitch, rv, rk, nullptr, nullptr); break;
     case 2048: k_unpack_form_norm_t<2048, true><<<grid, 256, 0, s>>>(zt, zpitch, C, amp, apitch, rv, rk, nullptr, nullptr); break;
@@ -1119,6 +1155,7 @@ int Fft4Plan::deredden(const float2* zt, size_t zpitch, int rows, float2* zo, si
     const float2* rk = d_tab + offRk;
     const MidArgs a{lev, m_stride, zap, parts, part_stride};
     switch (R) {
+    case 256: k_deredden_t<256><<<grid, 256, 0, s>>>(zt, zpitch, C, zo, opitch, rv, rk, a); break;
     case 768: k_deredden_t<768><<<grid, 256, 0, s>>>(zt, zpitch, C, zo, opitch, rv, rk, a); break;
     case 1024: k_deredden_t<1024><<<grid, 256, 0, s>>>(zt, zpitch, C, zo, opitch, rv, rk, a); break;
     case 2048: k_deredden_t<2048><<<grid, 256, 0, s>>>(zt, zpitch, C, zo, opitch, rv, rk, a); break;

@@ -1,7 +1,7 @@
 // psx_fft4.cuh -- the batched search's own forward transform: for each
 // acceleration trial, the complex DFT of length M = N/2 of the resampled
 // series read as interleaved pairs, z[m] = x'[2m] + i x'[2m+1], in two
-// passes over HBM (four-step split M = R * C, R = 1024 or 768), with the
+// passes over HBM (four-step split M = R * C, R = 256 to 4096), with the
 // resample gather done by the first pass's loads; and the unpack +
 // interbin + normalise pass that reads its transposed output.
 #pragma once
@@ -16,15 +16,15 @@ struct ColArgs;
 
 struct Fft4Plan {
     size_t n = 0;      // real samples N
-    unsigned R = 1024; // rows of the four-step split: 768 for 3 * 2^k, 1024
-                       // up to N = 2^25, 2048 at 2^26, 4096 at 2^27
+    unsigned R = 1024; // rows of the four-step split: 256 up to N = 2^18, 768
+                       // for 3 * 2^k, 1024 up to 2^25, 2048 at 2^26, 4096 at 2^27
     unsigned C = 0;    // row length of the second pass (M / R)
     int logc = 0;
     float2* d_tab = nullptr;  // twiddle tables (offsets below, in float2)
     size_t tab_len = 0;
     unsigned offA2 = 0, offA3 = 0, offQ = 0, offP = 0, offI = 0, offB = 0, offRv = 0, offRk = 0;
 
-    // N = 2^19 .. 2^27 (R = 1024, 2048, 4096) or 3 * 2^17 .. 3 * 2^23
+    // N = 2^17 .. 2^27 (R = 256, 1024, 2048, 4096) or 3 * 2^17 .. 3 * 2^23
     // (R = 768), i.e. C = 2^8 .. 2^14.
     static bool supported(size_t n);
     static unsigned rows_for(size_t n);

@@ -1937,7 +1937,9 @@ static int check_config(const psx_search_config* c)
         set_error("search: fft_form must be 0..3");
         return PSX_ERR_INVALID;
     }
-    if (c->fft_form == 3 && (c->mode != PSX_MODE_BATCHED || !Fft4Plan::supported(c->fft_size))) {
+    // (2^17 and 2^18 points take the two-pass transform by default only)
+    if (c->fft_form == 3 && (c->mode != PSX_MODE_BATCHED || !Fft4Plan::supported(c->fft_size) ||
+                             c->fft_size < ((size_t)3 << 17))) {
         set_error("search: fft_form 3 needs the batched mode and "
                   "fft_size 2^19 .. 2^27 or 3 * 2^17 .. 3 * 2^23");
         return PSX_ERR_INVALID;

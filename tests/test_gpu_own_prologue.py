@@ -99,3 +99,36 @@ def test_retarget_replaces_the_birdies(cuda):
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[3], want[3])
         del keep
     s.close()
+
+
+@pytest.mark.parametrize("n", [1 << 17, 1 << 18])
+def test_short_lengths_take_it_by_default(cuda, oracle, n):
+    """2^17 and 2^18 points (256-row columns): the default form; series and
+    statistics against cuFFT's prologue, the trials' gathered series bit for
+    bit and their spectra against 64 bits (1e-5, as the longer lengths'), and
+    an explicit fft_form 3 refused there as before."""
+    from test_gpu_fft4 import _fp64_spectrum, err_vs_mag_or_rms
+    from peasoup_b200 import search, synth
+    from peasoup_b200._lib import PsxError
+    from peasoup_b200.transforms import AccelerationPlan
+    x = _series(n - 1001, 5, 70.0)
+    base = dict(fft_size=n, tsamp=64e-6, cfreq_hz=synth.CFREQ_HZ, ch_bw_hz=synth.CH_BW_HZ,
+                acc_lo=-300.0, acc_hi=300.0, nharmonics=2, min_snr=8.0,
+                birdie_freqs=BIRDIES, birdie_widths=np.full(len(BIRDIES), 0.3, np.float32))
+    with pytest.raises(PsxError):
+        search.AccelSearch(search.SearchParams(fft_form=3, **base))
+    want, wnorm, _ = _tap(n, x, 1, birdie_freqs=BIRDIES,
+                          birdie_widths=np.full(len(BIRDIES), 0.3, np.float32))
+    s = search.AccelSearch(search.SearchParams(**base))
+    s.search(x)
+    assert s.info()["fft_form"] == 3
+    accs = AccelerationPlan(-300.0, 300.0, 1.10, 64e-6, n, 64e-6, synth.CFREQ_HZ,
+                            synth.CH_BW_HZ).generate_accel_list(0.0, 0.0)
+    for t in sorted({0, len(accs) // 2, len(accs) - 1}):
+        tim, tr, ps, norm = s.debug_tap(t)
+        idx = oracle.resampleII_index(n, float(accs[t]), 64e-6)
+        assert np.array_equal(tr, tim[idx.astype(np.int64)])
+        assert err_vs_mag_or_rms(ps, _fp64_spectrum(tim, idx, norm)) < 1e-5
+    s.close()
+    assert np.max(np.abs(tim - want)) <= 1e-5 * np.sqrt(np.mean(want.astype(np.float64) ** 2))
+    assert np.all(np.abs(norm - wnorm) <= 1e-5 * np.abs(wnorm))
