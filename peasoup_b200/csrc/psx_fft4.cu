@@ -253,17 +253,28 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
             const float4 m = *reinterpret_cast<const float4*>(a.means + 4 * blockIdx.y);
             auto less = [&](float f) { return ((f - m.x) - m.y) - m.z; };
             const size_t s0 = 2 * ((size_t)t * C + c), step = 2 * (size_t)J * C;
-            const bool pairs = (reinterpret_cast<uintptr_t>(xr) & 7u) == 0;
+            if ((reinterpret_cast<uintptr_t>(xr) & 7u) == 0 && a.ncopy >= 2) {
+                // sixteen loads in flight: no branch around any of them, the
+                // ones past the series read its last pair and are zeroed
+                const size_t last = (a.ncopy & ~(size_t)1) - 2;
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const size_t i = s0 + q * step;
-                v[q] = make_float2(0.f, 0.f);
-                if (pairs && i + 1 < a.ncopy) {
-                    const float2 f = *reinterpret_cast<const float2*>(xr + i);
-                    v[q] = make_float2(less(f.x), less(f.y));
-                } else {
-                    if (i < a.ncopy) v[q].x = less(xr[i]);
-                    if (i + 1 < a.ncopy) v[q].y = less(xr[i + 1]);
+                for (int q = 0; q < 16; ++q)
+                    v[q] = *reinterpret_cast<const float2*>(xr + min(s0 + q * step, last));
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    v[q] = s0 + q * step <= last ? make_float2(less(v[q].x), less(v[q].y))
+                                                 : make_float2(0.f, 0.f);
+                if (a.ncopy & 1) {  // an odd series' last sample
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                        if (s0 + q * step == a.ncopy - 1) v[q].x = less(xr[a.ncopy - 1]);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    const size_t i = s0 + q * step;
+                    v[q].x = i < a.ncopy ? less(xr[i]) : 0.f;
+                    v[q].y = i + 1 < a.ncopy ? less(xr[i + 1]) : 0.f;
                 }
             }
         } else {
