@@ -174,11 +174,15 @@ int psx_find_peaks(const float* d_spec, int n, int start, float thresh,
                    int* d_idx, float* d_val, int cap, int* h_count,
                    psx_stream_t stream);
 
-/* psx_find_peaks with the peaks returned in host arrays: the count and up to
- * 1024 peaks come back in one copy.  PSX_ERR_OVERFLOW with the full count in
- * *h_count (and nothing written) when cap is too small. */
-int psx_find_peaks_host(const float* d_spec, int n, int start, float thresh, int* h_idx,
-                        float* h_val, int cap, int* h_count, psx_stream_t stream);
+/* psx_find_peaks over up to 8 spectra (a trial's spectrum, or its harmonic
+ * sums) with the peaks returned in host arrays: spectrum k's counts in
+ * h_counts[k], its peaks at h_idx + k cap and h_val + k cap.  One pair of
+ * launches; the counts and up to 512 peaks of each spectrum come back in one
+ * copy.  PSX_ERR_OVERFLOW with the full counts (and no peaks) when some
+ * spectrum has more than cap. */
+int psx_find_peaks_host(const float* const* d_specs, const int* n, const int* start, int nspec,
+                        float thresh, int* h_idx, float* h_val, int cap, int* h_counts,
+                        psx_stream_t stream);
 
 /* psx_find_peaks without any device allocation; no counterpart in the
    reference.  For callers that may not allocate GPU memory during a run

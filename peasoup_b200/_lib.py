@@ -149,7 +149,7 @@ SIGNATURES = {
     "psx_convert_i8_f32": (_i, [_vp, _vp, _sz, _vp]),
     "psx_harmonic_sum": (_i, [_vp, _vp, _sz, _i, _vp]),
     "psx_find_peaks": (_i, [_vp, _i, _i, _f, _vp, _vp, _i, C.POINTER(_i), _vp]),
-    "psx_find_peaks_host": (_i, [_vp, _i, _i, _f, _vp, _vp, _i, C.POINTER(_i), _vp]),
+    "psx_find_peaks_host": (_i, [_vp, _vp, _vp, _i, _f, _vp, _vp, _i, _vp, _vp]),
     "psx_find_peaks_noalloc": (_i, [_vp, _i, _i, _f, _vp, _vp, _i, C.POINTER(_i), _vp]),
     "psx_harmonic_peaks": (_i, [_vp, _sz, _sz, _i, _i, _vp, _vp, _f, _vp, _sz, C.POINTER(_sz),
                                 C.c_uint, C.c_uint, _vp]),

@@ -1312,11 +1312,26 @@ constexpr int kPeakRuns = 1024;
 constexpr int kPeakWarps = 8;
 constexpr int kPeakInts = kPeakRuns * (1 + kPeakWarps) + 1;  // scratch: runs, parts, total
 
-__global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_count(const float* __restrict__ x,
-                                                                 int start, int n, int run,
-                                                                 float thresh,
-                                                                 int* __restrict__ counts)
+// The spectra of one launch (grid y): a fold-by-fold search of a trial's
+// harmonic sums is one pair of launches and one read-back.
+constexpr int kPeakSpectra = 8;
+struct PeakJobs {
+    const float* x[kPeakSpectra];
+    int start[kPeakSpectra], n[kPeakSpectra], run[kPeakSpectra];
+    int* counts[kPeakSpectra];  // kPeakInts - 1 of scratch
+    int* total[kPeakSpectra];
+    int* idx[kPeakSpectra];
+    float* val[kPeakSpectra];
+};
+
+__global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_count(const __grid_constant__ PeakJobs job,
+                                                                 float thresh)
 {
+    const int sp = blockIdx.y, run = job.run[sp], start = job.start[sp], n = job.n[sp];
+    const float* __restrict__ x = job.x[sp];
+    int* __restrict__ counts = job.counts[sp];
+    const int runs = (int)(((long long)n - start + run - 1) / run);
+    if ((int)blockIdx.x >= runs) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x / 32, part = run / kPeakWarps;
     const long long a = start + (long long)blockIdx.x * run + (long long)warp * part;
     const int len = (int)max(0LL, min((long long)part, (long long)n - a));
@@ -1328,7 +1343,7 @@ __global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_count(const float* __
     __shared__ int sh[kPeakWarps];
     if (lane == 0) {
         sh[warp] = c;
-        counts[gridDim.x + blockIdx.x * kPeakWarps + warp] = c;
+        counts[runs + blockIdx.x * kPeakWarps + warp] = c;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1338,17 +1353,19 @@ __global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_count(const float* __
     }
 }
 
-__global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_write(const float* __restrict__ x,
-                                                                 int start, int n, int run,
-                                                                 float thresh,
-                                                                 const int* __restrict__ counts,
-                                                                 int* __restrict__ total,
-                                                                 int* __restrict__ idx,
-                                                                 float* __restrict__ val, int cap)
+__global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_write(const __grid_constant__ PeakJobs job,
+                                                                 float thresh, int cap)
 {
+    const int sp = blockIdx.y, run = job.run[sp], start = job.start[sp], n = job.n[sp];
+    const float* __restrict__ x = job.x[sp];
+    const int* __restrict__ counts = job.counts[sp];
+    int* __restrict__ idx = job.idx[sp];
+    float* __restrict__ val = job.val[sp];
+    const int runs = (int)(((long long)n - start + run - 1) / run);
+    if ((int)blockIdx.x >= runs) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x / 32, part = run / kPeakWarps;
     const int own = counts[blockIdx.x];
-    const bool last = blockIdx.x == gridDim.x - 1;
+    const bool last = (int)blockIdx.x == runs - 1;
     if (own == 0 && !last) return;
     __shared__ int sh[kPeakWarps];
     int c = 0;  // hits of the runs before this one
@@ -1358,8 +1375,8 @@ __global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_write(const float* __
     __syncthreads();
     int pos = 0;
     for (int w = 0; w < kPeakWarps; ++w) pos += sh[w];
-    if (last && threadIdx.x == 0) *total = pos + own;
-    const int* parts = counts + gridDim.x + blockIdx.x * kPeakWarps;
+    if (last && threadIdx.x == 0) *job.total[sp] = pos + own;
+    const int* parts = counts + runs + blockIdx.x * kPeakWarps;
     for (int w = 0; w < warp; ++w) pos += parts[w];
     int left = parts[warp];
     const long long a = start + (long long)blockIdx.x * run + (long long)warp * part;
@@ -1381,20 +1398,42 @@ __global__ void __launch_bounds__(32 * kPeakWarps) k_peaks_write(const float* __
     }
 }
 
-// Both kernels over [start, n), n > start; `scratch` holds kPeakInts ints, its
-// last one the total.
+// Bins per run of [start, n): at least 2048, so that a short spectrum's few
+// CTAs have work.
+static int peak_run(long long bins)
+{
+    const long long run = (bins + kPeakRuns - 1) / kPeakRuns;
+    return (int)(((run < 2048 ? 2048 : run) + 255) / 256 * 256);
+}
+
+// Both kernels over the first `count` spectra of the job (all with n > start).
+static int launch_peaks(PeakJobs& job, int count, float thresh, int cap, cudaStream_t s)
+{
+    unsigned g = 1;
+    for (int k = 0; k < count; ++k) {
+        const long long bins = (long long)job.n[k] - job.start[k];
+        job.run[k] = peak_run(bins);
+        g = std::max(g, (unsigned)((bins + job.run[k] - 1) / job.run[k]));
+    }
+    const dim3 grid(g, (unsigned)count);
+    k_peaks_count<<<grid, 32 * kPeakWarps, 0, s>>>(job, thresh);
+    k_peaks_write<<<grid, 32 * kPeakWarps, 0, s>>>(job, thresh, cap);
+    return launch_status("compaction kernels");
+}
+
+// One spectrum; `scratch` holds kPeakInts ints, its last one the total.
 static int launch_peaks(const float* d_spec, int n, int start, float thresh, int* scratch,
                         int* d_idx, float* d_val, int cap, cudaStream_t s)
 {
-    const long long bins = (long long)n - start;
-    // runs of at least 2048 bins, so that a short spectrum's few CTAs have work
-    long long run = (bins + kPeakRuns - 1) / kPeakRuns;
-    run = ((run < 2048 ? 2048 : run) + 255) / 256 * 256;
-    const unsigned g = (unsigned)((bins + run - 1) / run);
-    k_peaks_count<<<g, 32 * kPeakWarps, 0, s>>>(d_spec, start, n, (int)run, thresh, scratch);
-    k_peaks_write<<<g, 32 * kPeakWarps, 0, s>>>(d_spec, start, n, (int)run, thresh, scratch,
-                                                scratch + kPeakInts - 1, d_idx, d_val, cap);
-    return launch_status("compaction kernels");
+    PeakJobs job{};
+    job.x[0] = d_spec;
+    job.start[0] = start;
+    job.n[0] = n;
+    job.counts[0] = scratch;
+    job.total[0] = scratch + kPeakInts - 1;
+    job.idx[0] = d_idx;
+    job.val[0] = d_val;
+    return launch_peaks(job, 1, thresh, cap, s);
 }
 
 }  // namespace psx
@@ -1778,55 +1817,87 @@ int psx_find_peaks(const float* d_spec, int n, int start, float thresh, int* d_i
     return PSX_OK;
 }
 
-int psx_find_peaks_host(const float* d_spec, int n, int start, float thresh, int* h_idx,
-                        float* h_val, int cap, int* h_count, psx_stream_t stream)
+int psx_find_peaks_host(const float* const* d_specs, const int* n, const int* start, int nspec,
+                        float thresh, int* h_idx, float* h_val, int cap, int* h_counts,
+                        psx_stream_t stream)
 {
     clear_error();
-    if (!d_spec || !h_count || cap < 0 || (cap > 0 && (!h_idx || !h_val))) {
-        set_error("find_peaks_host: bad arguments");
+    if (!d_specs || !n || !start || nspec < 1 || nspec > kPeakSpectra || !h_counts || cap < 0 ||
+        (cap > 0 && (!h_idx || !h_val))) {
+        set_error("find_peaks_host: bad arguments (1 to %d spectra)", kPeakSpectra);
         return PSX_ERR_INVALID;
     }
-    if (start < 0) start = 0;
-    *h_count = 0;
-    if (n <= start) return PSX_OK;
+    for (int k = 0; k < nspec; ++k)
+        if (!d_specs[k]) {
+            set_error("find_peaks_host: null spectrum %d", k);
+            return PSX_ERR_INVALID;
+        }
     cudaStream_t s = cs(stream);
-    // the count and the first kFirst peaks come back in one copy
-    constexpr int kFirst = 1024;
+    // the counts and the first kFirst peaks of every spectrum come back in
+    // one copy: per spectrum [total, idx[kFirst], val[kFirst]]
+    constexpr int kFirst = 512, kRow = 1 + 2 * kFirst;
+    PeakJobs job{};
+    int which[kPeakSpectra], count = 0;
+    for (int k = 0; k < nspec; ++k) {
+        h_counts[k] = 0;
+        const int st = std::max(0, start[k]);
+        if (n[k] <= st) continue;
+        which[count] = k;
+        job.x[count] = d_specs[k];
+        job.start[count] = st;
+        job.n[count] = n[k];
+        ++count;
+    }
+    if (!count) return PSX_OK;
     int* scratch = nullptr;
-    PSX_CUDA(scratch_alloc((void**)&scratch, sizeof(int) * (kPeakInts + 2 * kFirst), s));
-    int* d_idx = scratch + kPeakInts;
-    float* d_val = reinterpret_cast<float*>(d_idx + kFirst);
-    int first[1 + 2 * kFirst];
-    int rc = launch_peaks(d_spec, n, start, thresh, scratch, d_idx, d_val, kFirst, s);
-    if (rc == PSX_OK)
-        rc = cuda_status(cudaMemcpyAsync(first, d_idx - 1, sizeof first, cudaMemcpyDeviceToHost, s),
-                         "find_peaks_host copy");
-    cudaFreeAsync(scratch, s);
-    if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "find_peaks_host");
-    if (rc != PSX_OK) return rc;
-    const int total = *h_count = first[0];
-    if (total > cap) {
-        set_error("find_peaks_host: %d values above threshold, buffer holds %d", total, cap);
-        return PSX_ERR_OVERFLOW;
+    PSX_CUDA(scratch_alloc((void**)&scratch,
+                           sizeof(int) * (size_t)count * (kPeakInts - 1 + kRow), s));
+    int* back = scratch + (size_t)count * (kPeakInts - 1);  // the rows read back
+    for (int c = 0; c < count; ++c) {
+        job.counts[c] = scratch + (size_t)c * (kPeakInts - 1);
+        job.total[c] = back + c * kRow;
+        job.idx[c] = job.total[c] + 1;
+        job.val[c] = reinterpret_cast<float*>(job.idx[c] + kFirst);
     }
-    if (total <= kFirst) {
-        if (total) std::memcpy(h_idx, first + 1, sizeof(int) * total);
-        if (total) std::memcpy(h_val, first + 1 + kFirst, sizeof(float) * total);
-        return PSX_OK;
-    }
-    PSX_CUDA(scratch_alloc((void**)&scratch, sizeof(int) * (kPeakInts + 2 * (size_t)total), s));
-    d_idx = scratch + kPeakInts;
-    d_val = reinterpret_cast<float*>(d_idx + total);
-    rc = launch_peaks(d_spec, n, start, thresh, scratch, d_idx, d_val, total, s);
+    int h[kPeakSpectra * kRow];
+    int rc = launch_peaks(job, count, thresh, kFirst, s);
     if (rc == PSX_OK)
-        rc = cuda_status(cudaMemcpyAsync(h_idx, d_idx, sizeof(int) * total, cudaMemcpyDeviceToHost, s),
-                         "find_peaks_host copy");
-    if (rc == PSX_OK)
-        rc = cuda_status(cudaMemcpyAsync(h_val, d_val, sizeof(float) * total,
+        rc = cuda_status(cudaMemcpyAsync(h, back, sizeof(int) * (size_t)count * kRow,
                                          cudaMemcpyDeviceToHost, s), "find_peaks_host copy");
     cudaFreeAsync(scratch, s);
     if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "find_peaks_host");
-    return rc;
+    if (rc != PSX_OK) return rc;
+    int most = 0;
+    for (int c = 0; c < count; ++c) most = std::max(most, h_counts[which[c]] = h[c * kRow]);
+    if (most > cap) {
+        set_error("find_peaks_host: %d values above threshold, buffer holds %d", most, cap);
+        return PSX_ERR_OVERFLOW;
+    }
+    for (int c = 0; c < count; ++c) {
+        const int k = which[c], total = h_counts[k];
+        int* oi = h_idx + (size_t)k * cap;
+        float* ov = h_val + (size_t)k * cap;
+        if (total <= kFirst) {
+            std::memcpy(oi, h + c * kRow + 1, sizeof(int) * total);
+            std::memcpy(ov, h + c * kRow + 1 + kFirst, sizeof(float) * total);
+            continue;
+        }
+        // more than came back: this spectrum again, into a buffer of its size
+        PSX_CUDA(scratch_alloc((void**)&scratch, sizeof(int) * (kPeakInts + 2 * (size_t)total), s));
+        int* d_idx = scratch + kPeakInts;
+        float* d_val = reinterpret_cast<float*>(d_idx + total);
+        rc = launch_peaks(job.x[c], job.n[c], job.start[c], thresh, scratch, d_idx, d_val, total, s);
+        if (rc == PSX_OK)
+            rc = cuda_status(cudaMemcpyAsync(oi, d_idx, sizeof(int) * total,
+                                             cudaMemcpyDeviceToHost, s), "find_peaks_host copy");
+        if (rc == PSX_OK)
+            rc = cuda_status(cudaMemcpyAsync(ov, d_val, sizeof(float) * total,
+                                             cudaMemcpyDeviceToHost, s), "find_peaks_host copy");
+        cudaFreeAsync(scratch, s);
+        if (rc == PSX_OK) rc = cuda_status(cudaStreamSynchronize(s), "find_peaks_host");
+        if (rc != PSX_OK) return rc;
+    }
+    return PSX_OK;
 }
 
 }  // extern "C"

@@ -430,42 +430,53 @@ class PeakFinder:
         self.min_freq = float(min_freq)
         self.max_freq = float(max_freq)
         self.min_gap = int(min_gap)
-        self.cap = 4096  # grown on demand
-        self._alloc()
+        self.cap = 4096  # peaks of one spectrum; grown on demand
+        self._spectra = 0
+        self._alloc(1)
 
-    def _alloc(self) -> None:
-        self._idx, self._pidx = np.empty(self.cap, np.int32), np.empty(self.cap, np.int32)
-        self._val, self._pval = np.empty(self.cap, np.float32), np.empty(self.cap, np.float32)
+    def _alloc(self, spectra: int) -> None:
+        self._spectra = spectra
+        self._idx = np.empty((spectra, self.cap), np.int32)
+        self._val = np.empty((spectra, self.cap), np.float32)
+        self._pidx = np.empty(self.cap, np.int32)
+        self._pval = np.empty(self.cap, np.float32)
 
     def find_candidates(self, spec, cands: SpectrumCandidates) -> None:
-        if isinstance(spec, HarmonicSums):
-            for s in spec.folds:
-                self.find_candidates(s, cands)
-            return
+        specs = spec.folds if isinstance(spec, HarmonicSums) else [spec]
+        for k in range(0, len(specs), 8):  # one call searches up to 8 spectra
+            self._find(specs[k:k + 8], cands)
+
+    def _find(self, specs, cands: SpectrumCandidates) -> None:
         L = load()
-        size = spec.get_nbins()
+        m = len(specs)
+        n, first, count = (C.c_int * m)(), (C.c_int * m)(), (C.c_int * m)()
+        ptrs = (C.c_void_p * m)()
+        factors = []
         start, end, factor = C.c_int(), C.c_int(), C.c_float()
-        check(L.psx_peak_range(size, spec.get_bin_width(), spec.get_nh(), self.min_freq,
-                               self.max_freq, C.byref(start), C.byref(end), C.byref(factor)),
-              "peak_range")
-        count = C.c_int()
+        for k, sp in enumerate(specs):
+            check(L.psx_peak_range(sp.get_nbins(), sp.get_bin_width(), sp.get_nh(), self.min_freq,
+                                   self.max_freq, C.byref(start), C.byref(end), C.byref(factor)),
+                  "peak_range")
+            ptrs[k], n[k], first[k] = _ptr(sp.data).value, end.value, start.value
+            factors.append(np.float32(factor.value))
+        if m > self._spectra:
+            self._alloc(m)
         while True:
-            rc = L.psx_find_peaks_host(_ptr(spec.data), end.value, start.value, self.threshold,
-                                       self._idx.ctypes.data, self._val.ctypes.data, self.cap,
-                                       C.byref(count), _stream())
+            rc = L.psx_find_peaks_host(ptrs, n, first, m, self.threshold, self._idx.ctypes.data,
+                                       self._val.ctypes.data, self.cap, count, _stream())
             if rc != _lib.PSX_ERR_OVERFLOW:
                 break
-            self.cap = int(count.value * 1.25) + 1024
-            self._alloc()
+            self.cap = int(max(count) * 1.25) + 1024
+            self._alloc(self._spectra)
         check(rc, "find_peaks")
-        n = count.value
-        if n == 0:
-            return
-        npk = L.psx_identify_unique_peaks(self._idx.ctypes.data, self._val.ctypes.data, n,
-                                          self.min_gap, self._pidx.ctypes.data,
-                                          self._pval.ctypes.data)
-        freqs = (self._pidx[:npk].astype(np.float32) * np.float32(factor.value)).astype(np.float32)
-        cands.append_peaks(self._pval[:npk].tolist(), freqs.tolist(), spec.get_nh())
+        for k, sp in enumerate(specs):
+            if count[k] == 0:
+                continue
+            npk = L.psx_identify_unique_peaks(self._idx[k].ctypes.data, self._val[k].ctypes.data,
+                                              count[k], self.min_gap, self._pidx.ctypes.data,
+                                              self._pval.ctypes.data)
+            freqs = (self._pidx[:npk].astype(np.float32) * factors[k]).astype(np.float32)
+            cands.append_peaks(self._pval[:npk].tolist(), freqs.tolist(), sp.get_nh())
 
 
 # --------------------------------------------------------------- distillers

@@ -67,12 +67,20 @@ def test_find_peaks_runs_against_definition(psx, cuda, n, start, every):
         assert np.array_equal(idx.cpu().numpy()[:cap], want[:cap])
         assert np.array_equal(val.cpu().numpy()[:cap], x[want[:cap]])
         assert np.all(idx.cpu().numpy()[cap:] == -1)
-        hi, hv = np.full(len(want) + 1, -1, np.int32), np.zeros(len(want) + 1, np.float32)
-        rc = psx.psx_find_peaks_host(C.c_void_p(d.data_ptr()), n, start, 4.0, hi.ctypes.data,
-                                     hv.ctypes.data, cap, C.byref(cnt), None)
-        assert rc == (0 if cap == len(want) else 5) and cnt.value == len(want)
+        # the same spectrum whole, from its middle, empty and again in one call
+        starts = (C.c_int * 4)(start, n // 2, n, start)
+        ptrs = (C.c_void_p * 4)(*[d.data_ptr()] * 4)
+        hi, hv = np.full((4, cap + 1), -1, np.int32), np.zeros((4, cap + 1), np.float32)
+        hi, hv = hi[:, :cap].copy(), hv[:, :cap].copy()
+        cnts = (C.c_int * 4)()
+        rc = psx.psx_find_peaks_host(ptrs, (C.c_int * 4)(*[n] * 4), starts, 4, 4.0,
+                                     hi.ctypes.data, hv.ctypes.data, cap, cnts, None)
+        half = want[want >= n // 2]
+        assert rc == (0 if cap == len(want) else 5)
+        assert list(cnts) == [len(want), len(half), 0, len(want)]
         if rc == 0:
-            assert np.array_equal(hi[:-1], want) and np.array_equal(hv[:-1], x[want])
+            for k, w in ((0, want), (1, half), (3, want)):
+                assert np.array_equal(hi[k, :len(w)], w) and np.array_equal(hv[k, :len(w)], x[w])
 
 
 @pytest.mark.parametrize("shift", [0, 1])
