@@ -268,6 +268,17 @@ constexpr HarmShape kHarmShapes[] = {
 };
 static_assert(sizeof(kHarmShapes) / sizeof(kHarmShapes[0]) == PSX_HARM_SHAPES, "shape table");
 constexpr int kHarmDefaultShape = 4;
+// With no shape asked for, launch groups of the two-pass transform at 2^20 to
+// 2^23 points take the three-row shape where its whole rows carry them.
+// Measured on B200 (us per trial, shape 4 against 6, 4 folds): 24 trials in a
+// group at 2^19 1.56/1.41 (5 folds 2.16/2.26), 2^21 4.95/4.14, 2^23
+// 18.6/14.6; groups of 8 at 2^23 19.3/17.6; groups of 4, where one trial is
+// left for a launch of its own, 6.72/8.56 at 2^21.  Every bin is read at 16
+// places of the search, from L2 while the rows searched together stay in it:
+// three rows of 2^26 points (400 MB) took 8.30 ms a call where one at a time
+// took 7.73.
+constexpr int kHarmRowsShape = 6;
+constexpr size_t kHarmRowsMinPoints = (size_t)1 << 20, kHarmRowsMaxPoints = (size_t)1 << 23;
 
 template <int F, int SH>
 struct HarmKernel {
@@ -609,6 +620,12 @@ struct psx_search {
     float* d_Xl[2] = {nullptr, nullptr};
     float* d_pl[2] = {nullptr, nullptr};
     HarmMaps hmaps[2] = {};  // per lane: the spectra as boxes of the multi-row shape's rows
+    bool harm_auto = false;  // no shape asked for: shape_for picks per launch group
+    int shape_for(int trials) const
+    {
+        const int rows = kHarmShapes[kHarmRowsShape - 1].rows;
+        return harm_auto && (trials % rows == 0 || trials >= 4 * rows) ? kHarmRowsShape : harm_shape;
+    }
     float* d_tr = nullptr;
     float* d_X = nullptr;
     float* d_p = nullptr;
@@ -1103,10 +1120,10 @@ int psx_search::trials_span(GroupSet& g, int cnt)
                         g.d_trow + t0));
         g.launches += 3;
         if (span) {  // as trials_range: leftover trials on the single-row shape
-            const int rows = kHarmShapes[harm_shape - 1].rows;
+            const int shape = shape_for(b), rows = kHarmShapes[shape - 1].rows;
             const int rem = rows > 1 ? b % rows : 0, bm = b - rem;
             if (bm > 0) {
-                PSX_TRY(launch_harm(F, harm_shape, pp, Bp, (unsigned)Bp, pk, t0, bm, g.d_rec,
+                PSX_TRY(launch_harm(F, shape, pp, Bp, (unsigned)Bp, pk, t0, bm, g.d_rec,
                                     g.d_cnt, (unsigned)g.rec_cap, st, &hmaps[0]));
                 ++g.launches;
             }
@@ -1500,10 +1517,10 @@ int psx_search::trials_range(Slot& s, int t_begin, int nacc, bool reset)
             // last b % rows trials go to the single-row default shape
             // instead of a tile padded with unused rows (every shape gives
             // the same records).
-            const int rows = kHarmShapes[harm_shape - 1].rows;
+            const int shape = shape_for(b), rows = kHarmShapes[shape - 1].rows;
             const int rem = rows > 1 ? b % rows : 0, bm = b - rem;
             if (bm > 0) {
-                PSX_TRY(launch_harm(F, harm_shape, pp, Bp, (unsigned)Bp, pk, t0, bm, s.d_rec,
+                PSX_TRY(launch_harm(F, shape, pp, Bp, (unsigned)Bp, pk, t0, bm, s.d_rec,
                                     s.d_count, (unsigned)s.rec_cap, ls, &hmaps[lane]));
                 ++s.launches;
             }
@@ -2073,6 +2090,9 @@ static void host_setup(psx_search* s, const psx_search_config* cfg)
     s->lanes = effective_lanes(cfg);
     s->harm_shape = cfg->harm_shape ? cfg->harm_shape : kHarmDefaultShape;
     s->use_f4 = effective_form(cfg) == 3;
+    s->harm_auto = !cfg->harm_shape && s->use_f4 && s->N >= kHarmRowsMinPoints &&
+                   s->N <= kHarmRowsMaxPoints &&
+                   s->batch >= kHarmShapes[kHarmRowsShape - 1].rows;
     {
         const double M = (double)(s->N / 2), pi = 3.14159265358979323846;
         for (int t = 0; t < 6; ++t)
@@ -2153,10 +2173,10 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
     s->d_tr = s->d_trl[0];
     s->d_X = s->d_Xl[0];
     s->d_p = s->d_pl[0];
-    if (kHarmShapes[s->harm_shape - 1].rows > 0)
+    const int map_rows = kHarmShapes[(s->harm_auto ? kHarmRowsShape : s->harm_shape) - 1].rows;
+    if (map_rows > 0)
         for (int l = 0; l < s->lanes; ++l)
-            if ((rc = encode_harm_maps(s->d_pl[l], Bp, (int)b, kHarmShapes[s->harm_shape - 1].rows,
-                                       &s->hmaps[l])) != PSX_OK)
+            if ((rc = encode_harm_maps(s->d_pl[l], Bp, (int)b, map_rows, &s->hmaps[l])) != PSX_OK)
                 return fail(rc);
     for (Slot& sl : s->slot) {
         ALLOC(sl.d_count, sizeof(unsigned) * 16);

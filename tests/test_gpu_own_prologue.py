@@ -132,3 +132,31 @@ def test_short_lengths_take_it_by_default(cuda, oracle, n):
     s.close()
     assert np.max(np.abs(tim - want)) <= 1e-5 * np.sqrt(np.mean(want.astype(np.float64) ** 2))
     assert np.all(np.abs(norm - wnorm) <= 1e-5 * np.abs(wnorm))
+
+
+def test_default_harmonic_shape_per_launch_group(cuda):
+    """With no harmonic shape asked for, launch groups of 2^20 points take
+    the three-row kernel where its rows carry them (multiples of 3, 12 and
+    more) and the single-row one otherwise: the same candidates, bit for bit,
+    as the single-row shape throughout."""
+    from peasoup_b200 import search, synth
+    from peasoup_b200.transforms import AccelerationPlan
+    n, ts = 1 << 20, 64e-6
+    x = synth.make_series_np(synth.SeriesSpec(
+        nsamps=n, tsamp=ts, pulsars=[synth.Pulsar(5.1e-3, 100.0, 0.05, 0.4)]), 2)
+    seen = set()
+    for acc in (50.0, 150.0, 300.0, 450.0, 800.0, 900.0):
+        base = dict(fft_size=n, tsamp=ts, cfreq_hz=synth.CFREQ_HZ, ch_bw_hz=synth.CH_BW_HZ,
+                    acc_lo=-acc, acc_hi=acc, nharmonics=4, min_snr=5.5, batch=14)
+        seen.add(len(AccelerationPlan(-acc, acc, 1.10, 64e-6, n, ts, synth.CFREQ_HZ,
+                                      synth.CH_BW_HZ).generate_accel_list(0.0, 0.0)))
+        got = []
+        for shape in (0, 4):
+            s = search.AccelSearch(search.SearchParams(harm_shape=shape, **base))
+            got.append(s.search(x, 1.0, 2, per_dm=False))
+            s.close()
+        assert len(got[0][0]) > 0
+        for a, b in zip(*got):
+            assert np.array_equal(a, b)
+    # group sizes on both sides of the rule
+    assert len({k % 3 for k in seen}) > 1, seen
