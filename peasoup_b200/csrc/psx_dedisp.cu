@@ -718,6 +718,7 @@ struct psx_dedisp_plan {
     bool dirty = true;
     int elem = 0;
     int kind = -1;          // sample class the tables were built for
+    bool few = false;       // and whether for few CTAs
     int nlive = 0, ndm_pad = 0, nblk = 0, group = 8, lwin = 0, cc = 0;
     size_t ngroups = 0, max_lo = 0;
     size_t scratch_limit = 4ull << 30;  // bytes of channel-major samples
@@ -748,9 +749,10 @@ struct psx_dedisp_plan {
     }
 
     // Shift tables and the window shape for one class of samples.
-    int build_tables(int sample_kind)
+    int build_tables(int sample_kind, bool few_ctas)
     {
-        if (!dirty && sample_kind == kind) return PSX_OK;
+        if (!dirty && sample_kind == kind && few_ctas == few) return PSX_OK;
+        few = few_ctas;
         const int el = sample_kind == kTr16 ? 2 : 1;
         kind = sample_kind;
         dirty = true;
@@ -773,7 +775,7 @@ struct psx_dedisp_plan {
                 shift[(size_t)d * nlive + i] = (int)std::nearbyint(p);
             }
         tile = dd_tile(el);
-        if (nlive > 0 && build_tree(el, chans, shift)) {
+        if (nlive > 0 && !few && build_tree(el, chans, shift)) {
             elem = el;
             dirty = true;  // tables must be uploaded
             return PSX_OK;
@@ -1132,8 +1134,15 @@ int prepare(psx_dedisp_plan* p, size_t nout, int nbits, cudaStream_t st, size_t*
 {
     const int kind = nbits == 16 ? kTr16 : nbits <= 4 ? kTrSmall : kTr8;
     const int el = nbits == 16 ? 2 : 1;
-    bool rebuilt = p->dirty || kind != p->kind;
-    PSX_TRY(p->build_tables(kind));
+    // Blocks of 32 DM trials leave most SMs without a CTA where the output is
+    // short: the direct kernel's blocks of 8 then (30,278 samples x 16
+    // channels to 50 DM trials, 60 blocks of 32, on B200: 26.1 us against
+    // 28.0; 42,314 x 248 to 75, 123 blocks: 90 against 52).
+    const size_t blocks = (nout + tr_tile(el) - 1) / tr_tile(el) *
+                          ((p->dms.size() + kTrMaxDms - 1) / kTrMaxDms);
+    const bool few = 2 * blocks < (size_t)sm_count();
+    bool rebuilt = p->dirty || kind != p->kind || few != p->few;
+    PSX_TRY(p->build_tables(kind, few));
     if (rebuilt) {
         size_t bytes = p->h_tab.size() * sizeof(int);
         PSX_TRY(grow(reinterpret_cast<void**>(&p->d_tab), &p->tab_cap, std::max<size_t>(bytes, 4),

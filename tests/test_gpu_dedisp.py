@@ -119,21 +119,24 @@ def test_dedisperse_equals_oracle(psx, cuda, oracle, case):
 # The form that sums subbands once per vector of relative shifts: blocks of
 # 1, 17, 32 and 33 DM trials, a last subband of 1 to 3 channels, several
 # stages of channels, more channels than a 16-bit sum holds (258 and 600 at
-# 8 bits, 4380 at 4), wide windows, equal and unsorted DM values, outputs of
-# one sample and around one and two tiles (1024 outputs, 512 at 16 bits)
+# 8 bits, 4380 at 4), wide windows, equal and unsorted DM values, last tiles
+# of 1, all but 1 and all outputs (1024 outputs a tile, 512 at 16 bits).
+# Enough tiles that the form is taken (74 blocks of 32 DM trials); against
+# the definition in whole numbers, and the mapping in float.
 SHARED = [
-    # nchans, nbits, DM trials, largest DM, outputs
-    (64, 8, 33, 8.0, 1025), (67, 8, 32, 8.0, 1023), (9, 8, 17, 3.0, 1), (258, 8, 40, 10.0, 2049),
-    (600, 8, 12, 4.0, 1500), (1024, 4, 64, 300.0, 1024), (4380, 4, 9, 3.0, 1100),
-    (64, 2, 200, 60.0, 2047), (136, 1, 70, 30.0, 3000), (64, 16, 33, 20.0, 513),
-    (70, 16, 64, 8.0, 512), (64, 8, 300, 20.0, 4100), (33, 8, 31, 0.0, 700),
+    # nchans, nbits, DM trials, largest DM, outputs past whole tiles
+    (64, 8, 33, 8.0, 1), (67, 8, 32, 8.0, 1023), (9, 8, 17, 3.0, 1), (258, 8, 40, 10.0, 0),
+    (600, 8, 12, 4.0, 500), (1024, 4, 64, 300.0, 1023), (4380, 4, 9, 3.0, 100),
+    (64, 2, 200, 60.0, 1023), (136, 1, 70, 30.0, 3), (64, 16, 33, 20.0, 1),
+    (70, 16, 64, 8.0, 511), (64, 8, 300, 20.0, 4), (33, 8, 31, 0.0, 700),
 ]
 
 
-@pytest.mark.parametrize("nchans,nbits,ndm,dmax,nout", SHARED)
-def test_shared_partial_sums_equal_oracle(psx, cuda, oracle, nchans, nbits, ndm, dmax, nout):
+@pytest.mark.parametrize("nchans,nbits,ndm,dmax,tail", SHARED)
+def test_shared_partial_sums_equal_definition(psx, cuda, oracle, nchans, nbits, ndm, dmax, tail):
     torch = cuda
     tsamp, fch1, foff = 64e-6, 1500.0, -200.0 / nchans
+    nout = (74 // -(-ndm // 32) + 1) * (512 if nbits == 16 else 1024) + tail
     h = _plan(psx, nchans, tsamp, fch1, foff)
     try:
         rng = np.random.default_rng(ndm)
@@ -143,17 +146,28 @@ def test_shared_partial_sums_equal_oracle(psx, cuda, oracle, nchans, nbits, ndm,
         assert psx.psx_dedisp_set_dm_list(h, dms.ctypes.data, dms.size) == 0
         delays = oracle.delay_table(nchans, tsamp, fch1, foff)
         ns = oracle.max_delay(delays, dms) + nout
-        v = rng.integers(0, 1 << nbits, (ns, nchans), dtype=np.uint32)
-        v[:, : nchans // 2] = (1 << nbits) - 1      # the largest sums
+        top = (1 << nbits) - 1
+        v = rng.integers(0, top + 1, (ns, nchans), dtype=np.uint32)
+        v[:, : nchans // 2] = top                   # the largest sums
         rows = sigproc.pack_samples(v, nbits)
+        x = torch.from_numpy(v.T.astype(np.int32)).cuda().contiguous()
+        shift = np.rint(dms[:, None] * delays[None, :]).astype(np.int64)
         km = (rng.random(nchans) > 0.1).astype(np.int32)
-        for mask in (None, km):
-            assert psx.psx_dedisp_set_killmask(
-                h, None if mask is None else mask.ctypes.data) == 0
-            for raw in (True, False):
-                want = oracle.dedisperse(rows, nbits, nchans, delays, dms, killmask=mask, raw=raw)
-                got = _run(psx, torch, h, rows, nbits, dms.size, nout, raw)
-                assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+        mid = np.float32(0.5 * nchans * top)
+        scale = np.float32(1.0 / (top * np.sqrt(float(nchans))))
+        for mask in (np.ones(nchans, np.int32), km):
+            assert psx.psx_dedisp_set_killmask(h, mask.ctypes.data) == 0
+            sums = np.empty((ndm, nout), np.int32)
+            for d in range(ndm):
+                acc = torch.zeros(nout, dtype=torch.int32, device="cuda")
+                for c in np.flatnonzero(mask):
+                    acc += x[c, shift[d, c]:shift[d, c] + nout]
+                sums[d] = acc.cpu().numpy()
+            want = sums.astype(np.float32)
+            assert np.array_equal(_run(psx, torch, h, rows, nbits, ndm, nout, True), want)
+            want = (((want - mid) * scale).astype(np.float32) + np.float32(0.5)).astype(np.float32)
+            got = _run(psx, torch, h, rows, nbits, ndm, nout, False, host=True)
+            assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
     finally:
         psx.psx_dedisp_destroy(h)
 
