@@ -397,6 +397,10 @@ static int launch_harm(int F, int shape, const float* p, size_t ppitch, unsigned
 }
 
 constexpr int kDeviceBaselinePasses = 4;
+// Records that come back with the counters: most DM trials have no more, and
+// a second copy with a wait of its own costs 15 to 20 us.
+constexpr size_t kFirstRecords = 1024;
+constexpr size_t kCounterBytes = 16 * sizeof(unsigned);
 // launches of prologue_own: baseline means, two forward passes, amplitudes,
 // medians, dereddening, statistics, two inverse passes
 constexpr int kOwnPrologueLaunches = 1 + kBaselineMeans + 8;
@@ -499,6 +503,8 @@ int default_batch(size_t n)
 
 // Per-DM state that must not be shared by two DMs in flight.
 struct Slot {
+    // Records, behind the counters in one buffer (one copy brings both back);
+    // a grouped slot's counters are a row of its set's.
     int4* d_rec = nullptr;
     // [0] hits, [1] kernel error, [2] baseline still active after the device
     // passes, [3] passes; [4] the loop's start flag, [5] pass counter, [6..]
@@ -713,10 +719,8 @@ struct psx_search {
         last_dm = nullptr;
         free_groups();
         for (Slot& s : slot) {
-            if (s.d_rec) cudaFree(s.d_rec);
             if (s.d_count) cudaFree(s.d_count);
             if (s.d_ktab) cudaFree(s.d_ktab);
-            if (s.h_rec) cudaFreeHost(s.h_rec);
             if (s.h_count) cudaFreeHost(s.h_count);
             if (s.h_ktab) cudaFreeHost(s.h_ktab);
             if (s.done) cudaEventDestroy(s.done);
@@ -855,15 +859,26 @@ int psx_search::grow_records(Slot& s, size_t need)
     const size_t cap = round_up(need + need / 4, 4096);
     PSX_CUDA(cudaStreamSynchronize(st));
     PSX_CUDA(cudaStreamSynchronize(cst));
-    if (s.d_rec) cudaFree(s.d_rec);
-    if (s.h_rec) cudaFreeHost(s.h_rec);
-    s.d_rec = nullptr;
-    s.h_rec = nullptr;
     s.rec_cap = 0;
-    PSX_CUDA(cudaMalloc(&s.d_rec, sizeof(int4) * cap));
-    PSX_CUDA(cudaMallocHost(&s.h_rec, sizeof(int4) * cap));
+    if (s.grouped) {
+        if (s.d_rec) cudaFree(s.d_rec);
+        if (s.h_rec) cudaFreeHost(s.h_rec);
+        s.d_rec = s.h_rec = nullptr;
+        PSX_CUDA(cudaMalloc(&s.d_rec, sizeof(int4) * cap));
+        PSX_CUDA(cudaMallocHost(&s.h_rec, sizeof(int4) * cap));
+    } else {
+        drop_graphs();  // captured schedules hold the old buffer
+        if (s.pst) PSX_CUDA(cudaStreamSynchronize(s.pst));
+        if (s.d_count) cudaFree(s.d_count);
+        if (s.h_count) cudaFreeHost(s.h_count);
+        s.d_count = s.h_count = nullptr;
+        s.d_rec = s.h_rec = nullptr;
+        PSX_CUDA(cudaMalloc((void**)&s.d_count, kCounterBytes + sizeof(int4) * cap));
+        PSX_CUDA(cudaMallocHost((void**)&s.h_count, kCounterBytes + sizeof(int4) * cap));
+        s.d_rec = reinterpret_cast<int4*>(reinterpret_cast<char*>(s.d_count) + kCounterBytes);
+        s.h_rec = reinterpret_cast<int4*>(reinterpret_cast<char*>(s.h_count) + kCounterBytes);
+    }
     s.rec_cap = cap;
-    if (!s.grouped) drop_graphs();  // captured schedules hold the old buffer
     return PSX_OK;
 }
 
@@ -1139,6 +1154,8 @@ int psx_search::trials_span(GroupSet& g, int cnt)
     // every row's prologue counters (baseline flags) and the hit counter
     PSX_CUDA(cudaMemcpyAsync(g.h_cnt, g.count, sizeof(unsigned) * (16 * g.slots.size() + 2),
                              cudaMemcpyDeviceToHost, st));
+    PSX_CUDA(cudaMemcpyAsync(g.h_rec, g.d_rec, sizeof(int4) * kFirstRecords, cudaMemcpyDeviceToHost,
+                             st));
     PSX_CUDA(cudaEventRecord(g.done, st));
     for (int i = 0; i < cnt; ++i) PSX_CUDA(cudaEventRecord(g.slots[i].done, st));
     return PSX_OK;
@@ -1169,9 +1186,10 @@ int psx_search::finish_span(GroupSet& g, int cnt, std::vector<DmRecords>& jobs)
         PSX_TRY(trials_span(g, cnt));
     }
     const size_t nrec = hits[0];
-    if (nrec) {
+    if (nrec > kFirstRecords) {
         PSX_CUDA(cudaStreamWaitEvent(cst, g.done, 0));
-        PSX_CUDA(cudaMemcpyAsync(g.h_rec, g.d_rec, sizeof(int4) * nrec, cudaMemcpyDeviceToHost,
+        PSX_CUDA(cudaMemcpyAsync(g.h_rec + kFirstRecords, g.d_rec + kFirstRecords,
+                                 sizeof(int4) * (nrec - kFirstRecords), cudaMemcpyDeviceToHost,
                                  cst));
         PSX_CUDA(cudaStreamSynchronize(cst));
     }
@@ -1656,7 +1674,10 @@ int psx_search::enqueue_trials(Slot& s)
     PSX_CUDA(cudaStreamWaitEvent(st, s.ready, 0));
     PSX_CUDA(cudaMemcpyAsync(s.d_ktab, s.h_ktab, sizeof(double) * nacc, cudaMemcpyHostToDevice, st));
     PSX_TRY(run_trials(s, nacc));
-    PSX_CUDA(cudaMemcpyAsync(s.h_count, s.d_count, sizeof(unsigned) * 4, cudaMemcpyDeviceToHost, st));
+    PSX_CUDA(cudaMemcpyAsync(s.h_count, s.d_count,
+                             s.grouped ? sizeof(unsigned) * 4
+                                       : kCounterBytes + sizeof(int4) * kFirstRecords,
+                             cudaMemcpyDeviceToHost, st));
     PSX_CUDA(cudaEventRecord(s.done, st));
     return PSX_OK;
 }
@@ -1864,9 +1885,11 @@ int psx_search::finish(Slot& s, DmRecords& job)
     const size_t nrec = s.h_count[0];
     info.baseline_passes = s.host_baseline ? -1 : (int)s.h_count[3];
     s.host_baseline = false;
-    if (nrec) {
+    const size_t here = s.grouped ? 0 : kFirstRecords;  // came with the counters
+    if (nrec > here) {
         PSX_CUDA(cudaStreamWaitEvent(cst, s.done, 0));
-        PSX_CUDA(cudaMemcpyAsync(s.h_rec, s.d_rec, sizeof(int4) * nrec, cudaMemcpyDeviceToHost, cst));
+        PSX_CUDA(cudaMemcpyAsync(s.h_rec + here, s.d_rec + here, sizeof(int4) * (nrec - here),
+                                 cudaMemcpyDeviceToHost, cst));
         PSX_CUDA(cudaEventRecord(s.copied, cst));
         PSX_CUDA(cudaEventSynchronize(s.copied));
     }
@@ -2179,7 +2202,6 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
             if ((rc = encode_harm_maps(s->d_pl[l], Bp, (int)b, map_rows, &s->hmaps[l])) != PSX_OK)
                 return fail(rc);
     for (Slot& sl : s->slot) {
-        ALLOC(sl.d_count, sizeof(unsigned) * 16);
         ALLOC(sl.d_tim, sizeof(float) * N);
         ALLOC(sl.d_Xp, sizeof(float) * 2 * Bp);
         ALLOC(sl.d_med, median_scratch_bytes(s->B));
@@ -2197,8 +2219,6 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
 #undef ALLOC
     if (cudaMallocHost(&s->h_mean, sizeof(float) * 4) != cudaSuccess) return fail(PSX_ERR_ALLOC);
     for (Slot& sl : s->slot) {
-        if (cudaMallocHost(&sl.h_count, sizeof(unsigned) * 4) != cudaSuccess)
-            return fail(PSX_ERR_ALLOC);
         if (cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&sl.copied, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&sl.ready, cudaEventDisableTiming) != cudaSuccess)
