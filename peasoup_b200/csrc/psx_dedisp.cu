@@ -420,9 +420,9 @@ __global__ void __launch_bounds__(kDdThreads) k_dedisperse(DedispArgs a)
 //
 // Bound: the shared-memory port (71 % of its wavefronts; 46 % of them the
 // second level's, 2 bytes per output, subband and DM trial), then issue
-// (62 %).  Measured on B200 (us, the whole call, before and after): 256 DM
-// trials x 2^22 samples x 64 channels, 8 bits: 6311, 3227; 100 x 400,000 x
-// 1024, 4 bits: 3408, 1789.  Subbands of 8 channels have three times the
+// (62 %).  Measured on B200 (us, the whole call, channel by channel and so):
+// 256 DM trials x 2^22 samples x 64 channels, 8 bits: 6311, 3033; 100 x
+// 400,000 x 1024, 4 bits: 3408, 1680.  Subbands of 8 channels have three times the
 // patterns; blocks of 64 DM trials leave half the warps.
 constexpr int kTrQ = 256;      // words of a row per (DM trial, YE or YO)
 constexpr int kTrWords = kTrQ / 32;
@@ -459,6 +459,14 @@ struct TreeArgs {
     int p8s;           // subbands a byte holds (1..4-bit samples)
     unsigned tile0;    // first output tile of the launch
 };
+
+// A warp's Y offsets of one subband.
+template <int DPW>
+__device__ __forceinline__ int2 yoffs(const int* p)
+{
+    if constexpr (DPW == 2) return *reinterpret_cast<const int2*>(p);
+    return make_int2(p[0], p[0]);
+}
 
 template <int MODE, int DPW, bool FLUSH>
 __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
@@ -541,7 +549,12 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
     for (int j = 0; j < DPW; ++j)
 #pragma unroll
         for (int k = 0; k < 2 * W; ++k) acc[j][k] = 0;
-    const int d0 = blk * a.ndb + warp;  // the warp's DM trials: d0, d0 + 16
+    // the warp's DM trials in the block: neighbours, which may read the same
+    // Y, or (1..4 bits, whose loop has no registers left to compare) 16 apart,
+    // so that a block that is not full leaves no warp without one
+    constexpr int kStep = MODE == kTrSmall ? kTrWarps : 1;
+    const int s0 = MODE == kTrSmall ? warp : DPW * warp;
+    const int d0 = blk * a.ndb + s0;
     const int dend = min(a.ndm, (blk + 1) * a.ndb);
     bool flushed = false;
     int since = 0;
@@ -596,7 +609,7 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
                 const uint32_t* x2 = pl + src.z + k;
                 const uint32_t* x3 = pl + src.w + k;
                 uint32_t* y = ysm + (32 * g + lane) * kYWords;
-#pragma unroll 4
+#pragma unroll 8
                 for (int m = 0; m < n; ++m) {
                     const uint32_t v0 = x0[32 * m], v1 = x1[32 * m], v2 = x2[32 * m],
                                    v3 = x3[32 * m];
@@ -629,8 +642,8 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
             if (since + nch > a.p16) {
 #pragma unroll
                 for (int j = 0; j < DPW; ++j) {
-                    if (d0 + j * kTrWarps < dend) {
-                        float* o = a.out + (size_t)a.dmrow[d0 + j * kTrWarps] * a.out_pitch + t0 + lane;
+                    if (d0 + j * kStep < dend) {
+                        float* o = a.out + (size_t)a.dmrow[d0 + j * kStep] * a.out_pitch + t0 + lane;
                         each(j, [&](int t, uint32_t v) {
                             o[t] = flushed ? o[t] + (float)v : (float)v;
                         });
@@ -644,13 +657,14 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
             since += nch;
         }
         // one Y per subband and DM trial
-        const int nb = (nch + S - 1) / S;
-        const int* sy = s_yoff + (q & 1) * nsb * kSlots + warp;
+        // (1..4 bits: tested below, per trial)
+        const int nb = MODE == kTrSmall || d0 < dend ? (nch + S - 1) / S : 0;
+        const int* sy = s_yoff + (q & 1) * nsb * kSlots + s0;
+        if constexpr (MODE == kTrSmall) {
+            // bytes as they stand while they cannot overflow
 #pragma unroll
-        for (int j = 0; j < DPW; ++j) {
-            if (d0 + j * kTrWarps >= dend) continue;
-            if constexpr (MODE == kTrSmall) {
-                // bytes as they stand while they cannot overflow
+            for (int j = 0; j < DPW; ++j) {
+                if (d0 + j * kStep >= dend) continue;
                 for (int b0 = 0; b0 < nb; b0 += a.p8s) {
                     uint32_t a8[W];
 #pragma unroll
@@ -658,7 +672,7 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
                     const int b1 = min(nb, b0 + a.p8s);
 #pragma unroll 2
                     for (int b = b0; b < b1; ++b) {
-                        const uint32_t* y = ysm + sy[b * kSlots + j * kTrWarps] + lane;
+                        const uint32_t* y = ysm + sy[b * kSlots + j * kStep] + lane;
 #pragma unroll
                         for (int k = 0; k < W; ++k) a8[k] += y[32 * k];
                     }
@@ -668,15 +682,32 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
                         acc[j][W + k] += __byte_perm(a8[k], 0, 0x4341);
                     }
                 }
-            } else {
-#pragma unroll 2
-                for (int b = 0; b < nb; ++b) {
-                    const uint2* y = reinterpret_cast<const uint2*>(ysm) + sy[b * kSlots + j * kTrWarps] + lane;
+            }
+        } else {
+            // A warp's two trials are neighbours and read the same Y where
+            // their offsets agree (18 % of them at survey spacing).  Not
+            // unrolled: two subbands at a time spilled registers.
+            const uint2* y2 = reinterpret_cast<const uint2*>(ysm) + lane;
+#pragma unroll 1
+            for (int b = 0; b < nb; ++b) {
+                const int2 off = yoffs<DPW>(sy + b * kSlots);
+                uint2 v[W];
+#pragma unroll
+                for (int k = 0; k < W; ++k) v[k] = y2[off.x + 32 * k];
+#pragma unroll
+                for (int k = 0; k < W; ++k) {
+                    acc[0][k] += v[k].x;
+                    acc[0][W + k] += v[k].y;
+                }
+                if constexpr (DPW == 2) {
+                    if (off.y != off.x) {
+#pragma unroll
+                        for (int k = 0; k < W; ++k) v[k] = y2[off.y + 32 * k];
+                    }
 #pragma unroll
                     for (int k = 0; k < W; ++k) {
-                        const uint2 v = y[32 * k];
-                        acc[j][k] += v.x;
-                        acc[j][W + k] += v.y;
+                        acc[1][k] += v[k].x;
+                        acc[1][W + k] += v[k].y;
                     }
                 }
             }
@@ -684,8 +715,8 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
     }
 #pragma unroll
     for (int j = 0; j < DPW; ++j) {
-        if (d0 + j * kTrWarps >= dend) continue;
-        float* o = a.out + (size_t)a.dmrow[d0 + j * kTrWarps] * a.out_pitch + t0 + lane;
+        if (d0 + j * kStep >= dend) continue;
+        float* o = a.out + (size_t)a.dmrow[d0 + j * kStep] * a.out_pitch + t0 + lane;
         each(j, [&](int t, uint32_t v) {
             if constexpr (FLUSH) {
                 if (flushed) v += (uint32_t)o[t];
@@ -1020,6 +1051,8 @@ struct psx_dedisp_plan {
                 for (int e = e0; e < e1; ++e)
                     row[e - e0] = ybase[which[(size_t)e * nsbt + b]] +
                                   shift[(size_t)order[e] * nlive + c0];
+                // a warp's missing second trial reads what its first one does
+                if (e1 - e0 < slots) row[e1 - e0] = row[e1 - e0 - 1];
                 at += n;
             }
         }
