@@ -415,7 +415,10 @@ typedef struct {
                                   fusion itself */
     int use_graph;             /* batched: capture the trial schedule */
     int harm_shape;            /* harmonic-kernel tile shape 1..PSX_HARM_SHAPES;
-                                  0 = default (psx_autotune picks one) */
+                                  0 = default: the three-row shape for fft_size
+                                  2^20 .. 2^23 where a launch group has its
+                                  rows, else the single-row one
+                                  (psx_autotune picks one by timing) */
     int lanes;                 /* batched: launch groups alternate over this
                                   many streams with their own buffers, so one
                                   group's harmonic sums overlap the next one's
@@ -435,14 +438,17 @@ typedef struct {
     int group_dms;             /* batched: DM trials of a psx_search_block
                                   call whose per-DM prologues (baseline
                                   removal through the inverse transform) run
-                                  as one batch of row-indexed launches and
-                                  batched cuFFT plans (with fft_form 3 their
-                                  acceleration trials then run as one list,
-                                  in launch groups across the DM trials).
-                                  0 = default: 4 when
+                                  as one batch of row-indexed launches
+                                  (with fft_form 3 on the library's own
+                                  transform, and their acceleration trials
+                                  then run as one list, in launch groups
+                                  across the DM trials; else on batched cuFFT
+                                  plans).  0 = default, when
                                   fft_size <= 2^22 and the call's DM trials
-                                  average at most 32 acceleration trials,
-                                  else off; 1 = off; 2..16 = that many
+                                  average at most 32 acceleration trials:
+                                  16 up to 2^19, 8 up to 2^21, else 4 (4 with
+                                  the other forms); otherwise off; 1 = off;
+                                  2..16 = that many
                                   whenever the call has more DM trials than
                                   that.  Results do not depend on it. */
 } psx_search_config;

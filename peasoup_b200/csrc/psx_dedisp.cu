@@ -23,7 +23,9 @@
 // two aligned 32-bit loads, one funnel shift, and (8-bit samples) two byte
 // permutes into packed 16-bit accumulators.  Consecutive CTAs take the same
 // time tile for successive DM blocks, so the window is read from HBM once
-// and from L2 after that.
+// and from L2 after that.  Where the DM trials of a block share most of their
+// relative shifts, subband sums formed once serve all of them instead
+// (k_dedisperse_tree, below, with the rule at build_tree).
 #include <algorithm>
 #include <climits>
 #include <cmath>

@@ -1,9 +1,10 @@
 // psx_fft4.cu -- the batched search's forward transform, written for
 // sm_100a: per acceleration trial the complex DFT of length M = N/2 of
 // z[m] = x'[2m] + i x'[2m+1] (x' the resampled series) as a four-step
-// transform M = R * C (R = 1024, or 768 for lengths 3 * 2^k) in two passes
-// over HBM, then the real-spectrum
-// unpack fused with interbinning and normalisation.
+// transform M = R * C (R = 1024; 256 for 2^17 and 2^18 points, 2048 and 4096
+// for 2^26 and 2^27, 768 for lengths 3 * 2^k) in two passes over HBM, then the
+// real-spectrum unpack fused with interbinning and normalisation.  The same
+// passes, with other loads, are the two transforms of the per-DM prologue.
 //
 // It replaces, on the batched path, the reference's resample kernel
 // (src/kernels.cu:364-380), its cuFFT R2C call (include/transforms/

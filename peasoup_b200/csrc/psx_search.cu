@@ -7,7 +7,11 @@
 //   before the host takes over) -> zero padding -> R2C -> amplitude ->
 //   5/25/125-bin running median fused with the division of the spectrum ->
 //   birdie zapping -> interbin statistics (device-resident mean*N, std*N)
-//   -> C2R into the resident dereddened series.
+//   -> C2R into the resident dereddened series.  By default (the lengths of
+//   the library's own transform, prologue_own) the baseline's means are
+//   subtracted and the padding made by the transform's loads, and division,
+//   zapping, statistics and both real-complex steps are one kernel; several
+//   DM trials at a time where a call groups them.
 // Per acceleration trial (the hot loop), in launch groups of `batch`:
 //   resample gather -> R2C (one batched cuFFT; by default the library's
 //   two-pass transform with the gather in its first pass) -> k_form_norm
@@ -956,9 +960,11 @@ int psx_search::make_zap_mask()
 // levels, one kernel from spectrum to dereddened spectrum with its
 // statistics, and the two inverse passes.  `tim` holds in turn the forward
 // intermediate, the amplitudes, the inverse's input and the series; src may
-// lie there.  Twelve launches and about 13 N floats of traffic per DM trial,
-// where cuFFT's transforms with the passes between them took 22 launches and
-// 22 N (103 us per DM trial at 2^22 points on B200, now 61).
+// lie there.  Nine launches (twelve where the means are not one cluster
+// kernel) and 13 N floats of traffic per DM trial; mostly bandwidth, launches
+// below 2^19.  Whole calls on B200, with cuFFT's transforms and the passes
+// between them, and so: 48 DM trials of 2^19 points with one acceleration
+// trial each 1654, 739 us; 24 of 2^22 points with a few each 5816, 5190.
 int psx_search::prologue_own(float* tim, float* Xp, void* med, double2* part, float* stat,
                              unsigned* count, float* mean, const SeriesRows& src, size_t ncopy,
                              int rows, bool host_baseline, cudaStream_t ps)

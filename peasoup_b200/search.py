@@ -56,15 +56,16 @@ class SearchParams:
     # (fft_form 3) gathers the resampled series in its first pass instead.
     fft_callback: bool = False
     graph: bool = True             # batched: CUDA-graph trial schedule
-    harm_shape: int = 0            # harmonic-kernel tile shape (0 = default)
+    harm_shape: int = 0            # harmonic-kernel tile shape (0: by length and launch group)
     lanes: int = 0                 # batched: streams the launch groups alternate over (0 = 1)
     fft_form: int = 0              # batched: 0 default (3 for 2^17..2^27, 3*2^17..3*2^23, else 1),
                                    # 1 cuFFT complex transform + fused unpack/interbin,
                                    # 2 the reference's real transform + interbin,
                                    # 3 the library's two-pass transform (resample in pass 1)
     group_dms: int = 0             # batched: DM trials whose prologues run as one batch
-                                   # (0 default: 4 for <= 2^22 points and few trials
-                                   # per DM trial; 1 off; 2..16 that many)
+                                   # (0 default: 16, 8 or 4 by length for <= 2^22 points
+                                   # and few trials per DM trial; 1 off;
+                                   # 2..16 that many)
 
     def to_c(self):
         cfg = SearchConfig()
