@@ -10,7 +10,7 @@
 // (src/kernels.cu:364-380), its cuFFT R2C call (include/transforms/
 // ffter.hpp:23-53) and the spectrum forming and normalising kernels
 // (src/kernels.cu:238-259, :496-507) with three launches:
-//   pass 1 (k_fft4_cols): CTA = 8 columns c of the R x C matrix
+//   pass 1 (k_fft4_cols): CTA = 8 (or 4) columns c of the R x C matrix
 //     z[r * C + c], 512 threads; each thread gathers 16 rows of its column
 //     straight from the dereddened series through the resample index (FP64,
 //     the same device function the resample kernel reads through), then Stockham
@@ -173,11 +173,15 @@ __device__ __forceinline__ void dft3(float2& a, float2& b, float2& c)
 // butterflies per thread; 16 elements (12 for R = 768) per thread.  W is at
 // least 4 so that every row a CTA reads or writes is one whole 32-byte
 // sector (the series of a long segment does not stay in L2): 512 threads
-// and 64 KB of shared memory for R <= 2048, 1024 threads and 128 KB (one
-// CTA per SM) for R = 4096.
+// and 64 KB of shared memory for R <= 1024, 1024 threads and 128 KB (one
+// CTA per SM) above.  Eight columns, 64-byte rows, for R = 2048 although only
+// one CTA is left on an SM: the gather of 2^26 points 574 us per trial on
+// B200 against 650 with four columns and two CTAs (the prologue's two passes
+// 202 and 182 us against 191 and 188).  At R = 1024, whose series stays in
+// L2, sixteen columns were slower (a launch group at 2^23: 1131 us against 1018).
 template <int R>
 struct ColShape {
-    static constexpr int W = R >= 2048 ? 4 : 8;
+    static constexpr int W = R >= 4096 ? 4 : 8;
     static constexpr int J = R / 16;
     static constexpr int TPC = R == 256 ? 16 : J < 64 ? 64 : J;
     static constexpr int R3 = R / 256;
