@@ -175,8 +175,8 @@ __device__ __forceinline__ void dft3(float2& a, float2& b, float2& c)
 // sector (the series of a long segment does not stay in L2): 512 threads
 // and 64 KB of shared memory for R <= 1024, 1024 threads and 128 KB (one
 // CTA per SM) above.  Eight columns, 64-byte rows, for R = 2048 although only
-// one CTA is left on an SM: the gather of 2^26 points 574 us per trial on
-// B200 against 650 with four columns and two CTAs (the prologue's two passes
+// one CTA is left on an SM: the gather of 10 trials of 2^26 points 1721 us on
+// B200 against 1952 with four columns and two CTAs (the prologue's two passes
 // 202 and 182 us against 191 and 188).  At R = 1024, whose series stays in
 // L2, sixteen columns were slower (a launch group at 2^23: 1131 us against 1018).
 template <int R>
@@ -438,6 +438,12 @@ struct RowShape {
     static constexpr int NST = LOGC / 4 + (REM ? 1 : 0);
     static constexpr int THREADS = T * RPC;
     static constexpr size_t SMEM = (size_t)RPC * (C + C / 16) * sizeof(float2);
+    // Rows of 2^14 leave one CTA on an SM, which neither loads nor stores
+    // while it computes: it asks L2 for the row that the SM's next CTA takes.
+    // At 2^26 points 300 us per launch on B200 against 339 (three launches of 3
+    // or 4 trials and the prologue's two); shorter rows, two CTAs and more on an
+    // SM, did not change (2^12: 344-348 against 348-354, inside the spread).
+    static constexpr bool AHEAD = LOGC >= 14;
     // twiddle table offset of the last stage (stage s >= 1 holds R_s * NS_s)
     static constexpr int OFF_LAST = NST == 2 ? 0 : NST == 3 ? 16 * R1 : 16 * R1 + 256 * R1;
 };
@@ -488,7 +494,8 @@ __device__ __forceinline__ void row_stage(float2* s, unsigned t, const float2* _
 template <int LOGC>
 __global__ void __launch_bounds__(RowShape<LOGC>::THREADS, 1024 / RowShape<LOGC>::THREADS)
     k_fft4_rows(const float2* y, size_t ypitch, float2* zt, size_t zpitch,
-                const float2* __restrict__ tw)  // zt may be y: a CTA reads its rows first
+                const float2* __restrict__ tw,  // zt may be y: a CTA reads its rows first
+                unsigned ahead)
 {
     using S = RowShape<LOGC>;
     constexpr int C = S::C, T = S::T;
@@ -501,6 +508,15 @@ __global__ void __launch_bounds__(RowShape<LOGC>::THREADS, 1024 / RowShape<LOGC>
     // stage 0: radix 16, span 1, from the row in HBM
 #pragma unroll
     for (int q = 0; q < 16; ++q) v[q] = yr[t + q * T];
+    if constexpr (S::AHEAD) {
+        // a line per thread of the row that this SM's next CTA takes
+        const unsigned nr = blockIdx.x + ahead, trial = blockIdx.y + nr / gridDim.x;
+        if (trial < gridDim.y) {
+            const float2* p = y + (size_t)trial * ypitch +
+                              ((size_t)(nr % gridDim.x) * S::RPC + lr) * C + 16 * t;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+        }
+    }
     dft<16>(v);
 #pragma unroll
     for (int q = 0; q < 16; ++q) s[pad16(t * 16 + q)] = v[q];
@@ -843,7 +859,8 @@ int launch_rows(unsigned nrows, const float2* y, size_t ypitch, float2* zt, size
 {
     using S = RowShape<LOGC>;
     dim3 grid(nrows / S::RPC, (unsigned)ntrials);
-    k_fft4_rows<LOGC><<<grid, S::THREADS, S::SMEM, s>>>(y, ypitch, zt, zpitch, tw);
+    const unsigned ahead = (unsigned)sm_count() * (1024 / S::THREADS);
+    k_fft4_rows<LOGC><<<grid, S::THREADS, S::SMEM, s>>>(y, ypitch, zt, zpitch, tw, ahead);
     return launch_status("fft4 row pass");
 }
 
