@@ -31,15 +31,20 @@ __device__ __forceinline__ float gather_at(const float* __restrict__ in,
     return idx < n ? in[idx] : 0.0f;
 }
 
-// resampleII read with the output index i given as an exact double and
-// n < 2^32: the expression of resampleII_index, rounded by the same mode to
+// resampleII index and read with the output index i given as an exact double
+// and n < 2^32: the expression of resampleII_index, rounded by the same mode to
 // a 32-bit index (both conversions clamp, so indices outside [0, n) read
 // zero in both forms).  The resample kernel and the gather of the two-pass
 // transform both read through this.
+__device__ __forceinline__ unsigned resampleII_index32(double i, double k, double size)
+{
+    return __double2uint_rn(i + i * k * (i - size));
+}
+
 __device__ __forceinline__ float resampleII_read(const float* __restrict__ in, double i, double k,
                                                  double size, unsigned n)
 {
-    const unsigned idx = __double2uint_rn(i + i * k * (i - size));
+    const unsigned idx = resampleII_index32(i, k, size);
     return idx < n ? in[idx] : 0.0f;
 }
 

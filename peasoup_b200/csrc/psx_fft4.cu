@@ -62,6 +62,7 @@ struct ColArgs {
     size_t ncopy;
     const float* means;      // kColSeries: 4 floats a row
     unsigned offI;           // kColInverse: table of W_M^(J c q)
+    unsigned ahead;          // trials: CTAs between one and the next on its SM
 };
 
 namespace {
@@ -188,7 +189,20 @@ struct ColShape {
     static constexpr int U = 256 / TPC;
     static constexpr int THREADS = W * TPC;
     static constexpr size_t SMEM = (size_t)R * W * sizeof(float2);
+    // A CTA alone on its SM neither loads nor stores while it computes, and
+    // the long series comes from HBM: one lane per row asks L2 for the samples
+    // that the SM's next CTA gathers.  10 trials of 2^26 points 1588 us on
+    // B200 against 1724; a search at 2^27 45.4 ms against 47.2.  All lanes
+    // asking: 1629.  Not for R = 1024 (two CTAs, series in L2: 1067 us a
+    // launch group at 2^23 against 1014), nor for the prologue's two passes
+    // (2^26: 212 and 216 us against 202 and 182).
+    static constexpr bool AHEAD = R >= 2048;
 };
+
+__device__ __forceinline__ void prefetch_l2(const void* p)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
 
 // Shared layout [e][col], e the row index 0..R-1; a row of W columns spans
 // 2W of the 32 banks.  XOR-ing the low bits of e with bits 4.. of e (16/W
@@ -212,6 +226,9 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
 {
     using S = ColShape<R>;
     constexpr bool TRIAL = KIND == kColGather || KIND == kColDump;
+    // the columns that this SM's next CTA takes, `next` pairs further on
+    const unsigned next = a.ahead * S::W;
+    const bool has_next = S::AHEAD && TRIAL && blockIdx.x + a.ahead < gridDim.x;
     if constexpr (TRIAL)
         if (a.trow) x += (size_t)a.trow[blockIdx.y] * a.xpitch;
     static_assert(R == 256 || R == 768 || R == 1024 || R == 2048 || R == 4096, "column length");
@@ -252,6 +269,11 @@ __global__ void __launch_bounds__(ColShape<R>::THREADS, 1024 / ColShape<R>::THRE
                 const double i0 = i_first + (double)q * i_step;  // exact: integers < 2^28
                 v[q].x = resampleII_read(x, i0, k, size, n32);
                 v[q].y = resampleII_read(x, i0 + 1.0, k, size, n32);
+                if constexpr (S::AHEAD && KIND == kColGather) {
+                    // the resampling shift changes slowly along the series
+                    const unsigned i = resampleII_index32(i0, k, size) + 2 * next;
+                    if (col == 0 && has_next && i < n32) prefetch_l2(x + i);
+                }
             }
         } else if constexpr (KIND == kColSeries) {
             const float* xr = a.src.p[blockIdx.y];
@@ -514,7 +536,7 @@ __global__ void __launch_bounds__(RowShape<LOGC>::THREADS, 1024 / RowShape<LOGC>
         if (trial < gridDim.y) {
             const float2* p = y + (size_t)trial * ypitch +
                               ((size_t)(nr % gridDim.x) * S::RPC + lr) * C + 16 * t;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+            prefetch_l2(p);
         }
     }
     dft<16>(v);
@@ -899,12 +921,14 @@ int configure_cols()
 }  // namespace
 
 template <int KIND>
-int Fft4Plan::launch_cols(const float* x, int rows, float2* y, size_t ypitch, const ColArgs& a,
+int Fft4Plan::launch_cols(const float* x, int rows, float2* y, size_t ypitch, const ColArgs& args,
                           cudaStream_t s) const
 {
     auto go = [&](auto kern, auto shape) {
         using S = decltype(shape);
         dim3 ga(C / S::W, (unsigned)rows);
+        ColArgs a = args;
+        a.ahead = (unsigned)sm_count() * (1024 / S::THREADS);
         kern<<<ga, S::THREADS, KIND == kColDump ? 0 : S::SMEM, s>>>(
             x, (unsigned long long)n, d_tab, offA2, offA3, offQ, offP, C, y, ypitch, a);
     };
