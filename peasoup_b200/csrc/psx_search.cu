@@ -629,12 +629,19 @@ struct psx_search {
     float* d_trl[2] = {nullptr, nullptr};
     float* d_Xl[2] = {nullptr, nullptr};
     float* d_pl[2] = {nullptr, nullptr};
-    HarmMaps hmaps[2] = {};  // per lane: the spectra as boxes of the multi-row shape's rows
+    HarmMaps hmaps[2] = {};  // per lane: the spectra as boxes of map_rows rows
+    int map_rows = 0;        // 0: not encoded
     bool harm_auto = false;  // no shape asked for: shape_for picks per launch group
     int shape_for(int trials) const
     {
         const int rows = kHarmShapes[kHarmRowsShape - 1].rows;
         return harm_auto && (trials % rows == 0 || trials >= 4 * rows) ? kHarmRowsShape : harm_shape;
+    }
+    // The maps a shape reads its rows through; null where they are not the
+    // ones it needs (its launch is then refused).
+    const HarmMaps* maps_for(int shape, int lane) const
+    {
+        return map_rows == kHarmShapes[shape - 1].rows ? &hmaps[lane] : nullptr;
     }
     float* d_tr = nullptr;
     float* d_X = nullptr;
@@ -711,6 +718,7 @@ struct psx_search {
         for (void* q : dev)
             if (q) cudaFree(q);
         for (int l = 0; l < 2; ++l) d_trl[l] = d_Xl[l] = d_pl[l] = nullptr;
+        map_rows = 0;
         d_tr = d_X = d_p = d_bf = d_bw = nullptr;
         d_zap = nullptr;
         if (ev_fork) cudaEventDestroy(ev_fork);
@@ -764,6 +772,7 @@ struct psx_search {
     int prologue(Slot& s);
     bool readable(const Slot& s) const;
     int make_zap_mask();
+    int make_harm_maps();
     int host_baseline_loop(Slot& s, size_t ncopy, cudaStream_t ps);
     int prologue_own(float* tim, float* Xp, void* med, double2* part, float* stat,
                      unsigned* count, float* mean, const SeriesRows& src, size_t ncopy, int rows,
@@ -951,6 +960,18 @@ int psx_search::make_zap_mask()
     if (!d_zap || bf.empty()) return PSX_OK;
     PSX_CUDA(cudaStreamSynchronize(nullptr));  // the birdie list's copies
     return launch_zap_mask(d_zap, d_bf, d_bw, bin_width_f, bf.size(), B, st);
+}
+
+// Tensor maps over the lanes' spectra for the multi-row shape that this
+// configuration asks for or may take by default.
+int psx_search::make_harm_maps()
+{
+    const int rows = kHarmShapes[(harm_auto ? kHarmRowsShape : harm_shape) - 1].rows;
+    if (rows == 0 || rows == map_rows) return PSX_OK;
+    map_rows = 0;
+    for (int l = 0; l < lanes; ++l) PSX_TRY(encode_harm_maps(d_pl[l], Bp, batch, rows, &hmaps[l]));
+    map_rows = rows;
+    return PSX_OK;
 }
 
 // src/pipeline_multi.cu:170-238 on the library's own transform, for `rows`
@@ -1145,7 +1166,7 @@ int psx_search::trials_span(GroupSet& g, int cnt)
             const int rem = rows > 1 ? b % rows : 0, bm = b - rem;
             if (bm > 0) {
                 PSX_TRY(launch_harm(F, shape, pp, Bp, (unsigned)Bp, pk, t0, bm, g.d_rec,
-                                    g.d_cnt, (unsigned)g.rec_cap, st, &hmaps[0]));
+                                    g.d_cnt, (unsigned)g.rec_cap, st, maps_for(shape, 0)));
                 ++g.launches;
             }
             if (rem > 0) {
@@ -1545,7 +1566,7 @@ int psx_search::trials_range(Slot& s, int t_begin, int nacc, bool reset)
             const int rem = rows > 1 ? b % rows : 0, bm = b - rem;
             if (bm > 0) {
                 PSX_TRY(launch_harm(F, shape, pp, Bp, (unsigned)Bp, pk, t0, bm, s.d_rec,
-                                    s.d_count, (unsigned)s.rec_cap, ls, &hmaps[lane]));
+                                    s.d_count, (unsigned)s.rec_cap, ls, maps_for(shape, lane)));
                 ++s.launches;
             }
             if (rem > 0) {
@@ -2202,11 +2223,7 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
     s->d_tr = s->d_trl[0];
     s->d_X = s->d_Xl[0];
     s->d_p = s->d_pl[0];
-    const int map_rows = kHarmShapes[(s->harm_auto ? kHarmRowsShape : s->harm_shape) - 1].rows;
-    if (map_rows > 0)
-        for (int l = 0; l < s->lanes; ++l)
-            if ((rc = encode_harm_maps(s->d_pl[l], Bp, (int)b, map_rows, &s->hmaps[l])) != PSX_OK)
-                return fail(rc);
+    if ((rc = s->make_harm_maps()) != PSX_OK) return fail(rc);
     for (Slot& sl : s->slot) {
         ALLOC(sl.d_tim, sizeof(float) * N);
         ALLOC(sl.d_Xp, sizeof(float) * 2 * Bp);
@@ -2401,6 +2418,7 @@ int psx_search_retarget(psx_search* s, const psx_search_config* cfg)
         PSX_CUDA(cudaMemcpy(s->d_bw, s->bw.data(), sizeof(float) * s->bw.size(),
                             cudaMemcpyHostToDevice));
     }
+    PSX_TRY(s->make_harm_maps());
     PSX_TRY(s->make_zap_mask());
     PSX_CUDA(cudaStreamSynchronize(s->st));  // the prologues run on streams of their own
     // captured schedules hold the old search ranges by value
