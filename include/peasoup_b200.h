@@ -598,7 +598,10 @@ int psx_search_debug_tap(psx_search* s, int trial, float* h_tim_dered,
    mode, batch, harmonic shape, lanes, transform path and prologue
    grouping rows (the things its buffers and plans depend on): fold count,
    acceleration range, tsamp, thresholds,
-   frequency limits and birdies may all change.  Waits for the instance's
+   frequency limits and birdies may all change.  Defaults match what they
+   are documented to stand for: harm_shape 0 and 4, group_dms 0 and 4 up to
+   2^22 points, fft_form 0 and 1 at 2^17 and 2^18 points; where the instance
+   holds something else for them, that part of it is made anew.  Waits for the instance's
    queued work first.  No counterpart in the reference (whose Worker builds
    its transforms once per process, src/pipeline_multi.cu:114-149). */
 int psx_search_retarget(psx_search* s, const psx_search_config* cfg);

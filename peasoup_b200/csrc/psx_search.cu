@@ -401,6 +401,9 @@ static int launch_harm(int F, int shape, const float* p, size_t ppitch, unsigned
 }
 
 constexpr int kDeviceBaselinePasses = 4;
+// Shortest length where the two-pass transform may be asked for by name
+// (fft_form 3); 2^17 and 2^18 points take it by default only.
+constexpr size_t kOwnAskedMinPoints = (size_t)3 << 17;
 // Records that come back with the counters: most DM trials have no more, and
 // a second copy with a wait of its own costs 15 to 20 us.
 constexpr size_t kFirstRecords = 1024;
@@ -713,7 +716,9 @@ struct psx_search {
             for (auto& p : m) delete p.second;
             m.clear();
         }
+        capture_failures.clear();
         r2c1.destroy();
+        f4.destroy();
         void* dev[] = {d_trl[0], d_Xl[0], d_pl[0], d_trl[1], d_Xl[1], d_pl[1], d_bf, d_bw, d_zap};
         for (void* q : dev)
             if (q) cudaFree(q);
@@ -721,6 +726,7 @@ struct psx_search {
         map_rows = 0;
         d_tr = d_X = d_p = d_bf = d_bw = nullptr;
         d_zap = nullptr;
+        bird_cap = 0;
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         ev_fork = ev_join = nullptr;
@@ -728,7 +734,6 @@ struct psx_search {
         call_start = nullptr;
         if (h_mean) cudaFreeHost(h_mean);
         h_mean = nullptr;
-        last_dm = nullptr;
         free_groups();
         for (Slot& s : slot) {
             if (s.d_count) cudaFree(s.d_count);
@@ -1328,6 +1333,7 @@ void psx_search::free_groups()
 {
     for (Slot& s : slot)
         if (s.pst) cudaStreamSynchronize(s.pst);
+    last_dm = nullptr;
     for (GroupSet& g : gset) {
         for (Slot& s : g.slots) {
             if (s.d_rec) cudaFree(s.d_rec);
@@ -1373,7 +1379,7 @@ void psx_search::free_groups()
 // beside another's trials.
 int psx_search::group_rows_for_call(const float* dms, int ndm) const
 {
-    const int G = group_rows_for(&cfg);
+    const int G = (int)gset[0].slots.size();
     if (cfg.group_dms >= 2) return ndm > G ? G : 0;
     if (G < 2 || ndm <= kGroupRowsDefault) return 0;
     const psx_search_config& c = cfg;
@@ -2006,7 +2012,7 @@ static int check_config(const psx_search_config* c)
     }
     // (2^17 and 2^18 points take the two-pass transform by default only)
     if (c->fft_form == 3 && (c->mode != PSX_MODE_BATCHED || !Fft4Plan::supported(c->fft_size) ||
-                             c->fft_size < ((size_t)3 << 17))) {
+                             c->fft_size < kOwnAskedMinPoints)) {
         set_error("search: fft_form 3 needs the batched mode and "
                   "fft_size 2^19 .. 2^27 or 3 * 2^17 .. 3 * 2^23");
         return PSX_ERR_INVALID;
@@ -2183,30 +2189,25 @@ static void host_setup(psx_search* s, const psx_search_config* cfg)
     s->pk.flags = 0;
 }
 
-int psx_search_create(const psx_search_config* cfg, psx_search** out)
+// Buffers, streams and plans of a new or released instance for cfg (checked)
+// on the current device.  A compute stream that is there already (the
+// caller's) is kept.
+static int make_instance(psx_search* s, const psx_search_config* cfg)
 {
-    clear_error();
-    if (!out) return PSX_ERR_INVALID;
-    *out = nullptr;
-    PSX_TRY(check_config(cfg));
-    psx_search* s = new (std::nothrow) psx_search;
-    if (!s) return PSX_ERR_ALLOC;
     host_setup(s, cfg);
 
     int rc = PSX_OK;
-    auto fail = [&](int code) {
-        delete s;
-        return code;
-    };
-    if ((rc = cuda_status(cudaGetDevice(&s->device), "cudaGetDevice")) != PSX_OK) return fail(rc);
-    if ((rc = configure_harm(s->F)) != PSX_OK) return fail(rc);
-    if ((rc = cuda_status(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking),
-                          "cudaStreamCreate")) != PSX_OK)
-        return fail(rc);
-    s->own_stream = true;
+    if ((rc = cuda_status(cudaGetDevice(&s->device), "cudaGetDevice")) != PSX_OK) return rc;
+    if ((rc = configure_harm(s->F)) != PSX_OK) return rc;
+    if (!s->st) {
+        if ((rc = cuda_status(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking),
+                              "cudaStreamCreate")) != PSX_OK)
+            return rc;
+        s->own_stream = true;
+    }
     if ((rc = cuda_status(cudaStreamCreateWithFlags(&s->cst, cudaStreamNonBlocking),
                           "cudaStreamCreate")) != PSX_OK)
-        return fail(rc);
+        return rc;
     const size_t N = s->N, Bp = s->Bp;
     const size_t b = (size_t)s->batch;
     s->med_floats = median_scratch_bytes(s->B) / sizeof(float);
@@ -2214,7 +2215,7 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
 #define ALLOC(ptr, bytes)                                                        \
     if ((rc = cuda_status(cudaMalloc((void**)&(ptr), (bytes)), "cudaMalloc")) != \
         PSX_OK)                                                                  \
-        return fail(rc == PSX_ERR_CUDA ? PSX_ERR_ALLOC : rc);
+        return rc == PSX_ERR_CUDA ? PSX_ERR_ALLOC : rc;
     for (int l = 0; l < s->lanes; ++l) {
         ALLOC(s->d_trl[l], sizeof(float) * N * b);
         ALLOC(s->d_Xl[l], sizeof(float) * 2 * Bp * b);
@@ -2223,7 +2224,7 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
     s->d_tr = s->d_trl[0];
     s->d_X = s->d_Xl[0];
     s->d_p = s->d_pl[0];
-    if ((rc = s->make_harm_maps()) != PSX_OK) return fail(rc);
+    if ((rc = s->make_harm_maps()) != PSX_OK) return rc;
     for (Slot& sl : s->slot) {
         ALLOC(sl.d_tim, sizeof(float) * N);
         ALLOC(sl.d_Xp, sizeof(float) * 2 * Bp);
@@ -2240,24 +2241,24 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
         s->bird_cap = s->bf.size();
     }
 #undef ALLOC
-    if (cudaMallocHost(&s->h_mean, sizeof(float) * 4) != cudaSuccess) return fail(PSX_ERR_ALLOC);
+    if (cudaMallocHost(&s->h_mean, sizeof(float) * 4) != cudaSuccess) return PSX_ERR_ALLOC;
     for (Slot& sl : s->slot) {
         if (cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&sl.copied, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&sl.ready, cudaEventDisableTiming) != cudaSuccess)
-            return fail(PSX_ERR_CUDA);
+            return PSX_ERR_CUDA;
         if ((rc = cuda_status(cudaStreamCreateWithFlags(&sl.pst, cudaStreamNonBlocking),
                               "cudaStreamCreate")) != PSX_OK)
-            return fail(rc);
+            return rc;
         if (!s->use_f4) {
             sl.r2c = new (std::nothrow) FftPlan;
             sl.c2r = new (std::nothrow) FftPlan;
-            if (!sl.r2c || !sl.c2r) return fail(PSX_ERR_ALLOC);
-            if ((rc = sl.r2c->create(N, 1, PSX_FFT_R2C, 0, 0)) != PSX_OK) return fail(rc);
-            if ((rc = sl.c2r->create(N, 1, PSX_FFT_C2R, 0, 0)) != PSX_OK) return fail(rc);
+            if (!sl.r2c || !sl.c2r) return PSX_ERR_ALLOC;
+            if ((rc = sl.r2c->create(N, 1, PSX_FFT_R2C, 0, 0)) != PSX_OK) return rc;
+            if ((rc = sl.c2r->create(N, 1, PSX_FFT_C2R, 0, 0)) != PSX_OK) return rc;
         }
-        if ((rc = s->grow_records(sl, (size_t)1 << 20)) != PSX_OK) return fail(rc);
-        if ((rc = s->grow_ktab(sl, 1024)) != PSX_OK) return fail(rc);
+        if ((rc = s->grow_records(sl, (size_t)1 << 20)) != PSX_OK) return rc;
+        if ((rc = s->grow_ktab(sl, 1024)) != PSX_OK) return rc;
     }
     if (!s->bf.empty()) {
         cudaMemcpy(s->d_bf, s->bf.data(), sizeof(float) * s->bf.size(), cudaMemcpyHostToDevice);
@@ -2271,27 +2272,27 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
     if (s->lanes > 1) {
         if ((rc = cuda_status(cudaStreamCreateWithFlags(&s->st2, cudaStreamNonBlocking),
                               "cudaStreamCreate")) != PSX_OK)
-            return fail(rc);
+            return rc;
         if (cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming) != cudaSuccess)
-            return fail(PSX_ERR_CUDA);
+            return PSX_ERR_CUDA;
     }
     for (Slot& sl : s->slot) {
         cudaMemsetAsync(sl.d_Xp, 0, sizeof(float) * 2 * Bp, s->st);
     }
     if (cudaEventCreateWithFlags(&s->call_start, cudaEventDisableTiming) != cudaSuccess)
-        return fail(PSX_ERR_CUDA);
-    if (!s->use_f4 && (rc = s->r2c1.create(N, 1, PSX_FFT_R2C, 0, 0)) != PSX_OK) return fail(rc);
-    if ((rc = s->make_zap_mask()) != PSX_OK) return fail(rc);
+        return PSX_ERR_CUDA;
+    if (!s->use_f4 && (rc = s->r2c1.create(N, 1, PSX_FFT_R2C, 0, 0)) != PSX_OK) return rc;
+    if ((rc = s->make_zap_mask()) != PSX_OK) return rc;
     if (s->fft4()) {
-        if ((rc = s->f4.create(N)) != PSX_OK) return fail(rc);
+        if ((rc = s->f4.create(N)) != PSX_OK) return rc;
     } else if (s->batched()) {
         FftPlan* p = nullptr;
         for (int l = 0; l < s->lanes; ++l)
-            if ((rc = s->get_plan(s->batch, &p, l)) != PSX_OK) return fail(rc);
+            if ((rc = s->get_plan(s->batch, &p, l)) != PSX_OK) return rc;
     }
     if ((rc = cuda_status(cudaStreamSynchronize(s->st), "search create")) != PSX_OK)
-        return fail(rc);
+        return rc;
     s->info.batch = s->batch;
     s->info.harm_shape = s->harm_shape;
     s->info.fft_callback = 0;
@@ -2301,7 +2302,22 @@ int psx_search_create(const psx_search_config* cfg, psx_search** out)
     for (int k = 0; k < 2; ++k) s->set_pst[0][k] = s->slot[k].pst;
     // group sets made now (their bytes are in the footprint), so a call
     // that groups does not pay for them on first use
-    if ((rc = s->alloc_groups()) != PSX_OK) return fail(rc);
+    return s->alloc_groups();
+}
+
+int psx_search_create(const psx_search_config* cfg, psx_search** out)
+{
+    clear_error();
+    if (!out) return PSX_ERR_INVALID;
+    *out = nullptr;
+    PSX_TRY(check_config(cfg));
+    psx_search* s = new (std::nothrow) psx_search;
+    if (!s) return PSX_ERR_ALLOC;
+    const int rc = make_instance(s, cfg);
+    if (rc != PSX_OK) {
+        delete s;
+        return rc;
+    }
     *out = s;
     return PSX_OK;
 }
@@ -2376,6 +2392,21 @@ int psx_harmonic_peaks(const float* d_spec, size_t pitch, size_t nbins, int rows
     return PSX_OK;
 }
 
+// What has to match between an instance and the configuration it is
+// retargeted to, with the defaults spelled out: no shape asked for counts as
+// the single-row one, no grouping asked for as kGroupRowsDefault rows up to
+// kGroupMaxPoints, and the lengths that take the two-pass transform by default
+// only (2^17 and 2^18 points) as cuFFT's.  Which rows, shape and transform a
+// default then stands for is the instance's own affair.
+static psx_search_config retarget_key(const psx_search_config* cfg)
+{
+    psx_search_config k = *cfg;
+    if (!k.harm_shape) k.harm_shape = kHarmDefaultShape;
+    if (!k.group_dms) k.group_dms = k.fft_size <= kGroupMaxPoints ? kGroupRowsDefault : 1;
+    if (!k.fft_form && k.fft_size < kOwnAskedMinPoints) k.fft_form = 1;
+    return k;
+}
+
 int psx_search_retarget(psx_search* s, const psx_search_config* cfg)
 {
     clear_error();
@@ -2384,12 +2415,12 @@ int psx_search_retarget(psx_search* s, const psx_search_config* cfg)
         return PSX_ERR_INVALID;
     }
     PSX_TRY(check_config(cfg));
-    const int shape = cfg->harm_shape ? cfg->harm_shape : kHarmDefaultShape;
-    if (cfg->fft_size != s->N || cfg->mode != s->cfg.mode ||
-        effective_batch(cfg) != s->batch || shape != s->harm_shape ||
-        effective_lanes(cfg) != s->lanes ||
-        effective_form(cfg) != effective_form(&s->cfg) ||
-        group_rows_for(cfg) != group_rows_for(&s->cfg)) {
+    const psx_search_config want = retarget_key(cfg), have = retarget_key(&s->cfg);
+    if (want.fft_size != have.fft_size || want.mode != have.mode ||
+        effective_batch(&want) != effective_batch(&have) || want.harm_shape != have.harm_shape ||
+        effective_lanes(&want) != effective_lanes(&have) ||
+        effective_form(&want) != effective_form(&have) ||
+        group_rows_for(&want) != group_rows_for(&have)) {
         set_error("search_retarget: fft_size, mode, batch, harmonic shape, lanes, "
                   "transform path and prologue grouping must match the instance");
         return PSX_ERR_INVALID;
@@ -2399,6 +2430,18 @@ int psx_search_retarget(psx_search* s, const psx_search_config* cfg)
     PSX_CUDA(cudaStreamSynchronize(s->st));
     PSX_CUDA(cudaStreamSynchronize(s->cst));
     for (Slot& sl : s->slot) PSX_CUDA(cudaStreamSynchronize(sl.pst));
+    if (effective_form(cfg) != effective_form(&s->cfg) || effective_batch(cfg) != s->batch) {
+        // another transform or launch group under the same key (the short
+        // lengths): made anew, on the caller's stream if it has one.  Where
+        // that fails the instance holds nothing and its calls return an error.
+        cudaStream_t own = s->own_stream ? nullptr : s->st;
+        s->release();
+        s->st = own;
+        const int rc = make_instance(s, cfg);
+        if (rc != PSX_OK) s->release();
+        return rc;
+    }
+    const int rows = group_rows_for(&s->cfg);
     // the fold count only selects the harmonic kernel's instantiation (no
     // buffer depends on it): opt that one into its shared memory
     PSX_TRY(configure_harm(cfg->nharmonics));
@@ -2417,6 +2460,10 @@ int psx_search_retarget(psx_search* s, const psx_search_config* cfg)
                             cudaMemcpyHostToDevice));
         PSX_CUDA(cudaMemcpy(s->d_bw, s->bw.data(), sizeof(float) * s->bw.size(),
                             cudaMemcpyHostToDevice));
+    }
+    if (group_rows_for(cfg) != rows) {
+        s->free_groups();
+        PSX_TRY(s->alloc_groups());
     }
     PSX_TRY(s->make_harm_maps());
     PSX_TRY(s->make_zap_mask());

@@ -51,11 +51,11 @@ def _equal_to_fresh(s, p, xs):
 
 @pytest.mark.parametrize("first,then", [(4, 0), (0, 4)])
 def test_harmonic_shape_asked_for_and_by_default(cuda, first, then):
-    """Groups of twelve trials at 2^20 points take the three-row shape by
+    """Groups of twelve trials at 2^21 points take the three-row shape by
     default: its tensor maps are there also where the instance was made for
     the single-row one."""
     from peasoup_b200 import search
-    n = 1 << 20
+    n = 1 << 21
     xs = _series(n, 1)
     kw = dict(batch=12)
     s = search.AccelSearch(_params(n, 800.0, harm_shape=first, **kw))
@@ -78,4 +78,41 @@ def test_what_does_not_match_stays_refused(cuda):
                 _params(n, 100.0, batch=12, mode="plain")):
         assert _retarget(s, bad) == _lib.PSX_ERR_INVALID
     _equal_to_fresh(s, _params(n, 100.0, **base), _series(n, 1))
+    s.close()
+
+
+@pytest.mark.parametrize("first,then", [(0, 4), (4, 0)])
+def test_grouping_asked_for_and_by_default(cuda, first, then):
+    """Four DM trials to a grouped prologue, by name or as the default's
+    least, match; what the default takes at this length (16) is made anew."""
+    from peasoup_b200 import search
+    n = 1 << 19
+    xs = _series(n, 26)
+    s = search.AccelSearch(_params(n, 0.0, group_dms=first))
+    for g in (then, first):
+        p = _params(n, 0.0, group_dms=g)
+        assert _retarget(s, p) == 0
+        assert _equal_to_fresh(s, p, xs)["group_dms"] == (4 if g else 9)
+    s.close()
+
+
+@pytest.mark.parametrize("own_stream", [True, False])
+def test_short_lengths_with_cufft_asked_for_and_by_default(cuda, own_stream):
+    """2^17 points: the default and cuFFT's transform by name match, and
+    launch groups count as its powers of two; birdies go along."""
+    from peasoup_b200 import search
+    n = 1 << 17
+    xs = _series(n, 7)
+    birdies = dict(birdie_freqs=np.array([50.0], np.float32),
+                   birdie_widths=np.array([0.5], np.float32))
+    s = search.AccelSearch(_params(n, 40.0, batch=16, **birdies))
+    st = cuda.cuda.Stream()
+    if not own_stream:
+        s.set_stream(st.cuda_stream)
+    for kw in (dict(batch=16, fft_form=1), dict(batch=24), dict(batch=24, fft_form=1, **birdies),
+               dict(batch=16, **birdies), dict(batch=16)):
+        p = _params(n, 40.0, **kw)
+        assert _retarget(s, p) == 0
+        info = _equal_to_fresh(s, p, xs)
+        assert info["fft_form"] == (1 if kw.get("fft_form") else 3)
     s.close()
