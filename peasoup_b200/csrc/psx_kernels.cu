@@ -753,27 +753,61 @@ __global__ void __launch_bounds__(kVecThreads) k_interbin_partials_v4(const floa
 
 int reduction_blocks() { return sm_count() * 2; }
 
-// Sum of (x - m0) - m1 over [0, n) by the CTAs of a row, with 128-bit loads
-// where x is 16-byte aligned (x - 0 is x).
-__device__ __forceinline__ double sum_less(const float* __restrict__ x, size_t n, float m0, float m1)
+// The means of the baseline loop are sums over fixed pieces of the series,
+// one warp to a piece, added in one order: the 16 pieces of a group, then the
+// groups, 32 apart to a lane.  A mean then depends on the samples alone and
+// not on the rows that share its launch, the CTAs of a row or the address of
+// the series, and with it the dereddened series of a DM trial, bit for bit.
+// 512 pieces up to 2^21 samples, one to a warp of a 16-CTA cluster; 2048, four
+// to such a warp, up to 2^23, the longest row a cluster takes; 4096 above,
+// where the series come from HBM (2^26 samples, whole search: 7151 us on B200
+// with 2048 pieces, 7106 with 4096; 12 series of 2^23: 2300 and 2455).
+constexpr size_t kMeanShort = (size_t)1 << 21, kMeanMedium = (size_t)1 << 23;
+constexpr unsigned kMeanGroup = 16;
+inline unsigned mean_pieces(size_t n)
 {
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t done = 0;
-    double s = 0.0;
+    return n <= kMeanShort ? 512u : n <= kMeanMedium ? 2048u : 4096u;
+}
+
+__device__ __forceinline__ double warp_total(double v, int width)
+{
+    for (int o = width / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Adds (x - m0) - m1 (x - 0 is x) over pieces first + k W, k < K, of
+// `pieces` to this lane's s[k].  Piece v holds the runs of 128 samples
+// v, v + pieces, ..., four consecutive samples to a lane; the n % 4 last
+// samples go to piece 0.
+template <int K>
+__device__ __forceinline__ void piece_sums(const float* __restrict__ x, size_t n, unsigned pieces,
+                                           unsigned first, unsigned W, float m0, float m1,
+                                           double (&s)[K])
+{
+    const unsigned lane = threadIdx.x & 31;
+    const size_t n4 = n / 4, steps = n4 / 32 / pieces;
     auto less = [&](float v) { return (double)((v - m0) - m1); };
-    if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
-        done = n / 4 * 4;
-        const float4* x4 = reinterpret_cast<const float4*>(x);
-#pragma unroll 8
-        for (size_t q = first; q < n / 4; q += stride) {
-            const float4 v = x4[q];
-            s += (less(v.x) + less(v.y)) + (less(v.z) + less(v.w));
-        }
-    }
-#pragma unroll 4
-    for (size_t i = done + first; i < n; i += stride) s += less(x[i]);
-    return s;
+    auto run = [&](auto load) {
+        auto add = [&](double& t, const float* p) {
+            const float4 v = load(p);
+            t += (less(v.x) + less(v.y)) + (less(v.z) + less(v.w));
+        };
+        const size_t step = (size_t)pieces * 128;
+        const unsigned next = W * 128;
+        const float* p = x + ((size_t)first * 32 + lane) * 4;
+#pragma unroll (8 / K)
+        for (size_t j = 0; j < steps; ++j, p += step)  // eight loads in flight
+#pragma unroll
+            for (int k = 0; k < K; ++k) add(s[k], p + k * next);
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if ((steps * pieces + first + k * W) * 32 + lane < n4) add(s[k], p + k * next);
+    };
+    if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0)
+        run([](const float* p) { return *reinterpret_cast<const float4*>(p); });
+    else
+        run([](const float* p) { return make_float4(p[0], p[1], p[2], p[3]); });
+    if (first == 0 && lane < n - 4 * n4) s[0] += less(x[4 * n4 + lane]);
 }
 
 // The device-side baseline loop (reference src/kernels.cu:463-479) without
@@ -781,27 +815,34 @@ __device__ __forceinline__ double sum_less(const float* __restrict__ x, size_t n
 // would subtract next, from the sums of the series less the means found so
 // far (the subtraction itself, in the same order and so with the same
 // roundings, is done by the transform's loads).  Pass 0 (FIRST) sums the
-// series; pass p forms mean p - 1 from the previous pass's partials and,
-// while |mean| > 5e-7 n, sums again.  Row blockIdx.y of a batch; `cnt` as
-// Slot::d_count (16 words a row: [2] still active after the last pass, [3]
-// passes, [6 + p] pass p's flag), `means` 4 floats a row.
+// series; pass p forms mean p - 1 from the previous pass's group sums and,
+// while |mean| > 5e-7 n, sums again.  A CTA sums one group of pieces.  Row
+// blockIdx.y of a batch; `cnt` as Slot::d_count (16 words a row: [2] still
+// active after the last pass, [3] passes, [6 + p] pass p's flag), `means` 4
+// floats a row.
+constexpr int kMeanGroupThreads = 32 * kMeanGroup;
+
 template <bool FIRST>
-__global__ void __launch_bounds__(kVecThreads) k_baseline_means(
-    SeriesRows rows, size_t n, double2* __restrict__ parts, size_t part_stride, int nparts,
+__global__ void __launch_bounds__(kMeanGroupThreads) k_baseline_means(
+    const __grid_constant__ SeriesRows rows, size_t n, double* __restrict__ sums, size_t sum_stride,
     unsigned* __restrict__ cnt, float* __restrict__ means, int pass, int last)
 {
     const float* x = rows.p[blockIdx.y];
     unsigned* c = cnt + 16 * blockIdx.y;
     float* m = means + 4 * blockIdx.y;
-    double2* out = parts + (size_t)blockIdx.y * part_stride + (pass & 1) * nparts;
-    double s = 0.0;
+    const unsigned groups = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    double* out = sums + (size_t)blockIdx.y * sum_stride;  // two halves: passes alternate
+    const double* in = out + ((pass - 1) & 1) * groups;
+    out += (pass & 1) * groups;
+    double s[1] = {0.0};
+    const unsigned first = blockIdx.x * kMeanGroup + warp, pieces = groups * kMeanGroup;
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     if constexpr (FIRST) {
         if (one) {
             c[6] = 1u;
             for (int k = 0; k < 4; ++k) m[k] = 0.f;
         }
-        s = sum_less(x, n, 0.f, 0.f);
+        piece_sums<1>(x, n, pieces, first, 0, 0.f, 0.f, s);
     } else {
         // (mean p - 1 is read by nobody else in this pass: every CTA forms it)
         const bool active = c[6 + pass - 1] != 0u;
@@ -813,11 +854,11 @@ __global__ void __launch_bounds__(kVecThreads) k_baseline_means(
             return;
         }
         __shared__ float s_mean;
-        if (threadIdx.x < 32) {
-            double a, b;
-            warp_sum_partials(parts + (size_t)blockIdx.y * part_stride + ((pass - 1) & 1) * nparts,
-                              nparts, a, b);
-            if (threadIdx.x == 0) s_mean = __fdiv_rn((float)a, (float)(double)n);
+        if (warp == 0) {
+            double t = 0.0;
+            for (unsigned g = lane; g < groups; g += 32) t += in[g];
+            t = warp_total(t, 32);
+            if (lane == 0) s_mean = __fdiv_rn((float)t, (float)(double)n);
         }
         __syncthreads();
         const float mean = s_mean;
@@ -829,52 +870,77 @@ __global__ void __launch_bounds__(kVecThreads) k_baseline_means(
             if (last) c[2] = more ? 1u : 0u;
         }
         if (!more || last) return;
-        s = pass > 1 ? sum_less(x, n, m[0], mean) : sum_less(x, n, mean, 0.f);
+        if (pass > 1)
+            piece_sums<1>(x, n, pieces, first, 0, m[0], mean, s);
+        else
+            piece_sums<1>(x, n, pieces, first, 0, mean, 0.f, s);
     }
-    block_partials<kVecThreads>(s, 0.0, out);
+    __shared__ double sh[kMeanGroup];
+    s[0] = warp_total(s[0], 32);
+    if (lane == 0) sh[warp] = s[0];
+    __syncthreads();
+    if (warp == 0) {
+        const double t = warp_total(lane < kMeanGroup ? sh[lane] : 0.0, kMeanGroup);
+        if (lane == 0) out[blockIdx.x] = t;
+    }
 }
 static_assert(kBaselineMeans == 3, "the third mean needs no sum after it");
 
-// The same loop in one launch: a cluster of CTAs per row sums, exchanges its
-// partial sums through distributed shared memory and goes round again while
-// the mean is above the threshold.  Clusters of 16 (8 for more than 8 rows,
-// where 16 would take two waves); a few SMs read a long row slower than the
-// whole device, so fewer than 4 rows take it up to 2^21 samples, 4 and more
-// up to 2^23.  A call of 1, 12 and 48 DM trials on B200 (us; four launches,
-// one with clusters of 8, of 16): 2^19: 171/162/164, 513/397/379,
-// 1225/744/793; 2^20: 173/170/164, 614/508/494, 1797/1370/1346; 2^21:
-// 178/187/176, 887/808/777, 2828/2497/2416; 2^22: 231/300/258,
-// 1428/1435/1356, 5093/5001/4872.
+// The same loop in one launch: a cluster of CTAs per row sums, K pieces to a
+// warp, exchanges its group sums through distributed shared memory and goes
+// round again while the mean is above the threshold.  Clusters of 16 (8 for
+// more than 8 rows up to 2^21 samples, where 16 would take two waves); a few
+// SMs read a long row slower than the whole device, so fewer than 4 rows take
+// it up to 2^21 samples, 4 and more up to 2^23.  A call of 1, 12 and 48 DM
+// trials on B200 (us; four launches, one with clusters of 8, of 16): 2^19:
+// 171/162/164, 513/397/379, 1225/744/793; 2^20: 173/170/164, 614/508/494,
+// 1797/1370/1346; 2^21: 178/187/176, 887/808/777, 2828/2497/2416; 2^22:
+// 231/300/258, 1428/1435/1356, 5093/5001/4872.  (With sums per CTA; pieces of
+// their own per warp take the same within 1 %, and the four launches at 2^23
+// 4 % less of a 12-DM call, 2355 against 2455.)
 constexpr int kMeanThreads = 1024;
-inline unsigned mean_ctas(int rows) { return rows > 8 ? 8u : 16u; }
-inline size_t mean_max_samples(int rows) { return (size_t)1 << (rows < 4 ? 21 : 23); }
+inline unsigned mean_ctas(int rows, size_t n) { return rows > 8 && n <= kMeanShort ? 8u : 16u; }
+inline size_t mean_max_samples(int rows) { return rows < 4 ? kMeanShort : kMeanMedium; }
 
+template <int K>
 __global__ void __launch_bounds__(kMeanThreads) k_baseline_means_cluster(
-    SeriesRows rows, size_t n, unsigned* __restrict__ cnt, float* __restrict__ means)
+    const __grid_constant__ SeriesRows rows, size_t n, unsigned* __restrict__ cnt,
+    float* __restrict__ means)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const float* x = rows.p[blockIdx.y];
-    __shared__ double warp_sum[kMeanThreads / 32];
-    __shared__ double part[kBaselineMeans];  // this CTA's sum of each pass
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    const unsigned W = cl.num_blocks() * (kMeanThreads / 32), pieces = K * W;
+    __shared__ double warp_sum[K][kMeanThreads / 32];
+    __shared__ double part[kBaselineMeans][2 * K];  // this CTA's group sums of each pass
+    static_assert(kMeanThreads / 32 == 2 * kMeanGroup, "two groups to the warps of a CTA");
     float m[kBaselineMeans] = {0.f, 0.f, 0.f};
     int pass = 0;
     bool more = true;
 #pragma unroll
     for (int p = 0; p < kBaselineMeans; ++p) {
         if (!more) break;  // the same in every thread of the cluster
-        double s = sum_less(x, n, m[0], m[1]);
-        for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x / 32] = s;
+        double s[K] = {};
+        piece_sums<K>(x, n, pieces, cl.block_rank() * (kMeanThreads / 32) + warp, W, m[0], m[1], s);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            s[k] = warp_total(s[k], 32);
+            if (lane == 0) warp_sum[k][warp] = s[k];
+        }
         __syncthreads();
-        if (threadIdx.x < 32) {
-            double t = warp_sum[threadIdx.x];
-            for (int o = 16; o; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-            if (threadIdx.x == 0) part[p] = t;
+        if (warp < K) {
+            const double t = warp_total(warp_sum[warp][lane], kMeanGroup);
+            if (lane % kMeanGroup == 0) part[p][2 * warp + lane / kMeanGroup] = t;
         }
         cl.sync();
+        // group g is half g % 2 of the warps that CTA (g / 2) % CTAs ran its
+        // k = g / 2 / CTAs on
         double total = 0.0;
-        for (unsigned c = 0; c < cl.num_blocks(); ++c) total += *cl.map_shared_rank(&part[p], c);
+        for (unsigned g = lane; g < pieces / kMeanGroup; g += 32)
+            total += *cl.map_shared_rank(&part[p][2 * (g / 2 / cl.num_blocks()) + g % 2],
+                                         g / 2 % cl.num_blocks());
+        total = warp_total(total, 32);
         m[p] = __fdiv_rn((float)total, (float)(double)n);
         more = fabsf(m[p]) > 5e-7 * (double)n;
         pass = p + 1;
@@ -888,34 +954,42 @@ __global__ void __launch_bounds__(kMeanThreads) k_baseline_means_cluster(
     cl.sync();  // no CTA leaves while another reads its partial sums
 }
 
-// Whether this device runs such clusters (asked once per device and size:
-// 16 is above the portable 8).
-static bool mean_clusters_fit(const cudaLaunchConfig_t* cfg, unsigned ctas)
+// Launches the cluster form with K pieces to a warp; false where this device
+// does not run such clusters (asked once per device and K: 16 is above the
+// portable 8).
+template <int K>
+static bool mean_cluster(cudaLaunchConfig_t cfg, const SeriesRows& rows, size_t n, unsigned* d_cnt,
+                         float* d_means, int* rc)
 {
     static std::mutex mu;
-    static int table[64][2] = {};  // 1 yes, 2 no
+    static int table[64] = {};  // 1 yes, 2 no
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    std::lock_guard<std::mutex> lock(mu);
-    int& known = table[dev][ctas > 8];
-    if (!known) {
-        int n = 0;
-        const bool ok = cudaFuncSetAttribute(k_baseline_means_cluster,
-                                             cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                             1) == cudaSuccess &&
-                        cudaOccupancyMaxActiveClusters(&n, k_baseline_means_cluster, cfg) ==
-                            cudaSuccess && n > 0;
-        (void)cudaGetLastError();
-        known = ok ? 1 : 2;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!table[dev]) {
+            int fit = 0;
+            const bool ok = cudaFuncSetAttribute(k_baseline_means_cluster<K>,
+                                                 cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                                 1) == cudaSuccess &&
+                            cudaOccupancyMaxActiveClusters(&fit, k_baseline_means_cluster<K>,
+                                                           &cfg) == cudaSuccess && fit > 0;
+            (void)cudaGetLastError();
+            table[dev] = ok ? 1 : 2;
+        }
+        if (table[dev] != 1) return false;
     }
-    return known == 1;
+    *rc = cuda_status(cudaLaunchKernelEx(&cfg, k_baseline_means_cluster<K>, rows, n, d_cnt, d_means),
+                      "baseline mean kernel");
+    return true;
 }
 
 int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* d_parts,
                           size_t part_stride, unsigned* d_cnt, float* d_means, cudaStream_t s)
 {
+    const unsigned pieces = mean_pieces(n);
     if (n <= mean_max_samples(nrows)) {
-        const unsigned ctas = mean_ctas(nrows);
+        const unsigned ctas = mean_ctas(nrows, n);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(ctas, nrows);
         cfg.blockDim = dim3(kMeanThreads);
@@ -925,19 +999,26 @@ int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* 
         at[0].val.clusterDim = {ctas, 1, 1};
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        if (mean_clusters_fit(&cfg, ctas))
-            return cuda_status(cudaLaunchKernelEx(&cfg, k_baseline_means_cluster, rows, n, d_cnt,
-                                                  d_means),
-                               "baseline mean kernel");
+        int rc = PSX_OK;
+        bool ran = false;
+        switch (pieces / (ctas * (kMeanThreads / 32))) {
+        case 1: ran = mean_cluster<1>(cfg, rows, n, d_cnt, d_means, &rc); break;
+        case 2: ran = mean_cluster<2>(cfg, rows, n, d_cnt, d_means, &rc); break;
+        default: ran = mean_cluster<4>(cfg, rows, n, d_cnt, d_means, &rc); break;
+        }
+        if (ran) return rc;
     }
-    const int nb = reduction_blocks();
-    const dim3 grid(nb, nrows);
-    k_baseline_means<true><<<grid, kVecThreads, 0, s>>>(rows, n, d_parts, part_stride, nb, d_cnt,
-                                                        d_means, 0, 0);
+    const dim3 grid(pieces / kMeanGroup, nrows);
+    double* sums = reinterpret_cast<double*>(d_parts);
+    if (part_stride < grid.x) {  // (a row's two halves, in double2)
+        set_error("baseline means: partial sums of a row hold %zu entries", part_stride);
+        return PSX_ERR_INVALID;
+    }
+    k_baseline_means<true><<<grid, kMeanGroupThreads, 0, s>>>(rows, n, sums, 2 * part_stride, d_cnt,
+                                                              d_means, 0, 0);
     for (int pass = 1; pass <= kBaselineMeans; ++pass)
-        k_baseline_means<false><<<grid, kVecThreads, 0, s>>>(rows, n, d_parts, part_stride, nb,
-                                                             d_cnt, d_means, pass,
-                                                             pass == kBaselineMeans);
+        k_baseline_means<false><<<grid, kMeanGroupThreads, 0, s>>>(
+            rows, n, sums, 2 * part_stride, d_cnt, d_means, pass, pass == kBaselineMeans);
     return launch_status("baseline mean kernels");
 }
 
