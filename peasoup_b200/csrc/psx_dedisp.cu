@@ -738,23 +738,16 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_dedisperse_tree(TreeArgs a)
 size_t round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }
 
 }  // namespace
-}  // namespace psx
 
-using namespace psx;
-
-struct psx_dedisp_plan {
-    size_t nchans = 0;
-    float tsamp = 0, fch1 = 0, foff = 0;
-    std::vector<float> delays, dms;
-    std::vector<int> live;  // 1 = channel summed
-    // derived tables for one sample width (elem bytes), rebuilt when dirty
-    bool dirty = true;
-    int elem = 0;
-    int kind = -1;          // sample class the tables were built for
-    bool few = false;       // and whether for few CTAs
+// Shift tables and launch shape of one form for one class of samples.
+struct DedispTables {
+    enum State { kNew, kBuilt, kNotTaken };  // kNotTaken: the direct form instead
+    State state = kNew;
+    bool uploaded = false;
+    int kind = 0;           // sample class (direct: any of this width)
+    int elem = 0;           // bytes a sample
     int nlive = 0, ndm_pad = 0, nblk = 0, group = 8, lwin = 0, cc = 0;
     size_t ngroups = 0, max_lo = 0;
-    size_t scratch_limit = 4ull << 30;  // bytes of channel-major samples
     size_t flush_bytes = 0;             // shared 32-bit sums above 257 channels
     // shared-partial-sum form (k_dedisperse_tree): 0 = the direct kernel,
     // else S; DM trials in order of DM, ndb per block, dpw per warp
@@ -764,6 +757,44 @@ struct psx_dedisp_plan {
     std::vector<int> h_tab;
     int* d_tab = nullptr;
     size_t tab_cap = 0;
+
+    // a stage's windows: the planar words' samples once, and per channel
+    // the parts after the first
+    static int raw_words(int c, int pm, int more, int el) { return pm / (el == 1 ? 4 : 2) + c * (more + 4); }
+
+    static size_t tree_bytes(int raw, int plen, int gmax, int yw, int pmax, int trials)
+    {
+        return 4ull * ((size_t)raw + plen + 32ull * gmax * yw + 2ull * pmax * kTrRec + 2ull * trials);
+    }
+
+    size_t smem_bytes() const
+    {
+        if (tree)
+            return tree_bytes(rawlen, plen, gmax, kind == kTrSmall ? 1 : 2, pmax,
+                              cc / kTrS * kTrWarps * dpw);
+        return 2ull * cc * (kDdWarps / group) * lwin * elem + 2ull * kDdWarps * cc * sizeof(int) +
+               flush_bytes;
+    }
+};
+
+}  // namespace psx
+
+using namespace psx;
+
+struct psx_dedisp_plan {
+    size_t nchans = 0;
+    float tsamp = 0, fch1 = 0, foff = 0;
+    std::vector<float> delays, dms;
+    std::vector<int> live;  // 1 = channel summed
+    // Derived tables: the shared-sum form's by sample class, then the direct
+    // form's by sample width.  Every one a call has needed is kept until the
+    // DM list or the channels change, so that calls which need different ones
+    // in turn (a short output after long ones, files of another sample width)
+    // do not build and upload them each time: 0.9 ms of host time at 1024
+    // channels x 100 DM trials, 9 ms at 4096 x 300.
+    DedispTables sets[5];
+    DedispTables* t = nullptr;          // the call's
+    size_t scratch_limit = 4ull << 30;  // bytes of channel-major samples
     void* d_cm = nullptr;
     size_t cm_cap = 0;
     uint8_t* d_stage = nullptr;
@@ -781,39 +812,68 @@ struct psx_dedisp_plan {
         return (size_t)std::floor((double)prod + 0.5);
     }
 
-    // Shift tables and the window shape for one class of samples.
-    int build_tables(int sample_kind, bool few_ctas)
+    void changed()
     {
-        if (!dirty && sample_kind == kind && few_ctas == few) return PSX_OK;
-        few = few_ctas;
-        const int el = sample_kind == kTr16 ? 2 : 1;
-        kind = sample_kind;
-        dirty = true;
+        for (DedispTables& x : sets) x.state = DedispTables::kNew;
+    }
+
+    // Takes the tables for one class of samples, building them where this DM
+    // list has not needed them yet.
+    int take_tables(int kind, bool few_ctas)
+    {
+        const int el = kind == kTr16 ? 2 : 1;
         if (dms.empty()) {
             set_error("psx_dedisp: no DM list set");
             return PSX_ERR_INVALID;
         }
-        std::vector<int> chans;
-        for (size_t c = 0; c < nchans; ++c)
-            if (live[c]) chans.push_back((int)c);
-        nlive = (int)chans.size();
-        const int ndm = (int)dms.size();
-        ndm_pad = (int)round_up((size_t)ndm, kDdWarps);
-        nblk = ndm_pad / kDdWarps;
-        const int align = 16 / el;  // window starts on 16-byte boundaries
-        std::vector<int> shift((size_t)ndm * std::max(nlive, 1));
-        for (int d = 0; d < ndm; ++d)
-            for (int i = 0; i < nlive; ++i) {
-                float p = dms[d] * delays[chans[i]];
-                shift[(size_t)d * nlive + i] = (int)std::nearbyint(p);
-            }
-        tile = dd_tile(el);
-        if (nlive > 0 && !few && build_tree(el, chans, shift)) {
-            elem = el;
-            dirty = true;  // tables must be uploaded
-            return PSX_OK;
+        DedispTables &shared = sets[kind], &direct = sets[3 + (el == 2)];
+        if (!few_ctas && shared.state == DedispTables::kNew) {
+            shared.kind = kind;
+            shared.elem = el;
+            shared.uploaded = false;
+            std::vector<int> chans, shift;
+            shifts(&chans, &shift);
+            shared.nlive = (int)chans.size();
+            shared.state = shared.nlive > 0 && build_tree(shared, chans, shift)
+                               ? DedispTables::kBuilt : DedispTables::kNotTaken;
         }
-        tree = 0;
+        t = !few_ctas && shared.state == DedispTables::kBuilt ? &shared : &direct;
+        if (t->state == DedispTables::kBuilt) return PSX_OK;
+        direct.kind = kind;
+        direct.elem = el;
+        direct.uploaded = false;
+        PSX_TRY(build_direct(direct));
+        direct.state = DedispTables::kBuilt;
+        return PSX_OK;
+    }
+
+    // Channels summed, and the shift of every (DM trial, such channel).
+    void shifts(std::vector<int>* chans, std::vector<int>* shift) const
+    {
+        for (size_t c = 0; c < nchans; ++c)
+            if (live[c]) chans->push_back((int)c);
+        const size_t nlive = chans->size(), ndm = dms.size();
+        shift->resize(ndm * std::max<size_t>(nlive, 1));
+        for (size_t d = 0; d < ndm; ++d)
+            for (size_t i = 0; i < nlive; ++i) {
+                float p = dms[d] * delays[(*chans)[i]];
+                (*shift)[d * nlive + i] = (int)std::nearbyint(p);
+            }
+    }
+
+    // Shift tables and the window shape of the direct form.
+    int build_direct(DedispTables& T)
+    {
+        const int el = T.elem;
+        std::vector<int> chans, shift;
+        shifts(&chans, &shift);
+        const int nlive = T.nlive = (int)chans.size();
+        const int ndm = (int)dms.size();
+        const int ndm_pad = T.ndm_pad = (int)round_up((size_t)ndm, kDdWarps);
+        T.nblk = ndm_pad / kDdWarps;
+        const int align = 16 / el;  // window starts on 16-byte boundaries
+        T.tile = dd_tile(el);
+        T.tree = 0;
         // window shape for groups of G trials: lo = min shift aligned down,
         // lwin covers 512 outputs past the largest shift plus the read-ahead
         auto shape = [&](int G, std::vector<int>* lo_out, int* lwin_out, size_t* max_lo_out) {
@@ -844,39 +904,37 @@ struct psx_dedisp_plan {
         size_t mlo8 = 0, mlo1 = 0;
         shape(8, &lo8, &lwin8, &mlo8);
         shape(1, &lo1, &lwin1, &mlo1);
-        group = (lwin8 <= kDdWarps * lwin1) ? 8 : 1;
-        std::vector<int>& lo = group == 8 ? lo8 : lo1;
-        lwin = group == 8 ? lwin8 : lwin1;
-        max_lo = group == 8 ? mlo8 : mlo1;
-        ngroups = (size_t)ndm_pad / group;
-        const int nwin = kDdWarps / group;
-        cc = 0;
-        flush_bytes = (el == 1 && nlive > 257) ? 4ull * (kDdTile8 / 32) * kDdThreads : 0;
+        T.group = (lwin8 <= kDdWarps * lwin1) ? 8 : 1;
+        std::vector<int>& lo = T.group == 8 ? lo8 : lo1;
+        T.lwin = T.group == 8 ? lwin8 : lwin1;
+        T.max_lo = T.group == 8 ? mlo8 : mlo1;
+        T.ngroups = (size_t)ndm_pad / T.group;
+        const int nwin = kDdWarps / T.group;
+        T.cc = 0;
+        T.flush_bytes = (el == 1 && nlive > 257) ? 4ull * (kDdTile8 / 32) * kDdThreads : 0;
         // with the flush sums, fewer channels per chunk keep 4 CTAs on an SM
-        const size_t cap = flush_bytes ? 56 * 1024 : 96 * 1024;
+        const size_t cap = T.flush_bytes ? 56 * 1024 : 96 * 1024;
         for (int c : {16, 8, 4, 2, 1}) {
-            size_t bytes = 2ull * c * nwin * lwin * el + 2ull * kDdWarps * c * sizeof(int) +
-                           flush_bytes;
+            size_t bytes = 2ull * c * nwin * T.lwin * el + 2ull * kDdWarps * c * sizeof(int) +
+                           T.flush_bytes;
             if (bytes <= cap || (c == 1 && bytes <= 200 * 1024)) {
-                cc = c;
+                T.cc = c;
                 break;
             }
         }
-        if (cc == 0) {
+        if (T.cc == 0) {
             set_error("psx_dedisp: DM trials of one block spread over %d samples; "
-                      "the shared-memory window does not fit", lwin);
+                      "the shared-memory window does not fit", T.lwin);
             return PSX_ERR_UNSUPPORTED;
         }
-        h_tab.assign((size_t)nlive + ngroups * nlive + (size_t)ndm_pad * nlive, 0);
-        std::copy(chans.begin(), chans.end(), h_tab.begin());
-        std::copy(lo.begin(), lo.begin() + ngroups * nlive, h_tab.begin() + nlive);
-        int* off = h_tab.data() + nlive + ngroups * nlive;
+        T.h_tab.assign((size_t)nlive + T.ngroups * nlive + (size_t)ndm_pad * nlive, 0);
+        std::copy(chans.begin(), chans.end(), T.h_tab.begin());
+        std::copy(lo.begin(), lo.begin() + T.ngroups * nlive, T.h_tab.begin() + nlive);
+        int* off = T.h_tab.data() + nlive + T.ngroups * nlive;
         for (int d = 0; d < ndm; ++d)
             for (int i = 0; i < nlive; ++i)
                 off[(size_t)d * nlive + i] =
-                    shift[(size_t)d * nlive + i] - lo[(size_t)(d / group) * nlive + i];
-        elem = el;
-        dirty = true;  // tables must be uploaded
+                    shift[(size_t)d * nlive + i] - lo[(size_t)(d / T.group) * nlive + i];
         return PSX_OK;
     }
 
@@ -890,9 +948,10 @@ struct psx_dedisp_plan {
     // form, 64-128 channels x 500k samples, by that ratio, 8 / 2 / 16 bits):
     // 0.50: 766/416, 661/351, 1496/829; 0.69: 146/120, 122/104, 260/192;
     // 1.08: 145/157, 121/143, 261/263; 1.53: 155/208, 133/200, 321/357.
-    bool build_tree(int el, const std::vector<int>& chans, const std::vector<int>& shift)
+    bool build_tree(DedispTables& T, const std::vector<int>& chans, const std::vector<int>& shift)
     {
         constexpr int S = kTrS;
+        const int el = T.elem, nlive = T.nlive;
         const int ndm = (int)dms.size();
         if (el == 1 && (double)nlive * 255.0 >= 16777216.0) return false;
         std::vector<int> order(ndm);
@@ -972,7 +1031,7 @@ struct psx_dedisp_plan {
                             16.0 * (double)nquads;
         if (cost >= 0.9 * cost_direct) return false;
         // channels per stage: the most that leave two CTAs on an SM
-        const int yw = kind == kTrSmall ? 1 : 2;
+        const int yw = T.kind == kTrSmall ? 1 : 2;
         int c_ = 0, pm = 0, gm = 0, nm = 0;
         const int more = el == 1 ? 3 * kTrQ / 4 : kTrQ / 2;
         for (int c : {32, 16, 8, 4}) {
@@ -992,8 +1051,8 @@ struct psx_dedisp_plan {
                 }
             // the last group of a pattern may read up to 31 words past a
             // channel's: into the next one's, or the zeros
-            const size_t b = tree_bytes(raw_words(c, pm, more, el), pm + 4 * most + 32, gm, yw, nm,
-                                        c / S * slots);
+            const size_t b = DedispTables::tree_bytes(DedispTables::raw_words(c, pm, more, el),
+                                                      pm + 4 * most + 32, gm, yw, nm, c / S * slots);
             if (b <= 112 * 1024 || (c == 4 && b <= 220 * 1024)) {
                 c_ = c;
                 break;
@@ -1003,26 +1062,26 @@ struct psx_dedisp_plan {
         const int nq_ = (nlive + c_ - 1) / c_, sbs = c_ / S;
         // tables: channel records, output rows, per stage the first pattern
         // and the groups, pattern records, the trials' Y offsets
-        tab_row = 4 * (size_t)blocks * nlive;
-        tab_ps = tab_row + round_up((size_t)ndm, 4);
-        tab_gt = tab_ps + round_up((size_t)blocks * nq_ + 1, 4);
-        tab_pat = tab_gt + round_up((size_t)blocks * nq_, 4);
-        tab_yoff = tab_pat + pats.size() * kTrRec;
-        h_tab.assign(tab_yoff + (size_t)blocks * nq_ * sbs * slots, 0);
+        T.tab_row = 4 * (size_t)blocks * nlive;
+        T.tab_ps = T.tab_row + round_up((size_t)ndm, 4);
+        T.tab_gt = T.tab_ps + round_up((size_t)blocks * nq_ + 1, 4);
+        T.tab_pat = T.tab_gt + round_up((size_t)blocks * nq_, 4);
+        T.tab_yoff = T.tab_pat + pats.size() * kTrRec;
+        T.h_tab.assign(T.tab_yoff + (size_t)blocks * nq_ * sbs * slots, 0);
         for (int g = 0; g < blocks; ++g)
             for (int i = 0, at = 0; i < nlive; ++i) {
                 if (i % c_ == 0) at = 0;
-                int* ch = h_tab.data() + 4 * ((size_t)g * nlive + i);
+                int* ch = T.h_tab.data() + 4 * ((size_t)g * nlive + i);
                 ch[0] = chans[i];
                 ch[1] = lo[(size_t)g * nlive + i];
                 ch[2] = at;
                 ch[3] = quads[(size_t)g * nlive + i];
                 at += 4 * ch[3];
             }
-        std::copy(order.begin(), order.end(), h_tab.begin() + tab_row);
-        int* ps = h_tab.data() + tab_ps;
-        int* gt = h_tab.data() + tab_gt;
-        int* yo = h_tab.data() + tab_yoff;
+        std::copy(order.begin(), order.end(), T.h_tab.begin() + T.tab_row);
+        int* ps = T.h_tab.data() + T.tab_ps;
+        int* gt = T.h_tab.data() + T.tab_gt;
+        int* yo = T.h_tab.data() + T.tab_yoff;
         size_t at = 0;  // next pattern
         for (int g = 0; g < blocks; ++g) {
             const int e0 = g * per, e1 = std::min(ndm, e0 + per);
@@ -1037,10 +1096,10 @@ struct psx_dedisp_plan {
                 for (int p = 0; p < n; ++p) {
                     const Pat& pt = pats[at + p];
                     const int* u = &shift[(size_t)order[pt.first] * nlive];
-                    int* rec = h_tab.data() + tab_pat + (at + p) * kTrRec;
+                    int* rec = T.h_tab.data() + T.tab_pat + (at + p) * kTrRec;
                     for (int c = 0; c < S; ++c) {
                         const int i = c0 + c;
-                        const int* ch = h_tab.data() + 4 * ((size_t)g * nlive + i);
+                        const int* ch = T.h_tab.data() + 4 * ((size_t)g * nlive + i);
                         rec[c] = i < nlive ? ch[2] + pt.lo + (u[i] - u[c0]) - ch[1]
                                            : pm;  // the zeros
                     }
@@ -1059,45 +1118,28 @@ struct psx_dedisp_plan {
             }
         }
         ps[blocks * nq_] = (int)at;
-        tree = S;
-        dpw = dw;
-        ndb = per;
-        nblk = blocks;
-        cc = c_;
-        nq = nq_;
-        zero = pm;
-        zlen = 4 * most + 32;
-        plen = zero + zlen;
-        gmax = gm;
-        pmax = nm;
-        rawlen = raw_words(c_, pm, more, el);
-        lwin = 4 * most + (el == 1 ? 3 : 1) * kTrQ;
-        max_lo = mlo;
-        tile = tr_tile(el);
+        T.tree = S;
+        T.dpw = dw;
+        T.ndb = per;
+        T.nblk = blocks;
+        T.cc = c_;
+        T.nq = nq_;
+        T.zero = pm;
+        T.zlen = 4 * most + 32;
+        T.plen = T.zero + T.zlen;
+        T.gmax = gm;
+        T.pmax = nm;
+        T.rawlen = DedispTables::raw_words(c_, pm, more, el);
+        T.lwin = 4 * most + (el == 1 ? 3 : 1) * kTrQ;
+        T.max_lo = mlo;
+        T.tile = tr_tile(el);
         return true;
-    }
-
-    // a stage's windows: the planar words' samples once, and per channel
-    // the parts after the first
-    static int raw_words(int c, int pm, int more, int el) { return pm / (el == 1 ? 4 : 2) + c * (more + 4); }
-
-    static size_t tree_bytes(int raw, int plen, int gmax, int yw, int pmax, int trials)
-    {
-        return 4ull * ((size_t)raw + plen + 32ull * gmax * yw + 2ull * pmax * kTrRec + 2ull * trials);
-    }
-
-    size_t smem_bytes() const
-    {
-        if (tree)
-            return tree_bytes(rawlen, plen, gmax, kind == kTrSmall ? 1 : 2, pmax,
-                              cc / kTrS * kTrWarps * dpw);
-        return 2ull * cc * (kDdWarps / group) * lwin * elem + 2ull * kDdWarps * cc * sizeof(int) +
-               flush_bytes;
     }
 
     ~psx_dedisp_plan()
     {
-        if (d_tab) cudaFree(d_tab);
+        for (DedispTables& x : sets)
+            if (x.d_tab) cudaFree(x.d_tab);
         if (d_cm) cudaFree(d_cm);
         if (d_stage) cudaFree(d_stage);
         for (int i = 0; i < 2; ++i) {
@@ -1176,20 +1218,20 @@ int prepare(psx_dedisp_plan* p, size_t nout, int nbits, cudaStream_t st, size_t*
     const size_t blocks = (nout + tr_tile(el) - 1) / tr_tile(el) *
                           ((p->dms.size() + kTrMaxDms - 1) / kTrMaxDms);
     const bool few = 2 * blocks < (size_t)sm_count();
-    bool rebuilt = p->dirty || kind != p->kind || few != p->few;
-    PSX_TRY(p->build_tables(kind, few));
-    if (rebuilt) {
-        size_t bytes = p->h_tab.size() * sizeof(int);
-        PSX_TRY(grow(reinterpret_cast<void**>(&p->d_tab), &p->tab_cap, std::max<size_t>(bytes, 4),
+    PSX_TRY(p->take_tables(kind, few));
+    DedispTables& t = *p->t;
+    if (!t.uploaded) {
+        size_t bytes = t.h_tab.size() * sizeof(int);
+        PSX_TRY(grow(reinterpret_cast<void**>(&t.d_tab), &t.tab_cap, std::max<size_t>(bytes, 4),
                      "shift tables"));
-        PSX_CUDA(cudaMemcpyAsync(p->d_tab, p->h_tab.data(), bytes, cudaMemcpyHostToDevice, st));
-        p->dirty = false;
+        PSX_CUDA(cudaMemcpyAsync(t.d_tab, t.h_tab.data(), bytes, cudaMemcpyHostToDevice, st));
+        t.uploaded = true;
     }
-    const size_t tile = (size_t)p->tile;
+    const size_t tile = (size_t)p->t->tile;
     const size_t md = p->max_delay();
     auto pitch_for = [&](size_t g) {
         size_t nt = (g + tile - 1) / tile;
-        size_t need = (nt - 1) * tile + p->max_lo + (size_t)p->lwin;
+        size_t need = (nt - 1) * tile + p->t->max_lo + (size_t)p->t->lwin;
         return round_up(std::max(need, g + md), kUpRows);
     };
     size_t g = round_up(nout, tile);
@@ -1244,31 +1286,31 @@ int launch_tree(const TreeArgs& a, int dpw, unsigned grid, size_t smem, cudaStre
     return dpw == 1 ? go(k_dedisperse_tree<MODE, 1, FLUSH>) : go(k_dedisperse_tree<MODE, 2, FLUSH>);
 }
 
-// The shared-partial-sum form (p->tree), output tiles [tile0, tile1).
+// The shared-partial-sum form (p->t->tree), output tiles [tile0, tile1).
 int dedisperse_tree(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, float* d_out,
                     size_t out_pitch, int flags, size_t tile0, size_t tile1, cudaStream_t st)
 {
     TreeArgs a;
     a.cm = p->d_cm;
     a.pitch = pitch;
-    a.chan = reinterpret_cast<const int4*>(p->d_tab);
-    a.dmrow = p->d_tab + p->tab_row;
-    a.pstart = p->d_tab + p->tab_ps;
-    a.pat = reinterpret_cast<const int4*>(p->d_tab + p->tab_pat);
-    a.gtot = p->d_tab + p->tab_gt;
-    a.yoff = p->d_tab + p->tab_yoff;
-    a.nlive = p->nlive;
+    a.chan = reinterpret_cast<const int4*>(p->t->d_tab);
+    a.dmrow = p->t->d_tab + p->t->tab_row;
+    a.pstart = p->t->d_tab + p->t->tab_ps;
+    a.pat = reinterpret_cast<const int4*>(p->t->d_tab + p->t->tab_pat);
+    a.gtot = p->t->d_tab + p->t->tab_gt;
+    a.yoff = p->t->d_tab + p->t->tab_yoff;
+    a.nlive = p->t->nlive;
     a.ndm = (int)p->dms.size();
-    a.ndb = p->ndb;
-    a.nblk = p->nblk;
-    a.cc = p->cc;
-    a.nq = p->nq;
-    a.zero = p->zero;
-    a.zlen = p->zlen;
-    a.plen = p->plen;
-    a.gmax = p->gmax;
-    a.pmax = p->pmax;
-    a.rawlen = p->rawlen;
+    a.ndb = p->t->ndb;
+    a.nblk = p->t->nblk;
+    a.cc = p->t->cc;
+    a.nq = p->t->nq;
+    a.zero = p->t->zero;
+    a.zlen = p->t->zlen;
+    a.plen = p->t->plen;
+    a.gmax = p->t->gmax;
+    a.pmax = p->t->pmax;
+    a.rawlen = p->t->rawlen;
     a.out = d_out;
     a.out_pitch = out_pitch;
     a.nout = nout;
@@ -1279,41 +1321,41 @@ int dedisperse_tree(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, fl
     a.p16 = (int)(65535u / m);
     a.p8s = (int)(255u / m) / kTrS;
     a.tile0 = (unsigned)tile0;
-    const size_t nblocks = (tile1 - tile0) * (size_t)p->nblk;
+    const size_t nblocks = (tile1 - tile0) * (size_t)p->t->nblk;
     if (nblocks > 0x7fffffffull) {
         set_error("psx_dedisp: %zu blocks exceed one launch", nblocks);
         return PSX_ERR_UNSUPPORTED;
     }
-    const size_t smem = p->smem_bytes();
+    const size_t smem = p->t->smem_bytes();
     const unsigned grid = (unsigned)nblocks;
-    if (nbits == 16) return launch_tree<kTr16, false>(a, p->dpw, grid, smem, st);
-    const bool flush = p->nlive > a.p16;
+    if (nbits == 16) return launch_tree<kTr16, false>(a, p->t->dpw, grid, smem, st);
+    const bool flush = p->t->nlive > a.p16;
     if (nbits <= 4)
-        return flush ? launch_tree<kTrSmall, true>(a, p->dpw, grid, smem, st)
-                     : launch_tree<kTrSmall, false>(a, p->dpw, grid, smem, st);
-    return flush ? launch_tree<kTr8, true>(a, p->dpw, grid, smem, st)
-                 : launch_tree<kTr8, false>(a, p->dpw, grid, smem, st);
+        return flush ? launch_tree<kTrSmall, true>(a, p->t->dpw, grid, smem, st)
+                     : launch_tree<kTrSmall, false>(a, p->t->dpw, grid, smem, st);
+    return flush ? launch_tree<kTr8, true>(a, p->t->dpw, grid, smem, st)
+                 : launch_tree<kTr8, false>(a, p->t->dpw, grid, smem, st);
 }
 
 // Output tiles [tile0, tile1) of nout outputs (tile1 0: all the rest).
 int dedisperse(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, float* d_out,
                size_t out_pitch, int flags, cudaStream_t st, size_t tile0 = 0, size_t tile1 = 0)
 {
-    if (!tile1) tile1 = (nout + p->tile - 1) / p->tile;
-    if (p->tree)
+    if (!tile1) tile1 = (nout + p->t->tile - 1) / p->t->tile;
+    if (p->t->tree)
         return dedisperse_tree(p, nbits, pitch, nout, d_out, out_pitch, flags, tile0, tile1, st);
     DedispArgs a;  // with every channel killed the sums are zero
     a.cm = p->d_cm;
     a.pitch = pitch;
-    a.chan = p->d_tab;
-    a.lo = p->d_tab + p->nlive;
-    a.off = p->d_tab + p->nlive + p->ngroups * p->nlive;
-    a.nlive = p->nlive;
+    a.chan = p->t->d_tab;
+    a.lo = p->t->d_tab + p->t->nlive;
+    a.off = p->t->d_tab + p->t->nlive + p->t->ngroups * p->t->nlive;
+    a.nlive = p->t->nlive;
     a.ndm = (int)p->dms.size();
-    a.nblk = p->nblk;
-    a.cc = p->cc;
-    a.lwin = p->lwin;
-    a.group = p->group;
+    a.nblk = p->t->nblk;
+    a.cc = p->t->cc;
+    a.lwin = p->t->lwin;
+    a.group = p->t->group;
     a.out = d_out;
     a.out_pitch = out_pitch;
     a.nout = nout;
@@ -1324,12 +1366,12 @@ int dedisperse(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, float* 
     a.p8 = (int)(255u / m);
     a.p16 = (int)(65535u / m);
     a.tile0 = (unsigned)tile0;
-    size_t nblocks = (tile1 - tile0) * (size_t)p->nblk;
+    size_t nblocks = (tile1 - tile0) * (size_t)p->t->nblk;
     if (nblocks > 0x7fffffffull) {
         set_error("psx_dedisp: %zu blocks exceed one launch", nblocks);
         return PSX_ERR_UNSUPPORTED;
     }
-    size_t smem = p->smem_bytes();
+    size_t smem = p->t->smem_bytes();
     const unsigned grid = (unsigned)nblocks;
     if (nbits == 16) {
         PSX_CUDA(cudaFuncSetAttribute(k_dedisperse<uint16_t, false, false>,
@@ -1337,7 +1379,7 @@ int dedisperse(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, float* 
         k_dedisperse<uint16_t, false, false><<<grid, kDdThreads, smem, st>>>(a);
     } else {
         // 8 bits and below: the flush and small-sample variants
-        const bool flush = p->nlive > a.p16, small = nbits <= 4;
+        const bool flush = p->t->nlive > a.p16, small = nbits <= 4;
         auto kern = small ? (flush ? k_dedisperse<uint8_t, true, true>
                                    : k_dedisperse<uint8_t, false, true>)
                           : (flush ? k_dedisperse<uint8_t, true, false>
@@ -1399,7 +1441,7 @@ int psx_dedisp_set_dm_list(psx_dedisp_plan* p, const float* h_dms, size_t n)
             return PSX_ERR_INVALID;
         }
     p->dms.assign(h_dms, h_dms + n);
-    p->dirty = true;
+    p->changed();
     return PSX_OK;
 }
 
@@ -1434,7 +1476,7 @@ int psx_dedisp_generate_dm_list(psx_dedisp_plan* p, float dm_start, float dm_end
         }
     }
     p->dms.swap(list);
-    p->dirty = true;
+    p->changed();
     return PSX_OK;
 }
 
@@ -1463,7 +1505,7 @@ int psx_dedisp_set_killmask(psx_dedisp_plan* p, const int* h_mask)
 {
     if (!p) return PSX_ERR_INVALID;
     for (size_t c = 0; c < p->nchans; ++c) p->live[c] = h_mask ? (h_mask[c] != 0) : 1;
-    p->dirty = true;
+    p->changed();
     return PSX_OK;
 }
 
@@ -1547,11 +1589,11 @@ int psx_dedisp_execute_host(psx_dedisp_plan* p, size_t nsamps, const uint8_t* h_
             // From pinned rows on B200, one after the other against so: 2^22
             // samples x 64 channels of 8 bits to 256 DM trials 7984, 5291 us;
             // 400,000 x 1024 of 4 bits to 100 5344, 4823.
-            const size_t tile = (size_t)p->tile;
+            const size_t tile = (size_t)p->t->tile;
             const size_t ready = last || r0 + n <= md ? 0 : (r0 + n - md) / tile;
             if (last) {
                 PSX_TRY(dedisperse(p, nbits, pitch, n_out, d_out + g0, out_pitch, flags, st, done));
-            } else if (ready > done && (ready - done) * p->nblk >= 4 * (size_t)sm_count()) {
+            } else if (ready > done && (ready - done) * p->t->nblk >= 4 * (size_t)sm_count()) {
                 PSX_TRY(dedisperse(p, nbits, pitch, n_out, d_out + g0, out_pitch, flags, st, done,
                                    ready));
                 done = ready;
