@@ -25,7 +25,7 @@
 // time tile for successive DM blocks, so the window is read from HBM once
 // and from L2 after that.  Where the DM trials of a block share most of their
 // relative shifts, subband sums formed once serve all of them instead
-// (k_dedisperse_tree, below, with the rule at build_tree).
+// (k_dedisperse_tree, below, with the rule at kDedispWeights).
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -433,6 +433,7 @@ constexpr int kTrWords = kTrQ / 32;
 constexpr int kTrThreads = 512;
 constexpr int kTrWarps = 16;
 constexpr int kTrMaxDms = 32;  // DM trials per CTA: at most 2 per warp
+constexpr int kTrMinDms = 8;   // fewer take the direct form (kDedispWeights)
 // sample classes: 8-bit bytes (their sums need 16 bits at once), 1..4-bit
 // bytes (a subband's sum fits a byte), 16-bit samples (32-bit sums)
 enum { kTr8 = 0, kTrSmall = 1, kTr16 = 2 };
@@ -739,6 +740,45 @@ size_t round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }
 
 }  // namespace
 
+// When the shared sums are taken: predicted time over the direct form's below
+// one.  Of a full device, as a share of the direct form's (2Q words of shared
+// memory per DM trial and channel, DM trials in eights): the words of the
+// patterns' series (S + 2 each), one Y per subband and DM trial, a stage's
+// fixed time over its channels and DM trials, and what a CTA takes beside its
+// channels.  Of a device that is not full: an SM runs the CTAs of a launch two
+// (direct: four) at a time, and a lone shared-sum CTA takes 1.2 to 1.5 halves
+// of a pair's time, the direct form half to one CTA's time over its CTAs'.
+// The weights are least squares of the measured times (B200, kernel alone,
+// 2, 8 and 16 bits x 16 to 1024 channels x 8 to 100 DM trials of up to 20 to
+// 150 x 50 to 1200 CTAs, 8400 pairs, prediction within 12 % RMS): taken so,
+// 0.3 % of the pairs are more than 3 % slower than the direct form, against
+// 4 % with one line through the words and one through the CTAs.  Some of
+// those measured (us, direct and shared; channels, DM trials up to DM, bits):
+// 64, 32 to 60, 2: 18.5 and 28.7 at 74 CTAs, 71.8 and 65.9 at 400; 64, 32 to
+// 60, 8: 20.4 and 30.9 at 74, 35.0 and 31.7 at 148; 64, 32 to 90, 8: 83.9 and
+// 94.5 at 400; 1024, 32 to 60, 8: 307 and 264 at 74; 1024, 20 to 150, 8: 998
+// and 774 at 400.  Of 692 other lists of 8 to 400 DM trials (uneven spacing,
+// channels left out, 1 to 16 bits), 6 are more than 3 % slower so than with
+// the direct form, 1.16 times at most; of 189 lists of 2 to 7, 24, up to 1.42
+// times: those take the direct form.
+struct DedispWeights {
+    double patterns, sums, stage, channel, odd, fill;
+};
+constexpr DedispWeights kDedispWeights[3] = {
+    {1.07, 0.73, 46.0, 2.1, 0.26, 0.5},   // kTr8
+    {1.07, 0.86, 59.0, 2.6, 0.22, 0.5},   // kTrSmall
+    {0.95, 0.68, 58.0, 0.75, 0.48, 1.0},  // kTr16
+};
+
+// The second factor of that prediction, for the CTAs of both launches.
+inline double dedisp_occupancy(int kind, double ctas, double direct_ctas)
+{
+    const DedispWeights& w = kDedispWeights[kind];
+    const double sms = sm_count(), n = std::ceil(ctas / sms);
+    return (n + (std::fmod(n, 2.0) != 0.0 ? w.odd : 0.0)) / ctas /
+           ((std::ceil(direct_ctas / sms) + w.fill) / direct_ctas);
+}
+
 // Shift tables and launch shape of one form for one class of samples.
 struct DedispTables {
     enum State { kNew, kBuilt, kNotTaken };  // kNotTaken: the direct form instead
@@ -751,6 +791,7 @@ struct DedispTables {
     size_t flush_bytes = 0;             // shared 32-bit sums above 257 channels
     // shared-partial-sum form (k_dedisperse_tree): 0 = the direct kernel,
     // else S; DM trials in order of DM, ndb per block, dpw per warp
+    double rate = 0.0;      // predicted time of a full device over the direct form's
     int tree = 0, dpw = 0, ndb = 0, nq = 0, zero = 0, zlen = 0, plen = 0, gmax = 0, pmax = 0, rawlen = 0,
         tile = 0;
     size_t tab_row = 0, tab_ps = 0, tab_gt = 0, tab_pat = 0, tab_yoff = 0;  // in h_tab
@@ -817,9 +858,9 @@ struct psx_dedisp_plan {
         for (DedispTables& x : sets) x.state = DedispTables::kNew;
     }
 
-    // Takes the tables for one class of samples, building them where this DM
-    // list has not needed them yet.
-    int take_tables(int kind, bool few_ctas)
+    // Takes the tables for one class of samples and nout outputs, building
+    // them where this DM list has not needed them yet.
+    int take_tables(int kind, size_t nout)
     {
         const int el = kind == kTr16 ? 2 : 1;
         if (dms.empty()) {
@@ -827,7 +868,12 @@ struct psx_dedisp_plan {
             return PSX_ERR_INVALID;
         }
         DedispTables &shared = sets[kind], &direct = sets[3 + (el == 2)];
-        if (!few_ctas && shared.state == DedispTables::kNew) {
+        const double tiles = (double)((nout + tr_tile(el) - 1) / tr_tile(el));
+        const double direct_ctas = tiles * (double)((dms.size() + kDdWarps - 1) / kDdWarps);
+        const size_t blocks = (dms.size() + kTrMaxDms - 1) / kTrMaxDms;
+        const double full = dedisp_occupancy(kind, tiles * (double)blocks, direct_ctas);
+        // (no list's rate is below 0.3: not looked at where that cannot do)
+        if (0.3 * full < 1.0 && shared.state == DedispTables::kNew && dms.size() >= kTrMinDms) {
             shared.kind = kind;
             shared.elem = el;
             shared.uploaded = false;
@@ -837,7 +883,7 @@ struct psx_dedisp_plan {
             shared.state = shared.nlive > 0 && build_tree(shared, chans, shift)
                                ? DedispTables::kBuilt : DedispTables::kNotTaken;
         }
-        t = !few_ctas && shared.state == DedispTables::kBuilt ? &shared : &direct;
+        t = shared.state == DedispTables::kBuilt && shared.rate * full < 1.0 ? &shared : &direct;
         if (t->state == DedispTables::kBuilt) return PSX_OK;
         direct.kind = kind;
         direct.elem = el;
@@ -939,15 +985,11 @@ struct psx_dedisp_plan {
     }
 
     // Tables of the shared-partial-sum form, or false where the direct
-    // kernel is taken: the series do not fit shared memory, a sum could pass
-    // 2^24 where sums are kept as floats, or the patterns are so many (few
-    // or widely spaced DM trials) that it moves no fewer words through
-    // shared memory.  The words of a tile: S + 2 per pattern and word of its
-    // series, 2Q per DM trial and subband and 4 per planar word, against 2Q
-    // per DM trial and channel.  Measured on B200 (us, direct against this
-    // form, 64-128 channels x 500k samples, by that ratio, 8 / 2 / 16 bits):
-    // 0.50: 766/416, 661/351, 1496/829; 0.69: 146/120, 122/104, 260/192;
-    // 1.08: 145/157, 121/143, 261/263; 1.53: 155/208, 133/200, 321/357.
+    // kernel is taken whatever the outputs: the series do not fit shared
+    // memory, a sum could pass 2^24 where sums are kept as floats, or the
+    // patterns are so many (few or widely spaced DM trials) that no number of
+    // CTAs makes up for them (see kDedispWeights; its second factor is 0.66 at
+    // least).
     bool build_tree(DedispTables& T, const std::vector<int>& chans, const std::vector<int>& shift)
     {
         constexpr int S = kTrS;
@@ -971,7 +1013,7 @@ struct psx_dedisp_plan {
         std::vector<Pat> pats;                       // in (block, subband) order
         std::vector<uint8_t> which((size_t)ndm * nsbt);
         int most = 0;
-        size_t mlo = 0, ngroups_ = 0, nquads = 0;
+        size_t mlo = 0, ngroups_ = 0;
         for (int g = 0; g < blocks; ++g) {
             const int e0 = g * per, e1 = std::min(ndm, e0 + per);
             int* l = &lo[(size_t)g * nlive];
@@ -991,7 +1033,6 @@ struct psx_dedisp_plan {
                 const int qd = (int)round_up((size_t)(kTrQ + mx[i] - l[i]), 16) / 4;
                 quads[(size_t)g * nlive + i] = qd;
                 most = std::max(most, qd);
-                nquads += qd;
                 mlo = std::max(mlo, (size_t)l[i]);
             }
             for (int b = 0; b < nsbt; ++b) {
@@ -1026,10 +1067,6 @@ struct psx_dedisp_plan {
                 }
             }
         }
-        const double q2 = 2.0 * kTrQ, cost_direct = (double)nlive * ndm * q2;
-        const double cost = (double)ngroups_ * 32 * (S + 2) + (double)nsbt * blocks * slots * q2 +
-                            16.0 * (double)nquads;
-        if (cost >= 0.9 * cost_direct) return false;
         // channels per stage: the most that leave two CTAs on an SM
         const int yw = T.kind == kTrSmall ? 1 : 2;
         int c_ = 0, pm = 0, gm = 0, nm = 0;
@@ -1059,6 +1096,11 @@ struct psx_dedisp_plan {
             }
         }
         if (!c_) return false;
+        const DedispWeights& w = kDedispWeights[T.kind];
+        T.rate = (w.patterns * (double)ngroups_ * 32 * (S + 2) / (2.0 * kTrQ * nlive * ndm) +
+                  w.sums * nsbt / nlive + w.stage / ((double)c_ * per) + w.channel / nlive) *
+                 ndm / (double)round_up((size_t)ndm, kDdWarps);
+        if (T.rate >= 1.0 / 0.66) return false;
         const int nq_ = (nlive + c_ - 1) / c_, sbs = c_ / S;
         // tables: channel records, output rows, per stage the first pattern
         // and the groups, pattern records, the trials' Y offsets
@@ -1211,14 +1253,7 @@ int prepare(psx_dedisp_plan* p, size_t nout, int nbits, cudaStream_t st, size_t*
 {
     const int kind = nbits == 16 ? kTr16 : nbits <= 4 ? kTrSmall : kTr8;
     const int el = nbits == 16 ? 2 : 1;
-    // Blocks of 32 DM trials leave most SMs without a CTA where the output is
-    // short: the direct kernel's blocks of 8 then (30,278 samples x 16
-    // channels to 50 DM trials, 60 blocks of 32, on B200: 26.1 us against
-    // 28.0; 42,314 x 248 to 75, 123 blocks: 90 against 52).
-    const size_t blocks = (nout + tr_tile(el) - 1) / tr_tile(el) *
-                          ((p->dms.size() + kTrMaxDms - 1) / kTrMaxDms);
-    const bool few = 2 * blocks < (size_t)sm_count();
-    PSX_TRY(p->take_tables(kind, few));
+    PSX_TRY(p->take_tables(kind, nout));
     DedispTables& t = *p->t;
     if (!t.uploaded) {
         size_t bytes = t.h_tab.size() * sizeof(int);

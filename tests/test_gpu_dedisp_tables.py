@@ -9,9 +9,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _plan(psx, nchans, ndm, dmax):
+def _plan(psx, nchans, ndm, dmax, band=200.0):
     h = C.c_void_p()
-    assert psx.psx_dedisp_create(nchans, 64e-6, 1500.0, -200.0 / nchans, C.byref(h)) == 0
+    assert psx.psx_dedisp_create(nchans, 64e-6, 1500.0, -band / nchans, C.byref(h)) == 0
     dms = np.linspace(0.0, dmax, ndm).astype(np.float32)
     assert psx.psx_dedisp_set_dm_list(h, dms.ctypes.data, ndm) == 0
     return h, dms
@@ -85,3 +85,63 @@ def test_turns_and_changes_of_the_plan_equal_a_fresh_one(psx, cuda, nbits):
             assert np.array_equal(run(h, nout), run(fresh, nout))
             psx.psx_dedisp_destroy(fresh)
     psx.psx_dedisp_destroy(h)
+
+
+@pytest.mark.parametrize("nchans,nbits,ndm,dmax", [(9, 8, 17, 3.0), (64, 16, 33, 8.0),
+                                                   (64, 2, 32, 60.0), (256, 4, 64, 60.0),
+                                                   (136, 1, 50, 30.0), (64, 8, 40, 12.0)])
+def test_outputs_of_any_number_equal_definition(psx, cuda, oracle, nchans, nbits, ndm, dmax):
+    """Numbers of outputs on both sides of where the form changes (launches of
+    one to four CTAs an SM, whole and part tiles) through one plan: the
+    definition in whole numbers."""
+    from peasoup_b200 import sigproc
+    torch = cuda
+    tile = 512 if nbits == 16 else 1024
+    h, dms = _plan(psx, nchans, ndm, dmax)
+    md, most = psx.psx_dedisp_get_max_delay(h), 440 * tile
+    delays = oracle.delay_table(nchans, 64e-6, 1500.0, -200.0 / nchans)
+    v = np.random.default_rng(ndm).integers(0, 1 << nbits, (most + md, nchans), dtype=np.uint32)
+    v[:, : nchans // 2] = (1 << nbits) - 1  # the largest sums
+    x = torch.from_numpy(v.T.astype(np.int32)).cuda().contiguous()
+    rows = torch.from_numpy(sigproc.pack_samples(v, nbits)).cuda()
+    shift = np.rint(dms[:, None] * delays[None, :]).astype(np.int64)
+    want = torch.zeros((ndm, most), dtype=torch.int32, device="cuda")
+    for d in range(ndm):
+        for c in range(nchans):
+            want[d] += x[c, shift[d, c]:shift[d, c] + most]
+    want = want.float()
+    for tiles in (1, 36, 73, 74, 110, 148, 149, 222, 296, 297, 439):
+        for tail in (0, 1, tile - 1):
+            nout = tiles * tile + tail
+            out = torch.full((ndm, most + 4), -1.0, device="cuda")
+            assert psx.psx_dedisp_execute(h, nout + md, C.c_void_p(rows.data_ptr()), nbits,
+                                          C.c_void_p(out.data_ptr()), most + 4, 1, None) == 0
+            assert torch.equal(out[:, :nout], want[:, :nout]), (tiles, tail)
+            assert torch.all(out[:, nout:] == -1.0)
+    psx.psx_dedisp_destroy(h)
+
+
+@pytest.mark.parametrize("nbits", [2, 8])
+def test_half_a_device_of_ctas_is_no_step_in_time(psx, cuda, nbits):
+    """32 DM trials of 64 channels: a 74th tile of outputs is no reason for a
+    form whose 74 CTAs take half as long again as the direct form's 296."""
+    torch = cuda
+    h, _ = _plan(psx, 64, 32, 60.0, band=70.0)
+    md = psx.psx_dedisp_get_max_delay(h)
+    rows = torch.randint(0, 256, ((75 * 1024 + md) * 8 * nbits,), dtype=torch.uint8, device="cuda")
+    out = torch.empty((32, 75 * 1024), device="cuda")
+    best = {}
+    for _ in range(5):
+        for tiles in (73, 74):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            for k in range(24):
+                if k == 4:
+                    e[0].record()
+                assert psx.psx_dedisp_execute(h, tiles * 1024 + md, C.c_void_p(rows.data_ptr()),
+                                              nbits, C.c_void_p(out.data_ptr()), 75 * 1024, 0,
+                                              None) == 0
+            e[1].record()
+            torch.cuda.synchronize()
+            best[tiles] = min(best.get(tiles, 1e9), e[0].elapsed_time(e[1]))
+    psx.psx_dedisp_destroy(h)
+    assert best[74] < 1.25 * best[73], best
