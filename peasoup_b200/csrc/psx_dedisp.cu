@@ -45,6 +45,7 @@ constexpr int kDdTile8 = 1024; // output samples per CTA, 1..8-bit samples
 constexpr int kDdTile16 = 512; // output samples per CTA, 16-bit samples
 inline int dd_tile(int elem) { return elem == 1 ? kDdTile8 : kDdTile16; }
 constexpr int kUpRows = 64;    // unpack tile: samples
+constexpr int kUpThreads = 256;
 constexpr float kDmConst = 4.15e3f;
 
 template <int NBITS> struct Sample { using T = uint8_t; };
@@ -79,7 +80,7 @@ struct UnpackTile {
 };
 
 template <int NBITS>
-__global__ void __launch_bounds__(256) k_unpack_chanmajor(
+__global__ void __launch_bounds__(kUpThreads) k_unpack_chanmajor(
     const uint8_t* __restrict__ rows, size_t row_bytes, size_t nrows, size_t r0, size_t ncols,
     int nchans, typename Sample<NBITS>::T* __restrict__ cm, size_t pitch, int vec)
 {
@@ -90,7 +91,33 @@ __global__ void __launch_bounds__(256) k_unpack_chanmajor(
     const size_t seg = (size_t)c0 * NBITS / 8;  // first byte of the CTA's part of a row
     constexpr int kRows = NBITS == 16 ? 2 : 4;  // rows of a thread's step: one word of samples
     const int words = (int)min((size_t)U::kWords, (row_bytes - seg + 3) / 4);
-    for (int i = threadIdx.x; i < (kUpRows / kRows) * words; i += blockDim.x) {
+    bool turned = false;
+    if constexpr (NBITS == 16) {
+        // Two rows a step give a thread four steps: for a whole tile of rows
+        // of whole words all their loads first (400,000 x 64 on B200: 28.8 us
+        // step by step, 18.7; 40,000 x 64: 6.1, 4.1).
+        if (vec && words == U::kWords && col0 + kUpRows <= nrows) {
+            constexpr int kSteps = (kUpRows / kRows) * U::kWords / kUpThreads;
+            const int q = threadIdx.x % U::kWords, g0 = threadIdx.x / U::kWords;
+            const uint8_t* p = rows + (col0 + kRows * g0) * row_bytes + seg + 4 * q;
+            const size_t step = (size_t)(kRows * (kUpThreads / U::kWords)) * row_bytes;
+            uint32_t w[kSteps][kRows];
+#pragma unroll
+            for (int j = 0; j < kSteps; ++j)
+#pragma unroll
+                for (int r = 0; r < kRows; ++r)
+                    w[j][r] = *reinterpret_cast<const uint32_t*>(p + j * step + r * row_bytes);
+            uint32_t* t = tile + (q * U::kPer) * U::kChanWords;
+#pragma unroll
+            for (int j = 0; j < kSteps; ++j) {
+                const int at = (g0 + j * (kUpThreads / U::kWords)) ^ (q & (U::kChanWords - 1));
+                t[at] = __byte_perm(w[j][0], w[j][1], 0x5410);
+                t[U::kChanWords + at] = __byte_perm(w[j][0], w[j][1], 0x7632);
+            }
+            turned = true;
+        }
+    }
+    for (int i = threadIdx.x; !turned && i < (kUpRows / kRows) * words; i += blockDim.x) {
         const int q = i % words, g = i / words;  // row word, group of rows
         const size_t byte = seg + 4 * (size_t)q;
         uint32_t w[kRows];
@@ -1291,7 +1318,7 @@ int launch_unpack(const uint8_t* rows, size_t nrows, size_t r0, size_t ncols, ps
     // word loads when every row starts 4-byte aligned; channels past the
     // last whole word of a row then read as zero and are never stored
     const int vec = (row_bytes % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 3) == 0) ? 1 : 0;
-    k_unpack_chanmajor<NBITS><<<grid, 256, 0, st>>>(rows, row_bytes, nrows, r0, ncols,
+    k_unpack_chanmajor<NBITS><<<grid, kUpThreads, 0, st>>>(rows, row_bytes, nrows, r0, ncols,
                                                     (int)p->nchans, static_cast<T*>(p->d_cm), pitch,
                                                     vec);
     return launch_status("k_unpack_chanmajor");

@@ -145,3 +145,27 @@ def test_half_a_device_of_ctas_is_no_step_in_time(psx, cuda, nbits):
             best[tiles] = min(best.get(tiles, 1e9), e[0].elapsed_time(e[1]))
     psx.psx_dedisp_destroy(h)
     assert best[74] < 1.25 * best[73], best
+
+
+@pytest.mark.parametrize("nchans", [62, 64, 66, 130])
+@pytest.mark.parametrize("nsamps", [1, 63, 64, 65, 192])
+@pytest.mark.parametrize("shift", [0, 2])
+def test_16_bit_rows_turned_whole_and_in_part(psx, cuda, nchans, nsamps, shift):
+    """64 samples x 64 channels at a time with every load first, where a tile
+    is whole and rows are whole words; word by word or byte by byte elsewhere:
+    each channel alone comes out as it went in."""
+    torch = cuda
+    h, _ = _plan(psx, nchans, 1, 0.0)
+    rng = np.random.default_rng(nsamps)
+    v = rng.integers(0, 1 << 16, (nsamps, nchans), dtype=np.uint16)
+    buf = torch.zeros(v.nbytes + 16, dtype=torch.uint8, device="cuda")
+    buf[shift:shift + v.nbytes] = torch.from_numpy(v.view(np.uint8).reshape(-1)).cuda()
+    out = torch.empty((1, (nsamps + 3) // 4 * 4), device="cuda")
+    for c in (0, 1, 31, 61, nchans - 1):
+        km = np.zeros(nchans, np.int32)
+        km[c] = 1
+        assert psx.psx_dedisp_set_killmask(h, km.ctypes.data) == 0
+        assert psx.psx_dedisp_execute(h, nsamps, C.c_void_p(buf.data_ptr() + shift), 16,
+                                      C.c_void_p(out.data_ptr()), out.shape[1], 1, None) == 0
+        assert np.array_equal(out[0, :nsamps].cpu().numpy(), v[:, c].astype(np.float32))
+    psx.psx_dedisp_destroy(h)
