@@ -1335,15 +1335,18 @@ __device__ __forceinline__ void add_fractions(const float* __restrict__ in, unsi
 
 // The running sums in the reference's order (src/kernels.cu:41-96): a warp
 // takes 32 K consecutive bins, lane l the bins l + 32 k.  Bound by the loads'
-// L1 wavefronts (one or two per 32 reads); one bin per thread with every
-// index formed anew took 44 us at 2^21 bins and 5 folds on B200, this 19.
-constexpr int kHsBins = 4;
+// L1 wavefronts (one or two per 32 reads) where the spectrum fills the
+// device, and by a lane's chain of reads below that: two bins to a lane up to
+// kHsLongBins, four above.  Measured on B200 (us, 5 folds; one bin per thread
+// with every index formed anew, K = 2, 4): 24,577 bins 4.48, 4.29, 5.60;
+// 131,073: 5.19, 4.77, 6.14; 262,145: 7.36, 5.47, 6.40; 524,289: 11.9, 7.81,
+// 7.33; 2^20: 22.3, 12.8, 10.4; 2^22: 82.8, 46.7, 36.6.
+constexpr size_t kHsLongBins = (size_t)3 << 17;
 
-template <int NH>
+template <int NH, int K>
 __global__ void __launch_bounds__(256) k_harmonic_sum(const float* __restrict__ in, FoldPtrs out,
                                                       unsigned n)
 {
-    constexpr int K = kHsBins;
     const unsigned warps = gridDim.x * (blockDim.x / 32);
     const unsigned nw = n / (32 * K) + (n % (32 * K) != 0);
     for (unsigned w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; w < nw; w += warps) {
@@ -1856,14 +1859,19 @@ int psx_harmonic_sum(const float* d_in, float* const* h_out_ptrs, size_t n, int 
         }
         o.p[h] = h_out_ptrs[h];
     }
-    const unsigned g = grid_for((n + kHsBins - 1) / kHsBins, 256);
     cudaStream_t s = cs(stream);
+    auto go = [&](auto two, auto four) {
+        if (n <= kHsLongBins)
+            two<<<grid_for((n + 1) / 2, 256), 256, 0, s>>>(d_in, o, (unsigned)n);
+        else
+            four<<<grid_for((n + 3) / 4, 256), 256, 0, s>>>(d_in, o, (unsigned)n);
+    };
     switch (nharms) {
-    case 1: k_harmonic_sum<1><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
-    case 2: k_harmonic_sum<2><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
-    case 3: k_harmonic_sum<3><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
-    case 4: k_harmonic_sum<4><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
-    default: k_harmonic_sum<5><<<g, 256, 0, s>>>(d_in, o, (unsigned)n); break;
+    case 1: go(k_harmonic_sum<1, 2>, k_harmonic_sum<1, 4>); break;
+    case 2: go(k_harmonic_sum<2, 2>, k_harmonic_sum<2, 4>); break;
+    case 3: go(k_harmonic_sum<3, 2>, k_harmonic_sum<3, 4>); break;
+    case 4: go(k_harmonic_sum<4, 2>, k_harmonic_sum<4, 4>); break;
+    default: go(k_harmonic_sum<5, 2>, k_harmonic_sum<5, 4>); break;
     }
     return launch_status("harmonic sum kernel");
 }
