@@ -985,7 +985,8 @@ static bool mean_cluster(cudaLaunchConfig_t cfg, const SeriesRows& rows, size_t 
 }
 
 int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* d_parts,
-                          size_t part_stride, unsigned* d_cnt, float* d_means, cudaStream_t s)
+                          size_t part_stride, unsigned* d_cnt, float* d_means, cudaStream_t s,
+                          int* launches)
 {
     const unsigned pieces = mean_pieces(n);
     if (n <= mean_max_samples(nrows)) {
@@ -1006,7 +1007,10 @@ int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* 
         case 2: ran = mean_cluster<2>(cfg, rows, n, d_cnt, d_means, &rc); break;
         default: ran = mean_cluster<4>(cfg, rows, n, d_cnt, d_means, &rc); break;
         }
-        if (ran) return rc;
+        if (ran) {
+            ++*launches;
+            return rc;
+        }
     }
     const dim3 grid(pieces / kMeanGroup, nrows);
     double* sums = reinterpret_cast<double*>(d_parts);
@@ -1014,6 +1018,7 @@ int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* 
         set_error("baseline means: partial sums of a row hold %zu entries", part_stride);
         return PSX_ERR_INVALID;
     }
+    *launches += 1 + kBaselineMeans;
     k_baseline_means<true><<<grid, kMeanGroupThreads, 0, s>>>(rows, n, sums, 2 * part_stride, d_cnt,
                                                               d_means, 0, 0);
     for (int pass = 1; pass <= kBaselineMeans; ++pass)

@@ -408,9 +408,9 @@ constexpr size_t kOwnAskedMinPoints = (size_t)3 << 17;
 // a second copy with a wait of its own costs 15 to 20 us.
 constexpr size_t kFirstRecords = 1024;
 constexpr size_t kCounterBytes = 16 * sizeof(unsigned);
-// launches of prologue_own: baseline means, two forward passes, amplitudes,
-// medians, dereddening, statistics, two inverse passes
-constexpr int kOwnPrologueLaunches = 1 + kBaselineMeans + 8;
+// launches of prologue_own after the baseline means: two forward passes,
+// amplitudes, medians, dereddening, statistics, two inverse passes
+constexpr int kOwnPrologueLaunches = 8;
 
 // Grouped prologue: DM trials per group by default, the largest transform
 // it applies to by default, and the most acceleration trials per DM trial
@@ -781,7 +781,7 @@ struct psx_search {
     int host_baseline_loop(Slot& s, size_t ncopy, cudaStream_t ps);
     int prologue_own(float* tim, float* Xp, void* med, double2* part, float* stat,
                      unsigned* count, float* mean, const SeriesRows& src, size_t ncopy, int rows,
-                     bool host_baseline, cudaStream_t ps);
+                     bool host_baseline, cudaStream_t ps, int* launches);
     int prologue_group(GroupSet& g, int count, cudaStream_t ps);
     int prologue_done(GroupSet& g, int count, int launches, int ffts, cudaStream_t ps);
     int prep(Slot& s, const float* series, size_t nsamps, bool on_device, float dm, int dm_idx);
@@ -993,15 +993,16 @@ int psx_search::make_harm_maps()
 // trial each 1654, 739 us; 24 of 2^22 points with a few each 5816, 5190.
 int psx_search::prologue_own(float* tim, float* Xp, void* med, double2* part, float* stat,
                              unsigned* count, float* mean, const SeriesRows& src, size_t ncopy,
-                             int rows, bool host_baseline, cudaStream_t ps)
+                             int rows, bool host_baseline, cudaStream_t ps, int* launches)
 {
+    *launches += kOwnPrologueLaunches;
     float2* z = reinterpret_cast<float2*>(Xp);
     float2* t2 = reinterpret_cast<float2*>(tim);
     float* m = static_cast<float*>(med);
     if (host_baseline)
         PSX_CUDA(cudaMemsetAsync(mean, 0, sizeof(float) * 4 * (size_t)rows, ps));
     else
-        PSX_TRY(launch_baseline_means(src, rows, ncopy, part, part_len, count, mean, ps));
+        PSX_TRY(launch_baseline_means(src, rows, ncopy, part, part_len, count, mean, ps, launches));
     PSX_TRY(f4.exec_series(src, rows, ncopy, mean, t2, N / 2, z, Bp, ps));
     PSX_TRY(f4.amplitudes(z, Bp, rows, tim, N, ps));
     PSX_TRY(launch_scrunch_rows(tim, N, rows, B, m, med_floats, ps));
@@ -1038,8 +1039,7 @@ int psx_search::prologue(Slot& s)
         }
         if (s.host_baseline) PSX_TRY(host_baseline_loop(s, ncopy, ps));
         PSX_TRY(prologue_own(s.d_tim, s.d_Xp, s.d_med, s.d_part, s.d_stat, s.d_count, s.d_mean,
-                             src, ncopy, 1, s.host_baseline, ps));
-        s.launches += s.host_baseline ? 8 : kOwnPrologueLaunches;
+                             src, ncopy, 1, s.host_baseline, ps, &s.launches));
         if (s.profiled) PSX_CUDA(cudaEventRecord(s.ev[1], ps));
         PSX_CUDA(cudaEventRecord(s.ready, ps));
         return PSX_OK;
@@ -1417,9 +1417,10 @@ int psx_search::prologue_group(GroupSet& g, int count, cudaStream_t ps)
                                      ps));
             src.p[i] = sl.d_tim;
         }
+        int launches = 0;
         PSX_TRY(prologue_own(g.tim, g.Xp, g.med, g.part, g.stat, g.count, g.mean, src, ncopy, count,
-                             false, ps));
-        return prologue_done(g, count, kOwnPrologueLaunches, 0, ps);
+                             false, ps, &launches));
+        return prologue_done(g, count, launches, 0, ps);
     }
     for (int i = 0; i < count; ++i) {
         Slot& sl = g.slots[i];

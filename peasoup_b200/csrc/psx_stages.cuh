@@ -16,10 +16,11 @@ struct MedianLevels;
 // The grouped (and per-DM) prologue on the library's own transform: the means
 // the baseline loop subtracts (at most kBaselineMeans), the median levels of
 // amplitude rows, the statistics of many partials and the mask of the zapped
-// bins.
+// bins.  (The kernels launched, one or more, are added to *launches.)
 constexpr int kBaselineMeans = 3;
 int launch_baseline_means(const SeriesRows& rows, int nrows, size_t n, double2* d_parts,
-                          size_t part_stride, unsigned* d_cnt, float* d_means, cudaStream_t s);
+                          size_t part_stride, unsigned* d_cnt, float* d_means, cudaStream_t s,
+                          int* launches);
 int launch_scrunch_rows(const float* d_amp, size_t stride, int rows, size_t nbins, float* d_scratch,
                         size_t scratch_stride, cudaStream_t s);
 int launch_finish_stats_rows(const double2* d_partials, int nparts, size_t part_stride, int rows,

@@ -1,0 +1,31 @@
+"""What psx_search_last_info reports is what ran."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _search(n, **kw):
+    from peasoup_b200 import search, synth
+    return search.AccelSearch(search.SearchParams(
+        fft_size=n, tsamp=64e-6, cfreq_hz=synth.CFREQ_HZ, ch_bw_hz=synth.CH_BW_HZ, nharmonics=4,
+        min_snr=30.0, **kw))
+
+
+# A trial's four kernels and the prologue's eight beside the means: one kernel
+# up to 2^21 samples (from four rows 2^23), four above.  Five DM trials of 2^22
+# points go in groups of four and one, eight of 2^19 in two of four, with one
+# launch of each of a trial's kernels to a group.
+@pytest.mark.parametrize("n,ndm,want", [
+    (1 << 17, 1, 13), (1 << 19, 1, 13), (1 << 21, 1, 13), (1 << 22, 1, 16), (1 << 22, 3, 48),
+    (1 << 22, 5, 13 + 16), (1 << 19, 8, 2 * 13)])
+def test_kernel_launches(cuda, n, ndm, want):
+    torch = cuda
+    s = _search(n)
+    x = torch.randn(ndm, n, device="cuda")
+    for _ in range(2):
+        s.search_block([x[d] for d in range(ndm)], np.zeros(ndm, np.float32))
+        info = s.info()
+        assert info["ntrials"] == ndm and info["fft_launches"] == 0
+        assert info["kernel_launches"] == want, info
+    s.close()
