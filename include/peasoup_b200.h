@@ -536,7 +536,8 @@ typedef struct {
     int graph;            /* 1 if the trial schedule ran as a CUDA graph */
     int batch;            /* trials per launch used */
     int baseline_passes;  /* mean-removal passes of the last DM (-1: host loop) */
-    int harm_shape;       /* harmonic-kernel tile shape in use */
+    int harm_shape;       /* harmonic-kernel tile shape of the last call's
+                             largest launch group */
     int capture_fallbacks; /* schedules launched directly because their
                               graph capture was invalidated */
     int fft_form;         /* transform path of the trials: 1 cuFFT complex

@@ -640,6 +640,14 @@ struct psx_search {
         const int rows = kHarmShapes[kHarmRowsShape - 1].rows;
         return harm_auto && (trials % rows == 0 || trials >= 4 * rows) ? kHarmRowsShape : harm_shape;
     }
+    int info_trials = 0;  // trials of the call's largest launch group so far
+    // info.harm_shape: the shape of the call's largest launch group
+    void note_group(int trials)
+    {
+        if (trials <= info_trials) return;
+        info_trials = trials;
+        info.harm_shape = shape_for(trials);
+    }
     // The maps a shape reads its rows through; null where they are not the
     // ones it needs (its launch is then refused).
     const HarmMaps* maps_for(int shape, int lane) const
@@ -1168,6 +1176,7 @@ int psx_search::trials_span(GroupSet& g, int cnt)
         g.launches += 3;
         if (span) {  // as trials_range: leftover trials on the single-row shape
             const int shape = shape_for(b), rows = kHarmShapes[shape - 1].rows;
+            note_group(b);
             const int rem = rows > 1 ? b % rows : 0, bm = b - rem;
             if (bm > 0) {
                 PSX_TRY(launch_harm(F, shape, pp, Bp, (unsigned)Bp, pk, t0, bm, g.d_rec,
@@ -1570,6 +1579,7 @@ int psx_search::trials_range(Slot& s, int t_begin, int nacc, bool reset)
             // instead of a tile padded with unused rows (every shape gives
             // the same records).
             const int shape = shape_for(b), rows = kHarmShapes[shape - 1].rows;
+            note_group(b);
             const int rem = rows > 1 ? b % rows : 0, bm = b - rem;
             if (bm > 0) {
                 PSX_TRY(launch_harm(F, shape, pp, Bp, (unsigned)Bp, pk, t0, bm, s.d_rec,
@@ -1668,6 +1678,7 @@ int psx_search::run_trials(Slot& s, int nacc)
         it = graphs.emplace(key, ge).first;
     }
     PSX_CUDA(cudaGraphLaunch(it->second.exec, st));
+    note_group(std::min(batch, upto));
     s.launches += it->second.launches;
     s.ffts += it->second.ffts;
     s.groups = it->second.groups;
@@ -2534,6 +2545,7 @@ int psx_search_block(psx_search* s, const float* const* series, size_t nsamps,
     s->info.batch = bp;
     s->info.fft_callback = cbk;
     s->info.harm_shape = s->harm_shape;
+    s->info_trials = 0;
     s->info.fft_form = effective_form(&s->cfg);
     s->info.graph = s->batched() && s->cfg.use_graph && !s->profile ? 1 : 0;
     // prologues wait for the caller's work queued on the compute stream so far

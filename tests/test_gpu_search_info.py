@@ -1,4 +1,5 @@
-"""What psx_search_last_info reports is what ran."""
+"""What psx_search_last_info reports is what ran: kernel launches and the
+harmonic kernel's shape."""
 import numpy as np
 import pytest
 
@@ -28,4 +29,15 @@ def test_kernel_launches(cuda, n, ndm, want):
         info = s.info()
         assert info["ntrials"] == ndm and info["fft_launches"] == 0
         assert info["kernel_launches"] == want, info
+    s.close()
+
+
+@pytest.mark.parametrize("batch,shape,want", [(12, 0, 6), (4, 0, 4), (12, 4, 4), (12, 6, 6)])
+def test_harmonic_shape_of_the_largest_group(cuda, batch, shape, want):
+    n = 1 << 21
+    s = _search(n, acc_lo=-200.0, acc_hi=200.0, batch=batch, harm_shape=shape)
+    x = cuda.randn(n, device="cuda")
+    for _ in range(3):  # launched, captured and replayed
+        s.search(x)
+        assert s.info()["ntrials"] >= batch and s.info()["harm_shape"] == want
     s.close()
