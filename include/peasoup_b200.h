@@ -416,8 +416,8 @@ typedef struct {
     int use_graph;             /* batched: capture the trial schedule */
     int harm_shape;            /* harmonic-kernel tile shape 1..PSX_HARM_SHAPES;
                                   0 = default: the three-row shape for fft_size
-                                  2^20 .. 2^23 where a launch group has its
-                                  rows, else the single-row one
+                                  2^20 .. 2^23 where a launch group searches
+                                  enough bins for it, else the single-row one
                                   (psx_autotune picks one by timing) */
     int lanes;                 /* batched: launch groups alternate over this
                                   many streams with their own buffers, so one

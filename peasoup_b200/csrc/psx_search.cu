@@ -273,16 +273,26 @@ constexpr HarmShape kHarmShapes[] = {
 static_assert(sizeof(kHarmShapes) / sizeof(kHarmShapes[0]) == PSX_HARM_SHAPES, "shape table");
 constexpr int kHarmDefaultShape = 4;
 // With no shape asked for, launch groups of the two-pass transform at 2^20 to
-// 2^23 points take the three-row shape where its whole rows carry them.
-// Measured on B200 (us per trial, shape 4 against 6, 4 folds): 24 trials in a
-// group at 2^19 1.56/1.41 (5 folds 2.16/2.26), 2^21 4.95/4.14, 2^23
-// 18.6/14.6; groups of 8 at 2^23 19.3/17.6; groups of 4, where one trial is
-// left for a launch of its own, 6.72/8.56 at 2^21.  Every bin is read at 16
-// places of the search, from L2 while the rows searched together stay in it:
-// three rows of 2^26 points (400 MB) took 8.30 ms a call where one at a time
-// took 7.73.
+// 2^23 points take the three-row shape where it is the faster one: by the bins
+// a group searches (below kHarmRowsBins its items leave the one CTA per SM
+// short of work, and the more so the fewer folds), and further up where one or
+// two trials are left over, whose launch of their own costs 5 us and more.
+// Measured on B200 (us per trial, shape 4 and 6, three to 32 trials in a
+// group, 1 to 5 folds): 2^20 points, 4 folds: 6 trials 3.75/4.10, 12
+// 3.07/3.24, 16 2.94/3.14, 24 2.65/2.52, 32 2.56/2.53; 3 * 2^19: 3 6.83/7.17,
+// 9 4.55/4.10, 16 3.97/4.03, 32 3.71/3.42; 2^21: 3 7.51/7.85, 6 6.15/5.63,
+// 14 5.27/5.05, 20 5.02/4.66, 3 folds 14 3.88/4.02; 2^22: 3 12.3/11.6, 8
+// 10.2/10.1, 10 10.0/9.3; 2^23: 4 20.5/20.2, 8 19.2/17.5, 12 19.1/15.2; one
+// fold at 2^23: 12 3.93/4.01, 16 3.71/4.03; two folds: 12 7.68/7.42, 14
+// 7.61/7.83.  Every bin is read at 16 places of the search, from L2 while the
+// rows searched together stay in it: three rows of 2^26 points (400 MB) took
+// 8.30 ms a call where one at a time took 7.73.
 constexpr int kHarmRowsShape = 6;
 constexpr size_t kHarmRowsMinPoints = (size_t)1 << 20, kHarmRowsMaxPoints = (size_t)1 << 23;
+// Bins of a group in whole rows (more where a row is short: each bin has its
+// windows' reads beside it), and of one with trials left over.
+constexpr double kHarmRowsBins = 3 << 21, kHarmRowsShortBins = 1 << 23, kHarmRestBins = 5 << 22;
+constexpr size_t kHarmRowsShortPoints = (size_t)3 << 19;
 
 template <int F, int SH>
 struct HarmKernel {
@@ -637,8 +647,12 @@ struct psx_search {
     bool harm_auto = false;  // no shape asked for: shape_for picks per launch group
     int shape_for(int trials) const
     {
-        const int rows = kHarmShapes[kHarmRowsShape - 1].rows;
-        return harm_auto && (trials % rows == 0 || trials >= 4 * rows) ? kHarmRowsShape : harm_shape;
+        if (!harm_auto) return harm_shape;
+        const double bins = (double)trials * (double)(pk.hi - pk.lo);
+        const bool whole = trials % kHarmShapes[kHarmRowsShape - 1].rows == 0;
+        const double least = !whole ? kHarmRestBins
+                             : N < kHarmRowsShortPoints ? kHarmRowsShortBins : kHarmRowsBins;
+        return F >= (whole ? 2 : 3) && bins >= least ? kHarmRowsShape : harm_shape;
     }
     int info_trials = 0;  // trials of the call's largest launch group so far
     // info.harm_shape: the shape of the call's largest launch group

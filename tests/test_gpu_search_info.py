@@ -41,3 +41,41 @@ def test_harmonic_shape_of_the_largest_group(cuda, batch, shape, want):
         s.search(x)
         assert s.info()["ntrials"] >= batch and s.info()["harm_shape"] == want
     s.close()
+
+
+@pytest.mark.parametrize("lg,folds,batch,want", [
+    (20, 4, 3, 4), (20, 4, 12, 4), (20, 5, 16, 4), (20, 4, 24, 6), (20, 4, 32, 4), (21, 4, 3, 4),
+    (21, 4, 6, 6), (21, 3, 14, 4), (21, 4, 20, 6), (22, 4, 3, 6), (22, 4, 8, 4), (22, 4, 10, 6),
+    (22, 1, 12, 4), (22, 2, 14, 4), (23, 4, 8, 6)])
+def test_default_harmonic_shape(cuda, lg, folds, batch, want):
+    """Per launch group, the shape that was measured to be the faster one."""
+    from peasoup_b200 import search, synth
+    n = 1 << lg
+    s = search.AccelSearch(search.SearchParams(
+        fft_size=n, tsamp=76e-6, cfreq_hz=synth.CFREQ_HZ, ch_bw_hz=synth.CH_BW_HZ, acc_lo=-2000.0,
+        acc_hi=2000.0 if lg < 22 else -1800.0, nharmonics=folds, min_snr=30.0, batch=batch,
+        group_dms=1))
+    s.search(cuda.randn(n, device="cuda"))
+    assert s.info()["ntrials"] >= batch and s.info()["harm_shape"] == want
+    s.close()
+
+
+@pytest.mark.parametrize("acc", [60.0, 100.0, 150.0, 250.0, 300.0])
+def test_default_harmonic_shape_equals_the_single_row_one(cuda, acc):
+    """2^21 points in groups of up to 20 and 6 trials: the same candidates,
+    bit for bit, whichever shape the groups take."""
+    from peasoup_b200 import search, synth
+    n = 1 << 21
+    x = synth.make_series_np(synth.SeriesSpec(
+        nsamps=n, tsamp=64e-6, pulsars=[synth.Pulsar(5.1e-3, 100.0, 0.05, 0.4)]), 2)
+    for batch in (20, 6):
+        got = []
+        for shape in (0, 4):
+            s = search.AccelSearch(search.SearchParams(
+                fft_size=n, tsamp=64e-6, cfreq_hz=synth.CFREQ_HZ, ch_bw_hz=synth.CH_BW_HZ,
+                acc_lo=-acc, acc_hi=acc, nharmonics=4, min_snr=5.5, batch=batch, harm_shape=shape))
+            got.append(s.search(x, 1.0, 2, per_dm=False))
+            s.close()
+        assert len(got[0][0]) > 0
+        for a, b in zip(*got):
+            assert np.array_equal(a, b)
