@@ -500,6 +500,9 @@ namespace {
 
 size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 
+// Records a buffer is made for that has to hold `need`.
+size_t record_capacity(size_t need) { return round_up(need + need / 4, 4096); }
+
 double ms_since(std::chrono::steady_clock::time_point t)
 {
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t).count();
@@ -896,7 +899,7 @@ int psx_search::apply_priority()
 int psx_search::grow_records(Slot& s, size_t need)
 {
     if (need <= s.rec_cap) return PSX_OK;
-    const size_t cap = round_up(need + need / 4, 4096);
+    const size_t cap = record_capacity(need);
     PSX_CUDA(cudaStreamSynchronize(st));
     PSX_CUDA(cudaStreamSynchronize(cst));
     s.rec_cap = 0;
@@ -1128,7 +1131,7 @@ int psx_search::prologue(Slot& s)
 int psx_search::grow_span_records(GroupSet& g, size_t need)
 {
     if (need <= g.rec_cap) return PSX_OK;
-    const size_t cap = round_up(need + need / 4, 4096);
+    const size_t cap = record_capacity(need);
     PSX_CUDA(cudaStreamSynchronize(st));
     PSX_CUDA(cudaStreamSynchronize(cst));
     if (g.d_rec) cudaFree(g.d_rec);
@@ -2124,27 +2127,32 @@ size_t psx_search_footprint(const psx_search_config* c)
     bytes += L * sizeof(float) * N * b;               // resampled series, per lane
     bytes += L * sizeof(float) * 2 * Bp * b;          // complex spectra, per lane
     bytes += L * sizeof(float) * Bp * b;              // normalised spectra, per lane
-    bytes += 2 * sizeof(int4) * ((size_t)1 << 20);    // two initial record slots
+    const bool own = effective_form(c) == 3;
+    // two initial record slots
+    bytes += 2 * sizeof(int4) * (own ? record_capacity((size_t)1 << 20) : (size_t)1 << 20);
     // cuFFT work areas: about one transform's worth per batched plan size and
     // lane, plus the batch-1 plans of the two slots' prologues and the plain
     // path (the two-pass transform has twiddle tables instead)
-    const bool own = effective_form(c) == 3;
     bytes += 2 * sizeof(double2) * part_len_for(c);   // partial sums, per slot
     if (own)
         bytes += sizeof(float2) * Fft4Plan::table_floats2(N) + B / 8 + 4;  // and the zap mask
     else
         bytes += sizeof(float) * 2 * Bp * (2 * b * L + 6);
-    // two group sets of G rows (made with the instance): series,
-    // prologue spectra, median scratch, each slot's first record buffer, and
-    // about one batch's worth of transform work area per batch-G plan
+    // two group sets of G rows (made with the instance): series, prologue
+    // spectra, median scratch and partial sums; with the two-pass transform
+    // each set's record buffer, and a quarter more for records (the buffers
+    // grow with a call's hits, and a DM trial run again alone makes its slot's
+    // own); else each slot's first records, and about one batch's worth of
+    // transform work area per batch-G plan
     const size_t G = (size_t)group_rows_for(c);
-    if (G >= 2)
-        bytes += 2 * G *
-                     (sizeof(float) * (N + 2 * Bp) + median_scratch_bytes(B) +
-                      sizeof(int4) * ((size_t)1 << 18) + sizeof(double2) * part_len_for(c) +
-                      2 * sizeof(float) * 2 * Bp) +
-                 // the spanning schedule's first record buffer per set
-                 (own ? 2 * sizeof(int4) * ((size_t)1 << 20) : 0);
+    if (G >= 2) {
+        const size_t row = sizeof(float) * (N + 2 * Bp) + median_scratch_bytes(B) +
+                           sizeof(double2) * part_len_for(c);
+        if (own)
+            bytes += 2 * (G * row + sizeof(int4) * record_capacity((size_t)1 << 20)) / 4 * 5;
+        else
+            bytes += 2 * G * (row + sizeof(int4) * ((size_t)1 << 18) + 2 * sizeof(float) * 2 * Bp);
+    }
     return bytes;
 }
 
