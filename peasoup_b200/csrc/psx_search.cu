@@ -967,13 +967,10 @@ int psx_search::host_baseline_loop(Slot& s, size_t ncopy, cudaStream_t ps)
     return PSX_OK;
 }
 
-// src/pipeline_multi.cu:170-238 for one series, on the slot's own stream.
-// It starts once the caller's work queued before this call (call_start)
-// and the slot's previous DM (whose trials read s.d_tim) are done, and
-// records s.ready; the trials wait for s.ready on the compute stream.  So
-// the prologue of DM d+1 runs alongside the trials of DM d.
 // Whether the kernels can read the job's series where it lies: this
-// device's own memory, whole floats.  Anything else is copied first.
+// device's own memory, whole floats.  Anything else is copied first (a series
+// called the device's may be another device's, managed or mapped host memory:
+// the copy finds out).
 bool psx_search::readable(const Slot& s) const
 {
     if (!s.on_device || (reinterpret_cast<uintptr_t>(s.series) & 3u)) return false;
@@ -1039,6 +1036,11 @@ int psx_search::prologue_own(float* tim, float* Xp, void* med, double2* part, fl
     return f4.exec_inverse(t2, N / 2, rows, ps);
 }
 
+// src/pipeline_multi.cu:170-238 for one series, on the slot's own stream.
+// It starts once the caller's work queued before this call (call_start)
+// and the slot's previous DM (whose trials read s.d_tim) are done, and
+// records s.ready; the trials wait for s.ready on the compute stream.  So
+// the prologue of DM d+1 runs alongside the trials of DM d.
 int psx_search::prologue(Slot& s)
 {
     if (!s.r2c && !use_f4) {  // a grouped slot run on its own (a retry): batch-1 plans on first need
@@ -1058,7 +1060,7 @@ int psx_search::prologue(Slot& s)
         src.p[0] = s.series;
         if (s.host_baseline || !readable(s)) {
             PSX_CUDA(cudaMemcpyAsync(s.d_tim, s.series, sizeof(float) * ncopy,
-                                     s.on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                                     s.on_device ? cudaMemcpyDefault : cudaMemcpyHostToDevice,
                                      ps));
             src.p[0] = s.d_tim;
         }
@@ -1439,7 +1441,7 @@ int psx_search::prologue_group(GroupSet& g, int count, cudaStream_t ps)
             src.p[i] = sl.series;
             if (readable(sl)) continue;
             PSX_CUDA(cudaMemcpyAsync(sl.d_tim, sl.series, sizeof(float) * ncopy,
-                                     sl.on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                                     sl.on_device ? cudaMemcpyDefault : cudaMemcpyHostToDevice,
                                      ps));
             src.p[i] = sl.d_tim;
         }
