@@ -79,3 +79,21 @@ def test_default_harmonic_shape_equals_the_single_row_one(cuda, acc):
         assert len(got[0][0]) > 0
         for a, b in zip(*got):
             assert np.array_equal(a, b)
+
+
+def test_host_baseline_loop_takes_over(cuda):
+    """A mean of 1e12 leaves residual means above the threshold after every
+    float subtraction that the device makes: on either transform the host's
+    loop goes on from there."""
+    from peasoup_b200 import search, synth
+    n = 1 << 19
+    x = (np.random.default_rng(3).standard_normal(n) * 1e9 + 1e12).astype(np.float32)
+    for form in (3, 1):
+        s = search.AccelSearch(search.SearchParams(
+            fft_size=n, tsamp=64e-6, cfreq_hz=synth.CFREQ_HZ, ch_bw_hz=synth.CH_BW_HZ,
+            nharmonics=2, min_snr=8.0, batch=2, fft_form=form))
+        s.search(x)
+        assert s.info()["baseline_passes"] == -1
+        s.search((x - np.float32(1e12)) / np.float32(1e9))
+        assert s.info()["baseline_passes"] in (1, 2, 3)
+        s.close()

@@ -57,3 +57,27 @@ def test_short_harmonic_sums_keep_a_lane_s_chain_short(psx, cuda):
             torch.cuda.synchronize()
             best[n] = min(best.get(n, 1e9), e[0].elapsed_time(e[1]) * 10.0)
     assert best[24577] < 0.72 * best[LONG + 1], best
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("n", [3, 5, 1003, 300001, (1 << 20) + 3])
+def test_rms_and_deviation(psx, cuda, n, shift):
+    """Both forms of the statistics against 64 bits.  The float results: a
+    few roundings of mean and rms (2^-22 relative), and for the deviation the
+    roundings of rms^2 and mean^2 before their difference."""
+    torch = cuda
+    x = (np.random.default_rng(n).standard_normal(n) * 3 + 5).astype(np.float32)
+    for first in (0, 2):
+        buf = torch.zeros(n + 8, device="cuda")
+        buf[shift:shift + n] = torch.from_numpy(x)
+        m, r, s = C.c_float(), C.c_float(), C.c_float()
+        assert psx.psx_stats(C.c_void_p(buf.data_ptr() + 4 * shift), n, first, C.byref(m),
+                             C.byref(r), C.byref(s), None) == 0
+        y = x[first:].astype(np.float64)
+        cnt = float(n - first)
+        mean, rms = y.sum() / cnt, np.sqrt((y * y).sum() / cnt)
+        std = np.sqrt(max(rms * rms - mean * mean, 0.0))
+        assert abs(m.value - mean) <= 2.0 ** -22 * abs(mean)
+        assert abs(r.value - rms) <= 2.0 ** -22 * rms
+        if std > 1e-3 * rms:
+            assert abs(s.value - std) <= 2.0 ** -22 * ((rms * rms + mean * mean) / std + std)
