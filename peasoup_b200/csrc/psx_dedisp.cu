@@ -47,6 +47,7 @@ inline int dd_tile(int elem) { return elem == 1 ? kDdTile8 : kDdTile16; }
 constexpr int kUpRows = 64;    // unpack tile: samples
 constexpr int kUpThreads = 256;
 constexpr float kDmConst = 4.15e3f;
+constexpr size_t kDdMaxSmem = 220 * 1024;  // dynamic shared memory of a launch at most
 
 template <int NBITS> struct Sample { using T = uint8_t; };
 template <> struct Sample<16> { using T = uint16_t; };
@@ -1117,7 +1118,7 @@ struct psx_dedisp_plan {
             // channel's: into the next one's, or the zeros
             const size_t b = DedispTables::tree_bytes(DedispTables::raw_words(c, pm, more, el),
                                                       pm + 4 * most + 32, gm, yw, nm, c / S * slots);
-            if (b <= 112 * 1024 || (c == 4 && b <= 220 * 1024)) {
+            if (b <= 112 * 1024 || (c == 4 && b <= kDdMaxSmem)) {
                 c_ = c;
                 break;
             }
@@ -1336,12 +1337,22 @@ int unpack(int nbits, const uint8_t* rows, size_t nrows, size_t r0, size_t ncols
     }
 }
 
+// Opts a kernel into kDdMaxSmem: always the same value, since plans in other
+// threads launch the same kernel with windows of their own between one
+// thread's setting and its launch.
+template <class Kernel>
+int allow_smem(Kernel kern)
+{
+    PSX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kDdMaxSmem));
+    return PSX_OK;
+}
+
 template <int MODE, bool FLUSH>
 int launch_tree(const TreeArgs& a, int dpw, unsigned grid, size_t smem, cudaStream_t st)
 {
     auto go = [&](auto kern) -> int {
-        PSX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+        PSX_TRY(allow_smem(kern));
         kern<<<grid, kTrThreads, smem, st>>>(a);
         return launch_status("k_dedisperse_tree");
     };
@@ -1436,8 +1447,7 @@ int dedisperse(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, float* 
     size_t smem = p->t->smem_bytes();
     const unsigned grid = (unsigned)nblocks;
     if (nbits == 16) {
-        PSX_CUDA(cudaFuncSetAttribute(k_dedisperse<uint16_t, false, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PSX_TRY(allow_smem(k_dedisperse<uint16_t, false, false>));
         k_dedisperse<uint16_t, false, false><<<grid, kDdThreads, smem, st>>>(a);
     } else {
         // 8 bits and below: the flush and small-sample variants
@@ -1446,8 +1456,7 @@ int dedisperse(psx_dedisp_plan* p, int nbits, size_t pitch, size_t nout, float* 
                                    : k_dedisperse<uint8_t, false, true>)
                           : (flush ? k_dedisperse<uint8_t, true, false>
                                    : k_dedisperse<uint8_t, false, false>);
-        PSX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+        PSX_TRY(allow_smem(kern));
         kern<<<grid, kDdThreads, smem, st>>>(a);
     }
     return launch_status("k_dedisperse");

@@ -169,3 +169,39 @@ def test_16_bit_rows_turned_whole_and_in_part(psx, cuda, nchans, nsamps, shift):
                                       C.c_void_p(out.data_ptr()), out.shape[1], 1, None) == 0
         assert np.array_equal(out[0, :nsamps].cpu().numpy(), v[:, c].astype(np.float32))
     psx.psx_dedisp_destroy(h)
+
+
+@pytest.mark.parametrize("ndm", [32, 3])
+def test_plans_of_several_threads_launch_one_kernel(psx, cuda, ndm):
+    """Threads, each with a plan and a stream of its own, whose windows need
+    different amounts of shared memory of the same kernel: every launch
+    succeeds."""
+    import threading
+    torch = cuda
+    nchans, nout = 64, 4096
+    rows = torch.randint(0, 256, ((nout + 8192) * nchans,), dtype=torch.uint8, device="cuda")
+    bad = []
+
+    def work(k):
+        h = _plan(psx, nchans, ndm, (5.0, 60.0)[k % 2], band=70.0)[0]
+        o = torch.empty((ndm, nout), device="cuda")
+        st = torch.cuda.Stream()
+        md = psx.psx_dedisp_get_max_delay(h)
+        args = (h, nout + md, C.c_void_p(rows.data_ptr()), 8, C.c_void_p(o.data_ptr()), nout, 0,
+                C.c_void_p(st.cuda_stream))
+        for i in range(4000):
+            rc = psx.psx_dedisp_execute(*args)
+            if rc:
+                bad.append((k, i, rc, psx.psx_last_error()))
+                break
+            if i % 50 == 49:
+                st.synchronize()
+        st.synchronize()
+        psx.psx_dedisp_destroy(h)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
