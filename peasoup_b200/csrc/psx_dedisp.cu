@@ -448,9 +448,9 @@ __global__ void __launch_bounds__(kDdThreads) k_dedisperse(DedispArgs a)
 // number of words, so no load needs a funnel shift and a warp's loads are
 // consecutive.
 //
-// Bound: the shared-memory port (71 % of its wavefronts; 46 % of them the
-// second level's, 2 bytes per output, subband and DM trial), then issue
-// (62 %).  Measured on B200 (us, the whole call, channel by channel and so):
+// Bound: the shared-memory port (71 % of its wavefronts at 8 bits, 64 % at 4;
+// 45 % of the shared-memory ones the second level's, 2 bytes per output,
+// subband and DM trial) and issue (67 %, 69 %).  Measured on B200 (us, the whole call, channel by channel and so):
 // 256 DM trials x 2^22 samples x 64 channels, 8 bits: 6311, 3033; 100 x
 // 400,000 x 1024, 4 bits: 3408, 1680.  Subbands of 8 channels have three times the
 // patterns; blocks of 64 DM trials leave half the warps.

@@ -208,8 +208,9 @@ __global__ void __launch_bounds__(256) k_scrunch5(const float* __restrict__ in, 
     }
 }
 
-// The median spliced from its three levels (median_at); with X given the spectrum is divided by the median in place (bins 0..4 zeroed),
-// otherwise the median itself is written.
+// The median spliced from its three levels (median_at); with X given the
+// spectrum is divided by the median in place (bins 0..4 zeroed), otherwise the
+// median itself is written.
 __global__ void __launch_bounds__(256) k_median_apply(MedianLevels L, size_t nbins,
                                                       float* __restrict__ median_out,
                                                       float* __restrict__ X, size_t x_stride = 0,
@@ -291,9 +292,9 @@ MedianLevels median_levels(size_t nbins, double bin_width, float b5, float b25, 
 }
 
 // The three median-of-5 levels of the amplitudes of a complex spectrum X
-// (AMP), or of the powers X as they are, in one pass: a CTA takes groups of 125 bins (5 * 25) at a time, so
-// every value of the 5-, 25- and 125-bin levels it writes is formed from
-// its own bins; the levels stop where the reference's floor(count / 5)
+// (AMP), or of the powers X as they are, in one pass: a CTA takes groups of
+// 125 bins (5 * 25) at a time, so every value of the 5-, 25- and 125-bin levels
+// it writes is formed from its own bins; the levels stop where the reference's floor(count / 5)
 // stops them.  The amplitudes themselves are never written.  (One launch in
 // place of three for the powers: at 2^20 bins on B200 6.4 us of three
 // latency-bound kernels became 3.7.)
