@@ -809,7 +809,8 @@ inline double dedisp_occupancy(int kind, double ctas, double direct_ctas)
 
 // Shift tables and launch shape of one form for one class of samples.
 struct DedispTables {
-    enum State { kNew, kBuilt, kNotTaken };  // kNotTaken: the direct form instead
+    // kRated: only `rate`, at least, known so far; kNotTaken: the direct form instead
+    enum State { kNew, kRated, kBuilt, kNotTaken };
     State state = kNew;
     bool uploaded = false;
     int kind = 0;           // sample class (direct: any of this width)
@@ -900,23 +901,28 @@ struct psx_dedisp_plan {
         const double direct_ctas = tiles * (double)((dms.size() + kDdWarps - 1) / kDdWarps);
         const size_t blocks = (dms.size() + kTrMaxDms - 1) / kTrMaxDms;
         const double full = dedisp_occupancy(kind, tiles * (double)blocks, direct_ctas);
-        // (no list's rate is below 0.3: not looked at where that cannot do)
-        if (0.3 * full < 1.0 && shared.state == DedispTables::kNew && dms.size() >= kTrMinDms) {
+        std::vector<int> chans, shift;
+        // The rate of a list is not looked at (0.4 ms of host time at 1024
+        // channels x 100 DM trials) where it had to be below a half: less than
+        // half the device's SMs have a CTA then, and little is to be gained.
+        if (dms.size() >= kTrMinDms && full < 2.0 &&
+            (shared.state == DedispTables::kNew ||
+             (shared.state == DedispTables::kRated && shared.rate * full < 1.0))) {
             shared.kind = kind;
             shared.elem = el;
             shared.uploaded = false;
-            std::vector<int> chans, shift;
             shifts(&chans, &shift);
             shared.nlive = (int)chans.size();
-            shared.state = shared.nlive > 0 && build_tree(shared, chans, shift)
-                               ? DedispTables::kBuilt : DedispTables::kNotTaken;
+            shared.state = shared.nlive > 0 ? build_tree(shared, chans, shift, full)
+                                            : DedispTables::kNotTaken;
         }
         t = shared.state == DedispTables::kBuilt && shared.rate * full < 1.0 ? &shared : &direct;
         if (t->state == DedispTables::kBuilt) return PSX_OK;
+        if (shift.empty()) shifts(&chans, &shift);
         direct.kind = kind;
         direct.elem = el;
         direct.uploaded = false;
-        PSX_TRY(build_direct(direct));
+        PSX_TRY(build_direct(direct, chans, shift));
         direct.state = DedispTables::kBuilt;
         return PSX_OK;
     }
@@ -936,11 +942,9 @@ struct psx_dedisp_plan {
     }
 
     // Shift tables and the window shape of the direct form.
-    int build_direct(DedispTables& T)
+    int build_direct(DedispTables& T, const std::vector<int>& chans, const std::vector<int>& shift)
     {
         const int el = T.elem;
-        std::vector<int> chans, shift;
-        shifts(&chans, &shift);
         const int nlive = T.nlive = (int)chans.size();
         const int ndm = (int)dms.size();
         const int ndm_pad = T.ndm_pad = (int)round_up((size_t)ndm, kDdWarps);
@@ -1012,18 +1016,19 @@ struct psx_dedisp_plan {
         return PSX_OK;
     }
 
-    // Tables of the shared-partial-sum form, or false where the direct
-    // kernel is taken whatever the outputs: the series do not fit shared
-    // memory, a sum could pass 2^24 where sums are kept as floats, or the
-    // patterns are so many (few or widely spaced DM trials) that no number of
-    // CTAs makes up for them (see kDedispWeights; its second factor is 0.66 at
-    // least).
-    bool build_tree(DedispTables& T, const std::vector<int>& chans, const std::vector<int>& shift)
+    // Rate and, where the call's CTAs (`full`) want them, tables of the
+    // shared-partial-sum form; kNotTaken where the direct kernel is taken
+    // whatever the outputs: the series do not fit shared memory, a sum could
+    // pass 2^24 where sums are kept as floats, or the patterns are so many (few
+    // or widely spaced DM trials) that no number of CTAs makes up for them (see
+    // kDedispWeights; its second factor is 0.66 at least).
+    DedispTables::State build_tree(DedispTables& T, const std::vector<int>& chans,
+                                   const std::vector<int>& shift, double full)
     {
         constexpr int S = kTrS;
         const int el = T.elem, nlive = T.nlive;
         const int ndm = (int)dms.size();
-        if (el == 1 && (double)nlive * 255.0 >= 16777216.0) return false;
+        if (el == 1 && (double)nlive * 255.0 >= 16777216.0) return DedispTables::kNotTaken;
         std::vector<int> order(ndm);
         for (int d = 0; d < ndm; ++d) order[d] = d;
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return dms[x] < dms[y]; });
@@ -1095,6 +1100,14 @@ struct psx_dedisp_plan {
                 }
             }
         }
+        const DedispWeights& w = kDedispWeights[T.kind];
+        auto rate_at = [&](int c) {  // with c channels a stage
+            return (w.patterns * (double)ngroups_ * 32 * (S + 2) / (2.0 * kTrQ * nlive * ndm) +
+                    w.sums * nsbt / nlive + w.stage / ((double)c * per) + w.channel / nlive) *
+                   ndm / (double)round_up((size_t)ndm, kDdWarps);
+        };
+        T.rate = rate_at(32);
+        if (T.rate * full >= 1.0) return DedispTables::kRated;
         // channels per stage: the most that leave two CTAs on an SM
         const int yw = T.kind == kTrSmall ? 1 : 2;
         int c_ = 0, pm = 0, gm = 0, nm = 0;
@@ -1123,12 +1136,10 @@ struct psx_dedisp_plan {
                 break;
             }
         }
-        if (!c_) return false;
-        const DedispWeights& w = kDedispWeights[T.kind];
-        T.rate = (w.patterns * (double)ngroups_ * 32 * (S + 2) / (2.0 * kTrQ * nlive * ndm) +
-                  w.sums * nsbt / nlive + w.stage / ((double)c_ * per) + w.channel / nlive) *
-                 ndm / (double)round_up((size_t)ndm, kDdWarps);
-        if (T.rate >= 1.0 / 0.66) return false;
+        if (!c_) return DedispTables::kNotTaken;
+        T.rate = rate_at(c_);
+        if (T.rate >= 1.0 / 0.66) return DedispTables::kNotTaken;
+        if (T.rate * full >= 1.0) return DedispTables::kRated;
         const int nq_ = (nlive + c_ - 1) / c_, sbs = c_ / S;
         // tables: channel records, output rows, per stage the first pattern
         // and the groups, pattern records, the trials' Y offsets
@@ -1203,7 +1214,7 @@ struct psx_dedisp_plan {
         T.lwin = 4 * most + (el == 1 ? 3 : 1) * kTrQ;
         T.max_lo = mlo;
         T.tile = tr_tile(el);
-        return true;
+        return DedispTables::kBuilt;
     }
 
     ~psx_dedisp_plan()
