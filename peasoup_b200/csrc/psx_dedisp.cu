@@ -1293,6 +1293,17 @@ int prepare(psx_dedisp_plan* p, size_t nout, int nbits, cudaStream_t st, size_t*
     const int kind = nbits == 16 ? kTr16 : nbits <= 4 ? kTrSmall : kTr8;
     const int el = nbits == 16 ? 2 : 1;
     PSX_TRY(p->take_tables(kind, nout));
+    if (!p->t->uploaded) {
+        // Nothing can be allocated or copied from here while the stream is
+        // captured: the form whose tables are on the device then, as good as
+        // the other but for its time.
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        PSX_CUDA(cudaStreamIsCapturing(st, &capture));
+        DedispTables& other = p->t == &p->sets[kind] ? p->sets[3 + (el == 2)] : p->sets[kind];
+        if (capture != cudaStreamCaptureStatusNone && other.state == DedispTables::kBuilt &&
+            other.uploaded)
+            p->t = &other;
+    }
     DedispTables& t = *p->t;
     if (!t.uploaded) {
         size_t bytes = t.h_tab.size() * sizeof(int);

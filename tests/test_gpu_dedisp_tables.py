@@ -205,3 +205,39 @@ def test_plans_of_several_threads_launch_one_kernel(psx, cuda, ndm):
     for t in threads:
         t.join()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("nbits", [2, 8, 16])
+def test_captured_after_a_call_of_another_size(psx, cuda, nbits):
+    """A call is capturable once the plan has run, whatever outputs that call
+    had: short outputs (the direct form) are captured after long ones, run
+    again after further calls and replayed."""
+    torch = cuda
+    nchans, ndm, long_, short = 64, 64, 120 * 1024, 4 * 1024
+    h, _ = _plan(psx, nchans, ndm, 20.0)
+    md = psx.psx_dedisp_get_max_delay(h)
+    rows = torch.randint(0, 256, ((long_ + md) * nchans * nbits // 8,), dtype=torch.uint8,
+                         device="cuda")
+    out, cap = torch.empty((ndm, long_), device="cuda"), torch.zeros((ndm, short), device="cuda")
+
+    def run(o, nout, stream):
+        return psx.psx_dedisp_execute(h, nout + md, C.c_void_p(rows.data_ptr()), nbits,
+                                      C.c_void_p(o.data_ptr()), o.shape[1], 0,
+                                      C.c_void_p(stream))
+
+    assert run(out, long_, 0) == 0
+    torch.cuda.synchronize()
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(g, stream=s):
+        rc = run(cap, short, s.cuda_stream)
+    assert rc == 0
+    want = torch.empty_like(cap)
+    for _ in range(2):
+        cap.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert run(want, short, 0) == 0 and run(out, long_, 0) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(cap, want) and torch.equal(out[:, :short], want)
+    del g
+    psx.psx_dedisp_destroy(h)
